@@ -336,7 +336,7 @@ int mb_mul_rows_gather(int64_t n_rows, const float* x, const float* s, const int
  * matris/model/interaction_block.py:123, 270-273): out[u] = 0.5*(y[u2d[u]] + y[rev[u2d[u]]]) + res_w*res[u] */
 int mb_pair_mean_res(int32_t n_bonds, const int32_t* u2d, const int32_t* rev, const float* y, const float* res,
                      const float* res_w, float* out, void* stream);
-/* y = a*x (elementwise per channel weight a[128]) ; accumulate != 0: y += a*x */
+/* y = a*x (elementwise per channel weight a[128], NULL: 1) ; accumulate != 0: y += a*x */
 int mb_scale_rows(int64_t n_rows, const float* x, const float* a, float* y, int32_t accumulate, void* stream);
 
 /* K <= 16 linear layers (edge_linear1 / learnable_envelope: K=7, angle_embedding: K=16;
@@ -451,6 +451,120 @@ int mb_fourier_basis_fwd(int64_t n_trip, const int32_t* line_graph, const float*
                          float* basis, void* stream);
 int mb_fourier_basis_bwd(int64_t n_trip, const int32_t* line_graph, const float* unit, const float* freq,
                          const float* dbasis, float* dunit, void* stream);
+
+/* ------------------------------------------------------------------ whole evaluation
+ * The model's parameters as device pointers: every 128-wide weight with its operand splits, all in one layout
+ * (see mb_colblock).  ..t members are the transposes the data-gradient products contract with. */
+typedef struct mb_weight {
+  const float* W; const float* W_hi; const float* W_lo;
+  const uint16_t* W_hi16; const uint16_t* W_lo16;
+  int64_t ldw;
+} mb_weight;
+
+/* One update block (matris/model/functions.py:245-311): kind MB_UPDATE_GATED = GatedMLP, w1 [256,K] and w2 [256,128] =
+ * core rows then gate rows, w1t [K,256], w2t [256,128] = the two transposes stacked, b1 / b2 [256], nc / ng the norm
+ * weights; kind MB_UPDATE_MLP = MLP + RMSNorm (matris/model/interaction_block.py:39-62), w1 [128,K], w2 [128,128],
+ * b1 / b2 [128] or NULL, nc the norm weight. */
+#define MB_UPDATE_GATED 0
+#define MB_UPDATE_MLP 1
+typedef struct mb_update {
+  int32_t kind, k;
+  mb_weight w1, w2, w1t, w2t;
+  const float* b1; const float* b2; const float* nc; const float* ng;
+} mb_update;
+
+typedef struct mb_ffn { mb_weight w1, w2, w1t, w2t; const float* b1; const float* b2; } mb_ffn;
+
+/* Graph_Attention_Layer (matris/model/interaction_block.py:87-143): wst [256,128] = source then target logits */
+typedef struct mb_attn_params {
+  mb_update node, edge;
+  mb_weight wst, wstt;
+  const float* wn; const float* we;   /* residual weights */
+} mb_attn_params;
+
+/* Refinement (matris/model/interaction_block.py:218-278) */
+typedef struct mb_refine_params {
+  mb_update edge;
+  mb_ffn nffn, effn;
+  const float* wenv; const float* wn; const float* we;
+  int32_t smoothed_edge, pad;
+} mb_refine_params;
+
+typedef struct mb_layer_params {
+  mb_attn_params attn_atom, attn_line;
+  mb_refine_params refine_atom, refine_line;
+} mb_layer_params;
+
+typedef struct mb_model_params {
+  const mb_layer_params* layers; int32_t n_layers;
+  int32_t gaussian, fourier, envelope_exponent;
+  float cut2, cut3, coeff2, coeff3, sph_factor; int32_t pad;
+  const float* emb_table; mb_weight emb_w;
+  const float* freq2; const float* freq3;       /* Bessel frequencies or Gaussian offsets [7] */
+  const float* e_w1; mb_weight e_w2, e_w3, e_w2t, e_w3t; const float* e_lnw; const float* e_lnb;
+  const float* t_freq; const float* t_wa; mb_weight t_wb, t_wbt;
+  const float* out_norm;
+  mb_weight h_w0, h_w3, h_w0t, h_w3t; const float* h_b0; const float* h_b3; const float* h_w6; const float* h_b6;
+  mb_weight m_w0; const float* m_b0; const float* m_w3; const float* m_b3;
+  const float* ref_table; int32_t n_species;    /* AtomRef energies by atomic number - 1, or NULL */
+  int32_t is_intensive;
+} mb_model_params;
+
+/* One of the two message-passing graphs.  Atom graph (is_atom): rows = directed edges, nodes = atoms, edge features per
+ * bond (row r reads emap[r]); line graph: rows = triplets = edge features, nodes = bonds, ctr = centre atom of a row. */
+typedef struct mb_row_graph {
+  int64_t n_rows, n_nodes, n_edge_rows, n_ctr;
+  int32_t is_atom, pad;
+  const int32_t* tgt; const int32_t* src; const int32_t* ctr;
+  const int32_t* tgt_ptr; const int32_t* src_ptr; const int32_t* src_perm;
+  const int32_t* emap; const int32_t* u2d; const int32_t* rev;
+} mb_row_graph;
+
+/* One sub-block, forward and - when the gradients are wanted - backward, for a caller that composes its own model.
+ * ws == NULL: nothing runs, *ws_bytes receives the workspace size; otherwise *ws_bytes is the size of ws.
+ * d_node_out == NULL: forward only.  The backward recomputes the internals from the inputs. */
+int mb_attention_layer(const mb_attn_params* p, const mb_row_graph* g, const float* node, const float* edge, float* node_out,
+                       float* edge_out, const float* d_node_out, const float* d_edge_out, float* d_node, float* d_edge,
+                       void* ws, size_t* ws_bytes, void* stream);
+/* rbf [bonds,7]; atom_feat / d_atom (line graph only) are indexed by ctr, d_atom is accumulated into.  edge_out == NULL:
+ * the edge update is not computed (d_edge_out must then be NULL too).  d_rbf is accumulated into. */
+int mb_refine_layer(const mb_refine_params* p, const mb_row_graph* g, const float* node, const float* edge, const float* rbf,
+                    const float* atom_feat, float* node_out, float* edge_out, const float* d_node_out,
+                    const float* d_edge_out, float* d_node, float* d_edge, float* d_rbf, float* d_atom, void* ws,
+                    size_t* ws_bytes, void* stream);
+
+/* MatRIS.forward (matris/model/model.py:183-250) on a batch graph: energies, and forces / virial through the backward
+ * pass when f or s is given, as one call that queues every kernel.  mb_evaluate_workspace gives the most memory that is in
+ * use at any time for a number of layers whose internals are kept for the backward pass (the earlier layers' are
+ * recomputed), which is also the size of a workspace.  All outputs but e are optional. */
+typedef void* (*mb_alloc_fn)(size_t bytes);     /* device memory, 256-byte aligned, NULL when there is none */
+typedef void (*mb_free_fn)(void* p);            /* may be called while work that uses p is still queued on the stream */
+typedef struct mb_eval {
+  const mb_model_params* model;
+  int32_t n_atoms, n_struct; int64_t n_edges, n_bonds, n_triplets;
+  int32_t keep_layers, n_launches;              /* n_launches (out): kernels and memory operations queued */
+  const float* cart; const float* lattice; const float* volume;
+  const int32_t* atom_struct; const int32_t* atom_ptr; const int32_t* numbers;
+  const int32_t* center; const int32_t* neighbor; const int32_t* image; const int32_t* edge_ptr;
+  const int32_t* rev; const int32_t* d2u; const int32_t* u2d;
+  const int32_t* trip_ptr; const int32_t* trip_src_ptr; const int32_t* trip_src_perm;
+  const int32_t* line_graph;                    /* [T,5] */
+  const int32_t* lg_cols;                       /* [5,T] the same, column-major */
+  float* e;                                     /* [n_struct] energy (per atom when intensive) + reference energy */
+  float* ref;                                   /* [n_struct] reference energy */
+  int32_t* atoms_per_struct;                    /* [n_struct] */
+  float* f; float* s; float* m;                 /* [n_atoms,3] forces; [n_struct,9] stress in GPa; [n_atoms] moments */
+  void* ws; size_t ws_bytes;                    /* one workspace, or NULL: every buffer comes from alloc / release */
+  mb_alloc_fn alloc; mb_free_fn release;
+} mb_eval;
+int mb_evaluate_workspace(const mb_eval* e, size_t* bytes);
+int mb_evaluate(mb_eval* e, void* stream);
+
+/* Per-operation device times of mb_evaluate (CUDA events around every operation): switch on, evaluate, then read the
+ * records (synchronises); switching off drops what was not read. */
+typedef struct mb_op_record { char name[32]; float ms; int32_t fused; double flops, bytes; int64_t rows; int32_t k, n; } mb_op_record;
+int mb_profile_enable(int on);
+int mb_profile_read(mb_op_record* out, int32_t capacity, int32_t* n);
 
 #ifdef __cplusplus
 }

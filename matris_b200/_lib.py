@@ -73,6 +73,72 @@ class MbGatedMlp(C.Structure):
     ]
 
 
+class MbWeight(C.Structure):
+    _fields_ = [("W", _vp), ("W_hi", _vp), ("W_lo", _vp), ("W_hi16", _vp), ("W_lo16", _vp), ("ldw", _i64)]
+
+
+class MbUpdate(C.Structure):
+    _fields_ = [("kind", _i32), ("k", _i32), ("w1", MbWeight), ("w2", MbWeight), ("w1t", MbWeight), ("w2t", MbWeight),
+                ("b1", _vp), ("b2", _vp), ("nc", _vp), ("ng", _vp)]
+
+
+class MbFfn(C.Structure):
+    _fields_ = [("w1", MbWeight), ("w2", MbWeight), ("w1t", MbWeight), ("w2t", MbWeight), ("b1", _vp), ("b2", _vp)]
+
+
+class MbAttnParams(C.Structure):
+    _fields_ = [("node", MbUpdate), ("edge", MbUpdate), ("wst", MbWeight), ("wstt", MbWeight), ("wn", _vp), ("we", _vp)]
+
+
+class MbRefineParams(C.Structure):
+    _fields_ = [("edge", MbUpdate), ("nffn", MbFfn), ("effn", MbFfn), ("wenv", _vp), ("wn", _vp), ("we", _vp),
+                ("smoothed_edge", _i32), ("pad", _i32)]
+
+
+class MbLayerParams(C.Structure):
+    _fields_ = [("attn_atom", MbAttnParams), ("attn_line", MbAttnParams), ("refine_atom", MbRefineParams),
+                ("refine_line", MbRefineParams)]
+
+
+class MbModelParams(C.Structure):
+    _fields_ = [
+        ("layers", C.POINTER(MbLayerParams)), ("n_layers", _i32), ("gaussian", _i32), ("fourier", _i32),
+        ("envelope_exponent", _i32), ("cut2", _f32), ("cut3", _f32), ("coeff2", _f32), ("coeff3", _f32), ("sph_factor", _f32),
+        ("pad", _i32), ("emb_table", _vp), ("emb_w", MbWeight), ("freq2", _vp), ("freq3", _vp), ("e_w1", _vp),
+        ("e_w2", MbWeight), ("e_w3", MbWeight), ("e_w2t", MbWeight), ("e_w3t", MbWeight), ("e_lnw", _vp), ("e_lnb", _vp),
+        ("t_freq", _vp), ("t_wa", _vp), ("t_wb", MbWeight), ("t_wbt", MbWeight), ("out_norm", _vp),
+        ("h_w0", MbWeight), ("h_w3", MbWeight), ("h_w0t", MbWeight), ("h_w3t", MbWeight), ("h_b0", _vp), ("h_b3", _vp),
+        ("h_w6", _vp), ("h_b6", _vp), ("m_w0", MbWeight), ("m_b0", _vp), ("m_w3", _vp), ("m_b3", _vp),
+        ("ref_table", _vp), ("n_species", _i32), ("is_intensive", _i32),
+    ]
+
+
+class MbRowGraph(C.Structure):
+    _fields_ = [("n_rows", _i64), ("n_nodes", _i64), ("n_edge_rows", _i64), ("n_ctr", _i64), ("is_atom", _i32), ("pad", _i32),
+                ("tgt", _vp), ("src", _vp), ("ctr", _vp), ("tgt_ptr", _vp), ("src_ptr", _vp), ("src_perm", _vp),
+                ("emap", _vp), ("u2d", _vp), ("rev", _vp)]
+
+
+ALLOC_FN = C.CFUNCTYPE(_vp, C.c_size_t)
+FREE_FN = C.CFUNCTYPE(None, _vp)
+
+
+class MbEval(C.Structure):
+    _fields_ = [
+        ("model", C.POINTER(MbModelParams)), ("n_atoms", _i32), ("n_struct", _i32), ("n_edges", _i64), ("n_bonds", _i64),
+        ("n_triplets", _i64), ("keep_layers", _i32), ("n_launches", _i32), ("cart", _vp), ("lattice", _vp), ("volume", _vp),
+        ("atom_struct", _vp), ("atom_ptr", _vp), ("numbers", _vp), ("center", _vp), ("neighbor", _vp), ("image", _vp),
+        ("edge_ptr", _vp), ("rev", _vp), ("d2u", _vp), ("u2d", _vp), ("trip_ptr", _vp), ("trip_src_ptr", _vp),
+        ("trip_src_perm", _vp), ("line_graph", _vp), ("lg_cols", _vp), ("e", _vp), ("ref", _vp), ("atoms_per_struct", _vp),
+        ("f", _vp), ("s", _vp), ("m", _vp), ("ws", _vp), ("ws_bytes", C.c_size_t), ("alloc", ALLOC_FN), ("release", FREE_FN),
+    ]
+
+
+class MbOpRecord(C.Structure):
+    _fields_ = [("name", C.c_char * 32), ("ms", _f32), ("fused", _i32), ("flops", C.c_double), ("bytes", C.c_double),
+                ("rows", _i64), ("k", _i32), ("n", _i32)]
+
+
 # name -> argtypes (every function returns int status unless listed in _OTHER)
 _SIGNATURES = {
     "mb_graph_build": [C.POINTER(MbGraph), _vp],
@@ -120,6 +186,12 @@ _SIGNATURES = {
     "mb_gaussian_bwd": [_i32, _vp, _vp, _vp, _f32, _vp, _f32, _vp, _vp, _vp, _vp],
     "mb_fourier_basis_fwd": [_i64, _vp, _vp, _vp, _vp, _vp],
     "mb_fourier_basis_bwd": [_i64, _vp, _vp, _vp, _vp, _vp, _vp],
+    "mb_attention_layer": [C.POINTER(MbAttnParams), C.POINTER(MbRowGraph)] + [_vp] * 9 + [C.POINTER(C.c_size_t), _vp],
+    "mb_refine_layer": [C.POINTER(MbRefineParams), C.POINTER(MbRowGraph)] + [_vp] * 13 + [C.POINTER(C.c_size_t), _vp],
+    "mb_evaluate_workspace": [C.POINTER(MbEval), C.POINTER(C.c_size_t)],
+    "mb_evaluate": [C.POINTER(MbEval), _vp],
+    "mb_profile_enable": [C.c_int],
+    "mb_profile_read": [C.POINTER(MbOpRecord), _i32, C.POINTER(C.c_int32)],
 }
 _OTHER = {
     "mb_version": (C.c_int, []),
@@ -192,6 +264,41 @@ def call(name: str, *args) -> None:
     e1.record()
     profile.append((name, e0, e1, profile_meta))
     profile_meta = None
+
+
+class _Elapsed:
+    """Stands for a pair of CUDA events in ``profile`` records whose time the library has measured itself."""
+
+    def __init__(self, ms=0.0):
+        self.ms = ms
+
+    def elapsed_time(self, other):
+        return other.ms - self.ms
+
+
+def evaluate(e: MbEval, stream) -> None:
+    """mb_evaluate, with its operations counted and - while ``profile`` is a list - timed one by one."""
+    global launch_count
+    lib = load()
+    if profile is None:
+        status = lib.mb_evaluate(C.byref(e), stream)
+        launch_count += e.n_launches
+        if status:
+            check(status, "mb_evaluate")
+        return
+    lib.mb_profile_enable(1)
+    try:
+        check(lib.mb_evaluate(C.byref(e), stream), "mb_evaluate")
+        launch_count += e.n_launches
+        n = C.c_int32(0)
+        lib.mb_profile_read(None, 0, C.byref(n))
+        recs = (MbOpRecord * max(n.value, 1))()
+        check(lib.mb_profile_read(recs, len(recs), C.byref(n)), "mb_profile_read")
+    finally:
+        lib.mb_profile_enable(0)
+    for r in recs[:n.value]:
+        meta = dict(flops=r.flops, bytes=r.bytes, rows=r.rows, k=r.k, n=r.n, fused=bool(r.fused)) if r.rows else None
+        profile.append((r.name.decode(), _Elapsed(), _Elapsed(r.ms), meta))
 
 
 def ptr(t):

@@ -13,7 +13,7 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 LIB_PATH = os.path.join(PKG, "libmatris_b200.so")
-SOURCES = ["api.cu", "graph.cu", "gemm.cu", "rowwise.cu", "geometry.cu"]
+SOURCES = ["api.cu", "graph.cu", "gemm.cu", "rowwise.cu", "geometry.cu", "evaluate.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-I", INCLUDE, "-I", CSRC]
 

@@ -29,6 +29,8 @@ void set_cuda_error(cudaError_t e, const char* where);
 
 static inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 
+int gemm_mode();  // the contraction core selected with mb_set_gemm_mode
+
 // exclusive scan of n int32 values into out[0..n] (out[n] = total); tmp holds
 // mb_graph_scan_tmp_len(n) ints.  in may alias out.
 int scan_exclusive(const int32_t* in, int32_t* out, int64_t n, int32_t* tmp, cudaStream_t s);

@@ -567,6 +567,7 @@ k_gemm_tc(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ TcMaps
 
 // 0: persistent tcgen05 3xBF16 (default), 1: fp32 SIMT, 2: one-tile-per-CTA tcgen05 3xTF32, 3: persistent tcgen05 3xTF32
 static int g_gemm_mode = 0;
+int gemm_mode() { return g_gemm_mode; }
 
 // TMA descriptor of a [rows, k] float32 weight block (row stride ldw), box 128 rows x 32 columns, 128-byte swizzle.
 // Encoding depends only on (address, stride, k, rows), so descriptors are cached per host thread.

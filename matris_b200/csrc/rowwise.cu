@@ -298,7 +298,8 @@ __global__ void k_pair_mean_res(int n_bonds, const int32_t* __restrict__ u2d, co
 __global__ void k_scale_rows(int64_t n_rows, const float* __restrict__ x, const float* __restrict__ a,
                              float* __restrict__ y, int accumulate) {
   MB_ROW_PROLOGUE(n_rows)
-  float4 o = mul4(ld4(a + c), ld4(x + row * 128 + c));
+  float4 o = ld4(x + row * 128 + c);
+  if (a) o = mul4(ld4(a + c), o);
   if (accumulate) o = add4(o, ld4(y + row * 128 + c));
   st4(y + row * 128 + c, o);
 }
@@ -544,7 +545,7 @@ extern "C" int mb_pair_mean_res(int32_t n_bonds, const int32_t* u2d, const int32
 
 extern "C" int mb_scale_rows(int64_t n_rows, const float* x, const float* a, float* y, int32_t accumulate,
                              void* stream) {
-  MB_REQUIRE(n_rows >= 0 && x && a && y);
+  MB_REQUIRE(n_rows >= 0 && x && y);
   if (n_rows == 0) return MB_OK;
   k_scale_rows<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, x, a, y, accumulate);
   MB_LAUNCH_CHECK("k_scale_rows");

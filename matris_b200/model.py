@@ -4,20 +4,21 @@ Host-side mirror of the reference's ``MatRIS`` module
 (matris/model/model.py:30-317): same constructor arguments, ``config``,
 ``state_dict`` key names, ``from_dict`` / ``load`` checkpoint interface,
 ``graph_converter`` attribute and ``forward(graphs, task, is_training)`` result
-dictionary.  All arithmetic runs in the CUDA kernels behind the C ABI; the
-sub-blocks are ``torch.autograd.Function``s whose backward passes are
-hand-written kernel sequences (data gradients only: weights are frozen at
-inference), so forces = -dE/dr and stress = (1/V) dE/d(strain) come out of
-``torch.autograd.grad`` exactly as in the reference's conservative head
-(matris/model/readout.py:202-224).
+dictionary.  All arithmetic runs in the CUDA kernels behind the C ABI, and the sequence of
+kernels of an evaluation - forward and the hand-written backward pass (data
+gradients only: weights are frozen at inference) that gives forces = -dE/dr and
+stress = (1/V) dE/d(strain), the reference's conservative head
+(matris/model/readout.py:202-224) - is queued by one library call.
+``AttentionFn`` / ``RefineFn`` expose the two sub-blocks to torch.autograd.
 
 Memory policy: a sub-block always keeps its inputs for the backward pass.  Its
-internals are kept too while they fit in a fraction of the free device memory;
-beyond that they are recomputed in the backward pass (the reference switches to
+internals are kept too for as many of the last layers as fit in memory; those of
+the earlier layers are recomputed in the backward pass (the reference switches to
 recomputation above 60,000 triplets, matris/model/interaction_block.py:15, 400-403).
 """
 from __future__ import annotations
 
+import ctypes as C
 import os
 from collections.abc import Sequence
 from types import SimpleNamespace
@@ -27,321 +28,209 @@ import torch
 from torch import nn
 from torch.autograd.function import once_differentiable
 
-from . import ops
+from . import _lib, ops
 from ._lib import MbError
 from .graph import BatchedGraph, GraphConverter, RadiusGraph, build_batched_graph, as_arrays
-from .ops import B, OUT_ADD, OUT_ATOMIC, OUT_STORE, S, gemm
 from .weights import BUFFER_KEYS, check_supported, full_config, random_state_dict, schema
 
 GPA_PER_EV_A3 = 160.21766208  # matris/model/readout.py:215
-D = 128
+# Evaluations that need at most this much memory take it as one block: one allocation, and a block the allocator can place
+# again at the next call.  Larger ones ask for their buffers one by one, so that a block of a large part of the device is
+# never wanted in one piece; their host time is far below their device time.
+WORKSPACE_LIMIT = 4 << 30
 
 
 # ------------------------------------------------------------------ packed parameters
-def _pack_gated(get, prefix, dev):
-    """GatedMLP weights in kernel layout: first layers of core|gate stacked to
-    [256,K], second layers stacked to [256,128], plus the transposes the backward
-    GEMMs contract with."""
-    c, g = prefix + "mlp_core.layers.", prefix + "mlp_gate.layers."
-    w1 = torch.cat([get(c + "0.weight"), get(g + "0.weight")], 0).contiguous()
-    w2 = torch.cat([get(c + "3.weight"), get(g + "3.weight")], 0).contiguous()
-    SW = ops.SplitWeight
-    return SimpleNamespace(
-        w1=SW(w1), b1=torch.cat([get(c + "0.bias"), get(g + "0.bias")]).contiguous(),
-        w2=SW(w2), b2=torch.cat([get(c + "3.bias"), get(g + "3.bias")]).contiguous(),
-        w1t=SW(w1.t()),                                                           # [K,256]
-        w2t=SW(torch.cat([get(c + "3.weight").t(), get(g + "3.weight").t()], 0)),  # [256,128]
-        nc=get(prefix + "core_norm.weight").contiguous(), ng=get(prefix + "gate_norm.weight").contiguous(),
-        k=w1.shape[1])
+class _Packer:
+    """Parameters as the library's structs of device pointers.  The tensors behind the pointers are kept in ``alive``."""
 
+    def __init__(self, sd: dict, device):
+        self.sd, self.device, self.alive = sd, device, []
 
-def _pack_mlp(get, prefix, bias):
-    """The plain-MLP variant of an update block (graph_conv_mlp = "MLP"): nn.Sequential(MLP, RMSNorm)
-    (matris/model/interaction_block.py:39-62, 172-184): weights, transposes for the backward products, norm weight."""
-    w1, w2 = get(prefix + "0.layers.0.weight"), get(prefix + "0.layers.3.weight")
-    SW = ops.SplitWeight
-    return SimpleNamespace(
-        kind="mlp", w1=SW(w1), w2=SW(w2), w1t=SW(w1.t()), w2t=SW(w2.t()),
-        b1=get(prefix + "0.layers.0.bias").contiguous() if bias else None,
-        b2=get(prefix + "0.layers.3.bias").contiguous() if bias else None,
-        nw=get(prefix + "1.weight").contiguous(), k=w1.shape[1])
+    def get(self, key) -> torch.Tensor:
+        return self.sd[key].detach().to(device=self.device, dtype=torch.float32)
 
+    def vec(self, t) -> int | None:
+        """Device address of a contiguous copy (None for a parameter the configuration does not have)."""
+        if t is None:
+            return None
+        t = t.reshape(-1).contiguous()
+        self.alive.append(t)
+        return t.data_ptr()
 
-def _pack_ffn(get, prefix, bias):
-    """node_FFN / edge_FFN (matris/model/interaction_block.py:197-210): two linear layers, biases only with use_bias."""
-    w1, w2 = get(prefix + "layers.0.weight"), get(prefix + "layers.3.weight")
-    SW = ops.SplitWeight
-    b1 = get(prefix + "layers.0.bias").contiguous() if bias else None
-    b2 = get(prefix + "layers.3.bias").contiguous() if bias else None
-    return SimpleNamespace(w1=SW(w1), w2=SW(w2), w1t=SW(w1.t()), w2t=SW(w2.t()), b1=b1, b2=b2)
+    def weight(self, t) -> _lib.MbWeight:
+        sw = ops.SplitWeight(t)
+        self.alive.append(sw)
+        return _lib.MbWeight(*sw.ptrs, sw.ldw)
+
+    def gated(self, prefix) -> _lib.MbUpdate:
+        """GatedMLP: first layers of core|gate stacked to [256,K], second layers to [256,128], plus the transposes the
+        backward products contract with."""
+        get, c, g = self.get, prefix + "mlp_core.layers.", prefix + "mlp_gate.layers."
+        w1 = torch.cat([get(c + "0.weight"), get(g + "0.weight")], 0)
+        w2c, w2g = get(c + "3.weight"), get(g + "3.weight")
+        return _lib.MbUpdate(
+            kind=0, k=w1.shape[1], w1=self.weight(w1), w2=self.weight(torch.cat([w2c, w2g], 0)), w1t=self.weight(w1.t()),
+            w2t=self.weight(torch.cat([w2c.t(), w2g.t()], 0)), b1=self.vec(torch.cat([get(c + "0.bias"), get(g + "0.bias")])),
+            b2=self.vec(torch.cat([get(c + "3.bias"), get(g + "3.bias")])), nc=self.vec(get(prefix + "core_norm.weight")),
+            ng=self.vec(get(prefix + "gate_norm.weight")))
+
+    def mlp(self, prefix, bias) -> _lib.MbUpdate:
+        """The plain-MLP variant of an update block (graph_conv_mlp = "MLP"): nn.Sequential(MLP, RMSNorm)
+        (matris/model/interaction_block.py:39-62, 172-184)."""
+        get = self.get
+        w1, w2 = get(prefix + "0.layers.0.weight"), get(prefix + "0.layers.3.weight")
+        return _lib.MbUpdate(
+            kind=1, k=w1.shape[1], w1=self.weight(w1), w2=self.weight(w2), w1t=self.weight(w1.t()), w2t=self.weight(w2.t()),
+            b1=self.vec(get(prefix + "0.layers.0.bias")) if bias else None,
+            b2=self.vec(get(prefix + "0.layers.3.bias")) if bias else None, nc=self.vec(get(prefix + "1.weight")))
+
+    def ffn(self, prefix, bias) -> _lib.MbFfn:
+        """node_FFN / edge_FFN (matris/model/interaction_block.py:197-210): two linear layers, biases only with use_bias."""
+        w1, w2 = self.get(prefix + "layers.0.weight"), self.get(prefix + "layers.3.weight")
+        return _lib.MbFfn(
+            w1=self.weight(w1), w2=self.weight(w2), w1t=self.weight(w1.t()), w2t=self.weight(w2.t()),
+            b1=self.vec(self.get(prefix + "layers.0.bias")) if bias else None,
+            b2=self.vec(self.get(prefix + "layers.3.bias")) if bias else None)
+
+    def attention(self, prefix, update) -> _lib.MbAttnParams:
+        wst = torch.cat([self.get(prefix + "source_weight_linear.weight"), self.get(prefix + "target_weight_linear.weight")], 0)
+        return _lib.MbAttnParams(
+            node=update(prefix + "node_nonlinear_update."), edge=update(prefix + "edge_nonlinear_update."),
+            wst=self.weight(wst), wstt=self.weight(wst.t()), wn=self.vec(self.get(prefix + "node_res_weight")),
+            we=self.vec(self.get(prefix + "edge_res_weight")))
+
+    def refinement(self, prefix, update, bias, smoothed) -> _lib.MbRefineParams:
+        return _lib.MbRefineParams(
+            edge=update(prefix + "edge_nonlinear_update."), nffn=self.ffn(prefix + "node_FFN.", bias),
+            effn=self.ffn(prefix + "edge_FFN.", bias), wenv=self.vec(self.get(prefix + "learnable_envelope.weight")),
+            wn=self.vec(self.get(prefix + "node_res_weight")), we=self.vec(self.get(prefix + "edge_res_weight")),
+            smoothed_edge=int(smoothed))
 
 
 def pack_parameters(sd: dict, cfg: dict, device) -> SimpleNamespace:
-    def get(k):
-        return sd[k].detach().to(device=device, dtype=torch.float32)
-
-    P = SimpleNamespace()
-    P.emb_table = get("atom_embedding.embedding.weight").contiguous()
-    SW = ops.SplitWeight
-    P.emb_w = SW(get("atom_embedding.atom_swish_layer.linear.weight"))
+    """``.model``: the whole model as mb_model_params; ``.layers[i].attn_atom`` etc.: the sub-blocks' structs in it."""
+    k = _Packer(sd, device)
+    get, vec, weight = k.get, k.vec, k.weight
+    n_layers, bias = int(cfg["num_layers"]), bool(cfg["use_bias"])
+    M, layers = _lib.MbModelParams(), (_lib.MbLayerParams * n_layers)()
+    M.layers, M.n_layers = layers, n_layers
+    M.gaussian = str(cfg["distance_expansion"]).lower() == "gaussian"
+    M.fourier = str(cfg["three_body_expansion"]).lower() == "fourier"
+    M.envelope_exponent, M.cut2, M.cut3 = cfg["envelope_exponent"], cfg["pairwise_cutoff"], cfg["three_body_cutoff"]
+    M.emb_table = vec(get("atom_embedding.embedding.weight"))
+    M.emb_w = weight(get("atom_embedding.atom_swish_layer.linear.weight"))
     e = "edge_embedding."
-    P.gaussian = str(cfg["distance_expansion"]).lower() == "gaussian"
-    if P.gaussian:
+    if M.gaussian:
         # GaussianExpansion: the offsets are a buffer, the coefficient is derived from them at construction
         # (matris/model/basis_function.py:203-205: float32 spacing, then Python float arithmetic)
-        P.freq2, P.freq3 = get(e + "pairwise_rbf_expansion.offset").contiguous(), get(
-            e + "threebody_rbf_expansion.offset").contiguous()
-        P.coeff2, P.coeff3 = (-0.5 / (2.0 * (o[1] - o[0])).item() ** 2 for o in (P.freq2.cpu(), P.freq3.cpu()))
+        off = [get(e + n + "_rbf_expansion.offset") for n in ("pairwise", "threebody")]
+        M.freq2, M.freq3 = vec(off[0]), vec(off[1])
+        M.coeff2, M.coeff3 = (-0.5 / (2.0 * (o[1] - o[0])).item() ** 2 for o in (off[0].cpu(), off[1].cpu()))
     else:
-        P.freq2, P.freq3 = get(e + "pairwise_rbf_expansion.frequencies").contiguous(), get(
-            e + "threebody_rbf_expansion.frequencies").contiguous()
-    P.e_w1 = get(e + "edge_linear1.weight").contiguous()
-    P.e_w2 = SW(get(e + "edge_linear2.weight"))
-    P.e_w3 = SW(get(e + "swish_layer.linear.weight"))
-    P.e_w2t, P.e_w3t = P.e_w2.t(), P.e_w3.t()
-    P.e_lnw, P.e_lnb = get(e + "edge_init_norm.weight").contiguous(), get(e + "edge_init_norm.bias").contiguous()
+        M.freq2, M.freq3 = (vec(get(e + n + "_rbf_expansion.frequencies")) for n in ("pairwise", "threebody"))
+    M.e_w1 = vec(get(e + "edge_linear1.weight"))
+    w2, w3 = get(e + "edge_linear2.weight"), get(e + "swish_layer.linear.weight")
+    M.e_w2, M.e_w3, M.e_w2t, M.e_w3t = weight(w2), weight(w3), weight(w2.t()), weight(w3.t())
+    M.e_lnw, M.e_lnb = vec(get(e + "edge_init_norm.weight")), vec(get(e + "edge_init_norm.bias"))
     t = "three_body_embedding."
-    P.fourier = str(cfg["three_body_expansion"]).lower() == "fourier"
-    if P.fourier:
-        P.t_freq = get(t + "expansion.frequencies").contiguous()
+    if M.fourier:
+        M.t_freq = vec(get(t + "expansion.frequencies"))
     else:
-        P.sph_factor = float(sd[t + "expansion.factor"])
-    P.t_wa = get(t + "angle_embedding.weight").contiguous()
-    P.t_wb = SW(get(t + "swish_layer.linear.weight"))
-    P.t_wbt = P.t_wb.t()
-    P.layers = []
-    if str(cfg["graph_conv_mlp"]).lower() == "mlp":
-        pack_update = lambda prefix: _pack_mlp(get, prefix, bool(cfg["use_bias"]))  # noqa: E731
-    else:
-        pack_update = lambda prefix: _pack_gated(get, prefix, device)  # noqa: E731
-    for i in range(int(cfg["num_layers"])):
-        L = SimpleNamespace()
-        for gname in ("atom", "line"):
-            p = f"interaction_block.{i}.attn_block_{gname}_graph."
-            A = SimpleNamespace(node=pack_update(p + "node_nonlinear_update."),
-                                edge=pack_update(p + "edge_nonlinear_update."),
-                                wn=get(p + "node_res_weight").reshape(-1).contiguous(),
-                                we=get(p + "edge_res_weight").reshape(-1).contiguous())
-            A.wst = SW(torch.cat([get(p + "source_weight_linear.weight"), get(p + "target_weight_linear.weight")],
-                                 0))                  # [256,128]
-            A.wstt = A.wst.t()                        # [128,256]
-            setattr(L, "attn_" + gname, A)
-            p = f"interaction_block.{i}.refine_block_{gname}_graph."
-            R = SimpleNamespace(edge=pack_update(p + "edge_nonlinear_update."),
-                                nffn=_pack_ffn(get, p + "node_FFN.", bool(cfg["use_bias"])),
-                                effn=_pack_ffn(get, p + "edge_FFN.", bool(cfg["use_bias"])),
-                                smoothed_edge=bool(cfg["use_smoothed_for_delta_edge"]) and gname == "atom",
-                                wenv=get(p + "learnable_envelope.weight").contiguous(),
-                                wn=get(p + "node_res_weight").reshape(-1).contiguous(),
-                                we=get(p + "edge_res_weight").reshape(-1).contiguous())
-            setattr(L, "refine_" + gname, R)
-        P.layers.append(L)
-    P.out_norm = get("readout_norm.weight").contiguous()
+        M.sph_factor = float(sd[t + "expansion.factor"])
+    M.t_wa, wb = vec(get(t + "angle_embedding.weight")), get(t + "swish_layer.linear.weight")
+    M.t_wb, M.t_wbt = weight(wb), weight(wb.t())
+    update = (lambda p: k.mlp(p, bias)) if str(cfg["graph_conv_mlp"]).lower() == "mlp" else k.gated
+    for i, L in enumerate(layers):
+        p = f"interaction_block.{i}."
+        for g in ("atom", "line"):
+            setattr(L, "attn_" + g, k.attention(f"{p}attn_block_{g}_graph.", update))
+            smoothed = bool(cfg["use_smoothed_for_delta_edge"]) and g == "atom"
+            setattr(L, "refine_" + g, k.refinement(f"{p}refine_block_{g}_graph.", update, bias, smoothed))
+    M.out_norm = vec(get("readout_norm.weight"))
     h = "energy_head.energy_head.layers."
-    P.h_w0, P.h_b0 = SW(get(h + "0.weight")), get(h + "0.bias").contiguous()
-    P.h_w3, P.h_b3 = SW(get(h + "3.weight")), get(h + "3.bias").contiguous()
-    P.h_w0t, P.h_w3t = P.h_w0.t(), P.h_w3.t()
-    P.h_w6, P.h_b6 = get(h + "6.weight").reshape(-1).contiguous(), get(h + "6.bias").contiguous()
+    w0, w3 = get(h + "0.weight"), get(h + "3.weight")
+    M.h_w0, M.h_w3, M.h_w0t, M.h_w3t = weight(w0), weight(w3), weight(w0.t()), weight(w3.t())
+    M.h_b0, M.h_b3, M.h_w6, M.h_b6 = (vec(get(h + n)) for n in ("0.bias", "3.bias", "6.weight", "6.bias"))
     m = "magmom_head.magmom_head.layers."
-    P.m_w0, P.m_b0 = SW(get(m + "0.weight")), get(m + "0.bias").contiguous()
-    P.m_w3, P.m_b3 = get(m + "3.weight").reshape(-1).contiguous(), get(m + "3.bias").contiguous()
-    return P
+    M.m_w0 = weight(get(m + "0.weight"))
+    M.m_b0, M.m_w3, M.m_b3 = (vec(get(m + n)) for n in ("0.bias", "3.weight", "3.bias"))
+    if cfg["reference_energy"] is not None:
+        table = get("reference_energy.fc.weight")
+        M.ref_table, M.n_species = vec(table), table.numel()
+    M.is_intensive = int(bool(cfg["is_intensive"]))
+    return SimpleNamespace(model=M, layers=layers, alive=k.alive)
 
 
-# ------------------------------------------------------------------ row graphs
+# ------------------------------------------------------------------ sub-blocks as autograd functions
 def row_graphs(g: BatchedGraph):
-    """The two message-passing graphs in the form the kernels take: rows grouped by
-    target node (tgt_ptr), the source-side grouping as a permutation."""
-    if getattr(g, "_row_graphs", None) is None:
-        atom = SimpleNamespace(is_atom=True, n_rows=g.n_edges, n_nodes=g.n_atoms, n_edge_rows=g.n_bonds,
-                               tgt=g.center, src=g.neighbor, ctr=None, tgt_ptr=g.edge_ptr, src_ptr=g.edge_ptr,
-                               src_perm=g.rev, emap=g.d2u, u2d=g.u2d, rev=g.rev, keep=False, skip_edge_out=False)
-        line = None
-        if g.n_triplets:
-            c = g.lg_cols
-            line = SimpleNamespace(is_atom=False, n_rows=g.n_triplets, n_nodes=g.n_bonds, n_edge_rows=g.n_triplets,
-                                   ctr=c[0], tgt=c[1], src=c[3], tgt_ptr=g.trip_ptr, src_ptr=g.trip_src_ptr,
-                                   src_perm=g.trip_src_perm, emap=None, u2d=None, rev=None, keep=False,
-                                   skip_edge_out=False)
-        g._row_graphs = (atom, line)
-    return g._row_graphs
+    """The two message-passing graphs of a batch as the library takes them (rows grouped by target node, the source side
+    as a permutation)."""
+    p = _lib.ptr
+    atom = SimpleNamespace(n_bonds=g.n_bonds, skip_edge_out=False, alive=g, c=_lib.MbRowGraph(
+        n_rows=g.n_edges, n_nodes=g.n_atoms, n_edge_rows=g.n_bonds, is_atom=1, tgt=p(g.center), src=p(g.neighbor),
+        tgt_ptr=p(g.edge_ptr), src_ptr=p(g.edge_ptr), src_perm=p(g.rev), emap=p(g.d2u), u2d=p(g.u2d), rev=p(g.rev)))
+    line = None
+    if g.n_triplets:
+        cols = g.lg_cols
+        line = SimpleNamespace(n_bonds=g.n_bonds, skip_edge_out=False, alive=g, c=_lib.MbRowGraph(
+            n_rows=g.n_triplets, n_nodes=g.n_bonds, n_edge_rows=g.n_triplets, n_ctr=g.n_atoms, ctr=p(cols[0]),
+            tgt=p(cols[1]), src=p(cols[3]), tgt_ptr=p(g.trip_ptr), src_ptr=p(g.trip_src_ptr), src_perm=p(g.trip_src_perm)))
+    return atom, line
 
 
-# ------------------------------------------------------------------ gated MLP building block
-def gated_fwd(p, n_rows, srcs, want_h=True, res=None, res_w=None, save=True):
-    """GatedMLP.forward (matris/model/functions.py:300-311) in one kernel: returns (z1, z2, h, out2) with
-    z1 = X W1^T + b1 (core|gate pre-activations) and z2 = SiLU(z1) W2^T + b2 (pre-norm) only when ``save``."""
-    if getattr(p, "kind", "gated") == "mlp":
-        return _mlp_fwd(p, n_rows, srcs, want_h, res, res_w)
-    return ops.gated_mlp_fwd(p, n_rows, srcs, want_h=want_h, res=res, res_w=res_w, save=save)
-
-
-def _mlp_fwd(p, n_rows, srcs, want_h, res, res_w):
-    """The plain-MLP variant of an update block: h = RMSNorm(W2 SiLU(W1 x + b1) + b2); same return convention, with
-    z1 / z2 the two [rows,128] pre-activation / pre-norm tensors (always produced: they are the intermediates)."""
-    like = srcs[0][0]
-    z1, z2 = ops.new(n_rows, D, like), ops.new(n_rows, D, like)
-    gemm(n_rows, [B(srcs, p.w1, bias=p.b1, out=z1)])
-    gemm(n_rows, [B([S(z1, None, 0, 1)], p.w2, bias=p.b2, out=z2)])
-    h = ops.rmsnorm_fwd(z2, p.nw)
-    out2 = None
-    if res is not None:
-        out2 = h.clone()
-        ops.scale_rows(res, res_w, y=out2, accumulate=True)
-    return z1, z2, (h if want_h else None), out2
-
-
-def _gate_args(p, z2):
-    """What the kernels that produce a gated MLP's dh need to apply the tail adjoint themselves (None for the
-    plain-MLP variant, whose tail is an RMSNorm handled in ``gated_bwd``)."""
-    return None if getattr(p, "kind", "gated") == "mlp" else (z2, p.nc, p.ng)
-
-
-def gated_bwd(p, n_rows, z1, z2, dh, dests, dz2=None):
-    """Backward through the gated MLP: dests[c] = (tensor, idx, mode[, res, res_w]) for K segment c.  With ``res``
-    the block stores ``gemm + res_w * res`` (the residual branch's gradient joins in the epilogue instead of in a
-    separate scaling pass followed by an accumulate).  ``dz2``: the tail adjoint, where the producer of dh has
-    already applied it (then ``dh`` is not read)."""
-    if getattr(p, "kind", "gated") == "mlp":
-        dy = ops.rmsnorm_bwd(z2, p.nw, dh.contiguous())
-        da1 = torch.empty_like(z1)
-        gemm(n_rows, [B([S(dy)], p.w2t, gate=z1, out=da1)])
-        blocks, srcs = [], [S(da1)]  # one list of sources for all column blocks
-        for c, dest in enumerate(dests):
-            t, idx, mode = dest[:3]
-            if t is None:
-                continue
-            res, res_w = (dest[3], dest[4]) if len(dest) > 3 else (None, None)
-            blocks.append(B(srcs, p.w1t, w_row=D * c, out=t, out_idx=idx, mode=mode, res=res, res_w=res_w))
-        gemm(n_rows, blocks)
-        return
-    if dz2 is None:
-        dz2 = ops.gate_bwd(z2, p.nc, p.ng, dh)
-    dz1 = torch.empty_like(z1)
-    gemm(n_rows, [B([S(dz2, None, D * j)], p.w2t, w_row=D * j, gate=z1, gate_col=D * j, out=dz1, out_col=D * j)
-                  for j in (0, 1)])
-    del dz2
-    blocks, srcs = [], [S(dz1, None, 0), S(dz1, None, D)]  # one list of sources for all column blocks
-    for c, dest in enumerate(dests):
-        t, idx, mode = dest[:3]
-        if t is None:
-            continue
-        res, res_w = (dest[3], dest[4]) if len(dest) > 3 else (None, None)
-        blocks.append(B(srcs, p.w1t, w_row=D * c, out=t, out_idx=idx, mode=mode, res=res, res_w=res_w))
-    gemm(n_rows, blocks)
-
-
-# ------------------------------------------------------------------ attention layer
-def _attn_forward(P, rg, node, edge, save=True):
-    """``save``: also return the internals the backward pass reads (z1, z2 of both gated MLPs are then written)."""
-    R, Nn, Ne = rg.n_rows, rg.n_nodes, rg.n_edge_rows
-    srcs = [S(edge, rg.emap), S(node, rg.tgt), S(node, rg.src)]
-    if rg.is_atom:
-        z1, z2, h, _ = gated_fwd(P.edge, R, srcs, save=save)
-        edge_out = ops.pair_mean_res(Ne, rg.u2d, rg.rev, h, edge, P.we)
-    else:
-        z1, z2, h, edge_out = gated_fwd(P.edge, R, srcs, res=edge, res_w=P.we, save=save)
-    logits = ops.linear(edge, P.wst)                      # [Ne,256]: source | target logits
-    agg_t, agg_s, stats = ops.seg_attn_fwd(Nn, rg.tgt_ptr, rg.src_ptr, rg.src_perm, rg.emap, logits, h)
-    z1n, z2n, _, node_out = gated_fwd(P.node, Nn, [S(node), S(agg_t), S(agg_s)], want_h=False, res=node, res_w=P.wn,
-                                      save=save)
-    return node_out, edge_out, (z1, z2, h, logits, agg_t, agg_s, stats, z1n, z2n)
+def _layer_call(entry, like, *args):
+    """Call a sub-block entry point with a workspace of the size it asks for."""
+    need = C.c_size_t(0)
+    _lib.call(entry, *args, None, C.byref(need), None)
+    ws = torch.empty(need.value, dtype=torch.uint8, device=like.device)
+    _lib.call(entry, *args, ws.data_ptr(), C.byref(need), ops._stream())
 
 
 class AttentionFn(torch.autograd.Function):
-    """Graph_Attention_Layer.forward (matris/model/interaction_block.py:87-143)."""
+    """Graph_Attention_Layer.forward (matris/model/interaction_block.py:87-143) and its data gradients."""
 
     @staticmethod
     def forward(ctx, node, edge, P, rg):
         node, edge = node.contiguous(), edge.contiguous()
-        keep = bool(rg.keep and any(ctx.needs_input_grad))
-        node_out, edge_out, inter = _attn_forward(P, rg, node, edge, save=keep)
+        node_out, edge_out = torch.empty_like(node), torch.empty_like(edge)
+        p = _lib.ptr
+        _layer_call("mb_attention_layer", node, C.byref(P), C.byref(rg.c), p(node), p(edge), p(node_out), p(edge_out), None,
+                    None, None, None)
         ctx.save_for_backward(node, edge)
         ctx.P, ctx.rg = P, rg
-        ctx.inter = inter if keep else None
         return node_out, edge_out
 
     @staticmethod
     @once_differentiable
     def backward(ctx, d_node_out, d_edge_out):
         node, edge = ctx.saved_tensors
-        P, rg = ctx.P, ctx.rg
-        R, Nn, Ne = rg.n_rows, rg.n_nodes, rg.n_edge_rows
         d_node_out, d_edge_out = d_node_out.contiguous(), d_edge_out.contiguous()
-        inter, ctx.inter = ctx.inter, None
-        if inter is None:  # internals were not kept: recompute them from the saved inputs
-            _, _, inter = _attn_forward(P, rg, node, edge)
-        z1, z2, h, logits, agg_t, agg_s, stats, z1n, z2n = inter
-        del inter
-        # node update
-        d_node = ops.scale_rows(d_node_out, P.wn)
-        dagg_t, dagg_s = ops.new(Nn, D, node), ops.new(Nn, D, node)
-        gated_bwd(P.node, Nn, z1n, z2n, d_node_out,
-                  [(d_node, None, OUT_ADD), (dagg_t, None, OUT_STORE), (dagg_s, None, OUT_STORE)])
-        del z1n, z2n
-        # softmax-weighted aggregation
-        # (the row gradient dh goes straight on through the gated MLP's tail adjoint: dz2 comes back instead)
-        gate = _gate_args(P.edge, z2)
-        dh, dlogits = ops.seg_attn_bwd(rg.tgt, rg.src, rg.emap, logits, h, agg_t, agg_s, stats, dagg_t, dagg_s,
-                                       d_edge_out, rg.emap, 0.5 if rg.is_atom else 1.0, gate=gate)
-        dz2, dh = (dh, None) if gate is not None else (None, dh)
-        del logits, h, agg_t, agg_s, stats, dagg_t, dagg_s
-        # edge update (line graph: rows map one to one, so the residual gradient we * d_edge_out rides in the
-        # epilogue of the store; atom graph: two directed rows add into one bond row, so it is laid down first)
-        emode = OUT_ATOMIC if rg.is_atom else OUT_ADD
-        if rg.is_atom:
-            d_edge = ops.scale_rows(d_edge_out, P.we)
-            edge_dest = (d_edge, rg.emap, OUT_ATOMIC)
-        else:
-            d_edge = torch.empty_like(d_edge_out)
-            edge_dest = (d_edge, None, OUT_STORE, d_edge_out, P.we)
-        gated_bwd(P.edge, R, z1, z2, dh, [edge_dest, (d_node, rg.tgt, OUT_ATOMIC), (d_node, rg.src, OUT_ATOMIC)],
-                  dz2=dz2)
-        del z1, z2, dh, dz2
-        gemm(R, [B([S(dlogits, None, 0), S(dlogits, None, D)], P.wstt, out=d_edge, out_idx=rg.emap, mode=emode)])
+        d_node, d_edge = torch.empty_like(node), torch.empty_like(edge)
+        p = _lib.ptr
+        _layer_call("mb_attention_layer", node, C.byref(ctx.P), C.byref(ctx.rg.c), p(node), p(edge), None, None,
+                    p(d_node_out), p(d_edge_out), p(d_node), p(d_edge))
         return d_node, d_edge, None, None
 
 
-# ------------------------------------------------------------------ refinement layer
-def _refine_forward(P, rg, node, edge, rbf, atom_feat, save=True, want_edge=True):
-    R, Nn, Ne = rg.n_rows, rg.n_nodes, rg.n_edge_rows
-    if rg.is_atom:
-        srcs = [S(edge, rg.emap), S(node, rg.tgt), S(node, rg.src)]
-    else:
-        srcs = [S(edge), S(atom_feat, rg.ctr), S(node, rg.tgt), S(node, rg.src)]
-    z1, z2, h, _ = gated_fwd(P.edge, R, srcs, save=save)
-    env = ops.small_linear_fwd(rbf, P.wenv)               # [bonds,128]
-    agg = ops.seg_smooth_sum_fwd(Nn, rg.tgt_ptr, rg.emap, None if rg.is_atom else rg.src, env, h)
-    zn, _, node_out = ops.ffn_fwd(P.nffn, agg, want_y=False, res=node, res_w=P.wn, save=save)
-    # the edge update reads the unsmoothed rows unless use_smoothed_for_delta_edge (atom graph only,
-    # interaction_block.py:262-266): then it reads h * s, s = the envelope row of the edge's bond
-    if not want_edge:  # the last layer's edge update feeds nothing
-        return node_out, None, (z1, z2, h, env, zn, None)
-    ffn_in = ops.mul_rows_gather(h, env, rg.emap) if P.smoothed_edge else h
-    if rg.is_atom:
-        ze, y, _ = ops.ffn_fwd(P.effn, ffn_in, save=save)
-        edge_out = ops.pair_mean_res(Ne, rg.u2d, rg.rev, y, edge, P.we)
-    else:
-        ze, _, edge_out = ops.ffn_fwd(P.effn, ffn_in, want_y=False, res=edge, res_w=P.we, save=save)
-    return node_out, edge_out, (z1, z2, h, env, zn, ze)
-
-
 class RefineFn(torch.autograd.Function):
-    """Refinement.forward (matris/model/interaction_block.py:218-278)."""
+    """Refinement.forward (matris/model/interaction_block.py:218-278) and its data gradients.  With ``rg.skip_edge_out``
+    the edge update is not computed; a placeholder nobody reads keeps the signature (node, edge)."""
 
     @staticmethod
     def forward(ctx, node, edge, rbf, atom_feat, P, rg):
         node, edge, rbf = node.contiguous(), edge.contiguous(), rbf.contiguous()
         if atom_feat is not None:
             atom_feat = atom_feat.contiguous()
-        keep = bool(rg.keep and any(ctx.needs_input_grad))
         want_edge = not rg.skip_edge_out
-        node_out, edge_out, inter = _refine_forward(P, rg, node, edge, rbf, atom_feat, save=keep, want_edge=want_edge)
+        node_out = torch.empty_like(node)
+        edge_out = torch.empty_like(edge) if want_edge else edge.new_empty(0)
+        p = _lib.ptr
+        _layer_call("mb_refine_layer", node, C.byref(P), C.byref(rg.c), p(node), p(edge), p(rbf), p(atom_feat), p(node_out),
+                    p(edge_out) if want_edge else None, None, None, None, None, None, None)
         ctx.save_for_backward(node, edge, rbf, atom_feat)
         ctx.P, ctx.rg, ctx.want_edge = P, rg, want_edge
-        ctx.inter = inter if keep else None
-        if not want_edge:  # a placeholder nobody reads, so that the signature stays (node, edge)
-            edge_out = edge.new_empty(0)
+        if not want_edge:
             ctx.mark_non_differentiable(edge_out)
         return node_out, edge_out
 
@@ -349,201 +238,13 @@ class RefineFn(torch.autograd.Function):
     @once_differentiable
     def backward(ctx, d_node_out, d_edge_out):
         node, edge, rbf, atom_feat = ctx.saved_tensors
-        P, rg = ctx.P, ctx.rg
-        R, Nn, Ne = rg.n_rows, rg.n_nodes, rg.n_edge_rows
-        want_edge = ctx.want_edge
-        d_node_out = d_node_out.contiguous()
-        d_edge_out = d_edge_out.contiguous() if want_edge else None
-        inter, ctx.inter = ctx.inter, None
-        if inter is None:
-            _, _, inter = _refine_forward(P, rg, node, edge, rbf, atom_feat, want_edge=want_edge)
-        z1, z2, h, env, zn, ze = inter
-        del inter
-        # node FFN
-        d_node = ops.scale_rows(d_node_out, P.wn)
-        dzn = ops.linear(d_node_out, P.nffn.w2t, gate=zn)
-        dagg = ops.linear(dzn, P.nffn.w1t)
-        del zn, dzn
-        # edge FFN (atom graph: the mean over the two directions is a gather * 0.5)
-        drow = None
-        if want_edge:
-            if rg.is_atom:
-                dze = ops.linear(d_edge_out, P.effn.w2t, gate=ze, scale=0.5, idx=rg.emap)
-            else:
-                dze = ops.linear(d_edge_out, P.effn.w2t, gate=ze)
-            dh = ops.linear(dze, P.effn.w1t)
-            del ze, dze
-            if P.smoothed_edge:  # dh so far is the gradient of the smoothed rows h * s
-                drow, dh = dh, ops.mul_rows_gather(dh, env, rg.emap)
-        else:
-            dh = ops.new(R, D, dagg)  # no edge update, no gradient from it: the aggregation's term starts the row
-        # smoothed aggregation
-        src = None if rg.is_atom else rg.src
-        dz2 = ops.seg_smooth_sum_bwd_rows(rg.tgt, src, rg.emap, env, dagg, dh, accumulate=want_edge,
-                                          gate=_gate_args(P.edge, z2))  # with a gate: dh is finished in registers
-        denv = ops.seg_smooth_sum_bwd_env(env.shape[0], rg.tgt_ptr, None if rg.is_atom else rg.src_ptr, rg.src_perm,
-                                          rg.tgt, src if src is not None else rg.src, rg.u2d, rg.rev, env, h, dagg,
-                                          drow=drow)
-        del drow
-        d_rbf = ops.small_linear_bwd(denv, P.wenv)
-        del env, denv, dagg, h
-        # gated MLP
-        if rg.is_atom:
-            d_atom = None
-            d_edge = ops.scale_rows(d_edge_out, P.we) if want_edge else torch.zeros_like(edge)
-            dests = [(d_edge, rg.emap, OUT_ATOMIC), (d_node, rg.tgt, OUT_ATOMIC), (d_node, rg.src, OUT_ATOMIC)]
-        else:
-            d_atom = torch.zeros_like(atom_feat)
-            d_edge = torch.empty_like(edge)  # stored once: gemm (+ we * d_edge_out in the epilogue)
-            edge_dest = (d_edge, None, OUT_STORE, d_edge_out, P.we) if want_edge else (d_edge, None, OUT_STORE)
-            dests = [edge_dest, (d_atom, rg.ctr, OUT_ATOMIC), (d_node, rg.tgt, OUT_ATOMIC), (d_node, rg.src, OUT_ATOMIC)]
-        gated_bwd(P.edge, R, z1, z2, dh, dests, dz2=dz2)
+        d_node_out, d_edge_out = d_node_out.contiguous(), d_edge_out.contiguous() if ctx.want_edge else None
+        d_node, d_edge, d_rbf = torch.empty_like(node), torch.empty_like(edge), torch.zeros_like(rbf)
+        d_atom = None if atom_feat is None else torch.zeros_like(atom_feat)
+        p = _lib.ptr
+        _layer_call("mb_refine_layer", node, C.byref(ctx.P), C.byref(ctx.rg.c), p(node), p(edge), p(rbf), p(atom_feat), None,
+                    None, p(d_node_out), p(d_edge_out), p(d_node), p(d_edge), p(d_rbf), p(d_atom))
         return d_node, d_edge, d_rbf, d_atom, None, None
-
-
-# ------------------------------------------------------------------ geometry, embeddings, readout
-class EdgeGeometryFn(torch.autograd.Function):
-    """Edge vectors / lengths / unit vectors and their adjoint: forces and virial
-    (matris/model/processgraph.py:169-199, matris/model/readout.py:202-224).  ``strain`` is the
-    zero strain leaf; the forward value does not depend on it, its gradient is sym(sum v (x) dE/dv)."""
-
-    @staticmethod
-    def forward(ctx, cart, strain, g):
-        vec, length, unit = ops.edge_geometry_fwd(cart.contiguous(), g.lattice32, g.atom_struct, g.center, g.neighbor,
-                                                  g.image)
-        ctx.save_for_backward(vec, length, unit)
-        ctx.g, ctx.has_strain = g, strain is not None
-        ctx.mark_non_differentiable(vec)
-        return length, unit, vec
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, dlen, dunit, _dvec):
-        vec, length, unit = ctx.saved_tensors
-        g = ctx.g
-        dcart, dstrain, _ = ops.edge_geometry_bwd(g.n_atoms, g.n_struct, g.edge_ptr, g.atom_ptr, g.rev, vec, length,
-                                                  unit, dlen.contiguous(), dunit.contiguous())
-        return dcart, (dstrain if ctx.has_strain else None), None
-
-
-def _rbf_forward(P, g, length, cfg):
-    if P.gaussian:
-        return ops.gaussian_fwd(g.u2d, length, P.freq2, P.coeff2, P.freq3, P.coeff3)
-    return ops.bessel_fwd(g.u2d, length, P.freq2, cfg["pairwise_cutoff"], P.freq3, cfg["three_body_cutoff"],
-                          cfg["envelope_exponent"])
-
-
-def _angle_basis(P, g, unit, cfg):
-    if P.fourier:
-        return ops.fourier_basis_fwd(g.line_graph, unit, P.t_freq)
-    return ops.angle_basis_fwd(g.line_graph, unit, P.sph_factor, cfg["pairwise_cutoff"])
-
-
-def _edge_embed_forward(P, g, length, cfg):
-    rbf2, rbf3 = _rbf_forward(P, g, length, cfg)
-    e1 = ops.small_linear_fwd(rbf2, P.e_w1)
-    e2 = ops.linear(e1, P.e_w2)
-    # both directed copies of a bond carry the same row, so their mean is the row itself:
-    # the expand-to-directed / average-back pair of the reference is the identity here
-    e3 = ops.layernorm_fwd(e2, P.e_lnw, P.e_lnb)
-    return rbf2, rbf3, e2, e3
-
-
-class EdgeEmbedFn(torch.autograd.Function):
-    """EdgeBasisEmbedding.forward (matris/model/feature_embed.py:114-148)."""
-
-    @staticmethod
-    def forward(ctx, length, P, g, cfg):
-        length = length.contiguous()
-        rbf2, rbf3, _, e3 = _edge_embed_forward(P, g, length, cfg)
-        edge = ops.linear(e3, P.e_w3, out_act=1)
-        ctx.save_for_backward(length)
-        ctx.P, ctx.g, ctx.cfg = P, g, cfg
-        return edge, rbf2, rbf3
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, d_edge, d_rbf2, d_rbf3):
-        (length,) = ctx.saved_tensors
-        P, g, cfg = ctx.P, ctx.g, ctx.cfg
-        _, _, e2, e3 = _edge_embed_forward(P, g, length, cfg)
-        z = ops.linear(e3, P.e_w3)
-        dz = ops.silu_bwd(d_edge.contiguous(), z)
-        de3 = ops.linear(dz, P.e_w3t)
-        de2 = ops.layernorm_bwd(e2, P.e_lnw, de3)
-        de1 = ops.linear(de2, P.e_w2t)
-        d2 = d_rbf2.contiguous().clone()
-        ops.small_linear_bwd(de1, P.e_w1, d2, accumulate=True)
-        if P.gaussian:
-            dlen = ops.gaussian_bwd(g.u2d, length, P.freq2, P.coeff2, P.freq3, P.coeff3, d2, d_rbf3.contiguous())
-        else:
-            dlen = ops.bessel_bwd(g.u2d, length, P.freq2, cfg["pairwise_cutoff"], P.freq3, cfg["three_body_cutoff"],
-                                  cfg["envelope_exponent"], d2, d_rbf3.contiguous())
-        return dlen, None, None, None
-
-
-class AngleEmbedFn(torch.autograd.Function):
-    """ThreebodyEmbedding.forward (matris/model/feature_embed.py:183-203)."""
-
-    @staticmethod
-    def forward(ctx, unit, P, g, cfg):
-        unit = unit.contiguous()
-        basis = _angle_basis(P, g, unit, cfg)
-        t1 = ops.small_linear_fwd(basis, P.t_wa)
-        trip = ops.linear(t1, P.t_wb, out_act=1)
-        ctx.save_for_backward(unit)
-        ctx.P, ctx.g, ctx.cfg = P, g, cfg
-        return trip
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, d_trip):
-        (unit,) = ctx.saved_tensors
-        P, g, cfg = ctx.P, ctx.g, ctx.cfg
-        basis = _angle_basis(P, g, unit, cfg)
-        t1 = ops.small_linear_fwd(basis, P.t_wa)
-        z = ops.linear(t1, P.t_wb)
-        del basis, t1
-        dz = ops.silu_bwd(d_trip.contiguous(), z)
-        dt1 = ops.linear(dz, P.t_wbt)
-        del z, dz
-        dbasis = ops.small_linear_bwd(dt1, P.t_wa)
-        if P.fourier:
-            dunit = ops.fourier_basis_bwd(g.line_graph, unit, P.t_freq, dbasis)
-        else:
-            dunit = ops.angle_basis_bwd(g.line_graph, unit, P.sph_factor, cfg["pairwise_cutoff"], dbasis)
-        return dunit, None, None, None
-
-
-class EnergyFn(torch.autograd.Function):
-    """readout_norm + EnergyHead + per-structure sum (matris/model/model.py:216-218,
-    matris/model/readout.py:66-75).  Also returns the normalised features for the magmom head."""
-
-    @staticmethod
-    def forward(ctx, node, P, g):
-        node = node.contiguous()
-        nn_ = ops.rmsnorm_fwd(node, P.out_norm)
-        z1 = ops.linear(nn_, P.h_w0, bias=P.h_b0)
-        z2 = ops.linear(z1, P.h_w3, bias=P.h_b3, in_act=1)
-        e_atom = ops.head_dot_fwd(z2, P.h_w6, P.h_b6)
-        energy = ops.segment_sum_scalar(g.n_struct, g.atom_ptr, e_atom)
-        ctx.save_for_backward(node)
-        ctx.P, ctx.g = P, g
-        ctx.mark_non_differentiable(nn_)
-        return energy, nn_
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, d_energy, _d_nn):
-        (node,) = ctx.saved_tensors
-        P, g = ctx.P, ctx.g
-        nn_ = ops.rmsnorm_fwd(node, P.out_norm)
-        z1 = ops.linear(nn_, P.h_w0, bias=P.h_b0)
-        z2 = ops.linear(z1, P.h_w3, bias=P.h_b3, in_act=1)
-        dz2 = ops.head_dot_bwd(z2, P.h_w6, d_energy.contiguous(), g.atom_struct)
-        dz1 = ops.linear(dz2, P.h_w3t, gate=z1)
-        dnn = ops.linear(dz1, P.h_w0t)
-        return ops.rmsnorm_bwd(node, P.out_norm, dnn), None, None
 
 
 # ------------------------------------------------------------------ the module
@@ -615,7 +316,6 @@ class MatRIS(nn.Module):
         for key, value in random_state_dict(cfg, seed=seed).items():
             self._register(key, value, buffer=key in BUFFER_KEYS, trainable=not key.startswith("reference_energy"))
         self._packed = None
-        self._ref_table = None
         self._packed_device = None
         self.last_batch = None
         # None: decide per call from free memory; True / False: keep / recompute all; n: keep the last n layers' internals
@@ -641,7 +341,6 @@ class MatRIS(nn.Module):
 
     def _apply(self, fn, *a, **k):
         self._packed = None
-        self._ref_table = None
         out = super()._apply(fn, *a, **k)
         # graphs are built where the weights live: a batch on another GPU would be read through peer pointers
         # (or fault without peer access) by kernels launched on this one
@@ -651,7 +350,6 @@ class MatRIS(nn.Module):
 
     def load_state_dict(self, state_dict, strict: bool = True, **kw):
         self._packed = None
-        self._ref_table = None
         return super().load_state_dict(state_dict, strict=strict, **kw)
 
     def packed(self, device):
@@ -775,19 +473,28 @@ class MatRIS(nn.Module):
             avail = min(avail, float(self.memory_limit_bytes))
         return avail
 
-    def kept_layers(self, n_triplets: int, n_edges: int, avail: float | None = None) -> int:
-        """How many (last) layers keep their sub-block internals for the backward pass on a batch with that many
-        triplet rows and directed edges; the internals of the earlier layers are recomputed there.  The internals
-        take ~6.7 KB per triplet row and ~6.2 KB per directed edge per layer and are consumed and released last
-        layer first: all layers are kept when that fits in 45 % of the available memory, otherwise as many as do,
-        within two more bounds (see below).  ``keep_activations`` overrides: True / False / a number of layers."""
-        n_layers = int(self.config["num_layers"])
-        keep = self.keep_activations
+    def _plan_memory(self, e: _lib.MbEval) -> int:
+        """Decide how many (last) layers keep their internals for the backward pass - as many as fit in memory, or what
+        ``keep_activations`` says - and set it in ``e``; returns the bytes the evaluation will use."""
+        def need(n):
+            e.keep_layers = n
+            _lib.check(_lib.load().mb_evaluate_workspace(C.byref(e), C.byref(size)), "mb_evaluate_workspace")
+            return size.value
+
+        size, n_layers, keep = C.c_size_t(0), e.model.contents.n_layers, self.keep_activations
         if keep is not None:
-            if isinstance(keep, bool):
-                return n_layers if keep else 0
-            return max(0, min(n_layers, int(keep)))
-        return kept_layers_for(n_layers, n_triplets, n_edges, self._available_bytes() if avail is None else avail)
+            n = (n_layers if keep else 0) if isinstance(keep, bool) else max(0, min(n_layers, int(keep)))
+            return need(n)
+        budget = 0.9 * self._available_bytes()
+        # the need grows with the number of kept layers: the largest that fits, by bisection
+        best = need(n_layers)
+        if best <= budget:
+            return best
+        lo, hi = 0, n_layers
+        while hi - lo > 1:
+            mid = (lo + hi) // 2
+            lo, hi = (mid, hi) if need(mid) <= budget else (lo, mid)
+        return need(lo)
 
     def split_for_memory(self, g: BatchedGraph, headroom: float = 0.93) -> list[tuple[int, int]]:
         """Contiguous ranges of the structures of batch ``g`` such that every range, evaluated as a batch of its own,
@@ -805,77 +512,53 @@ class MatRIS(nn.Module):
         return split_ranges(np.diff(tp), np.diff(ep), lambda t, e: kept_layers_for(n_layers, t, e, avail) == n_layers)
 
     def _evaluate(self, g: BatchedGraph, task: str):
-        cfg = self.config
-        P = self.packed(self.device)
-        atom_rg, line_rg = row_graphs(g)
-        want_f, want_s = "f" in task, "s" in task
-        need_grad = want_f or want_s
-        n_layers = len(P.layers)
-        n_keep = self.kept_layers(g.n_triplets, g.n_edges)
-        self.last_kept_layers = n_keep
-        out = {}
-        with torch.set_grad_enabled(need_grad):
-            cart = g.cart32.detach().clone().requires_grad_(need_grad)
-            strain = None
-            if want_s:
-                strain = torch.zeros(g.n_struct, 3, 3, dtype=torch.float32, device=cart.device, requires_grad=True)
-            length, unit, _ = EdgeGeometryFn.apply(cart, strain, g)
-            node = ops.linear(ops.embedding(g.numbers, -1, P.emb_table), P.emb_w, out_act=1)
-            edge, rbf2, rbf3 = EdgeEmbedFn.apply(length, P, g, cfg)
-            trip = AngleEmbedFn.apply(unit, P, g, cfg) if line_rg is not None else None
-            for i, L in enumerate(P.layers):
-                atom_rg.keep = i >= n_layers - n_keep
-                # after the last layer only the atom features are read (matris/model/model.py:215-231; the edge features
-                # go to the non-conservative force head only): its two refinements need no edge update
-                atom_rg.skip_edge_out = i == n_layers - 1
-                if line_rg is not None:
-                    line_rg.keep, line_rg.skip_edge_out = atom_rg.keep, atom_rg.skip_edge_out
-                e_att, t_att = edge, trip
-                if trip is not None:
-                    e_att, t_att = AttentionFn.apply(edge, trip, L.attn_line, line_rg)
-                n_att, e_att = AttentionFn.apply(node, e_att, L.attn_atom, atom_rg)
-                e_upd, t_upd = edge, trip
-                if trip is not None:
-                    e_upd, t_upd = RefineFn.apply(e_att, t_att, rbf3, n_att, L.refine_line, line_rg)
-                node, edge = RefineFn.apply(n_att, e_upd, rbf2, None, L.refine_atom, atom_rg)
-                trip = t_upd
-            energy, node_n = EnergyFn.apply(node, P, g)
-            if need_grad:
-                leaves = [cart] + ([strain] if want_s else [])
-                grads = torch.autograd.grad(energy.sum(), leaves)
-                if want_f:
-                    out["f"] = torch.split(-grads[0], g.atoms_per_graph)
-                if want_s:
-                    scale = (GPA_PER_EV_A3 / g.volume).view(-1, 1, 1)
-                    out["s"] = list(torch.unbind(grads[-1] * scale, dim=0))
-        energy = energy.detach()
-        if "m" in task:
-            zm = ops.linear(node_n, P.m_w0, bias=P.m_b0)
-            out["m"] = list(torch.split(ops.head_dot_fwd(zm, P.m_w3, P.m_b3, take_abs=True), g.atoms_per_graph))
-        apg = g.atom_ptr[1:] - g.atom_ptr[:-1]  # atoms per structure, on the device (no host copy, no synchronisation)
-        out["e"] = energy / apg if self.is_intensive else energy
-        out["atoms_per_graph"] = apg
-        ref = 0
-        if cfg["reference_energy"] is not None:
-            ref = self._reference_energy(g)
-        out["e"] = out["e"] + ref
-        out["ref_energy"] = ref
-        return out
+        dev, n_struct, n_atoms = self.device, g.n_struct, g.n_atoms
+        P = self.packed(dev)
+        want = {"f": 3 * n_atoms if "f" in task else 0, "s": 9 * n_struct if "s" in task else 0,
+                "m": n_atoms if "m" in task else 0}
+        e, p = _lib.MbEval(), _lib.ptr
+        e.model = C.pointer(P.model)
+        e.n_atoms, e.n_struct, e.n_edges, e.n_bonds, e.n_triplets = n_atoms, n_struct, g.n_edges, g.n_bonds, g.n_triplets
+        e.cart, e.lattice, e.volume = p(g.cart32), p(g.lattice32), p(g.volume)
+        e.atom_struct, e.atom_ptr, e.numbers = p(g.atom_struct), p(g.atom_ptr), p(g.numbers)
+        e.center, e.neighbor, e.image, e.edge_ptr = p(g.center), p(g.neighbor), p(g.image), p(g.edge_ptr)
+        e.rev, e.d2u, e.u2d = p(g.rev), p(g.d2u), p(g.u2d)
+        e.trip_ptr, e.trip_src_ptr, e.trip_src_perm = p(g.trip_ptr), p(g.trip_src_ptr), p(g.trip_src_perm)
+        e.line_graph, e.lg_cols = p(g.line_graph), p(g.lg_cols)
+        energy, ref = (torch.empty(n_struct, dtype=torch.float32, device=dev) for _ in range(2))
+        apg = torch.empty(n_struct, dtype=torch.int32, device=dev)
+        res = {k: torch.empty(n, dtype=torch.float32, device=dev) for k, n in want.items() if n}
+        e.e, e.ref, e.atoms_per_struct = p(energy), p(ref), p(apg)
+        e.f, e.s, e.m = (p(res.get(k)) for k in ("f", "s", "m"))
+        size = self._plan_memory(e)
+        self.last_kept_layers = e.keep_layers
+        if size <= WORKSPACE_LIMIT:
+            # sizes in steps of an eighth of their power of two, so that the slightly different graphs of successive steps
+            # find the block of the step before in the allocator's cache
+            step = 1 << max(12, size.bit_length() - 4)
+            size = (size + step - 1) // step * step
+            ws = torch.empty(size, dtype=torch.uint8, device=dev)
+            e.ws, e.ws_bytes = ws.data_ptr(), size
+        else:
+            stream = torch.cuda.current_stream(dev)
 
-    def _reference_energy(self, g: BatchedGraph):
-        """AtomRef.forward (matris/model/reference_energy.py:34-55): composition-weighted table sum, float32."""
-        # evaluated on the device from the batch's own index tensors: a host round trip here would synchronise the
-        # stream at the end of every evaluation
-        table = getattr(self, "_ref_table", None)
-        if table is None or table.device != g.numbers.device:
-            table = self._ref_table = (self.state_dict()["reference_energy.fc.weight"].detach().reshape(-1)
-                                       .to(device=g.numbers.device, dtype=torch.float32))
-        comp = torch.zeros(g.n_struct, table.numel(), dtype=torch.float32, device=table.device)
-        comp.index_put_((g.atom_struct.long(), (g.numbers - 1).long()),
-                        torch.ones(g.n_atoms, dtype=torch.float32, device=table.device), accumulate=True)
-        if self.is_intensive:
-            comp = comp / (g.atom_ptr[1:] - g.atom_ptr[:-1]).to(torch.float32)[:, None]
-        return comp @ table
+            def alloc(n):
+                try:
+                    return torch.cuda.caching_allocator_alloc(n, dev, stream)
+                except torch.cuda.OutOfMemoryError:  # comes back as a status code
+                    return None
+            e.alloc, e.release = _lib.ALLOC_FN(alloc), _lib.FREE_FN(torch.cuda.caching_allocator_delete)
+        _lib.evaluate(e, ops._stream())
+        out = {}
+        if "f" in res:
+            out["f"] = torch.split(res["f"].view(n_atoms, 3), g.atoms_per_graph)
+        if "s" in res:
+            out["s"] = list(torch.unbind(res["s"].view(n_struct, 3, 3), dim=0))
+        if "m" in res:
+            out["m"] = list(torch.split(res["m"], g.atoms_per_graph))
+        out["e"], out["atoms_per_graph"] = energy, apg
+        out["ref_energy"] = ref if self.config["reference_energy"] is not None else 0
+        return out
 
     # -- convenience ------------------------------------------------------------------------
     def plan_batches(self, structures) -> list[BatchedGraph]:
