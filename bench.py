@@ -38,7 +38,7 @@ if ROOT not in sys.path:
     sys.path.insert(0, ROOT)
 
 NUM_LAYERS = 10
-GEMM_CALLS = ("mb_gemm", "mb_gated_mlp_fwd")  # the tensor-core entry points
+GEMM_CALLS = ("mb_gemm", "mb_gated_mlp_fwd", "mb_mlp_bwd_data")  # the tensor-core entry points
 PER_GPU = {"perov512": 512, "random256": 256, "random64": 64}
 
 

@@ -224,9 +224,18 @@ int mb_selftest_wait_expiry(void* stream);
  * denominator the 3-pass tf32 GEMMs are judged against. */
 int mb_bench_mma_rate(int kind, int iters, float* elapsed_ms, int* n_sms, void* stream);
 
+/* A 128-wide weight matrix with its operand splits, all in one layout (see mb_colblock) */
+typedef struct mb_weight {
+  const float* W; const float* W_hi; const float* W_lo;
+  const uint16_t* W_hi16; const uint16_t* W_lo16;
+  int64_t ldw;
+} mb_weight;
+/* rows of a table of finished sums, gathered per row and added to layer 1 of a fused MLP */
+typedef struct mb_add { const float* ptr; const int32_t* idx; int64_t ld; } mb_add;
+
 /* ------------------------------------------------------------------ fused gated MLP (forward)
  * GatedMLP.forward (matris/model/functions.py:245-311) as ONE kernel per call:
- *   z1 = X W1^T + b1            X = up to four gathered 128-wide row segments (as in mb_gemm), W1 [256, K]:
+ *   z1 = X W1^T + b1 + sum_i add_i[idx_i]   X = up to four gathered 128-wide row segments (as in mb_gemm), W1 [256, K]:
  *                               rows 0..127 the core branch's first layer, 128..255 the gate branch's
  *   z2 = SiLU(z1) (.) W2^T + b2 W2 [256, 128]: rows 0..127 act on z1[:, :128] (core), 128..255 on z1[:, 128:] (gate)
  *   h  = SiLU(RMSNorm(z2[:, :128]) * norm_core) * sigmoid(RMSNorm(z2[:, 128:]) * norm_gate)
@@ -247,7 +256,7 @@ int mb_bench_mma_rate(int kind, int iters, float* elapsed_ms, int* n_sms, void* 
 #define MB_MLP_PLAIN 1
 typedef struct mb_gated_mlp {
   int64_t n_rows;
-  int32_t n_src;               /* 1..4 ; K = 128 * n_src */
+  int32_t n_src;               /* 1..4 ; K = 128 * n_src (MB_MLP_GATED with addends: 0..4) */
   int32_t kind;                /* MB_MLP_GATED or MB_MLP_PLAIN */
   mb_src src[4];               /* src[].act is honoured (SiLU on load) */
   const float* W1;             /* [256, K] row-major (SIMT mode) */
@@ -273,8 +282,33 @@ typedef struct mb_gated_mlp {
   const float* res_w;          /* [128] or NULL (= 1) */
   int64_t ld_res;
   float* out2; int64_t ld_out2;
+  int32_t n_add, pad;          /* 0..3 addends (MB_MLP_GATED only) */
+  mb_add add[3];
 } mb_gated_mlp;
 int mb_gated_mlp_fwd(const mb_gated_mlp* desc, void* stream);
+
+/* Data gradient of the same block as one kernel.
+ *   MB_MLP_GATED  dz1 = (dy W2 per branch) * silu'(z1)   dy = dz2 [R, 256] (mb_gate_bwd's result), W2t [256, 128] = the two
+ *                 branches' transposed second layers     dx = dz1 W1 + sum_e ext_e W3 + res_w * res
+ *                 for ONE 128-wide segment of the block's input: W1t [128, 256] = that segment's columns of W1, transposed;
+ *                 the gradients of gathered segments are sums of dz1 over the rows that gather a node, times their columns.
+ *                 ext (0..2 further 128-wide operands) with W3t [128, 128 n_ext] join the same accumulator.
+ *   MB_MLP_PLAIN  dz1 = scale * (dy W2) * silu'(z1)      dy [R, 128] (gathered when dy.idx is given)
+ *                 dx = dz1 W1 + res_w * res              W2t, W1t [128, 128]
+ * dz1 is written when the pointer is given (the modes of mb_set_gemm_mode other than 0 need it as scratch). */
+typedef struct mb_mlp_bwd {
+  int64_t n_rows;
+  int32_t kind, n_ext;
+  mb_src dy;                   /* gated: the core half, the gate half follows 128 columns on */
+  mb_src ext[2];
+  float scale; int32_t pad;
+  mb_weight W2t, W1t, W3t;
+  const float* z1; int64_t ld_z1;
+  float* dz1; int64_t ld_dz1;
+  const float* res; const float* res_w; int64_t ld_res;
+  float* dx; int64_t ld_dx;
+} mb_mlp_bwd;
+int mb_mlp_bwd_data(const mb_mlp_bwd* desc, void* stream);
 
 /* ------------------------------------------------------------------ row-wise model kernels
  * All feature tensors are float32 row-major with 128 channels unless noted.
@@ -453,13 +487,7 @@ int mb_fourier_basis_bwd(int64_t n_trip, const int32_t* line_graph, const float*
                          const float* dbasis, float* dunit, void* stream);
 
 /* ------------------------------------------------------------------ whole evaluation
- * The model's parameters as device pointers: every 128-wide weight with its operand splits, all in one layout
- * (see mb_colblock).  ..t members are the transposes the data-gradient products contract with. */
-typedef struct mb_weight {
-  const float* W; const float* W_hi; const float* W_lo;
-  const uint16_t* W_hi16; const uint16_t* W_lo16;
-  int64_t ldw;
-} mb_weight;
+ * The model's parameters as device pointers.  ..t members are the transposes the data-gradient products contract with. */
 
 /* One update block (matris/model/functions.py:245-311): kind MB_UPDATE_GATED = GatedMLP, w1 [256,K] and w2 [256,128] =
  * core rows then gate rows, w1t [K,256], w2t [256,128] = the two transposes stacked, b1 / b2 [256], nc / ng the norm

@@ -62,6 +62,10 @@ class MbGemmDesc(C.Structure):
     _fields_ = [("n_rows", _i64), ("n_blocks", _i32), ("pad", _i32), ("blk", MbColBlock * 4)]
 
 
+class MbAdd(C.Structure):
+    _fields_ = [("ptr", _vp), ("idx", _vp), ("ld", _i64)]
+
+
 class MbGatedMlp(C.Structure):
     _fields_ = [
         ("n_rows", _i64), ("n_src", _i32), ("kind", _i32), ("src", MbSrc * 4),
@@ -70,11 +74,18 @@ class MbGatedMlp(C.Structure):
         ("norm_core", _vp), ("norm_gate", _vp),
         ("z1", _vp), ("ld_z1", _i64), ("z2", _vp), ("ld_z2", _i64), ("h", _vp), ("ld_h", _i64),
         ("res", _vp), ("res_w", _vp), ("ld_res", _i64), ("out2", _vp), ("ld_out2", _i64),
+        ("n_add", _i32), ("pad", _i32), ("add", MbAdd * 3),
     ]
 
 
 class MbWeight(C.Structure):
     _fields_ = [("W", _vp), ("W_hi", _vp), ("W_lo", _vp), ("W_hi16", _vp), ("W_lo16", _vp), ("ldw", _i64)]
+
+
+class MbMlpBwd(C.Structure):
+    _fields_ = [("n_rows", _i64), ("kind", _i32), ("n_ext", _i32), ("dy", MbSrc), ("ext", MbSrc * 2), ("scale", _f32),
+                ("pad", _i32), ("W2t", MbWeight), ("W1t", MbWeight), ("W3t", MbWeight), ("z1", _vp), ("ld_z1", _i64),
+                ("dz1", _vp), ("ld_dz1", _i64), ("res", _vp), ("res_w", _vp), ("ld_res", _i64), ("dx", _vp), ("ld_dx", _i64)]
 
 
 class MbUpdate(C.Structure):
@@ -153,6 +164,7 @@ _SIGNATURES = {
     "mb_selftest_wait_expiry": [_vp],
     "mb_bench_mma_rate": [C.c_int, C.c_int, C.POINTER(C.c_float), C.POINTER(C.c_int), _vp],
     "mb_gated_mlp_fwd": [C.POINTER(MbGatedMlp), _vp],
+    "mb_mlp_bwd_data": [C.POINTER(MbMlpBwd), _vp],
     "mb_gate_fwd": [_i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "mb_gate_bwd": [_i64, _vp, _vp, _vp, _vp, _vp, _vp],
     "mb_seg_attn_fwd": [_i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],

@@ -327,6 +327,23 @@ static void ffn_fwd(Run& R, const mb_ffn& p, int64_t rows, const float* x, float
   run_mlp(R, m);
 }
 
+// dx = scale * ((dy W2) * silu'(z1)) W1 ; dy optionally gathered
+static void ffn_bwd(Run& R, const mb_ffn& p, int64_t rows, const float* dy, const int32_t* idx, float scale, const float* z1,
+                    float* dx) {
+  if (rows == 0) return;
+  Scope sc(R);
+  mb_mlp_bwd m;
+  memset(&m, 0, sizeof(m));
+  m.n_rows = rows; m.kind = MB_MLP_PLAIN;
+  m.dy = src(dy, idx);
+  m.scale = scale;
+  m.W2t = p.w2t; m.W1t = p.w1t;
+  m.z1 = z1; m.ld_z1 = 128; m.dx = dx; m.ld_dx = 128;
+  if (R.scratch) { m.dz1 = R.ar.bottom(rows * 128); m.ld_dz1 = 128; }
+  R.op("mb_mlp_bwd_data", [&] { return mb_mlp_bwd_data(&m, R.st); }, 4.0 * rows * 128 * 128, 4.0 * rows * 128 * 3, rows, 128,
+       128, 1);
+}
+
 // ------------------------------------------------------------------ attention layer
 struct AttnInter { float *z1, *z2, *h, *logits, *agg_t, *agg_s, *stats, *z1n, *z2n; };
 
@@ -447,28 +464,13 @@ static void refine_bwd(Run& R, const mb_refine_params& p, const mb_row_graph& g,
   // node FFN
   float* dagg = R.ar.bottom(nodes * 128);
   MB_OP(mb_scale_rows, g.n_nodes, d_node_out, p.wn, d_node, 0);
-  {
-    Scope s2(R);
-    float* dzn = R.ar.bottom(nodes * 128);
-    LinearOpt o;
-    o.gate = it.zn;
-    linear(R, g.n_nodes, d_node_out, p.nffn.w2t, 128, 128, dzn, o);
-    linear(R, g.n_nodes, dzn, p.nffn.w1t, 128, 128, dagg);
-  }
+  ffn_bwd(R, p.nffn, g.n_nodes, d_node_out, nullptr, 1.f, it.zn, dagg);
   // edge FFN (atom graph: the mean over the two directions is a gather * 0.5)
   float* dh = R.ar.bottom(rows * 128);
   const float* drow = nullptr;
   if (want_edge) {
     float* dx = p.smoothed_edge ? R.ar.bottom(rows * 128) : dh;
-    {
-      Scope s2(R);
-      float* dze = R.ar.bottom(rows * 128);
-      LinearOpt o;
-      o.gate = it.ze;
-      if (g.is_atom) { o.scale = 0.5f; o.idx = g.emap; }
-      linear(R, g.n_rows, d_edge_out, p.effn.w2t, 128, 128, dze, o);
-      linear(R, g.n_rows, dze, p.effn.w1t, 128, 128, dx);
-    }
+    ffn_bwd(R, p.effn, g.n_rows, d_edge_out, g.is_atom ? g.emap : nullptr, g.is_atom ? 0.5f : 1.f, it.ze, dx);
     if (p.smoothed_edge) {  // dx is the gradient of the smoothed rows h * s
       drow = dx;
       MB_OP(mb_mul_rows_gather, g.n_rows, dx, it.env, g.emap, dh);

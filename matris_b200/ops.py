@@ -165,15 +165,17 @@ def gemm(n_rows: int, blocks: list[dict]) -> None:
     call("mb_gemm", C.byref(_lib.MbGemmDesc.from_buffer(buf)), _stream())
 
 
-_GATED_FMT = struct.Struct("<qii" + "QQqii" * 4 + "QQQQQqQ" + "QQQQQqQ" + "QQ" + "Qq" * 3 + "QQq" + "Qq")
+_GATED_FMT = struct.Struct("<qii" + "QQqii" * 4 + "QQQQQqQ" + "QQQQQqQ" + "QQ" + "Qq" * 3 + "QQq" + "Qq" + "ii" + "QQq" * 3)
+_NO_ADDS = (0,) * 11
 assert _GATED_FMT.size == C.sizeof(_lib.MbGatedMlp)
 
 
-def gated_mlp_fwd(p, n_rows, srcs, want_h=True, res=None, res_w=None, save=True):
+def gated_mlp_fwd(p, n_rows, srcs, want_h=True, res=None, res_w=None, save=True, adds=()):
     """GatedMLP forward as one fused kernel (mb_gated_mlp_fwd).  ``p`` holds the packed weights (w1 [256,K], b1,
     w2 [256,128], b2, nc, ng).  Returns (z1, z2, h, out2); z1 / z2 only when ``save`` (the backward pass reads
-    them), h only when ``want_h``, out2 = h + res_w * res only when ``res`` is given."""
-    ref = srcs[0][0]
+    them), h only when ``want_h``, out2 = h + res_w * res only when ``res`` is given.  ``adds``: up to three (table
+    [*,256], idx) pairs whose gathered rows are added to layer 1 (``srcs`` may then be empty)."""
+    ref = srcs[0][0] if srcs else adds[0][0]
     n_rows = int(n_rows)
     # the composed path of the non-default GEMM modes uses z1 / z2 as scratch
     save = save or _gemm_mode != 0
@@ -190,7 +192,12 @@ def gated_mlp_fwd(p, n_rows, srcs, want_h=True, res=None, res_w=None, save=True)
     for _ in range(4 - len(srcs)):
         flat += _NO_SRC
     w1, w2 = as_split(p.w1), as_split(p.w2)
-    assert w1.shape[0] == 2 * D and w1.shape[1] == D * len(srcs) and tuple(w2.shape) == (2 * D, D)
+    assert w1.shape[0] == 2 * D and (not srcs or w1.shape[1] == D * len(srcs)) and tuple(w2.shape) == (2 * D, D)
+    extra = []
+    for t, idx in adds:
+        assert t.dtype == torch.float32 and t.stride(-1) == 1
+        extra += (t.data_ptr(), 0 if idx is None else idx.data_ptr(), t.stride(0))
+    extra += (0, 0, 0) * (3 - len(adds))
 
     def pl(t):
         return (0, 0) if t is None else (t.data_ptr(), t.stride(0))
@@ -203,7 +210,7 @@ def gated_mlp_fwd(p, n_rows, srcs, want_h=True, res=None, res_w=None, save=True)
         0 if p.b2 is None else p.b2.data_ptr(),
         p.nc.data_ptr(), p.ng.data_ptr(), *pl(z1), *pl(z2), *pl(h),
         0 if res is None else res.data_ptr(), 0 if res is None or res_w is None else res_w.data_ptr(),
-        0 if res is None else res.stride(0), *pl(out2))
+        0 if res is None else res.stride(0), *pl(out2), len(adds), 0, *extra)
     if _lib.profile is not None:
         cols = len(srcs) + (4 if z1 is not None else 0) + (h is not None) + 2 * (out2 is not None)
         _lib.profile_meta = dict(flops=2.0 * n_rows * 2 * D * D * (len(srcs) + 1), rows=n_rows, k=D * len(srcs),
@@ -244,13 +251,39 @@ def ffn_fwd(p, x, want_y=True, res=None, res_w=None, save=True):
         *w2.ptrs, w2.ldw, 0 if p.b2 is None else p.b2.data_ptr(),
         0, 0, *pl(z1), 0, 0, *pl(y),
         0 if res is None else res.data_ptr(), 0 if res is None or res_w is None else res_w.data_ptr(),
-        0 if res is None else res.stride(0), *pl(out2))
+        0 if res is None else res.stride(0), *pl(out2), *_NO_ADDS)
     if _lib.profile is not None:
         cols = n_src + (z1 is not None) + (y is not None) + 2 * (out2 is not None)
         _lib.profile_meta = dict(flops=2.0 * n_rows * D * D * (n_src + 1), rows=n_rows, k=k, n=D, fused=True,
                                  bytes=4.0 * n_rows * D * cols)
     call("mb_gated_mlp_fwd", C.byref(_lib.MbGatedMlp.from_buffer_copy(buf)), _stream())
     return z1, y, out2
+
+
+def mlp_bwd(dy, w2t, w1t, z1, gated, want_dz1=True, res=None, res_w=None, idx=None, scale=1.0, ext=None, w3t=None):
+    """Data gradient of a gated (dy = dz2 [rows,256]) or plain (dy [*,128], optionally gathered) two-layer MLP as one
+    launch (mb_mlp_bwd_data): returns (dz1, dx) with dx = dz1 W1 (+ ext W3) (+ res_w * res) for one input segment."""
+    n_rows, width = z1.shape
+    want_dz1 = want_dz1 or _gemm_mode != 0  # the composed path of the other GEMM modes uses it
+    dz1 = new(n_rows, width, z1) if want_dz1 else None
+    dx = new(n_rows, D, z1)
+    m = _lib.MbMlpBwd()
+    m.n_rows, m.kind, m.scale = n_rows, 0 if gated else 1, scale
+    m.dy = _lib.MbSrc(dy.data_ptr(), 0 if idx is None else idx.data_ptr(), dy.stride(0), 0, 0)
+    m.W2t, m.W1t = (_lib.MbWeight(*s.ptrs, s.ldw) for s in (as_split(w2t), as_split(w1t)))
+    if ext is not None:
+        m.n_ext = ext.shape[1] // D
+        for j in range(m.n_ext):
+            m.ext[j] = _lib.MbSrc(ext.data_ptr(), 0, ext.stride(0), D * j, 0)
+        w3 = as_split(w3t)
+        m.W3t = _lib.MbWeight(*w3.ptrs, w3.ldw)
+    m.z1, m.ld_z1, m.dx, m.ld_dx = z1.data_ptr(), z1.stride(0), dx.data_ptr(), dx.stride(0)
+    if dz1 is not None:
+        m.dz1, m.ld_dz1 = dz1.data_ptr(), dz1.stride(0)
+    if res is not None:
+        m.res, m.res_w, m.ld_res = res.data_ptr(), ptr(res_w), res.stride(0)
+    call("mb_mlp_bwd_data", C.byref(m), _stream())
+    return dz1, dx
 
 
 def linear(x, W, bias=None, out_act=0, in_act=0, gate=None, res=None, res_w=None, scale=1.0, idx=None, out=None):
