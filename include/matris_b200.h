@@ -370,6 +370,14 @@ int mb_mul_rows_gather(int64_t n_rows, const float* x, const float* s, const int
  * matris/model/interaction_block.py:123, 270-273): out[u] = 0.5*(y[u2d[u]] + y[rev[u2d[u]]]) + res_w*res[u] */
 int mb_pair_mean_res(int32_t n_bonds, const int32_t* u2d, const int32_t* rev, const float* y, const float* res,
                      const float* res_w, float* out, void* stream);
+/* Gradient of the per-node layer-1 tables of a gated MLP: out [n_nodes,512] = (sum of x [n_rows,256] over the rows whose
+ * target is n | ... whose source is n); with ctr [n_rows], ctr_out [*,256] additionally accumulates x by centre atom. */
+int mb_seg_sum(int32_t n_nodes, int64_t n_rows, const int32_t* tgt_ptr, const int32_t* src_ptr, const int32_t* src_perm,
+               const int32_t* ctr, const float* x, float* out, float* ctr_out, void* stream);
+/* per bond u with directed rows e1, e2: out[u] = a[e1] + a[e2] ([*,256]), with b != NULL out [n_bonds,512] = that | b[e1] +
+ * b[e2] */
+int mb_pair_sum(int32_t n_bonds, const int32_t* u2d, const int32_t* rev, const float* a, const float* b, float* out,
+                void* stream);
 /* y = a*x (elementwise per channel weight a[128], NULL: 1) ; accumulate != 0: y += a*x */
 int mb_scale_rows(int64_t n_rows, const float* x, const float* a, float* y, int32_t accumulate, void* stream);
 
@@ -499,6 +507,10 @@ typedef struct mb_update {
   int32_t kind, k;
   mb_weight w1, w2, w1t, w2t;
   const float* b1; const float* b2; const float* nc; const float* ng;
+  /* edge updates of kind MB_UPDATE_GATED, layer 1 by the origin of its columns (w1, w1t are then unused): we [256,128] the
+   * edge's own, wts [512,128] those of the target and of the source node (rows core | gate each), wc [256,128] of the centre
+   * atom (line-graph refinement); wet [128,256], wtst [128,512], wct [128,256] their transposes */
+  mb_weight we, wts, wc, wet, wtst, wct;
 } mb_update;
 
 typedef struct mb_ffn { mb_weight w1, w2, w1t, w2t; const float* b1; const float* b2; } mb_ffn;
@@ -507,6 +519,7 @@ typedef struct mb_ffn { mb_weight w1, w2, w1t, w2t; const float* b1; const float
 typedef struct mb_attn_params {
   mb_update node, edge;
   mb_weight wst, wstt;
+  mb_weight welt;                     /* [128,512]: edge.wet | wstt (atom graph, gated) */
   const float* wn; const float* we;   /* residual weights */
 } mb_attn_params;
 

@@ -90,7 +90,8 @@ class MbMlpBwd(C.Structure):
 
 class MbUpdate(C.Structure):
     _fields_ = [("kind", _i32), ("k", _i32), ("w1", MbWeight), ("w2", MbWeight), ("w1t", MbWeight), ("w2t", MbWeight),
-                ("b1", _vp), ("b2", _vp), ("nc", _vp), ("ng", _vp)]
+                ("b1", _vp), ("b2", _vp), ("nc", _vp), ("ng", _vp), ("we", MbWeight), ("wts", MbWeight), ("wc", MbWeight),
+                ("wet", MbWeight), ("wtst", MbWeight), ("wct", MbWeight)]
 
 
 class MbFfn(C.Structure):
@@ -98,7 +99,8 @@ class MbFfn(C.Structure):
 
 
 class MbAttnParams(C.Structure):
-    _fields_ = [("node", MbUpdate), ("edge", MbUpdate), ("wst", MbWeight), ("wstt", MbWeight), ("wn", _vp), ("we", _vp)]
+    _fields_ = [("node", MbUpdate), ("edge", MbUpdate), ("wst", MbWeight), ("wstt", MbWeight), ("welt", MbWeight),
+                ("wn", _vp), ("we", _vp)]
 
 
 class MbRefineParams(C.Structure):
@@ -174,6 +176,8 @@ _SIGNATURES = {
     "mb_seg_smooth_sum_bwd_rows": [_i64, _vp, _vp, _i32, _vp, _vp, _vp, _vp, _i32, _vp, _vp, _vp, _vp, _vp],
     "mb_seg_smooth_sum_bwd_env": [_i32, _vp, _vp, _vp, _vp, _vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "mb_mul_rows_gather": [_i64, _vp, _vp, _vp, _vp, _vp],
+    "mb_seg_sum": [_i32, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
+    "mb_pair_sum": [_i32, _vp, _vp, _vp, _vp, _vp, _vp],
     "mb_pair_mean_res": [_i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "mb_scale_rows": [_i64, _vp, _vp, _vp, _i32, _vp],
     "mb_small_linear_fwd": [_i64, _i32, _vp, _vp, _vp, _vp],

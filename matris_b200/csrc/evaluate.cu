@@ -271,6 +271,110 @@ static void update_fwd(Run& R, const mb_update& p, int64_t rows, std::initialize
   run_mlp(R, m);
 }
 
+// Edge update of a gated kind: layer 1 from tables of finished sums per node (P = node [Wt | Ws]^T), per bond (atom graph:
+// bonds We^T, the directed rows only gather) and per centre atom (line-graph refinement).  With `logits` the attention logits
+// of the edge features come out of the same launch as the bond table (atom graph) or of one of their own.
+static void edge_update_fwd(Run& R, const mb_update& p, const mb_row_graph& g, const float* node, const float* edge,
+                            const float* ctr_feat, const mb_weight* wst, float* logits, float* z1, float* z2, float* h,
+                            const float* res_w, float* out2) {
+  if (p.kind == MB_UPDATE_MLP) {
+    if (g.is_atom || !ctr_feat)
+      update_fwd(R, p, g.n_rows, {src(edge, g.emap), src(node, g.tgt), src(node, g.src)}, z1, z2, h, edge, res_w, out2);
+    else
+      update_fwd(R, p, g.n_rows, {src(edge), src(ctr_feat, g.ctr), src(node, g.tgt), src(node, g.src)}, z1, z2, h, edge, res_w,
+                 out2);
+    if (logits) linear(R, g.n_edge_rows, edge, *wst, 256, 128, logits);
+    return;
+  }
+  Scope sc(R);
+  float* P = R.ar.bottom((size_t)g.n_nodes * 512);
+  float* Pc = ctr_feat ? R.ar.bottom((size_t)g.n_ctr * 256) : nullptr;
+  float* Pe = g.is_atom ? R.ar.bottom((size_t)g.n_edge_rows * 256) : nullptr;
+  if (R.scratch) {
+    if (!z1) z1 = R.ar.bottom((size_t)g.n_rows * 256);
+    if (!z2) z2 = R.ar.bottom((size_t)g.n_rows * 256);
+  }
+  linear(R, g.n_nodes, node, p.wts, 512, 128, P);
+  if (Pc) linear(R, g.n_ctr, ctr_feat, p.wc, 256, 128, Pc);
+  Gemm e(g.n_edge_rows);
+  if (Pe)
+    for (int j = 0; j < 2; ++j) e.block({src(edge)}, p.we, 128 * j, Pe, 256, 128 * j);
+  if (logits)
+    for (int j = 0; j < 2; ++j) e.block({src(edge)}, *wst, 128 * j, logits, 256, 128 * j);
+  e.run(R);
+  mb_gated_mlp m;
+  if (g.is_atom) fill_mlp(m, g.n_rows, {}, p.we, p.w2, p.b1, p.b2);
+  else fill_mlp(m, g.n_rows, {src(edge)}, p.we, p.w2, p.b1, p.b2);
+  m.norm_core = p.nc; m.norm_gate = p.ng;
+  m.z1 = z1; m.ld_z1 = 256; m.z2 = z2; m.ld_z2 = 256; m.h = h; m.ld_h = 128;
+  m.res = out2 ? edge : nullptr; m.res_w = out2 ? res_w : nullptr; m.ld_res = 128; m.out2 = out2; m.ld_out2 = 128;
+  auto add = [&](const float* t, const int32_t* idx, int64_t ld) { m.add[m.n_add++] = mb_add{t, idx, ld}; };
+  add(P, g.tgt, 512);
+  add(P + 256, g.src, 512);
+  if (Pe) add(Pe, g.emap, 256);
+  if (Pc) add(Pc, g.ctr, 256);
+  run_mlp(R, m);
+}
+
+// Backward of the same from dz2 (and dlogits): d_edge = ... + edge_w * edge_res, d_node (+)= ... + node_w * node_res, the centre
+// atoms' gradient is accumulated into d_ctr.
+static void edge_update_bwd(Run& R, const mb_update& p, const mb_row_graph& g, const float* z1, const float* dz2,
+                            const float* dlogits, const mb_weight* w_log, const float* edge_res, const float* edge_w,
+                            float* d_edge, const float* node_res, const float* node_w, float* d_node, float* d_ctr) {
+  Scope sc(R);
+  float* dz1 = R.ar.bottom((size_t)g.n_rows * 256);
+  if (g.is_atom) {
+    Gemm a(g.n_rows);
+    for (int j = 0; j < 2; ++j) {
+      mb_colblock& b = a.block({src(dz2, nullptr, 128 * j, 256)}, p.w2t, 128 * j, dz1, 256, 128 * j);
+      b.gate = z1; b.ld_gate = 256; b.col_gate = 128 * j;
+    }
+    a.run(R);
+    Scope s2(R);
+    const int ld = dlogits ? 512 : 256;
+    float* pair = R.ar.bottom((size_t)g.n_edge_rows * ld);
+    MB_OP(mb_pair_sum, (int32_t)g.n_edge_rows, g.u2d, g.rev, dz1, dlogits, pair);
+    Gemm e(g.n_edge_rows);
+    mb_colblock& b = e.block({src(pair, nullptr, 0, ld), src(pair, nullptr, 128, ld)}, dlogits ? *w_log : p.wet, 0, d_edge, 128);
+    if (dlogits) {
+      b.src[b.n_src++] = src(pair, nullptr, 256, ld);
+      b.src[b.n_src++] = src(pair, nullptr, 384, ld);
+    }
+    b.res = edge_res; b.res_w = edge_w; b.ld_res = 128;
+    e.run(R);
+  } else {
+    mb_mlp_bwd m;
+    memset(&m, 0, sizeof(m));
+    m.n_rows = g.n_rows; m.kind = MB_MLP_GATED;
+    m.dy = src(dz2, nullptr, 0, 256);
+    m.W2t = p.w2t; m.W1t = p.wet;
+    m.z1 = z1; m.ld_z1 = 256; m.dz1 = dz1; m.ld_dz1 = 256; m.dx = d_edge; m.ld_dx = 128;
+    m.res = edge_res; m.res_w = edge_w; m.ld_res = 128;
+    if (dlogits) {
+      m.n_ext = 2;
+      for (int j = 0; j < 2; ++j) m.ext[j] = src(dlogits, nullptr, 128 * j, 256);
+      m.W3t = *w_log;
+    }
+    const double k = dlogits ? 768 : 512;
+    R.op("mb_mlp_bwd_data", [&] { return mb_mlp_bwd_data(&m, R.st); }, 2.0 * g.n_rows * 128 * k,
+         4.0 * g.n_rows * 128 * (7 + (edge_res != nullptr) + (dlogits ? 2 : 0)), g.n_rows, 256, 256, 1);
+  }
+  float* dP = R.ar.bottom((size_t)g.n_nodes * 512);
+  float* dPc = d_ctr ? R.ar.bottom((size_t)g.n_ctr * 256) : nullptr;
+  if (dPc) R.zero(dPc, (size_t)g.n_ctr * 1024);
+  MB_OP(mb_seg_sum, (int32_t)g.n_nodes, g.n_rows, g.tgt_ptr, g.src_ptr, g.src_perm, d_ctr ? g.ctr : nullptr, dz1, dP, dPc);
+  Gemm n(g.n_nodes);
+  mb_colblock& b = n.block({src(dP, nullptr, 0, 512), src(dP, nullptr, 128, 512), src(dP, nullptr, 256, 512),
+                            src(dP, nullptr, 384, 512)}, p.wtst, 0, d_node, 128, 0, nullptr, node_res ? MB_OUT_STORE : MB_OUT_ADD);
+  b.res = node_res; b.res_w = node_w; b.ld_res = 128;
+  n.run(R);
+  if (dPc) {
+    Gemm c(g.n_ctr);
+    c.block({src(dPc, nullptr, 0, 256), src(dPc, nullptr, 128, 256)}, p.wct, 0, d_ctr, 128, 0, nullptr, MB_OUT_ADD);
+    c.run(R);
+  }
+}
+
 struct Dest {  // where the gradient of one 128-wide K segment goes
   float* t; const int32_t* idx; int mode; const float* res; const float* res_w;
 };
@@ -363,14 +467,8 @@ static void attn_fwd(Run& R, const mb_attn_params& p, const mb_row_graph& g, con
   it.stats = get(nodes * 512);
   it.z1n = mode == NONE ? nullptr : get(nodes * update_width(p.node));
   it.z2n = mode == NONE ? nullptr : get(nodes * update_width(p.node));
-  const std::initializer_list<mb_src> srcs = {src(edge, g.emap), src(node, g.tgt), src(node, g.src)};
-  if (g.is_atom) {
-    update_fwd(R, p.edge, g.n_rows, srcs, it.z1, it.z2, it.h, nullptr, nullptr, nullptr);
-    if (edge_out) MB_OP(mb_pair_mean_res, (int32_t)g.n_edge_rows, g.u2d, g.rev, it.h, edge, p.we, edge_out);
-  } else {
-    update_fwd(R, p.edge, g.n_rows, srcs, it.z1, it.z2, it.h, edge, p.we, edge_out);
-  }
-  linear(R, g.n_edge_rows, edge, p.wst, 256, 128, it.logits);  // source | target logits
+  edge_update_fwd(R, p.edge, g, node, edge, nullptr, &p.wst, it.logits, it.z1, it.z2, it.h, p.we, g.is_atom ? nullptr : edge_out);
+  if (g.is_atom && edge_out) MB_OP(mb_pair_mean_res, (int32_t)g.n_edge_rows, g.u2d, g.rev, it.h, edge, p.we, edge_out);
   MB_OP(mb_seg_attn_fwd, (int32_t)g.n_nodes, g.tgt_ptr, g.src_ptr, g.src_perm, g.emap, it.logits, it.h, it.agg_t, it.agg_s,
         it.stats);
   Scope sc(R);
@@ -385,9 +483,8 @@ static void attn_bwd(Run& R, const mb_attn_params& p, const mb_row_graph& g, con
   // node update
   float* dagg_t = R.ar.bottom(nodes * 128);
   float* dagg_s = R.ar.bottom(nodes * 128);
-  MB_OP(mb_scale_rows, g.n_nodes, d_node_out, p.wn, d_node, 0);
   update_bwd(R, p.node, g.n_nodes, it.z1n, it.z2n, d_node_out, nullptr,
-             {{d_node, nullptr, MB_OUT_ADD, nullptr, nullptr}, {dagg_t, nullptr, MB_OUT_STORE, nullptr, nullptr},
+             {{d_node, nullptr, MB_OUT_STORE, d_node_out, p.wn}, {dagg_t, nullptr, MB_OUT_STORE, nullptr, nullptr},
               {dagg_s, nullptr, MB_OUT_STORE, nullptr, nullptr}});
   // softmax-weighted aggregation; dh goes straight on through the gated MLP's tail adjoint (dz2 instead)
   const bool gated = p.edge.kind == MB_UPDATE_GATED;
@@ -397,6 +494,11 @@ static void attn_bwd(Run& R, const mb_attn_params& p, const mb_row_graph& g, con
   MB_OP(mb_seg_attn_bwd, g.n_rows, g.tgt, g.src, 1, g.emap, it.logits, it.h, it.agg_t, it.agg_s, it.stats, dagg_t, dagg_s,
         d_edge_out, g.emap, g.is_atom ? 0.5f : 1.f, dh, dlogits, gated ? it.z2 : nullptr, gated ? p.edge.nc : nullptr,
         gated ? p.edge.ng : nullptr, dz2);
+  if (gated) {
+    edge_update_bwd(R, p.edge, g, it.z1, dz2, dlogits, g.is_atom ? &p.welt : &p.wstt, d_edge_out, p.we, d_edge, nullptr,
+                    nullptr, d_node, nullptr);
+    return;
+  }
   // edge update (line graph: rows map one to one, so the residual gradient we * d_edge_out rides in the epilogue of the
   // store; atom graph: two directed rows add into one bond row, so it is laid down first)
   const Dest to_tgt{d_node, g.tgt, MB_OUT_ATOMIC, nullptr, nullptr}, to_src{d_node, g.src, MB_OUT_ATOMIC, nullptr, nullptr};
@@ -426,12 +528,8 @@ static void refine_fwd(Run& R, const mb_refine_params& p, const mb_row_graph& g,
   it.env = get((size_t)n_bonds * 128);
   it.zn = mode == NONE ? nullptr : get(nodes * 128);
   it.ze = mode == NONE || !want_edge ? nullptr : get(rows * 128);
-  if (g.is_atom)
-    update_fwd(R, p.edge, g.n_rows, {src(edge, g.emap), src(node, g.tgt), src(node, g.src)}, it.z1, it.z2, it.h, nullptr,
-               nullptr, nullptr);
-  else
-    update_fwd(R, p.edge, g.n_rows, {src(edge), src(atom_feat, g.ctr), src(node, g.tgt), src(node, g.src)}, it.z1, it.z2, it.h,
-               nullptr, nullptr, nullptr);
+  edge_update_fwd(R, p.edge, g, node, edge, g.is_atom ? nullptr : atom_feat, nullptr, nullptr, it.z1, it.z2, it.h, nullptr,
+                  nullptr);
   Scope sc(R);
   float* agg = R.ar.bottom(nodes * 128);
   MB_OP(mb_small_linear_fwd, n_bonds, 7, rbf, p.wenv, it.env);
@@ -463,7 +561,6 @@ static void refine_bwd(Run& R, const mb_refine_params& p, const mb_row_graph& g,
   const bool want_edge = d_edge_out != nullptr, gated = p.edge.kind == MB_UPDATE_GATED;
   // node FFN
   float* dagg = R.ar.bottom(nodes * 128);
-  MB_OP(mb_scale_rows, g.n_nodes, d_node_out, p.wn, d_node, 0);
   ffn_bwd(R, p.nffn, g.n_nodes, d_node_out, nullptr, 1.f, it.zn, dagg);
   // edge FFN (atom graph: the mean over the two directions is a gather * 0.5)
   float* dh = R.ar.bottom(rows * 128);
@@ -488,7 +585,12 @@ static void refine_bwd(Run& R, const mb_refine_params& p, const mb_row_graph& g,
           g.u2d, g.rev, it.env, it.h, dagg, drow, denv);
     MB_OP(mb_small_linear_bwd, n_bonds, 7, denv, p.wenv, d_rbf, 1);
   }
-  // gated MLP
+  // edge update
+  if (gated) {
+    edge_update_bwd(R, p.edge, g, it.z1, dz2, nullptr, nullptr, d_edge_out, p.we, d_edge, d_node_out, p.wn, d_node, d_atom);
+    return;
+  }
+  MB_OP(mb_scale_rows, g.n_nodes, d_node_out, p.wn, d_node, 0);
   const Dest to_tgt{d_node, g.tgt, MB_OUT_ATOMIC, nullptr, nullptr}, to_src{d_node, g.src, MB_OUT_ATOMIC, nullptr, nullptr};
   if (g.is_atom) {
     if (want_edge) MB_OP(mb_scale_rows, g.n_edge_rows, d_edge_out, p.we, d_edge, 0);

@@ -280,6 +280,94 @@ __global__ void k_smooth_env_bwd_line(int n_nodes, const int32_t* __restrict__ t
   st4(denv + row * 128 + c, acc);
 }
 
+// ------------------------------------------------------------------ sums of row gradients over a node's rows
+// out[n, 0:256] = sum of x over the rows whose target is n (contiguous), out[n, 256:512] = over the rows whose source is n
+// (through the permutation); with ctr, ctr_out[ctr[r]] += x[r] on top (the rows of a target bond change their centre atom
+// at most once, so that is one or two reductions a segment).  The gradient of a node's layer-1 table is exactly these sums: the
+// products with the weights then run once per node instead of scattering 128 finished columns per row.
+// WARPS warps share a segment: one for the line graph's short segments, eight for an atom's 30 - 80 edges, whose few
+// segments would otherwise be walked by a handful of warps.
+template <int WARPS>
+__global__ void k_seg_sum(int n_nodes, const int32_t* __restrict__ tgt_ptr, const int32_t* __restrict__ src_ptr,
+                          const int32_t* __restrict__ src_perm, const int32_t* __restrict__ ctr,
+                          const float* __restrict__ x, float* __restrict__ out, float* __restrict__ ctr_out) {
+  constexpr int NB = 4;  // rows in flight per warp
+  __shared__ float4 part[WARPS > 1 ? WARPS : 1][WARPS > 1 ? 64 : 1];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t item = WARPS > 1 ? (int64_t)blockIdx.x : ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t node = item >> 1;
+  const int side = (int)(item & 1), c = lane * 4;
+  if (node >= n_nodes) return;
+  const int32_t* ptr = side == 0 ? tgt_ptr : src_ptr;
+  const int q0 = ptr[node], q1 = ptr[node + 1];
+  float4 a = zero4(), b = zero4(), ca = zero4(), cb = zero4();
+  const bool by_ctr = WARPS == 1 && side == 0 && ctr != nullptr;
+  int cur = -1;
+  auto flush = [&]() {
+    if (cur < 0) return;
+    atomicAdd(reinterpret_cast<float4*>(ctr_out + (int64_t)cur * 256 + c), ca);
+    atomicAdd(reinterpret_cast<float4*>(ctr_out + (int64_t)cur * 256 + 128 + c), cb);
+    ca = cb = zero4();
+  };
+  for (int q = q0 + (WARPS > 1 ? w * NB : 0); q < q1; q += NB * WARPS) {
+    int64_t r[NB];
+    float4 va[NB], vb[NB];
+    int ct[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int qq = q + i < q1 ? q + i : q1 - 1;
+      r[i] = side == 0 ? qq : src_perm[qq];
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      va[i] = ld4(x + r[i] * 256 + c);
+      vb[i] = ld4(x + r[i] * 256 + 128 + c);
+      ct[i] = by_ctr ? ctr[r[i]] : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      if (q + i >= q1) break;
+      a = add4(a, va[i]);
+      b = add4(b, vb[i]);
+      if (by_ctr) {
+        if (ct[i] != cur) { flush(); cur = ct[i]; }
+        ca = add4(ca, va[i]);
+        cb = add4(cb, vb[i]);
+      }
+    }
+  }
+  if (by_ctr) flush();
+  float* const o = out + node * 512 + side * 256;
+  if (WARPS > 1) {
+    part[w][lane] = a;
+    part[w][32 + lane] = b;
+    __syncthreads();
+    if (threadIdx.x < 64) {
+      float4 s = part[0][threadIdx.x];
+#pragma unroll
+      for (int k = 1; k < WARPS; ++k) s = add4(s, part[k][threadIdx.x]);
+      st4(o + 4 * threadIdx.x, s);
+    }
+  } else {
+    st4(o + c, a);
+    st4(o + 128 + c, b);
+  }
+}
+
+// out[u, 0:256] = a[e1] + a[e2] and, with b, out[u, 256:512] = b[e1] + b[e2]: the two directed rows e1, e2 of bond u
+__global__ void k_pair_sum(int n_bonds, const int32_t* __restrict__ u2d, const int32_t* __restrict__ rev,
+                           const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out, int ld) {
+  MB_ROW_PROLOGUE(n_bonds)
+  const int64_t e1 = u2d[row], e2 = rev[e1];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    st4(out + row * ld + 128 * h + c, add4(ld4(a + e1 * 256 + 128 * h + c), ld4(a + e2 * 256 + 128 * h + c)));
+  if (!b) return;
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    st4(out + row * ld + 256 + 128 * h + c, add4(ld4(b + e1 * 256 + 128 * h + c), ld4(b + e2 * 256 + 128 * h + c)));
+}
+
 // ------------------------------------------------------------------ pair mean / scaling
 __global__ void k_pair_mean_res(int n_bonds, const int32_t* __restrict__ u2d, const int32_t* __restrict__ rev,
                                 const float* __restrict__ y, const float* __restrict__ res,
@@ -531,6 +619,30 @@ extern "C" int mb_mul_rows_gather(int64_t n_rows, const float* x, const float* s
   if (n_rows == 0) return MB_OK;
   k_mul_rows_gather<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, x, s, idx, y);
   MB_LAUNCH_CHECK("k_mul_rows_gather");
+  return MB_OK;
+}
+
+extern "C" int mb_seg_sum(int32_t n_nodes, int64_t n_rows, const int32_t* tgt_ptr, const int32_t* src_ptr,
+                          const int32_t* src_perm, const int32_t* ctr, const float* x, float* out, float* ctr_out,
+                          void* stream) {
+  MB_REQUIRE(n_nodes >= 0 && n_rows >= 0 && tgt_ptr && src_ptr && src_perm && x && out && (!ctr || ctr_out));
+  if (n_nodes == 0) return MB_OK;
+  // long segments on average (and no per-centre sums, which follow the order of the rows): a block per segment and side
+  if (!ctr && n_rows >= 16 * (int64_t)n_nodes)
+    k_seg_sum<8><<<2 * (unsigned)n_nodes, 256, 0, STREAM>>>(n_nodes, tgt_ptr, src_ptr, src_perm, ctr, x, out, ctr_out);
+  else
+    k_seg_sum<1><<<row_grid(2 * (int64_t)n_nodes), RW_THREADS, 0, STREAM>>>(n_nodes, tgt_ptr, src_ptr, src_perm, ctr, x, out,
+                                                                           ctr_out);
+  MB_LAUNCH_CHECK("k_seg_sum");
+  return MB_OK;
+}
+
+extern "C" int mb_pair_sum(int32_t n_bonds, const int32_t* u2d, const int32_t* rev, const float* a, const float* b, float* out,
+                           void* stream) {
+  MB_REQUIRE(n_bonds >= 0 && u2d && rev && a && out);
+  if (n_bonds == 0) return MB_OK;
+  k_pair_sum<<<row_grid(n_bonds), RW_THREADS, 0, STREAM>>>(n_bonds, u2d, rev, a, b, out, b ? 512 : 256);
+  MB_LAUNCH_CHECK("k_pair_sum");
   return MB_OK;
 }
 

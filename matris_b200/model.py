@@ -63,19 +63,29 @@ class _Packer:
         self.alive.append(sw)
         return _lib.MbWeight(*sw.ptrs, sw.ldw)
 
-    def gated(self, prefix) -> _lib.MbUpdate:
+    def gated(self, prefix, roles=()) -> _lib.MbUpdate:
         """GatedMLP: first layers of core|gate stacked to [256,K], second layers to [256,128], plus the transposes the
-        backward products contract with."""
+        backward products contract with.  ``roles`` names the origin of each 128 columns of layer 1 for an edge update
+        ("edge", "ctr", "tgt", "src"): the library then forms the node terms once per node."""
         get, c, g = self.get, prefix + "mlp_core.layers.", prefix + "mlp_gate.layers."
         w1 = torch.cat([get(c + "0.weight"), get(g + "0.weight")], 0)
         w2c, w2g = get(c + "3.weight"), get(g + "3.weight")
+        if roles:
+            part = {r: w1[:, 128 * i:128 * i + 128] for i, r in enumerate(roles)}
+            ts = torch.cat([part["tgt"], part["src"]], 0)
+            first = dict(we=self.weight(part["edge"]), wet=self.weight(part["edge"].t()), wts=self.weight(ts),
+                         wtst=self.weight(ts.t()))
+            if "ctr" in part:
+                first.update(wc=self.weight(part["ctr"]), wct=self.weight(part["ctr"].t()))
+        else:
+            first = dict(w1=self.weight(w1), w1t=self.weight(w1.t()))
         return _lib.MbUpdate(
-            kind=0, k=w1.shape[1], w1=self.weight(w1), w2=self.weight(torch.cat([w2c, w2g], 0)), w1t=self.weight(w1.t()),
+            kind=0, k=w1.shape[1], **first, w2=self.weight(torch.cat([w2c, w2g], 0)),
             w2t=self.weight(torch.cat([w2c.t(), w2g.t()], 0)), b1=self.vec(torch.cat([get(c + "0.bias"), get(g + "0.bias")])),
             b2=self.vec(torch.cat([get(c + "3.bias"), get(g + "3.bias")])), nc=self.vec(get(prefix + "core_norm.weight")),
             ng=self.vec(get(prefix + "gate_norm.weight")))
 
-    def mlp(self, prefix, bias) -> _lib.MbUpdate:
+    def mlp(self, prefix, bias, roles=()) -> _lib.MbUpdate:
         """The plain-MLP variant of an update block (graph_conv_mlp = "MLP"): nn.Sequential(MLP, RMSNorm)
         (matris/model/interaction_block.py:39-62, 172-184)."""
         get = self.get
@@ -95,14 +105,18 @@ class _Packer:
 
     def attention(self, prefix, update) -> _lib.MbAttnParams:
         wst = torch.cat([self.get(prefix + "source_weight_linear.weight"), self.get(prefix + "target_weight_linear.weight")], 0)
+        edge, more = update(prefix + "edge_nonlinear_update.", ("edge", "tgt", "src")), {}
+        if edge.kind == 0:
+            c, g = (self.get(f"{prefix}edge_nonlinear_update.mlp_{b}.layers.0.weight")[:, :128] for b in ("core", "gate"))
+            more["welt"] = self.weight(torch.cat([c.t(), g.t(), wst.t()], 1))
         return _lib.MbAttnParams(
-            node=update(prefix + "node_nonlinear_update."), edge=update(prefix + "edge_nonlinear_update."),
+            node=update(prefix + "node_nonlinear_update."), edge=edge, **more,
             wst=self.weight(wst), wstt=self.weight(wst.t()), wn=self.vec(self.get(prefix + "node_res_weight")),
             we=self.vec(self.get(prefix + "edge_res_weight")))
 
-    def refinement(self, prefix, update, bias, smoothed) -> _lib.MbRefineParams:
+    def refinement(self, prefix, update, bias, smoothed, line) -> _lib.MbRefineParams:
         return _lib.MbRefineParams(
-            edge=update(prefix + "edge_nonlinear_update."), nffn=self.ffn(prefix + "node_FFN.", bias),
+            edge=update(prefix + "edge_nonlinear_update.", ("edge", "ctr", "tgt", "src") if line else ("edge", "tgt", "src")), nffn=self.ffn(prefix + "node_FFN.", bias),
             effn=self.ffn(prefix + "edge_FFN.", bias), wenv=self.vec(self.get(prefix + "learnable_envelope.weight")),
             wn=self.vec(self.get(prefix + "node_res_weight")), we=self.vec(self.get(prefix + "edge_res_weight")),
             smoothed_edge=int(smoothed))
@@ -140,13 +154,13 @@ def pack_parameters(sd: dict, cfg: dict, device) -> SimpleNamespace:
         M.sph_factor = float(sd[t + "expansion.factor"])
     M.t_wa, wb = vec(get(t + "angle_embedding.weight")), get(t + "swish_layer.linear.weight")
     M.t_wb, M.t_wbt = weight(wb), weight(wb.t())
-    update = (lambda p: k.mlp(p, bias)) if str(cfg["graph_conv_mlp"]).lower() == "mlp" else k.gated
+    update = (lambda p, roles=(): k.mlp(p, bias, roles)) if str(cfg["graph_conv_mlp"]).lower() == "mlp" else k.gated
     for i, L in enumerate(layers):
         p = f"interaction_block.{i}."
         for g in ("atom", "line"):
             setattr(L, "attn_" + g, k.attention(f"{p}attn_block_{g}_graph.", update))
             smoothed = bool(cfg["use_smoothed_for_delta_edge"]) and g == "atom"
-            setattr(L, "refine_" + g, k.refinement(f"{p}refine_block_{g}_graph.", update, bias, smoothed))
+            setattr(L, "refine_" + g, k.refinement(f"{p}refine_block_{g}_graph.", update, bias, smoothed, g == "line"))
     M.out_norm = vec(get("readout_norm.weight"))
     h = "energy_head.energy_head.layers."
     w0, w3 = get(h + "0.weight"), get(h + "3.weight")

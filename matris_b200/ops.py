@@ -370,6 +370,22 @@ def mul_rows_gather(x, s, idx=None):
     return y
 
 
+def seg_sum(n_nodes, tgt_ptr, src_ptr, src_perm, x, ctr=None, ctr_out=None):
+    """[n_nodes,512]: sums of the rows of x [*,256] by target node | by source node; ``ctr_out`` [*,256] accumulates them
+    by centre atom."""
+    out = new(n_nodes, 4 * D, x)
+    call("mb_seg_sum", n_nodes, x.shape[0], ptr(tgt_ptr), ptr(src_ptr), ptr(src_perm), ptr(ctr), ptr(x), ptr(out), ptr(ctr_out),
+         _stream())
+    return out
+
+
+def pair_sum(n_bonds, u2d, rev, a, b=None):
+    """[n_bonds,256]: sum of the two directed rows of every bond, with ``b`` [n_bonds,512]: of both tensors."""
+    out = new(n_bonds, 2 * D if b is None else 4 * D, a)
+    call("mb_pair_sum", n_bonds, ptr(u2d), ptr(rev), ptr(a), ptr(b), ptr(out), _stream())
+    return out
+
+
 def pair_mean_res(n_bonds, u2d, rev, y, res=None, res_w=None):
     out = new(n_bonds, D, y)
     call("mb_pair_mean_res", n_bonds, ptr(u2d), ptr(rev), ptr(y), ptr(res), ptr(res_w), ptr(out), _stream())
