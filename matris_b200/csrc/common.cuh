@@ -27,6 +27,26 @@ void set_cuda_error(cudaError_t e, const char* where);
     }                                                        \
   } while (0)
 
+// Kernels of an evaluation are launched with programmatic stream serialization: a kernel may be scheduled, and set itself up,
+// while its predecessor is still running, and waits in pdl_sync() before it touches anything a predecessor wrote (or read).
+// Launch gaps and prologues (tensor-memory allocation, barriers, weight tiles) then overlap; on small systems, where a kernel
+// lasts a few microseconds, they are most of the time.  Every kernel so launched must call pdl_sync().
+template <typename... P, typename... A>
+static inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // errors surface in MB_LAUNCH_CHECK
+}
+// wait for the preceding kernels' results, then let the next kernel be scheduled
+__device__ __forceinline__ void pdl_sync() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+}
+
 static inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 int gemm_mode();  // the contraction core selected with mb_set_gemm_mode

@@ -28,6 +28,7 @@ constexpr int FIN_WARPS = 4, FIN_SPECIES = 128;
 __global__ void k_energy_finish(int n_struct, const int32_t* __restrict__ atom_ptr, const float* __restrict__ e_atom,
                                 const int32_t* __restrict__ numbers, const float* __restrict__ table, int n_species,
                                 int intensive, float* __restrict__ e, float* __restrict__ ref, int32_t* __restrict__ apg) {
+  pdl_sync();
   __shared__ int count[FIN_WARPS][FIN_SPECIES];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int b = blockIdx.x * FIN_WARPS + w;
@@ -62,6 +63,7 @@ __global__ void k_energy_finish(int n_struct, const int32_t* __restrict__ atom_p
 __global__ void k_force_stress_finish(int n_atoms, int n_struct, const float* __restrict__ dcart,
                                       const float* __restrict__ dstrain, const float* __restrict__ volume,
                                       float* __restrict__ f, float* __restrict__ s) {
+  pdl_sync();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (f && i < 3 * (int64_t)n_atoms) f[i] = -dcart[i];
   if (s && i < 9 * (int64_t)n_struct) s[i] = dstrain[i] * (160.21766208f / volume[i / 9]);
@@ -762,8 +764,7 @@ static int evaluate(Run& R, mb_eval& E) {
     linear(R, E.n_atoms, z1, M.h_w3, 128, 128, z2, o);
     MB_OP(mb_head_dot_fwd, E.n_atoms, 128, z2, M.h_w6, M.h_b6, 0, ea);
     R.op("energy_finish", [&] {
-      k_energy_finish<<<cdiv(E.n_struct, FIN_WARPS), 32 * FIN_WARPS, 0, R.st>>>(
-          E.n_struct, E.atom_ptr, ea, E.numbers, M.ref_table, M.n_species, M.is_intensive, E.e, E.ref, E.atoms_per_struct);
+      launch(k_energy_finish, cdiv(E.n_struct, FIN_WARPS), 32 * FIN_WARPS, 0, R.st, E.n_struct, E.atom_ptr, ea, E.numbers, M.ref_table, M.n_species, M.is_intensive, E.e, E.ref, E.atoms_per_struct);
       MB_LAUNCH_CHECK("k_energy_finish");
       return (int)MB_OK;
     });
@@ -882,7 +883,7 @@ static int evaluate(Run& R, mb_eval& E) {
         dcart, virial, dstrain);
   R.op("force_stress_finish", [&] {
     const long long n = 3LL * E.n_atoms > 9LL * E.n_struct ? 3LL * E.n_atoms : 9LL * E.n_struct;
-    k_force_stress_finish<<<cdiv(n, 256), 256, 0, R.st>>>(E.n_atoms, E.n_struct, dcart, dstrain, E.volume, E.f, E.s);
+    launch(k_force_stress_finish, cdiv(n, 256), 256, 0, R.st, E.n_atoms, E.n_struct, dcart, dstrain, E.volume, E.f, E.s);
     MB_LAUNCH_CHECK("k_force_stress_finish");
     return (int)MB_OK;
   });

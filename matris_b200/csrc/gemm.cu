@@ -860,8 +860,8 @@ extern "C" int mb_gemm(const mb_gemm_desc* desc, void* stream_) {
       const long long n_items = shared_a ? gx : n_tiles;
       const unsigned grid = (unsigned)(n_items < n_sm ? n_items : n_sm);
       const int sa = shared_a ? 1 : 0;
-      if (bf16) mb::k_gemm_ps<true><<<grid, mb::PS_THREADS, mb::PS_SMEM_BYTES, (cudaStream_t)stream_>>>(*desc, maps, sa);
-      else mb::k_gemm_ps<false><<<grid, mb::PS_THREADS, mb::PS_SMEM_BYTES, (cudaStream_t)stream_>>>(*desc, maps, sa);
+      if (bf16) mb::launch(mb::k_gemm_ps<true>, grid, mb::PS_THREADS, mb::PS_SMEM_BYTES, (cudaStream_t)stream_, *desc, maps, sa);
+      else mb::launch(mb::k_gemm_ps<false>, grid, mb::PS_THREADS, mb::PS_SMEM_BYTES, (cudaStream_t)stream_, *desc, maps, sa);
     } else {
       mb::k_gemm_tc<<<(unsigned)n_tiles, mb::TC_THREADS, mb::TC_SMEM_BYTES, (cudaStream_t)stream_>>>(*desc, maps);
     }
@@ -1005,8 +1005,8 @@ extern "C" int mb_gated_mlp_fwd(const mb_gated_mlp* g, void* stream_) {
   const long long n_tiles = (g->n_rows + 127) / 128;
   const unsigned grid = (unsigned)(n_tiles < n_sm ? n_tiles : n_sm);
   cudaStream_t st = (cudaStream_t)stream_;
-  if (plain) mb::k_mlp<mb::MLP_PLAIN_FWD><<<grid, mb::ML_THREADS, mb::ML_SMEM_BYTES, st>>>(a, maps);
-  else mb::k_mlp<mb::MLP_GATED_FWD><<<grid, mb::ML_THREADS, mb::ML_SMEM_BYTES, st>>>(a, maps);
+  if (plain) mb::launch(mb::k_mlp<mb::MLP_PLAIN_FWD>, grid, mb::ML_THREADS, mb::ML_SMEM_BYTES, st, a, maps);
+  else mb::launch(mb::k_mlp<mb::MLP_GATED_FWD>, grid, mb::ML_THREADS, mb::ML_SMEM_BYTES, st, a, maps);
   MB_LAUNCH_CHECK("k_mlp forward");
   return MB_OK;
 }
@@ -1110,8 +1110,8 @@ extern "C" int mb_mlp_bwd_data(const mb_mlp_bwd* g, void* stream_) {
   const long long n_tiles = (g->n_rows + 127) / 128;
   const unsigned grid = (unsigned)(n_tiles < n_sm ? n_tiles : n_sm);
   cudaStream_t st = (cudaStream_t)stream_;
-  if (plain) mb::k_mlp<mb::MLP_PLAIN_BWD><<<grid, mb::ML_THREADS, mb::ML_SMEM_BYTES, st>>>(a, maps);
-  else mb::k_mlp<mb::MLP_GATED_BWD><<<grid, mb::ML_THREADS, mb::ML_SMEM_BYTES, st>>>(a, maps);
+  if (plain) mb::launch(mb::k_mlp<mb::MLP_PLAIN_BWD>, grid, mb::ML_THREADS, mb::ML_SMEM_BYTES, st, a, maps);
+  else mb::launch(mb::k_mlp<mb::MLP_GATED_BWD>, grid, mb::ML_THREADS, mb::ML_SMEM_BYTES, st, a, maps);
   MB_LAUNCH_CHECK("k_mlp backward");
   return MB_OK;
 }

@@ -304,6 +304,7 @@ k_gemm_ps(const __grid_constant__ mb_gemm_desc d_param, const __grid_constant__ 
                  :: "r"(smem_u32(tmem_slot)), "r"(PS_TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   } else if (warp >= PS_PROD_WARP0 && warp < PS_EPI_WARP0) {
+    pdl_sync();  // (the MMA warp touches nothing but this CTA's own memory)
     resolve_rows(first_rt, first_jb, 0);
     gather_next();
   }
@@ -363,6 +364,7 @@ k_gemm_ps(const __grid_constant__ mb_gemm_desc d_param, const __grid_constant__ 
   } else if (warp == PS_TMA_WARP) {
     // ---------------------------------------------------------------- TMA warp: W_hi / W_lo tiles, up to 4 chunks ahead
     // (warp-uniform loop, one elected lane issues: same reason as in the MMA warp)
+    pdl_sync();
     uint32_t elected;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
     const uint32_t ring_u = __shfl_sync(0xffffffffu, ring, 0);
@@ -400,6 +402,7 @@ k_gemm_ps(const __grid_constant__ mb_gemm_desc d_param, const __grid_constant__ 
     // straight from the tcgen05.ld layout: thread = row, 32 columns per load, global accesses of 32 bytes (one full
     // sector) per thread with 256-bit loads and stores.  No shared-memory staging: every sector is still written
     // exactly once, and the row's sixteen sectors merge in L2.
+    pdl_sync();
     const int e = warp - PS_EPI_WARP0, quarter_e = warp & 3, half = e >> 2;
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter_e * 32) << 16) + (uint32_t)(half * 64);
     bool alive = true;

@@ -14,6 +14,7 @@ __global__ void k_edge_geometry_fwd(int64_t n_edges, const float* __restrict__ c
                                     const int32_t* __restrict__ atom_struct, const int32_t* __restrict__ center,
                                     const int32_t* __restrict__ neighbor, const int32_t* __restrict__ image,
                                     float* __restrict__ vec, float* __restrict__ len, float* __restrict__ unit) {
+  pdl_sync();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n_edges) return;
   const int i = center[e], j = neighbor[e];
@@ -37,6 +38,7 @@ __global__ void k_edge_geometry_fwd(int64_t n_edges, const float* __restrict__ c
 // g_e = dE/dv_e from dE/dlen and dE/dunit:  d len/dv = u ; d unit/dv = (I - u u^T)/len
 __global__ void k_edge_grad(int64_t n_edges, const float* __restrict__ len, const float* __restrict__ unit,
                             const float* __restrict__ dlen, const float* __restrict__ dunit, float* __restrict__ g) {
+  pdl_sync();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n_edges) return;
   const float ux = unit[3 * e], uy = unit[3 * e + 1], uz = unit[3 * e + 2];
@@ -52,6 +54,7 @@ __global__ void k_edge_grad(int64_t n_edges, const float* __restrict__ len, cons
 __global__ void k_atom_grad(int n_atoms, const int32_t* __restrict__ edge_ptr, const int32_t* __restrict__ rev,
                             const float* __restrict__ vec, const float* __restrict__ g, float* __restrict__ dcart,
                             float* __restrict__ virial_atom) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (i >= n_atoms) return;
@@ -85,6 +88,7 @@ __global__ void k_atom_grad(int n_atoms, const int32_t* __restrict__ edge_ptr, c
 // warp per structure: dE/dstrain = 0.5 (G + G^T), G = sum over the structure's atoms of the partials
 __global__ void k_struct_virial(int n_struct, const int32_t* __restrict__ atom_ptr,
                                 const float* __restrict__ virial_atom, float* __restrict__ dstrain) {
+  pdl_sync();
   const int lane = threadIdx.x & 31;
   const int b = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (b >= n_struct) return;
@@ -137,6 +141,7 @@ __device__ __forceinline__ void bessel_eval(float d, float cut, const float* __r
 __global__ void k_bessel_fwd(int n_bonds, const int32_t* __restrict__ u2d, const float* __restrict__ len,
                              const float* __restrict__ fa, float ca, const float* __restrict__ fb, float cb, int p,
                              float* __restrict__ ra, float* __restrict__ rb) {
+  pdl_sync();
   const int u = blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= n_bonds) return;
   const float d = len[u2d[u]];
@@ -152,6 +157,7 @@ __global__ void k_bessel_fwd(int n_bonds, const int32_t* __restrict__ u2d, const
 __global__ void k_bessel_bwd(int n_bonds, const int32_t* __restrict__ u2d, const float* __restrict__ len,
                              const float* __restrict__ fa, float ca, const float* __restrict__ fb, float cb, int p,
                              const float* __restrict__ dra, const float* __restrict__ drb, float* __restrict__ dlen) {
+  pdl_sync();
   const int u = blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= n_bonds) return;
   const int e = u2d[u];
@@ -171,6 +177,7 @@ __global__ void k_bessel_bwd(int n_bonds, const int32_t* __restrict__ u2d, const
 __global__ void k_gaussian_fwd(int n_bonds, const int32_t* __restrict__ u2d, const float* __restrict__ len,
                                const float* __restrict__ off_a, float coeff_a, const float* __restrict__ off_b,
                                float coeff_b, float* __restrict__ ra, float* __restrict__ rb) {
+  pdl_sync();
   const int u = blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= n_bonds) return;
   const float d = len[u2d[u]];
@@ -186,6 +193,7 @@ __global__ void k_gaussian_bwd(int n_bonds, const int32_t* __restrict__ u2d, con
                                const float* __restrict__ off_a, float coeff_a, const float* __restrict__ off_b,
                                float coeff_b, const float* __restrict__ dra, const float* __restrict__ drb,
                                float* __restrict__ dlen) {
+  pdl_sync();
   const int u = blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= n_bonds) return;
   const int e = u2d[u];
@@ -246,6 +254,7 @@ __device__ __forceinline__ void radial16(float x, float factor, float* r) {
 
 __global__ void k_angle_basis_fwd(int64_t n_trip, const int32_t* __restrict__ lg, const float* __restrict__ unit,
                                   float factor, float cutoff, float* __restrict__ basis) {
+  pdl_sync();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n_trip) return;
   const int64_t a = lg[5 * t + 2], b = lg[5 * t + 4];
@@ -266,6 +275,7 @@ __global__ void k_angle_basis_fwd(int64_t n_trip, const int32_t* __restrict__ lg
 __global__ void k_angle_basis_bwd(int64_t n_trip, const int32_t* __restrict__ lg, const float* __restrict__ unit,
                                   float factor, float cutoff, const float* __restrict__ dbasis,
                                   float* __restrict__ dunit) {
+  pdl_sync();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n_trip) return;
   const int64_t a = lg[5 * t + 2], b = lg[5 * t + 4];
@@ -295,6 +305,7 @@ __global__ void k_angle_basis_bwd(int64_t n_trip, const int32_t* __restrict__ lg
 #define FOURIER_INV_SQRT_PI 0.5641895835477563f
 __global__ void k_fourier_fwd(int64_t n_trip, const int32_t* __restrict__ lg, const float* __restrict__ unit,
                               const float* __restrict__ freq, float* __restrict__ basis) {
+  pdl_sync();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n_trip) return;
   const int64_t a = lg[5 * t + 2], b = lg[5 * t + 4];
@@ -314,6 +325,7 @@ __global__ void k_fourier_fwd(int64_t n_trip, const int32_t* __restrict__ lg, co
 __global__ void k_fourier_bwd(int64_t n_trip, const int32_t* __restrict__ lg, const float* __restrict__ unit,
                               const float* __restrict__ freq, const float* __restrict__ dbasis,
                               float* __restrict__ dunit) {
+  pdl_sync();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n_trip) return;
   const int64_t a = lg[5 * t + 2], b = lg[5 * t + 4];
@@ -344,7 +356,7 @@ extern "C" int mb_edge_geometry_fwd(int64_t n_edges, const float* cart, const fl
                                     const int32_t* image, float* vec, float* len, float* unit, void* stream) {
   MB_REQUIRE(n_edges >= 0 && cart && lattice && atom_struct && center && neighbor && image && vec && len && unit);
   if (n_edges == 0) return MB_OK;
-  k_edge_geometry_fwd<<<grid1(n_edges), GEO_THREADS, 0, STREAM>>>(n_edges, cart, lattice, atom_struct, center, neighbor,
+  launch(k_edge_geometry_fwd, grid1(n_edges), GEO_THREADS, 0, STREAM, n_edges, cart, lattice, atom_struct, center, neighbor,
                                                                 image, vec, len, unit);
   MB_LAUNCH_CHECK("k_edge_geometry_fwd");
   return MB_OK;
@@ -356,10 +368,10 @@ extern "C" int mb_edge_geometry_bwd(int32_t n_atoms, int32_t n_struct, int64_t n
                                     float* dcart, float* virial_atom, float* dstrain, void* stream) {
   MB_REQUIRE(n_atoms > 0 && n_struct > 0 && n_edges > 0 && edge_ptr && atom_ptr && rev && vec && len && unit && dlen &&
              dunit && g_edge && dcart && virial_atom && dstrain);
-  k_edge_grad<<<grid1(n_edges), GEO_THREADS, 0, STREAM>>>(n_edges, len, unit, dlen, dunit, g_edge);
-  k_atom_grad<<<grid1((int64_t)n_atoms * 32), GEO_THREADS, 0, STREAM>>>(n_atoms, edge_ptr, rev, vec, g_edge, dcart,
+  launch(k_edge_grad, grid1(n_edges), GEO_THREADS, 0, STREAM, n_edges, len, unit, dlen, dunit, g_edge);
+  launch(k_atom_grad, grid1((int64_t)n_atoms * 32), GEO_THREADS, 0, STREAM, n_atoms, edge_ptr, rev, vec, g_edge, dcart,
                                                                        virial_atom);
-  k_struct_virial<<<grid1((int64_t)n_struct * 32), GEO_THREADS, 0, STREAM>>>(n_struct, atom_ptr, virial_atom, dstrain);
+  launch(k_struct_virial, grid1((int64_t)n_struct * 32), GEO_THREADS, 0, STREAM, n_struct, atom_ptr, virial_atom, dstrain);
   MB_LAUNCH_CHECK("mb_edge_geometry_bwd");
   return MB_OK;
 }
@@ -408,10 +420,10 @@ extern "C" int mb_edge_geometry_bwd_static(int32_t n_atoms, int32_t n_struct, in
   if (!scratch) return status;
   float* g_edge = scratch;                                  // [n_edges,3]  written in full by k_edge_grad before it is read
   float* virial_atom = scratch + 3 * MB_STATIC_MAX_EDGES;   // [n_atoms,9]  written in full by k_atom_grad before it is read
-  k_edge_grad<<<grid1(n_edges), GEO_THREADS, 0, STREAM>>>(n_edges, len, unit, dlen, dunit, g_edge);
-  k_atom_grad<<<grid1((int64_t)n_atoms * 32), GEO_THREADS, 0, STREAM>>>(n_atoms, edge_ptr, rev, vec, g_edge, dcart,
+  launch(k_edge_grad, grid1(n_edges), GEO_THREADS, 0, STREAM, n_edges, len, unit, dlen, dunit, g_edge);
+  launch(k_atom_grad, grid1((int64_t)n_atoms * 32), GEO_THREADS, 0, STREAM, n_atoms, edge_ptr, rev, vec, g_edge, dcart,
                                                                        virial_atom);
-  k_struct_virial<<<grid1((int64_t)n_struct * 32), GEO_THREADS, 0, STREAM>>>(n_struct, atom_ptr, virial_atom, dstrain);
+  launch(k_struct_virial, grid1((int64_t)n_struct * 32), GEO_THREADS, 0, STREAM, n_struct, atom_ptr, virial_atom, dstrain);
   MB_LAUNCH_CHECK("mb_edge_geometry_bwd_static");
   return MB_OK;
 }
@@ -420,7 +432,7 @@ extern "C" int mb_bessel_fwd(int32_t n_bonds, const int32_t* u2d, const float* l
                              const float* freq_b, float cut_b, int32_t p, float* rbf_a, float* rbf_b, void* stream) {
   MB_REQUIRE(n_bonds >= 0 && u2d && len && freq_a && freq_b && rbf_a && rbf_b && p >= 1 && cut_a > 0 && cut_b > 0);
   if (n_bonds == 0) return MB_OK;
-  k_bessel_fwd<<<grid1(n_bonds), GEO_THREADS, 0, STREAM>>>(n_bonds, u2d, len, freq_a, cut_a, freq_b, cut_b, p, rbf_a,
+  launch(k_bessel_fwd, grid1(n_bonds), GEO_THREADS, 0, STREAM, n_bonds, u2d, len, freq_a, cut_a, freq_b, cut_b, p, rbf_a,
                                                          rbf_b);
   MB_LAUNCH_CHECK("k_bessel_fwd");
   return MB_OK;
@@ -431,7 +443,7 @@ extern "C" int mb_bessel_bwd(int32_t n_bonds, const int32_t* u2d, const float* l
                              float* dlen, void* stream) {
   MB_REQUIRE(n_bonds >= 0 && u2d && len && freq_a && freq_b && drbf_a && drbf_b && dlen && p >= 1);
   if (n_bonds == 0) return MB_OK;
-  k_bessel_bwd<<<grid1(n_bonds), GEO_THREADS, 0, STREAM>>>(n_bonds, u2d, len, freq_a, cut_a, freq_b, cut_b, p, drbf_a,
+  launch(k_bessel_bwd, grid1(n_bonds), GEO_THREADS, 0, STREAM, n_bonds, u2d, len, freq_a, cut_a, freq_b, cut_b, p, drbf_a,
                                                          drbf_b, dlen);
   MB_LAUNCH_CHECK("k_bessel_bwd");
   return MB_OK;
@@ -441,7 +453,7 @@ extern "C" int mb_gaussian_fwd(int32_t n_bonds, const int32_t* u2d, const float*
                                const float* off_b, float coeff_b, float* rbf_a, float* rbf_b, void* stream) {
   MB_REQUIRE(n_bonds >= 0 && u2d && len && off_a && off_b && rbf_a && rbf_b);
   if (n_bonds == 0) return MB_OK;
-  k_gaussian_fwd<<<grid1(n_bonds), GEO_THREADS, 0, STREAM>>>(n_bonds, u2d, len, off_a, coeff_a, off_b, coeff_b, rbf_a,
+  launch(k_gaussian_fwd, grid1(n_bonds), GEO_THREADS, 0, STREAM, n_bonds, u2d, len, off_a, coeff_a, off_b, coeff_b, rbf_a,
                                                            rbf_b);
   MB_LAUNCH_CHECK("k_gaussian_fwd");
   return MB_OK;
@@ -452,7 +464,7 @@ extern "C" int mb_gaussian_bwd(int32_t n_bonds, const int32_t* u2d, const float*
                                float* dlen, void* stream) {
   MB_REQUIRE(n_bonds >= 0 && u2d && len && off_a && off_b && drbf_a && drbf_b && dlen);
   if (n_bonds == 0) return MB_OK;
-  k_gaussian_bwd<<<grid1(n_bonds), GEO_THREADS, 0, STREAM>>>(n_bonds, u2d, len, off_a, coeff_a, off_b, coeff_b, drbf_a,
+  launch(k_gaussian_bwd, grid1(n_bonds), GEO_THREADS, 0, STREAM, n_bonds, u2d, len, off_a, coeff_a, off_b, coeff_b, drbf_a,
                                                            drbf_b, dlen);
   MB_LAUNCH_CHECK("k_gaussian_bwd");
   return MB_OK;
@@ -462,7 +474,7 @@ extern "C" int mb_fourier_basis_fwd(int64_t n_trip, const int32_t* line_graph, c
                                     float* basis, void* stream) {
   MB_REQUIRE(n_trip >= 0 && line_graph && unit && freq && basis);
   if (n_trip == 0) return MB_OK;
-  k_fourier_fwd<<<grid1(n_trip), GEO_THREADS, 0, STREAM>>>(n_trip, line_graph, unit, freq, basis);
+  launch(k_fourier_fwd, grid1(n_trip), GEO_THREADS, 0, STREAM, n_trip, line_graph, unit, freq, basis);
   MB_LAUNCH_CHECK("k_fourier_fwd");
   return MB_OK;
 }
@@ -471,7 +483,7 @@ extern "C" int mb_fourier_basis_bwd(int64_t n_trip, const int32_t* line_graph, c
                                     const float* dbasis, float* dunit, void* stream) {
   MB_REQUIRE(n_trip >= 0 && line_graph && unit && freq && dbasis && dunit);
   if (n_trip == 0) return MB_OK;
-  k_fourier_bwd<<<grid1(n_trip), GEO_THREADS, 0, STREAM>>>(n_trip, line_graph, unit, freq, dbasis, dunit);
+  launch(k_fourier_bwd, grid1(n_trip), GEO_THREADS, 0, STREAM, n_trip, line_graph, unit, freq, dbasis, dunit);
   MB_LAUNCH_CHECK("k_fourier_bwd");
   return MB_OK;
 }
@@ -480,7 +492,7 @@ extern "C" int mb_angle_basis_fwd(int64_t n_trip, const int32_t* line_graph, con
                                   float cutoff, float* basis, void* stream) {
   MB_REQUIRE(n_trip >= 0 && line_graph && unit && basis && cutoff > 0);
   if (n_trip == 0) return MB_OK;
-  k_angle_basis_fwd<<<grid1(n_trip), GEO_THREADS, 0, STREAM>>>(n_trip, line_graph, unit, factor, cutoff, basis);
+  launch(k_angle_basis_fwd, grid1(n_trip), GEO_THREADS, 0, STREAM, n_trip, line_graph, unit, factor, cutoff, basis);
   MB_LAUNCH_CHECK("k_angle_basis_fwd");
   return MB_OK;
 }
@@ -489,7 +501,7 @@ extern "C" int mb_angle_basis_bwd(int64_t n_trip, const int32_t* line_graph, con
                                   float cutoff, const float* dbasis, float* dunit, void* stream) {
   MB_REQUIRE(n_trip >= 0 && line_graph && unit && dbasis && dunit && cutoff > 0);
   if (n_trip == 0) return MB_OK;
-  k_angle_basis_bwd<<<grid1(n_trip), GEO_THREADS, 0, STREAM>>>(n_trip, line_graph, unit, factor, cutoff, dbasis, dunit);
+  launch(k_angle_basis_bwd, grid1(n_trip), GEO_THREADS, 0, STREAM, n_trip, line_graph, unit, factor, cutoff, dbasis, dunit);
   MB_LAUNCH_CHECK("k_angle_basis_bwd");
   return MB_OK;
 }

@@ -126,14 +126,6 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
                  side_empty = bar0 + 384, conv_full = bar0 + 512;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   float* const cst = reinterpret_cast<float*>(smem + ML_CONST_OFF);
-  for (int i = tid; i < 896; i += ML_THREADS) {
-    float v = 0.f;
-    if (i < 256) { if (FWD && d.b1 && (GATED || i < 128)) v = d.b1[i]; }
-    else if (i < 512) { if (FWD && d.b2 && (GATED || i < 384)) v = d.b2[i - 256]; }
-    else if (i < 768) { if (FWD && GATED) v = i < 640 ? d.norm_core[i - 512] : d.norm_gate[i - 640]; }
-    else v = d.res_w ? d.res_w[i - 768] : 1.f;
-    cst[i] = v;
-  }
   const int64_t n_rows = d.n_rows;
   const int n_row_tiles = (int)((n_rows + 127) >> 7);
   const int first_rt = (int)blockIdx.x, step_rt = (int)gridDim.x;
@@ -298,6 +290,7 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
     });
   } else if (warp == ML_TMA_WARP) {
     // ---------------------------------------------------------------- TMA warp: weight tiles, up to five ahead
+    pdl_sync();
     uint32_t elected;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
     const uint32_t ring_u = __shfl_sync(0xffffffffu, sm0, 0);
@@ -332,6 +325,16 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
     }
   } else if (warp >= ML_EPI_WARP0) {
     // ---------------------------------------------------------------- epilogue warps
+    pdl_sync();  // (the MMA warp touches nothing but this CTA's own memory)
+    for (int i = tid - 32 * ML_EPI_WARP0; i < 896; i += 256) {
+      float v = 0.f;
+      if (i < 256) { if (FWD && d.b1 && (GATED || i < 128)) v = d.b1[i]; }
+      else if (i < 512) { if (FWD && d.b2 && (GATED || i < 384)) v = d.b2[i - 256]; }
+      else if (i < 768) { if (FWD && GATED) v = i < 640 ? d.norm_core[i - 512] : d.norm_gate[i - 640]; }
+      else v = d.res_w ? d.res_w[i - 768] : 1.f;
+      cst[i] = v;
+    }
+    asm volatile("bar.sync 5, 512;" ::: "memory");  // the constants are there: epilogue and producer warps
     const int e = warp - ML_EPI_WARP0, q = warp & 3, grp = e >> 2;
     const uint32_t lane_q = tmem_base + ((uint32_t)(q * 32) << 16);
     const uint32_t side0 = sm0 + ML_SIDE_OFF + e * 2 * ML_PATCH, stage = sm0 + ML_STAGE_OFF + e * ML_PATCH;
@@ -535,6 +538,7 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
   } else {
     // ---------------------------------------------------------------- producers
     // Warp pw: lane quarter (warp & 3), K chunks of its parity; then the side patches of epilogue warp pw (same quarter).
+    pdl_sync();
     const int pw = warp - ML_PROD_WARP0, parity = pw >> 2, quarter = warp & 3;
     const int lr = lane >> 3, lc = lane & 7;
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
@@ -571,6 +575,7 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
       }
     };
     if (n_seg > 0 && is_direct(0)) request(0, 0, 0);
+    asm volatile("bar.sync 5, 512;" ::: "memory");  // the constants are there
     for (int t = 0; t < n_tiles; ++t) {
       const int64_t row0 = tile_row(t);
       // rows past the end repeat the last row; their results are never written

@@ -43,6 +43,7 @@ static inline unsigned row_grid(int64_t n_rows) { return (unsigned)((n_rows * 32
 __global__ void k_gate_fwd(int64_t n_rows, const float* __restrict__ z, const float* __restrict__ wc,
                            const float* __restrict__ wg, float* __restrict__ h, const float* __restrict__ res,
                            const float* __restrict__ res_w, float* __restrict__ out2) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
   const float4 xc = ld4(z + row * 256 + c), xg = ld4(z + row * 256 + 128 + c);
   const float rc = rsqrtf(warp_sum(dot4(xc, xc)) * (1.f / 128.f) + RMS_EPS);
@@ -87,6 +88,7 @@ __device__ __forceinline__ void gate_bwd_row(int64_t row, int c, const float* __
 
 __global__ void k_gate_bwd(int64_t n_rows, const float* __restrict__ z, const float* __restrict__ wc,
                            const float* __restrict__ wg, const float* __restrict__ dh, float* __restrict__ dz) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
   gate_bwd_row(row, c, z, wc, wg, ld4(dh + row * 128 + c), dz);
 }
@@ -97,6 +99,7 @@ __global__ void k_seg_attn_fwd(int n_nodes, const int32_t* __restrict__ tgt_ptr,
                                const int32_t* __restrict__ src_perm, const int32_t* __restrict__ emap,
                                const float* __restrict__ logits, const float* __restrict__ h,
                                float* __restrict__ agg_t, float* __restrict__ agg_s, float* __restrict__ stats) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_nodes)
   constexpr int NB = 8;  // rows in flight per warp: their index and data loads are issued together
 #pragma unroll
@@ -181,6 +184,7 @@ __global__ void k_seg_attn_bwd(int64_t n_rows, const int32_t* __restrict__ tgt, 
                                float* __restrict__ dh, float* __restrict__ dlogits, const float* __restrict__ gate_z,
                                const float* __restrict__ gate_wc, const float* __restrict__ gate_wg,
                                float* __restrict__ gate_dz) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
   const int64_t nt = tgt[row * idx_stride], ns = src[row * idx_stride];
   const int64_t er = emap ? emap[row] : row;
@@ -205,6 +209,7 @@ __global__ void k_seg_smooth_sum_fwd(int n_nodes, const int32_t* __restrict__ tg
                                      const int32_t* __restrict__ emap, const int32_t* __restrict__ src,
                                      int idx_stride, const float* __restrict__ env, const float* __restrict__ h,
                                      float* __restrict__ agg) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_nodes)
   const int q0 = tgt_ptr[row], q1 = tgt_ptr[row + 1];
   float4 acc = zero4();
@@ -225,6 +230,7 @@ __global__ void k_seg_smooth_sum_bwd_rows(int64_t n_rows, const int32_t* __restr
                                           const float* __restrict__ dagg, float* __restrict__ dh, int accumulate,
                                           const float* __restrict__ gate_z, const float* __restrict__ gate_wc,
                                           const float* __restrict__ gate_wg, float* __restrict__ gate_dz) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
   const int64_t nt = tgt[row * idx_stride];
   float4 s;
@@ -240,6 +246,7 @@ __global__ void k_smooth_env_bwd_atom(int n_bonds, const int32_t* __restrict__ u
                                       const int32_t* __restrict__ tgt, const float* __restrict__ h,
                                       const float* __restrict__ dagg, const float* __restrict__ drow,
                                       float* __restrict__ denv) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_bonds)
   const int64_t e1 = u2d[row], e2 = rev[e1];
   float4 g1 = ld4(dagg + (int64_t)tgt[e1] * 128 + c), g2 = ld4(dagg + (int64_t)tgt[e2] * 128 + c);
@@ -253,6 +260,7 @@ __global__ void k_smooth_env_bwd_atom(int n_bonds, const int32_t* __restrict__ u
 // y[r] = x[r] * s[idx[r]]  (rows scaled channel-wise by a gathered row)
 __global__ void k_mul_rows_gather(int64_t n_rows, const float* __restrict__ x, const float* __restrict__ s,
                                   const int32_t* __restrict__ idx, float* __restrict__ y) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
   const int64_t sr = idx ? idx[row] : row;
   st4(y + row * 128 + c, mul4(ld4(x + row * 128 + c), ld4(s + sr * 128 + c)));
@@ -263,6 +271,7 @@ __global__ void k_smooth_env_bwd_line(int n_nodes, const int32_t* __restrict__ t
                                       const int32_t* __restrict__ tgt, const int32_t* __restrict__ src,
                                       int idx_stride, const float* __restrict__ env, const float* __restrict__ h,
                                       const float* __restrict__ dagg, float* __restrict__ denv) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_nodes)
   float4 acc = zero4();
   const int q0 = tgt_ptr[row], q1 = tgt_ptr[row + 1];
@@ -291,6 +300,7 @@ template <int WARPS>
 __global__ void k_seg_sum(int n_nodes, const int32_t* __restrict__ tgt_ptr, const int32_t* __restrict__ src_ptr,
                           const int32_t* __restrict__ src_perm, const int32_t* __restrict__ ctr,
                           const float* __restrict__ x, float* __restrict__ out, float* __restrict__ ctr_out) {
+  pdl_sync();
   constexpr int NB = 4;  // rows in flight per warp
   __shared__ float4 part[WARPS > 1 ? WARPS : 1][WARPS > 1 ? 64 : 1];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -357,6 +367,7 @@ __global__ void k_seg_sum(int n_nodes, const int32_t* __restrict__ tgt_ptr, cons
 // out[u, 0:256] = a[e1] + a[e2] and, with b, out[u, 256:512] = b[e1] + b[e2]: the two directed rows e1, e2 of bond u
 __global__ void k_pair_sum(int n_bonds, const int32_t* __restrict__ u2d, const int32_t* __restrict__ rev,
                            const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out, int ld) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_bonds)
   const int64_t e1 = u2d[row], e2 = rev[e1];
 #pragma unroll
@@ -372,6 +383,7 @@ __global__ void k_pair_sum(int n_bonds, const int32_t* __restrict__ u2d, const i
 __global__ void k_pair_mean_res(int n_bonds, const int32_t* __restrict__ u2d, const int32_t* __restrict__ rev,
                                 const float* __restrict__ y, const float* __restrict__ res,
                                 const float* __restrict__ res_w, float* __restrict__ out) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_bonds)
   const int64_t e1 = u2d[row], e2 = rev[e1];
   float4 o = scl4(add4(ld4(y + e1 * 128 + c), ld4(y + e2 * 128 + c)), 0.5f);
@@ -385,6 +397,7 @@ __global__ void k_pair_mean_res(int n_bonds, const int32_t* __restrict__ u2d, co
 
 __global__ void k_scale_rows(int64_t n_rows, const float* __restrict__ x, const float* __restrict__ a,
                              float* __restrict__ y, int accumulate) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
   float4 o = ld4(x + row * 128 + c);
   if (a) o = mul4(ld4(a + c), o);
@@ -395,6 +408,7 @@ __global__ void k_scale_rows(int64_t n_rows, const float* __restrict__ x, const 
 // ------------------------------------------------------------------ K <= 16 linear layers
 __global__ void k_small_linear_fwd(int64_t n_rows, int k, const float* __restrict__ x, const float* __restrict__ w,
                                    float* __restrict__ y) {
+  pdl_sync();
   __shared__ float ws[16][128];
   for (int i = threadIdx.x; i < 128 * k; i += blockDim.x) ws[i % k][i / k] = w[i];
   __syncthreads();
@@ -409,6 +423,7 @@ __global__ void k_small_linear_fwd(int64_t n_rows, int k, const float* __restric
 
 __global__ void k_small_linear_bwd(int64_t n_rows, int k, const float* __restrict__ dy, const float* __restrict__ w,
                                    float* __restrict__ dx, int accumulate) {
+  pdl_sync();
   __shared__ float ws[16][128];
   for (int i = threadIdx.x; i < 128 * k; i += blockDim.x) ws[i % k][i / k] = w[i];
   __syncthreads();
@@ -428,6 +443,7 @@ __global__ void k_small_linear_bwd(int64_t n_rows, int k, const float* __restric
 // ------------------------------------------------------------------ norms
 __global__ void k_layernorm_fwd(int64_t n_rows, const float* __restrict__ x, const float* __restrict__ w,
                                 const float* __restrict__ b, float* __restrict__ y) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
   const float4 v = ld4(x + row * 128 + c);
   const float mean = warp_sum(v.x + v.y + v.z + v.w) * (1.f / 128.f);
@@ -438,6 +454,7 @@ __global__ void k_layernorm_fwd(int64_t n_rows, const float* __restrict__ x, con
 
 __global__ void k_layernorm_bwd(int64_t n_rows, const float* __restrict__ x, const float* __restrict__ w,
                                 const float* __restrict__ dy, float* __restrict__ dx) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
   const float4 v = ld4(x + row * 128 + c);
   const float mean = warp_sum(v.x + v.y + v.z + v.w) * (1.f / 128.f);
@@ -453,6 +470,7 @@ __global__ void k_layernorm_bwd(int64_t n_rows, const float* __restrict__ x, con
 
 __global__ void k_rmsnorm_fwd(int64_t n_rows, const float* __restrict__ x, const float* __restrict__ w,
                               float* __restrict__ y) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
   const float4 v = ld4(x + row * 128 + c);
   const float r = rsqrtf(warp_sum(dot4(v, v)) * (1.f / 128.f) + RMS_EPS);
@@ -461,6 +479,7 @@ __global__ void k_rmsnorm_fwd(int64_t n_rows, const float* __restrict__ x, const
 
 __global__ void k_rmsnorm_bwd(int64_t n_rows, const float* __restrict__ x, const float* __restrict__ w,
                               const float* __restrict__ dy, float* __restrict__ dx) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
   const float4 v = ld4(x + row * 128 + c);
   const float r = rsqrtf(warp_sum(dot4(v, v)) * (1.f / 128.f) + RMS_EPS);
@@ -472,6 +491,7 @@ __global__ void k_rmsnorm_bwd(int64_t n_rows, const float* __restrict__ x, const
 
 __global__ void k_embedding(int64_t n_rows, const int32_t* __restrict__ idx, int offset,
                             const float* __restrict__ table, float* __restrict__ y) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
   st4(y + row * 128 + c, ld4(table + (int64_t)(idx[row] + offset) * 128 + c));
 }
@@ -479,6 +499,7 @@ __global__ void k_embedding(int64_t n_rows, const int32_t* __restrict__ idx, int
 // ------------------------------------------------------------------ head projections
 __global__ void k_head_dot_fwd(int64_t n_rows, int k, const float* __restrict__ z, const float* __restrict__ w,
                                const float* __restrict__ b, int take_abs, float* __restrict__ out) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
   float s = 0.f;
   for (int j = c; j < k; j += 128) {
@@ -492,6 +513,7 @@ __global__ void k_head_dot_fwd(int64_t n_rows, int k, const float* __restrict__ 
 __global__ void k_head_dot_bwd(int64_t n_rows, int k, const float* __restrict__ z, const float* __restrict__ w,
                                const float* __restrict__ seed, const int32_t* __restrict__ seed_map,
                                float* __restrict__ dz) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
   const float g = seed ? seed[seed_map ? seed_map[row] : row] : 1.f;
   for (int j = c; j < k; j += 128) {
@@ -503,6 +525,7 @@ __global__ void k_head_dot_bwd(int64_t n_rows, int k, const float* __restrict__ 
 
 __global__ void k_silu_bwd(int64_t n_rows, const float* __restrict__ dy, const float* __restrict__ z,
                            float* __restrict__ dz) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
   const float4 g = ld4(dy + row * 128 + c), v = ld4(z + row * 128 + c);
   st4(dz + row * 128 + c, make_float4(g.x * silu_grad_f(v.x), g.y * silu_grad_f(v.y), g.z * silu_grad_f(v.z),
@@ -511,6 +534,7 @@ __global__ void k_silu_bwd(int64_t n_rows, const float* __restrict__ dy, const f
 
 __global__ void k_segment_sum_scalar(int n_seg, const int32_t* __restrict__ seg_ptr, const float* __restrict__ x,
                                      float* __restrict__ out) {
+  pdl_sync();
   MB_ROW_PROLOGUE(n_seg)
   float s = 0.f;
   for (int i = seg_ptr[row] + lane; i < seg_ptr[row + 1]; i += 32) s += x[i];
@@ -528,7 +552,7 @@ extern "C" int mb_gate_fwd(int64_t n_rows, const float* z, const float* w_core, 
                            const float* res, const float* res_w, float* out2, void* stream) {
   MB_REQUIRE(n_rows >= 0 && z && w_core && w_gate && (h || out2) && (!out2 || res));
   if (n_rows == 0) return MB_OK;
-  k_gate_fwd<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, z, w_core, w_gate, h, res, res_w, out2);
+  launch(k_gate_fwd, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, z, w_core, w_gate, h, res, res_w, out2);
   MB_LAUNCH_CHECK("k_gate_fwd");
   return MB_OK;
 }
@@ -537,7 +561,7 @@ extern "C" int mb_gate_bwd(int64_t n_rows, const float* z, const float* w_core, 
                            float* dz, void* stream) {
   MB_REQUIRE(n_rows >= 0 && z && w_core && w_gate && dh && dz);
   if (n_rows == 0) return MB_OK;
-  k_gate_bwd<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, z, w_core, w_gate, dh, dz);
+  launch(k_gate_bwd, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, z, w_core, w_gate, dh, dz);
   MB_LAUNCH_CHECK("k_gate_bwd");
   return MB_OK;
 }
@@ -547,7 +571,7 @@ extern "C" int mb_seg_attn_fwd(int32_t n_nodes, const int32_t* tgt_ptr, const in
                                float* agg_t, float* agg_s, float* stats, void* stream) {
   MB_REQUIRE(n_nodes >= 0 && tgt_ptr && src_ptr && src_perm && logits && h && agg_t && agg_s && stats);
   if (n_nodes == 0) return MB_OK;
-  k_seg_attn_fwd<<<row_grid(n_nodes), RW_THREADS, 0, STREAM>>>(n_nodes, tgt_ptr, src_ptr, src_perm, emap, logits, h,
+  launch(k_seg_attn_fwd, row_grid(n_nodes), RW_THREADS, 0, STREAM, n_nodes, tgt_ptr, src_ptr, src_perm, emap, logits, h,
                                                               agg_t, agg_s, stats);
   MB_LAUNCH_CHECK("k_seg_attn_fwd");
   return MB_OK;
@@ -562,7 +586,7 @@ extern "C" int mb_seg_attn_bwd(int64_t n_rows, const int32_t* tgt, const int32_t
   MB_REQUIRE(n_rows >= 0 && tgt && src && idx_stride > 0 && logits && h && agg_t && agg_s && stats && dagg_t &&
              dagg_s && dlogits && (gate_dz ? (gate_z && gate_wc && gate_wg) : dh != nullptr));
   if (n_rows == 0) return MB_OK;
-  k_seg_attn_bwd<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, tgt, src, idx_stride, emap, logits, h, agg_t,
+  launch(k_seg_attn_bwd, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, tgt, src, idx_stride, emap, logits, h, agg_t,
                                                              agg_s, stats, dagg_t, dagg_s, dh_in, dh_map, dh_scale,
                                                              dh, dlogits, gate_z, gate_wc, gate_wg, gate_dz);
   MB_LAUNCH_CHECK("k_seg_attn_bwd");
@@ -574,7 +598,7 @@ extern "C" int mb_seg_smooth_sum_fwd(int32_t n_nodes, const int32_t* tgt_ptr, co
                                      float* agg, void* stream) {
   MB_REQUIRE(n_nodes >= 0 && tgt_ptr && (emap || src) && env && h && agg && idx_stride > 0);
   if (n_nodes == 0) return MB_OK;
-  k_seg_smooth_sum_fwd<<<row_grid(n_nodes), RW_THREADS, 0, STREAM>>>(n_nodes, tgt_ptr, emap, src, idx_stride, env, h,
+  launch(k_seg_smooth_sum_fwd, row_grid(n_nodes), RW_THREADS, 0, STREAM, n_nodes, tgt_ptr, emap, src, idx_stride, env, h,
                                                                     agg);
   MB_LAUNCH_CHECK("k_seg_smooth_sum_fwd");
   return MB_OK;
@@ -587,7 +611,7 @@ extern "C" int mb_seg_smooth_sum_bwd_rows(int64_t n_rows, const int32_t* tgt, co
   MB_REQUIRE(n_rows >= 0 && tgt && (emap || src) && env && dagg && idx_stride > 0 && (dh || (gate_dz && !accumulate)) &&
              (!gate_dz || (gate_z && gate_wc && gate_wg)));
   if (n_rows == 0) return MB_OK;
-  k_seg_smooth_sum_bwd_rows<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, tgt, src, idx_stride, emap, env,
+  launch(k_seg_smooth_sum_bwd_rows, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, tgt, src, idx_stride, emap, env,
                                                                         dagg, dh, accumulate, gate_z, gate_wc, gate_wg,
                                                                         gate_dz);
   MB_LAUNCH_CHECK("k_seg_smooth_sum_bwd_rows");
@@ -603,10 +627,10 @@ extern "C" int mb_seg_smooth_sum_bwd_env(int32_t n_nodes, const int32_t* tgt_ptr
   if (n_nodes == 0) return MB_OK;
   if (!src_ptr) {
     MB_REQUIRE(u2d && rev && idx_stride == 1);
-    k_smooth_env_bwd_atom<<<row_grid(n_nodes), RW_THREADS, 0, STREAM>>>(n_nodes, u2d, rev, tgt, h, dagg, drow, denv);
+    launch(k_smooth_env_bwd_atom, row_grid(n_nodes), RW_THREADS, 0, STREAM, n_nodes, u2d, rev, tgt, h, dagg, drow, denv);
   } else {
     MB_REQUIRE(tgt_ptr && src_perm && src && env && !drow);
-    k_smooth_env_bwd_line<<<row_grid(n_nodes), RW_THREADS, 0, STREAM>>>(n_nodes, tgt_ptr, src_ptr, src_perm, tgt, src,
+    launch(k_smooth_env_bwd_line, row_grid(n_nodes), RW_THREADS, 0, STREAM, n_nodes, tgt_ptr, src_ptr, src_perm, tgt, src,
                                                                        idx_stride, env, h, dagg, denv);
   }
   MB_LAUNCH_CHECK("k_smooth_env_bwd");
@@ -617,7 +641,7 @@ extern "C" int mb_mul_rows_gather(int64_t n_rows, const float* x, const float* s
                                   void* stream) {
   MB_REQUIRE(n_rows >= 0 && x && s && y);
   if (n_rows == 0) return MB_OK;
-  k_mul_rows_gather<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, x, s, idx, y);
+  launch(k_mul_rows_gather, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, x, s, idx, y);
   MB_LAUNCH_CHECK("k_mul_rows_gather");
   return MB_OK;
 }
@@ -629,9 +653,9 @@ extern "C" int mb_seg_sum(int32_t n_nodes, int64_t n_rows, const int32_t* tgt_pt
   if (n_nodes == 0) return MB_OK;
   // long segments on average (and no per-centre sums, which follow the order of the rows): a block per segment and side
   if (!ctr && n_rows >= 16 * (int64_t)n_nodes)
-    k_seg_sum<8><<<2 * (unsigned)n_nodes, 256, 0, STREAM>>>(n_nodes, tgt_ptr, src_ptr, src_perm, ctr, x, out, ctr_out);
+    launch(k_seg_sum<8>, 2 * (unsigned)n_nodes, 256, 0, STREAM, n_nodes, tgt_ptr, src_ptr, src_perm, ctr, x, out, ctr_out);
   else
-    k_seg_sum<1><<<row_grid(2 * (int64_t)n_nodes), RW_THREADS, 0, STREAM>>>(n_nodes, tgt_ptr, src_ptr, src_perm, ctr, x, out,
+    launch(k_seg_sum<1>, row_grid(2 * (int64_t)n_nodes), RW_THREADS, 0, STREAM, n_nodes, tgt_ptr, src_ptr, src_perm, ctr, x, out,
                                                                            ctr_out);
   MB_LAUNCH_CHECK("k_seg_sum");
   return MB_OK;
@@ -641,7 +665,7 @@ extern "C" int mb_pair_sum(int32_t n_bonds, const int32_t* u2d, const int32_t* r
                            void* stream) {
   MB_REQUIRE(n_bonds >= 0 && u2d && rev && a && out);
   if (n_bonds == 0) return MB_OK;
-  k_pair_sum<<<row_grid(n_bonds), RW_THREADS, 0, STREAM>>>(n_bonds, u2d, rev, a, b, out, b ? 512 : 256);
+  launch(k_pair_sum, row_grid(n_bonds), RW_THREADS, 0, STREAM, n_bonds, u2d, rev, a, b, out, b ? 512 : 256);
   MB_LAUNCH_CHECK("k_pair_sum");
   return MB_OK;
 }
@@ -650,7 +674,7 @@ extern "C" int mb_pair_mean_res(int32_t n_bonds, const int32_t* u2d, const int32
                                 const float* res, const float* res_w, float* out, void* stream) {
   MB_REQUIRE(n_bonds >= 0 && u2d && rev && y && out);
   if (n_bonds == 0) return MB_OK;
-  k_pair_mean_res<<<row_grid(n_bonds), RW_THREADS, 0, STREAM>>>(n_bonds, u2d, rev, y, res, res_w, out);
+  launch(k_pair_mean_res, row_grid(n_bonds), RW_THREADS, 0, STREAM, n_bonds, u2d, rev, y, res, res_w, out);
   MB_LAUNCH_CHECK("k_pair_mean_res");
   return MB_OK;
 }
@@ -659,7 +683,7 @@ extern "C" int mb_scale_rows(int64_t n_rows, const float* x, const float* a, flo
                              void* stream) {
   MB_REQUIRE(n_rows >= 0 && x && y);
   if (n_rows == 0) return MB_OK;
-  k_scale_rows<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, x, a, y, accumulate);
+  launch(k_scale_rows, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, x, a, y, accumulate);
   MB_LAUNCH_CHECK("k_scale_rows");
   return MB_OK;
 }
@@ -667,7 +691,7 @@ extern "C" int mb_scale_rows(int64_t n_rows, const float* x, const float* a, flo
 extern "C" int mb_small_linear_fwd(int64_t n_rows, int32_t k, const float* x, const float* w, float* y, void* stream) {
   MB_REQUIRE(n_rows >= 0 && k >= 1 && k <= 16 && x && w && y);
   if (n_rows == 0) return MB_OK;
-  k_small_linear_fwd<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, k, x, w, y);
+  launch(k_small_linear_fwd, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, k, x, w, y);
   MB_LAUNCH_CHECK("k_small_linear_fwd");
   return MB_OK;
 }
@@ -676,7 +700,7 @@ extern "C" int mb_small_linear_bwd(int64_t n_rows, int32_t k, const float* dy, c
                                    int32_t accumulate, void* stream) {
   MB_REQUIRE(n_rows >= 0 && k >= 1 && k <= 16 && dy && w && dx);
   if (n_rows == 0) return MB_OK;
-  k_small_linear_bwd<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, k, dy, w, dx, accumulate);
+  launch(k_small_linear_bwd, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, k, dy, w, dx, accumulate);
   MB_LAUNCH_CHECK("k_small_linear_bwd");
   return MB_OK;
 }
@@ -685,7 +709,7 @@ extern "C" int mb_layernorm_fwd(int64_t n_rows, const float* x, const float* w, 
                                 void* stream) {
   MB_REQUIRE(n_rows >= 0 && x && w && b && y);
   if (n_rows == 0) return MB_OK;
-  k_layernorm_fwd<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, x, w, b, y);
+  launch(k_layernorm_fwd, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, x, w, b, y);
   MB_LAUNCH_CHECK("k_layernorm_fwd");
   return MB_OK;
 }
@@ -694,7 +718,7 @@ extern "C" int mb_layernorm_bwd(int64_t n_rows, const float* x, const float* w, 
                                 void* stream) {
   MB_REQUIRE(n_rows >= 0 && x && w && dy && dx);
   if (n_rows == 0) return MB_OK;
-  k_layernorm_bwd<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, x, w, dy, dx);
+  launch(k_layernorm_bwd, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, x, w, dy, dx);
   MB_LAUNCH_CHECK("k_layernorm_bwd");
   return MB_OK;
 }
@@ -702,7 +726,7 @@ extern "C" int mb_layernorm_bwd(int64_t n_rows, const float* x, const float* w, 
 extern "C" int mb_rmsnorm_fwd(int64_t n_rows, const float* x, const float* w, float* y, void* stream) {
   MB_REQUIRE(n_rows >= 0 && x && w && y);
   if (n_rows == 0) return MB_OK;
-  k_rmsnorm_fwd<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, x, w, y);
+  launch(k_rmsnorm_fwd, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, x, w, y);
   MB_LAUNCH_CHECK("k_rmsnorm_fwd");
   return MB_OK;
 }
@@ -711,7 +735,7 @@ extern "C" int mb_rmsnorm_bwd(int64_t n_rows, const float* x, const float* w, co
                               void* stream) {
   MB_REQUIRE(n_rows >= 0 && x && w && dy && dx);
   if (n_rows == 0) return MB_OK;
-  k_rmsnorm_bwd<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, x, w, dy, dx);
+  launch(k_rmsnorm_bwd, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, x, w, dy, dx);
   MB_LAUNCH_CHECK("k_rmsnorm_bwd");
   return MB_OK;
 }
@@ -720,7 +744,7 @@ extern "C" int mb_embedding(int64_t n_rows, const int32_t* idx, int32_t offset, 
                             void* stream) {
   MB_REQUIRE(n_rows >= 0 && idx && table && y);
   if (n_rows == 0) return MB_OK;
-  k_embedding<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, idx, offset, table, y);
+  launch(k_embedding, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, idx, offset, table, y);
   MB_LAUNCH_CHECK("k_embedding");
   return MB_OK;
 }
@@ -729,7 +753,7 @@ extern "C" int mb_head_dot_fwd(int64_t n_rows, int32_t k, const float* z, const 
                                int32_t take_abs, float* out, void* stream) {
   MB_REQUIRE(n_rows >= 0 && k > 0 && (k % 128) == 0 && z && w && b && out);
   if (n_rows == 0) return MB_OK;
-  k_head_dot_fwd<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, k, z, w, b, take_abs, out);
+  launch(k_head_dot_fwd, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, k, z, w, b, take_abs, out);
   MB_LAUNCH_CHECK("k_head_dot_fwd");
   return MB_OK;
 }
@@ -738,7 +762,7 @@ extern "C" int mb_head_dot_bwd(int64_t n_rows, int32_t k, const float* z, const 
                                const int32_t* seed_map, float* dz, void* stream) {
   MB_REQUIRE(n_rows >= 0 && k > 0 && (k % 128) == 0 && z && w && dz);
   if (n_rows == 0) return MB_OK;
-  k_head_dot_bwd<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, k, z, w, seed, seed_map, dz);
+  launch(k_head_dot_bwd, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, k, z, w, seed, seed_map, dz);
   MB_LAUNCH_CHECK("k_head_dot_bwd");
   return MB_OK;
 }
@@ -746,7 +770,7 @@ extern "C" int mb_head_dot_bwd(int64_t n_rows, int32_t k, const float* z, const 
 extern "C" int mb_silu_bwd(int64_t n_rows, const float* dy, const float* z, float* dz, void* stream) {
   MB_REQUIRE(n_rows >= 0 && dy && z && dz);
   if (n_rows == 0) return MB_OK;
-  k_silu_bwd<<<row_grid(n_rows), RW_THREADS, 0, STREAM>>>(n_rows, dy, z, dz);
+  launch(k_silu_bwd, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, dy, z, dz);
   MB_LAUNCH_CHECK("k_silu_bwd");
   return MB_OK;
 }
@@ -755,7 +779,7 @@ extern "C" int mb_segment_sum_scalar(int32_t n_seg, const int32_t* seg_ptr, cons
                                      void* stream) {
   MB_REQUIRE(n_seg >= 0 && seg_ptr && x && out);
   if (n_seg == 0) return MB_OK;
-  k_segment_sum_scalar<<<row_grid(n_seg), RW_THREADS, 0, STREAM>>>(n_seg, seg_ptr, x, out);
+  launch(k_segment_sum_scalar, row_grid(n_seg), RW_THREADS, 0, STREAM, n_seg, seg_ptr, x, out);
   MB_LAUNCH_CHECK("k_segment_sum_scalar");
   return MB_OK;
 }
