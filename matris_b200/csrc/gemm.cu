@@ -559,6 +559,7 @@ k_gemm_tc(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ TcMaps
 
 #include "gemm_persistent.cuh"
 #include "mlp_fused.cuh"
+#include "linear_tma.cuh"
 
 // 0: persistent tcgen05 3xBF16 (default), 1: fp32 SIMT, 2: one-tile-per-CTA tcgen05 3xTF32, 3: persistent tcgen05 3xTF32
 static int g_gemm_mode = 0;
@@ -637,6 +638,7 @@ static int device_config(int* n_sm) {
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_gemm_ps<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PS_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_gemm_ps<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PS_SMEM_BYTES));
+    MB_CUDA_CHECK(cudaFuncSetAttribute(k_linear, cudaFuncAttributeMaxDynamicSharedMemorySize, LN_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_GATED_FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_PLAIN_FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_GATED_BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
@@ -856,6 +858,42 @@ extern "C" int mb_gemm(const mb_gemm_desc* desc, void* stream_) {
         for (int s = 0; s < a.n_src && shared_a; ++s)
           shared_a = a.src[s].ptr == b.src[s].ptr && a.src[s].idx == b.src[s].idx && a.src[s].ld == b.src[s].ld &&
                      a.src[s].col == b.src[s].col && a.src[s].act == b.src[s].act;
+      }
+      // Outputs at their own rows and an A operand that is shared or 128 wide per block: the TMA kernel.  (Blocks of a wider
+      // shared A advance together, one accumulator region each, of which there are three.)
+      bool same_a = true, one_seg = true, direct = bf16;
+      for (int j = 0; j < desc->n_blocks; ++j) {
+        const mb_colblock& a = desc->blk[0], &b = desc->blk[j];
+        direct = direct && !b.out_idx && b.mode != MB_OUT_ATOMIC;
+        one_seg = one_seg && b.n_src == 1;
+        same_a = same_a && a.n_src == b.n_src;
+        for (int s = 0; s < a.n_src && same_a; ++s)
+          same_a = a.src[s].ptr == b.src[s].ptr && a.src[s].idx == b.src[s].idx && a.src[s].ld == b.src[s].ld &&
+                   a.src[s].col == b.src[s].col && a.src[s].act == b.src[s].act;
+      }
+      direct = direct && (same_a ? desc->blk[0].n_src == 1 || desc->n_blocks <= 3 : one_seg) && desc->n_rows <= 0x7fffff00LL;
+      if (direct) {
+        mb::LinMaps lm;
+        for (int j = 0; j < desc->n_blocks; ++j) {
+          const mb_colblock& b = desc->blk[j];
+          lm.w[j][0] = maps.m[j][0];
+          lm.w[j][1] = maps.m[j][1];
+          if (!same_a && !b.src[0].idx && (rc = mb::row_map(b.src[0].ptr + b.src[0].col, b.src[0].ld, 128, desc->n_rows, &lm.src[j])))
+            return rc;
+          if (b.gate && (rc = mb::row_map(b.gate + b.col_gate, b.ld_gate, 128, desc->n_rows, &lm.gate[j]))) return rc;
+          if (b.res && (rc = mb::row_map(b.res + b.col_res, b.ld_res, 128, desc->n_rows, &lm.res[j]))) return rc;
+          if ((rc = mb::row_map(b.out + b.col_out, b.ld_out, 128, desc->n_rows, &lm.out[j]))) return rc;
+        }
+        for (int s = 0; s < desc->blk[0].n_src && same_a; ++s) {
+          const mb_src& r = desc->blk[0].src[s];
+          if (!r.idx && (rc = mb::row_map(r.ptr + r.col, r.ld, 128, desc->n_rows, &lm.src[s]))) return rc;
+        }
+        const int split = n_tiles <= n_sm ? 1 : 0;
+        const long long items = split ? n_tiles : gx;
+        mb::launch(mb::k_linear, (unsigned)(items < n_sm ? items : n_sm), mb::LN_THREADS, mb::LN_SMEM_BYTES,
+                   (cudaStream_t)stream_, *desc, lm, same_a ? 1 : 0, split);
+        MB_LAUNCH_CHECK("k_linear");
+        return MB_OK;
       }
       const long long n_items = shared_a ? gx : n_tiles;
       const unsigned grid = (unsigned)(n_items < n_sm ? n_items : n_sm);

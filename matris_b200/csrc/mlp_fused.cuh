@@ -606,29 +606,32 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
             const float4 v = lds4(patch + lane * 128 + ((j ^ (lane & 7)) << 4));
             x[4 * j] = v.x; x[4 * j + 1] = v.y; x[4 * j + 2] = v.z; x[4 * j + 3] = v.w;
           }
-          __syncwarp();  // the patch has been read: the next chunk may arrive
-          const int s2 = k == 0 ? s : (s + 1 < n_seg ? s + 1 : 0), t2 = k == 1 && s + 1 == n_seg ? t + 1 : t;
-          if (t2 < n_tiles && is_direct(s2)) request(t2, s2, k ^ 1);
-          const uint32_t ab = g & 3, ta = lane_base + ML_A_BASE + 32u * ab;
           if (act) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) x[i] = silu_fast_f(x[i]);
           }
+          uint32_t hi[2][8], lo[2][8];
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
             float sx[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) sx[i] = x[16 * hh + i];
-            uint32_t hi[8], lo[8];
-            split_bf16(sx, hi, lo);
-            if (hh == 0) {
-              if (g >= 4 && alive) alive = mbar_wait(a_done + 8 * ab, ((g >> 2) - 1) & 1);  // A buffer ab is free again
-              alive = __all_sync(0xffffffffu, alive);
-              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            }
-            MB_TMEM_ST8(ta + 8 * hh, hi);
-            MB_TMEM_ST8(ta + 16 + 8 * hh, lo);
+            split_bf16(sx, hi[hh], lo[hh]);
           }
+          const uint32_t ab = g & 3, ta = lane_base + ML_A_BASE + 32u * ab;
+          if (g >= 4 && alive) alive = mbar_wait(a_done + 8 * ab, ((g >> 2) - 1) & 1);  // A buffer ab is free again
+          alive = __all_sync(0xffffffffu, alive);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {
+            MB_TMEM_ST8(ta + 8 * hh, hi[hh]);
+            MB_TMEM_ST8(ta + 16 + 8 * hh, lo[hh]);
+          }
+          // Every lane has used the values it read from the patch (the stores above depend on them): only now may the copy of the
+          // next chunk overwrite it.  Issued right after the reads it could overtake them.
+          __syncwarp();
+          const int s2 = k == 0 ? s : (s + 1 < n_seg ? s + 1 : 0), t2 = k == 1 && s + 1 == n_seg ? t + 1 : t;
+          if (t2 < n_tiles && is_direct(s2)) request(t2, s2, k ^ 1);
           asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
