@@ -94,85 +94,83 @@ __global__ void k_gate_bwd(int64_t n_rows, const float* __restrict__ z, const fl
 }
 
 // ------------------------------------------------------------------ attention aggregation
-// warp per node; side 0: target segment (contiguous rows), side 1: source segment (through perm)
+// One (node, side) per WARPS warps: side 0 the target segment (contiguous rows), side 1 the source segment (through perm).  A warp
+// takes batches of eight rows whose index and data loads are issued together and keeps a running maximum, so that every row is read
+// once whatever the segment's length; WARPS = 4 splits the long segments of an atom graph (30 - 80 edges), which a warp alone would
+// walk for tens of microseconds, and joins the partial softmax sums in shared memory.
+// Latency of the gathered rows bounds it.  9372 atoms / 234,096 edges: 357 -> 294 us (WARPS = 8: 379, blocks too short lived); bonds,
+// about 4 rows a segment: 125 -> 101 us.  Both measured against one warp per segment walking it in two passes.
+template <int WARPS>
 __global__ void k_seg_attn_fwd(int n_nodes, const int32_t* __restrict__ tgt_ptr, const int32_t* __restrict__ src_ptr,
                                const int32_t* __restrict__ src_perm, const int32_t* __restrict__ emap,
                                const float* __restrict__ logits, const float* __restrict__ h,
                                float* __restrict__ agg_t, float* __restrict__ agg_s, float* __restrict__ stats) {
   pdl_sync();
-  MB_ROW_PROLOGUE(n_nodes)
-  constexpr int NB = 8;  // rows in flight per warp: their index and data loads are issued together
+  constexpr int NB = 8;
+  __shared__ float4 part[WARPS > 1 ? 3 : 1][WARPS > 1 ? WARPS : 1][WARPS > 1 ? 32 : 1];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = lane * 4;
+  const int64_t item = WARPS > 1 ? (int64_t)blockIdx.x : ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t row = item >> 1;
+  const int side = (int)(item & 1);
+  if (row >= n_nodes) return;
+  const int32_t* ptr = side == 0 ? tgt_ptr : src_ptr;
+  const int q0 = ptr[row], q1 = ptr[row + 1];
+  const int lcol = side == 0 ? 128 : 0;
+  float4 mx = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+  float4 s = zero4(), acc = zero4();
+  for (int q = q0 + (WARPS > 1 ? w * NB : 0); q < q1; q += NB * WARPS) {
+    int64_t r[NB], er[NB];
 #pragma unroll
-  for (int side = 0; side < 2; ++side) {
-    const int32_t* ptr = side == 0 ? tgt_ptr : src_ptr;
-    const int q0 = ptr[row], q1 = ptr[row + 1];
-    const int lcol = side == 0 ? 128 : 0;
-    auto rows_of = [&](int q, int64_t (&r)[NB], int64_t (&er)[NB]) {
+    for (int i = 0; i < NB; ++i) {  // rows past the end repeat the last one
+      const int qq = q + i < q1 ? q + i : q1 - 1;
+      r[i] = side == 0 ? qq : src_perm[qq];
+    }
 #pragma unroll
-      for (int i = 0; i < NB; ++i) {
-        const int qq = q + i < q1 ? q + i : q1 - 1;
-        r[i] = side == 0 ? qq : src_perm[qq];
-      }
+    for (int i = 0; i < NB; ++i) er[i] = emap ? emap[r[i]] : r[i];
+    float4 x[NB], hv[NB];
 #pragma unroll
-      for (int i = 0; i < NB; ++i) er[i] = emap ? emap[r[i]] : r[i];
-    };
-    float4 mx = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
-    float4 s = zero4(), acc = zero4();
-    if (q1 - q0 <= NB) {  // the common case: the whole segment is held in registers, every row is read once
-      if (q1 > q0) {
-        int64_t r[NB], er[NB];
-        rows_of(q0, r, er);
-        float4 x[NB], hv[NB];
+    for (int i = 0; i < NB; ++i) x[i] = ld4(logits + er[i] * 256 + lcol + c);
 #pragma unroll
-        for (int i = 0; i < NB; ++i) x[i] = ld4(logits + er[i] * 256 + lcol + c);
+    for (int i = 0; i < NB; ++i) hv[i] = ld4(h + r[i] * 128 + c);
+    float4 m = mx;
 #pragma unroll
-        for (int i = 0; i < NB; ++i) hv[i] = ld4(h + r[i] * 128 + c);
+    for (int i = 0; i < NB; ++i) m = max4(m, x[i]);
+    if (q >= q0 + NB * WARPS) {  // a later batch: what has been summed so far was relative to the old maximum
+      const float4 f = exp4(sub4(mx, m));
+      s = mul4(s, f);
+      acc = mul4(acc, f);
+    }
+    mx = m;
 #pragma unroll
-        for (int i = 0; i < NB; ++i) mx = max4(mx, x[i]);  // rows past the end repeat the last one
-#pragma unroll
-        for (int i = 0; i < NB; ++i) {
-          if (q0 + i < q1) {
-            const float4 e = exp4(sub4(x[i], mx));
-            s = add4(s, e);
-            acc = fma4(e, hv[i], acc);
-          }
-        }
-      }
-    } else {
-      for (int q = q0; q < q1; q += NB) {
-        int64_t r[NB], er[NB];
-        rows_of(q, r, er);
-        float4 x[NB];
-#pragma unroll
-        for (int i = 0; i < NB; ++i) x[i] = ld4(logits + er[i] * 256 + lcol + c);
-#pragma unroll
-        for (int i = 0; i < NB; ++i) mx = max4(mx, x[i]);
-      }
-      for (int q = q0; q < q1; q += NB) {
-        int64_t r[NB], er[NB];
-        rows_of(q, r, er);
-        float4 x[NB], hv[NB];
-#pragma unroll
-        for (int i = 0; i < NB; ++i) x[i] = ld4(logits + er[i] * 256 + lcol + c);
-#pragma unroll
-        for (int i = 0; i < NB; ++i) hv[i] = ld4(h + r[i] * 128 + c);
-#pragma unroll
-        for (int i = 0; i < NB; ++i) {
-          if (q + i < q1) {
-            const float4 e = exp4(sub4(x[i], mx));
-            s = add4(s, e);
-            acc = fma4(e, hv[i], acc);
-          }
-        }
+    for (int i = 0; i < NB; ++i) {
+      if (q + i < q1) {
+        const float4 e = exp4(sub4(x[i], mx));
+        s = add4(s, e);
+        acc = fma4(e, hv[i], acc);
       }
     }
-    float4 inv = zero4();
-    if (q1 > q0) inv = make_float4(1.f / s.x, 1.f / s.y, 1.f / s.z, 1.f / s.w);
-    else mx = zero4();
-    st4((side == 0 ? agg_t : agg_s) + row * 128 + c, mul4(acc, inv));
-    st4(stats + row * 512 + side * 256 + c, mx);
-    st4(stats + row * 512 + side * 256 + 128 + c, inv);
   }
+  if (WARPS > 1) {
+    part[0][w][lane] = mx;
+    part[1][w][lane] = s;
+    part[2][w][lane] = acc;
+    __syncthreads();
+    if (w > 0) return;
+    const int used = (q1 - q0 + NB - 1) / NB < WARPS ? (q1 - q0 + NB - 1) / NB : WARPS;  // warps that had rows
+    for (int k = 1; k < used; ++k) mx = max4(mx, part[0][k][lane]);
+    s = acc = zero4();
+    for (int k = 0; k < used; ++k) {
+      const float4 f = exp4(sub4(part[0][k][lane], mx));
+      s = fma4(f, part[1][k][lane], s);
+      acc = fma4(f, part[2][k][lane], acc);
+    }
+  }
+  float4 inv = zero4();
+  if (q1 > q0) inv = make_float4(1.f / s.x, 1.f / s.y, 1.f / s.z, 1.f / s.w);
+  else mx = zero4();
+  st4((side == 0 ? agg_t : agg_s) + row * 128 + c, mul4(acc, inv));
+  st4(stats + row * 512 + side * 256 + c, mx);
+  st4(stats + row * 512 + side * 256 + 128 + c, inv);
 }
 
 __global__ void k_seg_attn_bwd(int64_t n_rows, const int32_t* __restrict__ tgt, const int32_t* __restrict__ src,
@@ -205,22 +203,44 @@ __global__ void k_seg_attn_bwd(int64_t n_rows, const int32_t* __restrict__ tgt, 
 }
 
 // ------------------------------------------------------------------ refinement aggregation
+// WARPS warps per node as in k_seg_attn_fwd (eight: a row costs less here), four rows of a warp in flight: 86 -> 65 us on average over
+// both graphs of 9372 atoms / 522,844 angles
+template <int WARPS>
 __global__ void k_seg_smooth_sum_fwd(int n_nodes, const int32_t* __restrict__ tgt_ptr,
                                      const int32_t* __restrict__ emap, const int32_t* __restrict__ src,
                                      int idx_stride, const float* __restrict__ env, const float* __restrict__ h,
                                      float* __restrict__ agg) {
   pdl_sync();
-  MB_ROW_PROLOGUE(n_nodes)
+  constexpr int NB = 4;
+  __shared__ float4 part[WARPS > 1 ? WARPS : 1][WARPS > 1 ? 32 : 1];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = lane * 4;
+  const int64_t row = WARPS > 1 ? (int64_t)blockIdx.x : ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (row >= n_nodes) return;
   const int q0 = tgt_ptr[row], q1 = tgt_ptr[row + 1];
   float4 acc = zero4();
-  float4 env_n = zero4();
-  if (src && q1 > q0) env_n = ld4(env + row * 128 + c);
-  for (int64_t r = q0; r < q1; ++r) {
-    float4 s;
-    if (src) s = mul4(ld4(env + (int64_t)src[r * idx_stride] * 128 + c), env_n);
-    else s = ld4(env + (int64_t)emap[r] * 128 + c);
-    acc = add4(acc, mul4(ld4(h + r * 128 + c), s));
+  for (int q = q0 + (WARPS > 1 ? w * NB : 0); q < q1; q += NB * WARPS) {
+    int64_t er[NB];
+    float4 hv[NB], ev[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int64_t r = q + i < q1 ? q + i : q1 - 1;
+      er[i] = src ? src[r * idx_stride] : emap[r];
+      hv[i] = ld4(h + r * 128 + c);
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i) ev[i] = ld4(env + er[i] * 128 + c);
+#pragma unroll
+    for (int i = 0; i < NB; ++i)
+      if (q + i < q1) acc = fma4(hv[i], ev[i], acc);
   }
+  if (WARPS > 1) {
+    part[w][lane] = acc;
+    __syncthreads();
+    if (w > 0) return;
+#pragma unroll
+    for (int k = 1; k < WARPS; ++k) acc = add4(acc, part[k][lane]);
+  }
+  if (src && q1 > q0) acc = mul4(acc, ld4(env + row * 128 + c));  // line graph: s = env[src] * env[target]
   st4(agg + row * 128 + c, acc);
 }
 
@@ -273,18 +293,41 @@ __global__ void k_smooth_env_bwd_line(int n_nodes, const int32_t* __restrict__ t
                                       const float* __restrict__ dagg, float* __restrict__ denv) {
   pdl_sync();
   MB_ROW_PROLOGUE(n_nodes)
+  constexpr int NB = 4;  // rows in flight
   float4 acc = zero4();
   const int q0 = tgt_ptr[row], q1 = tgt_ptr[row + 1];
-  if (q1 > q0) {
-    float4 inner = zero4();
-    for (int64_t r = q0; r < q1; ++r)
-      inner = fma4(ld4(h + r * 128 + c), ld4(env + (int64_t)src[r * idx_stride] * 128 + c), inner);
-    acc = mul4(ld4(dagg + row * 128 + c), inner);
+  for (int q = q0; q < q1; q += NB) {
+    float4 hv[NB], ev[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int64_t r = q + i < q1 ? q + i : q1 - 1;
+      ev[i] = ld4(env + (int64_t)src[r * idx_stride] * 128 + c);
+      hv[i] = ld4(h + r * 128 + c);
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i)
+      if (q + i < q1) acc = fma4(hv[i], ev[i], acc);
   }
-  for (int q = src_ptr[row]; q < src_ptr[row + 1]; ++q) {
-    const int64_t r = src_perm[q];
-    const int64_t nt = tgt[r * idx_stride];
-    acc = add4(acc, mul4(mul4(ld4(dagg + nt * 128 + c), ld4(h + r * 128 + c)), ld4(env + nt * 128 + c)));
+  if (q1 > q0) acc = mul4(ld4(dagg + row * 128 + c), acc);
+  const int s0 = src_ptr[row], s1 = src_ptr[row + 1];
+  for (int q = s0; q < s1; q += NB) {
+    int64_t r[NB], nt[NB];
+    float4 gv[NB], hv[NB], ev[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) r[i] = src_perm[q + i < s1 ? q + i : s1 - 1];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      nt[i] = tgt[r[i] * idx_stride];
+      hv[i] = ld4(h + r[i] * 128 + c);
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      gv[i] = ld4(dagg + nt[i] * 128 + c);
+      ev[i] = ld4(env + nt[i] * 128 + c);
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i)
+      if (q + i < s1) acc = fma4(mul4(gv[i], hv[i]), ev[i], acc);
   }
   st4(denv + row * 128 + c, acc);
 }
@@ -571,8 +614,13 @@ extern "C" int mb_seg_attn_fwd(int32_t n_nodes, const int32_t* tgt_ptr, const in
                                float* agg_t, float* agg_s, float* stats, void* stream) {
   MB_REQUIRE(n_nodes >= 0 && tgt_ptr && src_ptr && src_perm && logits && h && agg_t && agg_s && stats);
   if (n_nodes == 0) return MB_OK;
-  launch(k_seg_attn_fwd, row_grid(n_nodes), RW_THREADS, 0, STREAM, n_nodes, tgt_ptr, src_ptr, src_perm, emap, logits, h,
-                                                              agg_t, agg_s, stats);
+  // with an edge map the rows are directed edges and the nodes atoms: long segments
+  if (emap)
+    launch(k_seg_attn_fwd<4>, 2 * (unsigned)n_nodes, 128, 0, STREAM, n_nodes, tgt_ptr, src_ptr, src_perm, emap, logits, h, agg_t,
+           agg_s, stats);
+  else
+    launch(k_seg_attn_fwd<1>, row_grid(2 * (int64_t)n_nodes), RW_THREADS, 0, STREAM, n_nodes, tgt_ptr, src_ptr, src_perm, emap,
+           logits, h, agg_t, agg_s, stats);
   MB_LAUNCH_CHECK("k_seg_attn_fwd");
   return MB_OK;
 }
@@ -598,8 +646,11 @@ extern "C" int mb_seg_smooth_sum_fwd(int32_t n_nodes, const int32_t* tgt_ptr, co
                                      float* agg, void* stream) {
   MB_REQUIRE(n_nodes >= 0 && tgt_ptr && (emap || src) && env && h && agg && idx_stride > 0);
   if (n_nodes == 0) return MB_OK;
-  launch(k_seg_smooth_sum_fwd, row_grid(n_nodes), RW_THREADS, 0, STREAM, n_nodes, tgt_ptr, emap, src, idx_stride, env, h,
-                                                                    agg);
+  if (!src)
+    launch(k_seg_smooth_sum_fwd<8>, (unsigned)n_nodes, 256, 0, STREAM, n_nodes, tgt_ptr, emap, src, idx_stride, env, h, agg);
+  else
+    launch(k_seg_smooth_sum_fwd<1>, row_grid(n_nodes), RW_THREADS, 0, STREAM, n_nodes, tgt_ptr, emap, src, idx_stride, env, h,
+           agg);
   MB_LAUNCH_CHECK("k_seg_smooth_sum_fwd");
   return MB_OK;
 }
