@@ -31,6 +31,10 @@
 // r+1 as soon as L2 gate(t) is done, under the epilogue of t.  GATED_BWD: 0, 1 and 2.  PLAIN_*: tiles alternate between the
 // two epilogue groups, L1(t) -> 2t mod 3, L2(t) -> 2t+1 mod 3, issued L1(t+1) before L2(t).
 //
+// Measured, 573,894 rows with z1 and z2 kept: two addends and a residual 0.57 ms, three addends 0.54 (nothing kept: 0.43), no
+// contraction and three addends 0.48, K = 384 gathered with a residual 0.64; GATED_BWD with a residual 0.43, with E too 0.61; FFN
+// forward 0.22, backward 0.19.  One tile alone takes 30 us forward, 22 us backward: the chain of its stages.
+//
 // Warps: 0 MMA, 1 TMA (weights, 16 KB tiles of 64 K values, five slots), 2-9 producers, 10-17 epilogue (two groups of four; the
 // group's branch or tile parity, the warp's lane quarter).  Every mbarrier wait is bounded; on expiry the status word is set, the
 // role stops waiting and runs to the common exit.  Every waiter sees every phase of a barrier it waits on.
@@ -97,6 +101,11 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t pa
                :: "l"(reinterpret_cast<uint64_t>(map)), "r"(patch), "r"(x), "r"(y) : "memory");
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
+// rows y.., columns x.. of a tensor -> patch (one lane)
+__device__ __forceinline__ void load_patch(const CUtensorMap* map, uint32_t patch, uint32_t bar, int x, int y) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(ML_PATCH) : "memory");
+  tma_load_2d(patch, map, bar, x, y);
+}
 __device__ __forceinline__ void tmem_get(uint32_t addr, float (&x)[32]) {
   uint32_t v[32];
   MB_TMEM_LD32(addr, v);
@@ -105,10 +114,25 @@ __device__ __forceinline__ void tmem_get(uint32_t addr, float (&x)[32]) {
   for (int i = 0; i < 32; ++i) x[i] = __uint_as_float(v[i]);
 }
 
+// SiLU(a) sigmoid(b) = a / ((1 + e^-a) (1 + e^-b)): one reciprocal for both (the special-function pipe, a quarter of the rate of
+// the others, bounds this pass)
+__device__ __forceinline__ float gated_value(float a, float b) {
+  float ea, eb, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(ea) : "f"(a * -1.442695041f));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(eb) : "f"(b * -1.442695041f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((1.0f + ea) * (1.0f + eb)));
+  return a * r;
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(ML_THREADS, 1)
 k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
   constexpr bool GATED = MODE == MLP_GATED_FWD || MODE == MLP_GATED_BWD;
+  // Who asks for the residual's patches, which follow a tile's side patches in the same two buffers.  GATED_FWD: the epilogue warp
+  // itself when it is done with what a buffer held; left to the producer, whose addends are a latency-bound gather, the chunks of
+  // the next tile wait for that (0.65 against 0.59 ms for 573,894 rows).  The others: the producer (their epilogue is the busier side:
+  // 0.61 against 0.62 ms backward).
+  constexpr bool EPI_RES = MODE == MLP_GATED_FWD;
   constexpr bool FWD = MODE == MLP_GATED_FWD || MODE == MLP_PLAIN_FWD;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + ML_BAR_OFF);
@@ -358,6 +382,13 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
       __syncwarp();
       if (lane == 0 && alive && row0 < n_rows) tma_store_2d(map, stage, x, row0);
     };
+    uint32_t asked = 0;  // number after that of the last copy asked for
+    auto request = [&](uint32_t n, int k, int row0) {  // residual patch k (EPI_RES)
+      if (!alive) return;
+      asked = n + 1;
+      if (lane == 0)
+        load_patch(&maps.res, side0 + (n & 1) * ML_PATCH, my_full + 8 * (n & 1), 64 * grp + 32 * k, row0);
+    };
     // finished columns `col`..: h = v and / or out2 = v + res_w * res (the residual rows arrive as a side patch)
     auto finish = [&](float (&v)[32], int col, int row0) {
       if (d.h) write(&maps.h, v, col, row0);
@@ -372,7 +403,7 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
           v[4 * j + 2] = fmaf(w.z, x.z, v[4 * j + 2]); v[4 * j + 3] = fmaf(w.w, x.w, v[4 * j + 3]);
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(my_empty + 8 * (side_n & 1));
+        if ((has_side || !EPI_RES) && lane == 0) mbar_arrive(my_empty + 8 * (side_n & 1));
         ++side_n;
         write(&maps.out2, v, col, row0);
       }
@@ -391,6 +422,10 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
       } else {
         reg_a = (uint32_t)(2 * t) % 3u;
         reg_d = (uint32_t)(2 * t + 1) % 3u;
+      }
+      if (EPI_RES && has_res && !has_side) {
+        request(side_n, 0, row0);
+        request(side_n + 1, 1, row0);
       }
       // ------------------------------------------------ mid
       wait(d1_full + 8 * grp, par);
@@ -429,9 +464,11 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
             x[4 * j + 2] *= s * silu_grad_fast_f(v.z); x[4 * j + 3] *= s * silu_grad_fast_f(v.w);
           }
         }
-        if (has_side) {  // the side patch goes back to its producer
-          __syncwarp();
-          if (lane == 0) mbar_arrive(my_empty + 8 * (side_n & 1));
+        if (has_side) {
+          if (!EPI_RES || c < 2 || !has_res) {  // the side patch goes back to its producer
+            __syncwarp();
+            if (lane == 0) mbar_arrive(my_empty + 8 * (side_n & 1));
+          }
           ++side_n;
         }
 #pragma unroll
@@ -448,6 +485,7 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(mid_ready + 8 * (4 * grp + c));
+        if (EPI_RES && has_side && has_res && c >= 2) request(side_n + 1, c - 2, row0);
         if (d.z1) write(&maps.z1, x, 128 * br + 32 * c, row0);
       }
       if constexpr (MODE == MLP_GATED_FWD) {
@@ -484,11 +522,9 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
           tmem_get(core + 32u * j2, y);
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const float4 b = b2s[c4 + j], n = nws[c4 + j];
-            y[4 * j] = silu_fast_f((y[4 * j] + b.x) * rc * n.x);
-            y[4 * j + 1] = silu_fast_f((y[4 * j + 1] + b.y) * rc * n.y);
-            y[4 * j + 2] = silu_fast_f((y[4 * j + 2] + b.z) * rc * n.z);
-            y[4 * j + 3] = silu_fast_f((y[4 * j + 3] + b.w) * rc * n.w);
+            const float4 bc = b2s[c4 + j], nc = nws[c4 + j];
+            y[4 * j] = (y[4 * j] + bc.x) * (rc * nc.x); y[4 * j + 1] = (y[4 * j + 1] + bc.y) * (rc * nc.y);
+            y[4 * j + 2] = (y[4 * j + 2] + bc.z) * (rc * nc.z); y[4 * j + 3] = (y[4 * j + 3] + bc.w) * (rc * nc.w);
           }
           float z[32];
           tmem_get(gate + 32u * j2, z);
@@ -499,11 +535,11 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
           }
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const float4 b = b2s[32 + c4 + j], n = nws[32 + c4 + j];
-            y[4 * j] *= sigmoid_fast_f((z[4 * j] + b.x) * rg * n.x);
-            y[4 * j + 1] *= sigmoid_fast_f((z[4 * j + 1] + b.y) * rg * n.y);
-            y[4 * j + 2] *= sigmoid_fast_f((z[4 * j + 2] + b.z) * rg * n.z);
-            y[4 * j + 3] *= sigmoid_fast_f((z[4 * j + 3] + b.w) * rg * n.w);
+            const float4 bg = b2s[32 + c4 + j], ng = nws[32 + c4 + j];
+            y[4 * j] = gated_value(y[4 * j], (z[4 * j] + bg.x) * (rg * ng.x));
+            y[4 * j + 1] = gated_value(y[4 * j + 1], (z[4 * j + 1] + bg.y) * (rg * ng.y));
+            y[4 * j + 2] = gated_value(y[4 * j + 2], (z[4 * j + 2] + bg.z) * (rg * ng.z));
+            y[4 * j + 3] = gated_value(y[4 * j + 3], (z[4 * j + 3] + bg.w) * (rg * ng.w));
           }
           finish(y, 64 * grp + 32 * j2, row0);
         }
@@ -534,6 +570,9 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
         }
       }
     }
+    if (EPI_RES && !alive) {  // failure path only: no copy may still be in flight when the CTA's shared memory is released
+      for (uint32_t n = asked >= 2 ? asked - 2 : 0; n < asked; ++n) mbar_wait(my_full + 8 * (n & 1), (n >> 1) & 1);
+    }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   } else {
     // ---------------------------------------------------------------- producers
@@ -552,10 +591,6 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
       sts4(p + ((i & 1) ? put_odd : put_even) + 512u * i, v.x, v.y, v.z, v.w);
     };
     auto tile_row = [&](int t) { return (first_rt + t * step_rt) * 128 + quarter * 32; };
-    auto load_patch = [&](const CUtensorMap* map, uint32_t dst, uint32_t bar, int x, int y) {  // one lane
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(ML_PATCH) : "memory");
-      tma_load_2d(dst, map, bar, x, y);
-    };
     auto is_direct = [&](int s) { return (s < d.n_src ? d.src[s].idx : d.ext[s - d.n_src].idx) == nullptr; };
     auto request = [&](int t, int s, int k) {  // rows read in place: this warp's chunk k of segment s
       if (lane == 0 && alive)
@@ -572,6 +607,50 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
         if (lane == 0 && alive)
           load_patch(&maps.res, side0 + (side_n & 1) * ML_PATCH, side_full + 8 * (2 * pw + (side_n & 1)),
                      (GATED ? 64 * parity : 0) + 32 * c, tile_row(t));
+      }
+    };
+    // Addend sums of a tile.  The loads are latency bound, so as many as fit in the registers are requested together: three addends
+    // half a patch (16 rows) at a time (0.58 -> 0.54 ms for 573,894 rows), fewer one after the other with the whole patch each (two at
+    // once by halves: 0.68 instead of 0.60 ms).
+    auto gather = [&](auto count, int t, int col0) {
+      constexpr int N = decltype(count)::value, ROWS = N == 3 ? 4 : 8, AT_ONCE = N == 3 ? 3 : 1;
+      const int64_t row0 = tile_row(t);
+      int32_t ix[N][8];
+#pragma unroll
+      for (int a = 0; a < N; ++a)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int64_t r = row0 + lr + 4 * i < n_rows ? row0 + lr + 4 * i : n_rows - 1;
+          ix[a][i] = d.add[a].idx ? d.add[a].idx[r] : (int32_t)r;
+        }
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c, ++side_n) {
+        const int col = col0 + 32 * c + lc * 4;
+        const float4 b = reinterpret_cast<const float4*>(cst)[col >> 2];
+#pragma unroll
+        for (int i0 = 0; i0 < 8; i0 += ROWS) {
+          float4 sum[ROWS];
+#pragma unroll
+          for (int a0 = 0; a0 < N; a0 += AT_ONCE) {
+            float4 v[AT_ONCE][ROWS];
+#pragma unroll
+            for (int a = 0; a < AT_ONCE; ++a)
+#pragma unroll
+              for (int i = 0; i < ROWS; ++i) v[a][i] = ld4(d.add[a0 + a].ptr + (int64_t)ix[a0 + a][i0 + i] * d.add[a0 + a].ld + col);
+#pragma unroll
+            for (int a = 0; a < AT_ONCE; ++a)
+#pragma unroll
+              for (int i = 0; i < ROWS; ++i) {
+                const float4 o = a0 + a == 0 ? b : sum[i];
+                sum[i] = make_float4(o.x + v[a][i].x, o.y + v[a][i].y, o.z + v[a][i].z, o.w + v[a][i].w);
+              }
+          }
+          if (i0 == 0) wait_empty();
+#pragma unroll
+          for (int i = 0; i < ROWS; ++i) put(side0 + (side_n & 1) * ML_PATCH, i0 + i, sum[i]);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(side_full + 8 * (2 * pw + (side_n & 1)));
       }
     };
     if (n_seg > 0 && is_direct(0)) request(0, 0, 0);
@@ -648,37 +727,9 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
       if (has_side) {
         const int col0 = GATED ? 128 * parity : 0;
         if constexpr (FWD) {
-          int32_t ix[3][8];
-#pragma unroll
-          for (int a = 0; a < 3; ++a)
-            if (a < d.n_add) {
-#pragma unroll
-              for (int i = 0; i < 8; ++i) ix[a][i] = d.add[a].idx ? d.add[a].idx[row_of(i)] : (int32_t)row_of(i);
-            }
-#pragma unroll 1
-          for (int c = 0; c < 4; ++c, ++side_n) {
-            const int col = col0 + 32 * c + lc * 4;
-            float4 sum[8];
-            const float4 b = reinterpret_cast<const float4*>(cst)[col >> 2];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) sum[i] = ld4(d.add[0].ptr + (int64_t)ix[0][i] * d.add[0].ld + col);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) { sum[i].x += b.x; sum[i].y += b.y; sum[i].z += b.z; sum[i].w += b.w; }
-#pragma unroll
-            for (int a = 1; a < 3; ++a)
-              if (a < d.n_add) {
-                float4 v[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = ld4(d.add[a].ptr + (int64_t)ix[a][i] * d.add[a].ld + col);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) { sum[i].x += v[i].x; sum[i].y += v[i].y; sum[i].z += v[i].z; sum[i].w += v[i].w; }
-              }
-            wait_empty();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) put(side0 + (side_n & 1) * ML_PATCH, i, sum[i]);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(side_full + 8 * (2 * pw + (side_n & 1)));
-          }
+          if (d.n_add == 1) gather(std::integral_constant<int, 1>{}, t, col0);
+          else if (d.n_add == 2) gather(std::integral_constant<int, 2>{}, t, col0);
+          else gather(std::integral_constant<int, 3>{}, t, col0);
         } else {
           for (int c = 0; c < 4; ++c, ++side_n) {
             wait_empty();
@@ -688,12 +739,13 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
           }
         }
       }
-      if (GATED) residual(t);
+      if (MODE == MLP_GATED_BWD) residual(t);
     }
     if (!GATED && ((n_tiles - 1) & 1) == parity) residual(n_tiles - 1);
     if (!alive) {  // failure path only: no copy may still be in flight when the CTA's shared memory is released
       if (n_seg > 0) mbar_wait(my_conv, conv_n & 1);
-      for (uint32_t n = side_n >= 2 ? side_n - 2 : 0; n < side_n; ++n) mbar_wait(side_full + 8 * (2 * pw + (n & 1)), (n >> 1) & 1);
+      if (!EPI_RES)
+        for (uint32_t n = side_n >= 2 ? side_n - 2 : 0; n < side_n; ++n) mbar_wait(side_full + 8 * (2 * pw + (n & 1)), (n >> 1) & 1);
     }
   }
 
