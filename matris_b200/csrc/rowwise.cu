@@ -76,9 +76,10 @@ __device__ __forceinline__ void gate_bwd_row(int64_t row, int c, const float* __
   const float gv[4] = {g.x, g.y, g.z, g.w}, wcv[4] = {gwc.x, gwc.y, gwc.z, gwc.w}, wgv[4] = {gwg.x, gwg.y, gwg.z, gwg.w};
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const float core = silu_f(ycv[k]), gate = sigmoid_f(ygv[k]);
-    dnc[k] = gv[k] * gate * silu_grad_f(ycv[k]) * wcv[k];
-    dng[k] = gv[k] * core * gate * (1.f - gate) * wgv[k];
+    const float s = sigmoid_f(ycv[k]), gate = sigmoid_f(ygv[k]);
+    const float core = ycv[k] * s, gg = gv[k] * gate;
+    dnc[k] = gg * (s * (1.f + ycv[k] * (1.f - s))) * wcv[k];
+    dng[k] = gg * core * (1.f - gate) * wgv[k];
   }
   const float4 dn_c = make_float4(dnc[0], dnc[1], dnc[2], dnc[3]), dn_g = make_float4(dng[0], dng[1], dng[2], dng[3]);
   const float mc = warp_sum(dot4(dn_c, nc)) * (1.f / 128.f), mg = warp_sum(dot4(dn_g, ng)) * (1.f / 128.f);
@@ -95,18 +96,19 @@ __global__ void k_gate_bwd(int64_t n_rows, const float* __restrict__ z, const fl
 
 // ------------------------------------------------------------------ attention aggregation
 // One (node, side) per WARPS warps: side 0 the target segment (contiguous rows), side 1 the source segment (through perm).  A warp
-// takes batches of eight rows whose index and data loads are issued together and keeps a running maximum, so that every row is read
+// takes batches of rows whose index and data loads are issued together and keeps a running maximum, so that every row is read
 // once whatever the segment's length; WARPS = 4 splits the long segments of an atom graph (30 - 80 edges), which a warp alone would
 // walk for tens of microseconds, and joins the partial softmax sums in shared memory.
-// Latency of the gathered rows bounds it.  9372 atoms / 234,096 edges: 357 -> 294 us (WARPS = 8: 379, blocks too short lived); bonds,
-// about 4 rows a segment: 125 -> 101 us.  Both measured against one warp per segment walking it in two passes.
+// Latency of the gathered rows bounds it.  Line graph of 117,048 bonds / 522,844 angles (4.5 rows a segment): 350 us with one warp
+// walking a segment in two passes, 295 with batches of eight rows, 233 with four (64 registers, twice the warps).  Atom graph of
+// 9372 atoms / 234,096 edges 103 -> 105 us (eight warps: 124), of 32 atoms a third of the time.
 template <int WARPS>
-__global__ void k_seg_attn_fwd(int n_nodes, const int32_t* __restrict__ tgt_ptr, const int32_t* __restrict__ src_ptr,
+__global__ void __launch_bounds__(WARPS == 1 ? RW_THREADS : 128, WARPS == 1 ? 4 : 5) k_seg_attn_fwd(int n_nodes, const int32_t* __restrict__ tgt_ptr, const int32_t* __restrict__ src_ptr,
                                const int32_t* __restrict__ src_perm, const int32_t* __restrict__ emap,
                                const float* __restrict__ logits, const float* __restrict__ h,
                                float* __restrict__ agg_t, float* __restrict__ agg_s, float* __restrict__ stats) {
   pdl_sync();
-  constexpr int NB = 8;
+  constexpr int NB = WARPS == 1 ? 4 : 8;
   __shared__ float4 part[WARPS > 1 ? 3 : 1][WARPS > 1 ? WARPS : 1][WARPS > 1 ? 32 : 1];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = lane * 4;
   const int64_t item = WARPS > 1 ? (int64_t)blockIdx.x : ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -173,7 +175,9 @@ __global__ void k_seg_attn_fwd(int n_nodes, const int32_t* __restrict__ tgt_ptr,
   st4(stats + row * 512 + side * 256 + 128 + c, inv);
 }
 
-__global__ void k_seg_attn_bwd(int64_t n_rows, const int32_t* __restrict__ tgt, const int32_t* __restrict__ src,
+// Latency of the gathered rows bounds it (5 TB/s of DRAM traffic at half occupancy): six blocks per SM, even with a few spills, beat
+// what 62 registers allow.  522,844 angles 579 -> 526 us, 234,096 edges 252 -> 229; eight blocks 557 and 242.
+__global__ void __launch_bounds__(RW_THREADS, 6) k_seg_attn_bwd(int64_t n_rows, const int32_t* __restrict__ tgt, const int32_t* __restrict__ src,
                                int idx_stride, const int32_t* __restrict__ emap, const float* __restrict__ logits,
                                const float* __restrict__ h, const float* __restrict__ agg_t,
                                const float* __restrict__ agg_s, const float* __restrict__ stats,
@@ -203,8 +207,8 @@ __global__ void k_seg_attn_bwd(int64_t n_rows, const int32_t* __restrict__ tgt, 
 }
 
 // ------------------------------------------------------------------ refinement aggregation
-// WARPS warps per node as in k_seg_attn_fwd (eight: a row costs less here), four rows of a warp in flight: 86 -> 65 us on average over
-// both graphs of 9372 atoms / 522,844 angles
+// WARPS warps per node as in k_seg_attn_fwd (eight: a row costs less here), four rows of a warp in flight: 124 -> 82 us for the line
+// graph of 522,844 angles, 47 us as before for the atom graph of 9372 atoms
 template <int WARPS>
 __global__ void k_seg_smooth_sum_fwd(int n_nodes, const int32_t* __restrict__ tgt_ptr,
                                      const int32_t* __restrict__ emap, const int32_t* __restrict__ src,
@@ -244,7 +248,9 @@ __global__ void k_seg_smooth_sum_fwd(int n_nodes, const int32_t* __restrict__ tg
   st4(agg + row * 128 + c, acc);
 }
 
-__global__ void k_seg_smooth_sum_bwd_rows(int64_t n_rows, const int32_t* __restrict__ tgt,
+// Bounded by latency like k_seg_attn_bwd; the exponentials of the gate's adjoint come next.  522,844 angles with the adjoint: one
+// sigmoid per branch instead of three in all 351 -> 301 us, eight blocks per SM 274 us; 234,096 edges 156 -> 125.
+__global__ void __launch_bounds__(RW_THREADS, 8) k_seg_smooth_sum_bwd_rows(int64_t n_rows, const int32_t* __restrict__ tgt,
                                           const int32_t* __restrict__ src, int idx_stride,
                                           const int32_t* __restrict__ emap, const float* __restrict__ env,
                                           const float* __restrict__ dagg, float* __restrict__ dh, int accumulate,
@@ -286,7 +292,8 @@ __global__ void k_mul_rows_gather(int64_t n_rows, const float* __restrict__ x, c
   st4(y + row * 128 + c, mul4(ld4(x + row * 128 + c), ld4(s + sr * 128 + c)));
 }
 
-__global__ void k_smooth_env_bwd_line(int n_nodes, const int32_t* __restrict__ tgt_ptr,
+// Four rows in flight and six blocks per SM (40 registers): 180 -> 121 us for 117,048 bonds / 522,844 angles (four blocks 156).
+__global__ void __launch_bounds__(RW_THREADS, 6) k_smooth_env_bwd_line(int n_nodes, const int32_t* __restrict__ tgt_ptr,
                                       const int32_t* __restrict__ src_ptr, const int32_t* __restrict__ src_perm,
                                       const int32_t* __restrict__ tgt, const int32_t* __restrict__ src,
                                       int idx_stride, const float* __restrict__ env, const float* __restrict__ h,
@@ -339,8 +346,9 @@ __global__ void k_smooth_env_bwd_line(int n_nodes, const int32_t* __restrict__ t
 // products with the weights then run once per node instead of scattering 128 finished columns per row.
 // WARPS warps share a segment: one for the line graph's short segments, eight for an atom's 30 - 80 edges, whose few
 // segments would otherwise be walked by a handful of warps.
+// 117,048 bonds 178 -> 162 us with four blocks per SM (five: 193, spilling), 9372 atoms 73 -> 62 with eight.
 template <int WARPS>
-__global__ void k_seg_sum(int n_nodes, const int32_t* __restrict__ tgt_ptr, const int32_t* __restrict__ src_ptr,
+__global__ void __launch_bounds__(256, WARPS == 1 ? 4 : 8) k_seg_sum(int n_nodes, const int32_t* __restrict__ tgt_ptr, const int32_t* __restrict__ src_ptr,
                           const int32_t* __restrict__ src_perm, const int32_t* __restrict__ ctr,
                           const float* __restrict__ x, float* __restrict__ out, float* __restrict__ ctr_out) {
   pdl_sync();
@@ -449,37 +457,77 @@ __global__ void k_scale_rows(int64_t n_rows, const float* __restrict__ x, const 
 }
 
 // ------------------------------------------------------------------ K <= 16 linear layers
-__global__ void k_small_linear_fwd(int64_t n_rows, int k, const float* __restrict__ x, const float* __restrict__ w,
-                                   float* __restrict__ y) {
-  pdl_sync();
-  __shared__ float ws[16][128];
+// A lane owns four of the 128 columns with their KP (k padded to 8 or 16) weights in registers, loaded once per warp, and a warp takes
+// 32 / KP rows at a time: a row is then KP broadcasts and 4 KP products.  (One row per warp with the weights in shared memory, set
+// up by every block of eight rows, cost more than the rows: 69 -> 27 us forward and 71 -> 28 backward, on average over the calls of
+// 522,844 angles and 117,048 bonds.)
+template <int KP>
+__device__ __forceinline__ void small_linear_weights(const float* __restrict__ w, int k, int c, float4 (&wr)[KP]) {
+  __shared__ float ws[KP][128];  // transposed, so that a warp reads its weights a row at a time
   for (int i = threadIdx.x; i < 128 * k; i += blockDim.x) ws[i % k][i / k] = w[i];
   __syncthreads();
-  MB_ROW_PROLOGUE(n_rows)
-  float4 acc = zero4();
-  for (int j = 0; j < k; ++j) {
-    const float xv = x[row * k + j];
-    acc = fma4(make_float4(xv, xv, xv, xv), ld4(&ws[j][c]), acc);
-  }
-  st4(y + row * 128 + c, acc);
+#pragma unroll
+  for (int j = 0; j < KP; ++j) wr[j] = j < k ? ld4(&ws[j][c]) : zero4();
 }
 
-__global__ void k_small_linear_bwd(int64_t n_rows, int k, const float* __restrict__ dy, const float* __restrict__ w,
-                                   float* __restrict__ dx, int accumulate) {
+template <int KP>
+__global__ void __launch_bounds__(RW_THREADS, KP == 8 ? 4 : 2)
+k_small_linear_fwd(int64_t n_rows, int k, const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y) {
+  constexpr int ROWS = 32 / KP;
+  const int lane = threadIdx.x & 31, c = lane * 4, ri = lane / KP, rj = lane % KP;
+  const int64_t step = ((int64_t)gridDim.x * blockDim.x >> 5) * ROWS;
+  float4 wr[KP];
   pdl_sync();
-  __shared__ float ws[16][128];
-  for (int i = threadIdx.x; i < 128 * k; i += blockDim.x) ws[i % k][i / k] = w[i];
-  __syncthreads();
-  MB_ROW_PROLOGUE(n_rows)
-  const float4 g = ld4(dy + row * 128 + c);
-  float mine = 0.f;
-  for (int j = 0; j < k; ++j) {
-    const float s = warp_sum(dot4(g, ld4(&ws[j][c])));
-    if (lane == j) mine = s;
+  small_linear_weights<KP>(w, k, c, wr);
+  for (int64_t r0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * ROWS; r0 < n_rows; r0 += step) {
+    const float xv = rj < k && r0 + ri < n_rows ? x[(r0 + ri) * k + rj] : 0.f;
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      float4 acc = zero4();
+#pragma unroll
+      for (int j = 0; j < KP; ++j) {
+        const float v = __shfl_sync(0xffffffffu, xv, r * KP + j);
+        acc = fma4(make_float4(v, v, v, v), wr[j], acc);
+      }
+      if (r0 + r < n_rows) st4(y + (r0 + r) * 128 + c, acc);
+    }
   }
-  if (lane < k) {
-    if (accumulate) mine += dx[row * k + lane];
-    dx[row * k + lane] = mine;
+}
+
+// dx = dy W: every lane's 32 partial sums (32 / KP rows x KP) are reduced across the warp by halving, 31 shuffles in all, which leaves
+// lane l with the sum number l = row * KP + j (reduced one by one they were 5 shuffles each).
+template <int KP>
+__global__ void __launch_bounds__(RW_THREADS, KP == 8 ? 3 : 2)
+k_small_linear_bwd(int64_t n_rows, int k, const float* __restrict__ dy, const float* __restrict__ w, float* __restrict__ dx,
+                   int accumulate) {
+  constexpr int ROWS = 32 / KP;
+  const int lane = threadIdx.x & 31, c = lane * 4, ri = lane / KP, rj = lane % KP;
+  const int64_t step = ((int64_t)gridDim.x * blockDim.x >> 5) * ROWS;
+  float4 wr[KP];
+  pdl_sync();
+  small_linear_weights<KP>(w, k, c, wr);
+  for (int64_t r0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * ROWS; r0 < n_rows; r0 += step) {
+    float4 g[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) g[r] = ld4(dy + (r0 + r < n_rows ? r0 + r : n_rows - 1) * 128 + c);
+    const bool mine = rj < k && r0 + ri < n_rows;
+    float* const out = dx + (r0 + ri) * k + rj;
+    const float old = accumulate && mine ? *out : 0.f;
+    float v[32];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+      for (int j = 0; j < KP; ++j) v[r * KP + j] = dot4(g[r], wr[j]);
+#pragma unroll
+    for (int h = 16; h > 0; h >>= 1) {
+      const bool upper = lane & h;
+#pragma unroll
+      for (int i = 0; i < h; ++i) {
+        const float keep = upper ? v[i + h] : v[i], give = upper ? v[i] : v[i + h];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+      }
+    }
+    if (mine) *out = v[0] + old;
   }
 }
 
@@ -739,10 +787,17 @@ extern "C" int mb_scale_rows(int64_t n_rows, const float* x, const float* a, flo
   return MB_OK;
 }
 
+// a warp loads its weights once: no more blocks than are resident at a time, which walk the rows
+static inline unsigned small_linear_grid(int64_t n_rows, int rows_per_warp, int blocks_per_sm) {
+  const int64_t blocks = (n_rows + rows_per_warp * (RW_THREADS / 32) - 1) / (rows_per_warp * (RW_THREADS / 32));
+  return (unsigned)(blocks < 148 * blocks_per_sm ? blocks : 148 * blocks_per_sm);
+}
+
 extern "C" int mb_small_linear_fwd(int64_t n_rows, int32_t k, const float* x, const float* w, float* y, void* stream) {
   MB_REQUIRE(n_rows >= 0 && k >= 1 && k <= 16 && x && w && y);
   if (n_rows == 0) return MB_OK;
-  launch(k_small_linear_fwd, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, k, x, w, y);
+  if (k <= 8) launch(k_small_linear_fwd<8>, small_linear_grid(n_rows, 4, 4), RW_THREADS, 0, STREAM, n_rows, k, x, w, y);
+  else launch(k_small_linear_fwd<16>, small_linear_grid(n_rows, 2, 2), RW_THREADS, 0, STREAM, n_rows, k, x, w, y);
   MB_LAUNCH_CHECK("k_small_linear_fwd");
   return MB_OK;
 }
@@ -751,7 +806,8 @@ extern "C" int mb_small_linear_bwd(int64_t n_rows, int32_t k, const float* dy, c
                                    int32_t accumulate, void* stream) {
   MB_REQUIRE(n_rows >= 0 && k >= 1 && k <= 16 && dy && w && dx);
   if (n_rows == 0) return MB_OK;
-  launch(k_small_linear_bwd, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, k, dy, w, dx, accumulate);
+  if (k <= 8) launch(k_small_linear_bwd<8>, small_linear_grid(n_rows, 4, 3), RW_THREADS, 0, STREAM, n_rows, k, dy, w, dx, accumulate);
+  else launch(k_small_linear_bwd<16>, small_linear_grid(n_rows, 2, 2), RW_THREADS, 0, STREAM, n_rows, k, dy, w, dx, accumulate);
   MB_LAUNCH_CHECK("k_small_linear_bwd");
   return MB_OK;
 }
