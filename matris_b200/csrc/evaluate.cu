@@ -15,6 +15,7 @@
 #include <string.h>
 #include <array>
 #include <initializer_list>
+#include <mutex>
 #include <vector>
 #include "common.cuh"
 
@@ -118,9 +119,87 @@ struct Arena {
   float* top(size_t floats) { return take(high, hi, floats, true); }
 };
 
+// ------------------------------------------------------------------ side streams
+// Two more streams for work that does not feed the next kernel of the caller's stream.  A small system is bound by the chain of its
+// 660 launches, most of which leave most SMs idle: off the chain go a layer's centre and node tables, the logits, the envelopes and
+// the other of two feed-forward blocks, in the backward pass the node sums beside the edge gradients.  Device time of an evaluation:
+// 32 atoms 6.5 -> 5.5 ms, 256 atoms 10.4 -> 9.4; 16,000 atoms 624 -> 608 (tails of one launch filled by another), so for all sizes.
+// Taken from a pool for one call and given back when its work is queued (a later user of the same streams queues behind it); the
+// pool keeps no more than eight sets.
+struct Side {
+  int device = -1;
+  cudaStream_t st[2] = {};
+  cudaEvent_t ev = nullptr;
+};
+static std::mutex g_side_mutex;
+static std::vector<Side> g_side_pool;
+
+static void side_free(Side& s) {
+  for (cudaStream_t t : s.st)
+    if (t) cudaStreamDestroy(t);  // (work still queued there runs to its end)
+  if (s.ev) cudaEventDestroy(s.ev);
+}
+static bool side_take(Side& s) {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  {
+    std::lock_guard<std::mutex> lock(g_side_mutex);
+    for (size_t i = 0; i < g_side_pool.size(); ++i)
+      if (g_side_pool[i].device == dev) {
+        s = g_side_pool[i];
+        g_side_pool.erase(g_side_pool.begin() + i);
+        return true;
+      }
+  }
+  s.device = dev;
+  for (cudaStream_t& t : s.st)
+    if (cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking) != cudaSuccess) { side_free(s); return false; }
+  if (cudaEventCreateWithFlags(&s.ev, cudaEventDisableTiming) != cudaSuccess) { side_free(s); return false; }
+  return true;
+}
+static void side_give(Side& s) {
+  {
+    std::lock_guard<std::mutex> lock(g_side_mutex);
+    if (g_side_pool.size() < 8) {
+      g_side_pool.push_back(s);
+      return;
+    }
+  }
+  side_free(s);
+}
+
 struct Run {
   Arena ar;
   cudaStream_t st = nullptr;
+  Side* sides = nullptr;  // NULL: everything on the caller's stream
+  bool pending[2] = {};
+  int on = 0;             // 0: the caller's stream, 1 + k: side stream k
+  bool behind[3] = {};    // the last thing queued there is a wait for another stream's event
+
+  // f's launches on side stream k, after everything queued on the caller's stream so far.  The buffers they touch must live, and
+  // must not be written or (where f writes) read on the caller's stream, until join(k).
+  template <typename F> void side(int k, F f) {
+    if (!sides || !go()) {
+      f();
+      return;
+    }
+    const cudaStream_t main = st;
+    after(1 + k, sides->st[k], main);
+    st = sides->st[k]; on = 1 + k;
+    f();
+    st = main; on = 0;
+    pending[k] = true;
+  }
+  void join(int k) {
+    if (!pending[k]) return;
+    pending[k] = false;
+    after(0, st, sides->st[k]);
+  }
+  void after(int which, cudaStream_t later, cudaStream_t earlier) {
+    if (cudaEventRecord(sides->ev, earlier) != cudaSuccess || cudaStreamWaitEvent(later, sides->ev, 0) != cudaSuccess)
+      rc = rc == MB_OK ? MB_ERR_CUDA : rc;
+    behind[which] = true;
+  }
   int rc = MB_OK, launches = 0;
   bool scratch = false;  // the contraction mode composes a gated MLP from separate launches, which need z1 / z2
 
@@ -133,7 +212,10 @@ struct Run {
     if (!go()) return;
     ++launches;
     if (!g_times.on) {
+      launch_after_event = behind[on];
       rc = f();
+      behind[on] = launch_after_event;  // (a memset or copy leaves it)
+      launch_after_event = false;
       return;
     }
     OpTimes::Rec rec{};
@@ -164,8 +246,13 @@ struct Run {
 struct Scope {
   Run& R;
   size_t mark;
+  bool open = true;
   explicit Scope(Run& r) : R(r), mark(r.ar.low.size()) {}
-  ~Scope() { R.ar.drop(R.ar.low, R.ar.lo, mark); }
+  ~Scope() { if (open) close(); }
+  void close() {
+    open = false;
+    R.ar.drop(R.ar.low, R.ar.lo, mark);
+  }
 };
 
 // ------------------------------------------------------------------ contractions
@@ -296,14 +383,22 @@ static void edge_update_fwd(Run& R, const mb_update& p, const mb_row_graph& g, c
     if (!z1) z1 = R.ar.bottom((size_t)g.n_rows * 256);
     if (!z2) z2 = R.ar.bottom((size_t)g.n_rows * 256);
   }
-  linear(R, g.n_nodes, node, p.wts, 512, 128, P);
-  if (Pc) linear(R, g.n_ctr, ctr_feat, p.wc, 256, 128, Pc);
+  if (Pc) R.side(0, [&] { linear(R, g.n_ctr, ctr_feat, p.wc, 256, 128, Pc); });
+  auto node_table = [&] { linear(R, g.n_nodes, node, p.wts, 512, 128, P); };
   Gemm e(g.n_edge_rows);
   if (Pe)
     for (int j = 0; j < 2; ++j) e.block({src(edge)}, p.we, 128 * j, Pe, 256, 128 * j);
   if (logits)
     for (int j = 0; j < 2; ++j) e.block({src(edge)}, *wst, 128 * j, logits, 256, 128 * j);
-  e.run(R);
+  if (g.is_atom) {
+    R.side(0, node_table);
+    e.run(R);
+    R.join(0);
+  } else {  // e holds the logits at most, which the caller waits for
+    if (e.d.n_blocks) R.side(0, [&] { e.run(R); });
+    node_table();
+    if (Pc) R.join(0);
+  }
   mb_gated_mlp m;
   if (g.is_atom) fill_mlp(m, g.n_rows, {}, p.we, p.w2, p.b1, p.b2);
   else fill_mlp(m, g.n_rows, {src(edge)}, p.we, p.w2, p.b1, p.b2);
@@ -325,6 +420,19 @@ static void edge_update_bwd(Run& R, const mb_update& p, const mb_row_graph& g, c
                             float* d_edge, const float* node_res, const float* node_w, float* d_node, float* d_ctr) {
   Scope sc(R);
   float* dz1 = R.ar.bottom((size_t)g.n_rows * 256);
+  float* dP = R.ar.bottom((size_t)g.n_nodes * 512);
+  float* dPc = d_ctr ? R.ar.bottom((size_t)g.n_ctr * 256) : nullptr;
+  if (dPc) R.zero(dPc, (size_t)g.n_ctr * 1024);
+  auto node_sums = [&] {
+    MB_OP(mb_seg_sum, (int32_t)g.n_nodes, g.n_rows, g.tgt_ptr, g.src_ptr, g.src_perm, d_ctr ? g.ctr : nullptr, dz1, dP, dPc);
+  };
+  auto node_grad = [&] {
+    Gemm n(g.n_nodes);
+    mb_colblock& b = n.block({src(dP, nullptr, 0, 512), src(dP, nullptr, 128, 512), src(dP, nullptr, 256, 512),
+                              src(dP, nullptr, 384, 512)}, p.wtst, 0, d_node, 128, 0, nullptr, node_res ? MB_OUT_STORE : MB_OUT_ADD);
+    b.res = node_res; b.res_w = node_w; b.ld_res = 128;
+    n.run(R);
+  };
   if (g.is_atom) {
     Gemm a(g.n_rows);
     for (int j = 0; j < 2; ++j) {
@@ -332,7 +440,10 @@ static void edge_update_bwd(Run& R, const mb_update& p, const mb_row_graph& g, c
       b.gate = z1; b.ld_gate = 256; b.col_gate = 128 * j;
     }
     a.run(R);
-    Scope s2(R);
+    R.side(0, [&] {
+      node_sums();
+      node_grad();
+    });
     const int ld = dlogits ? 512 : 256;
     float* pair = R.ar.bottom((size_t)g.n_edge_rows * ld);
     MB_OP(mb_pair_sum, (int32_t)g.n_edge_rows, g.u2d, g.rev, dz1, dlogits, pair);
@@ -361,20 +472,17 @@ static void edge_update_bwd(Run& R, const mb_update& p, const mb_row_graph& g, c
     R.op("mb_mlp_bwd_data", [&] { return mb_mlp_bwd_data(&m, R.st); }, 2.0 * g.n_rows * 128 * k,
          4.0 * g.n_rows * 128 * (7 + (edge_res != nullptr) + (dlogits ? 2 : 0)), g.n_rows, 256, 256, 1);
   }
-  float* dP = R.ar.bottom((size_t)g.n_nodes * 512);
-  float* dPc = d_ctr ? R.ar.bottom((size_t)g.n_ctr * 256) : nullptr;
-  if (dPc) R.zero(dPc, (size_t)g.n_ctr * 1024);
-  MB_OP(mb_seg_sum, (int32_t)g.n_nodes, g.n_rows, g.tgt_ptr, g.src_ptr, g.src_perm, d_ctr ? g.ctr : nullptr, dz1, dP, dPc);
-  Gemm n(g.n_nodes);
-  mb_colblock& b = n.block({src(dP, nullptr, 0, 512), src(dP, nullptr, 128, 512), src(dP, nullptr, 256, 512),
-                            src(dP, nullptr, 384, 512)}, p.wtst, 0, d_node, 128, 0, nullptr, node_res ? MB_OUT_STORE : MB_OUT_ADD);
-  b.res = node_res; b.res_w = node_w; b.ld_res = 128;
-  n.run(R);
-  if (dPc) {
-    Gemm c(g.n_ctr);
-    c.block({src(dPc, nullptr, 0, 256), src(dPc, nullptr, 128, 256)}, p.wct, 0, d_ctr, 128, 0, nullptr, MB_OUT_ADD);
-    c.run(R);
+  if (!g.is_atom) {
+    node_sums();
+    if (dPc)
+      R.side(0, [&] {
+        Gemm c(g.n_ctr);
+        c.block({src(dPc, nullptr, 0, 256), src(dPc, nullptr, 128, 256)}, p.wct, 0, d_ctr, 128, 0, nullptr, MB_OUT_ADD);
+        c.run(R);
+      });
+    node_grad();
   }
+  R.join(0);
 }
 
 struct Dest {  // where the gradient of one 128-wide K segment goes
@@ -470,12 +578,15 @@ static void attn_fwd(Run& R, const mb_attn_params& p, const mb_row_graph& g, con
   it.z1n = mode == NONE ? nullptr : get(nodes * update_width(p.node));
   it.z2n = mode == NONE ? nullptr : get(nodes * update_width(p.node));
   edge_update_fwd(R, p.edge, g, node, edge, nullptr, &p.wst, it.logits, it.z1, it.z2, it.h, p.we, g.is_atom ? nullptr : edge_out);
-  if (g.is_atom && edge_out) MB_OP(mb_pair_mean_res, (int32_t)g.n_edge_rows, g.u2d, g.rev, it.h, edge, p.we, edge_out);
+  R.join(0);  // the logits
+  if (g.is_atom && edge_out)
+    R.side(0, [&] { MB_OP(mb_pair_mean_res, (int32_t)g.n_edge_rows, g.u2d, g.rev, it.h, edge, p.we, edge_out); });
   MB_OP(mb_seg_attn_fwd, (int32_t)g.n_nodes, g.tgt_ptr, g.src_ptr, g.src_perm, g.emap, it.logits, it.h, it.agg_t, it.agg_s,
         it.stats);
   Scope sc(R);
   float* out = node_out ? node_out : R.ar.bottom(nodes * 128);  // a recomputation wants the internals only
   update_fwd(R, p.node, g.n_nodes, {src(node), src(it.agg_t), src(it.agg_s)}, it.z1n, it.z2n, nullptr, node, p.wn, out);
+  R.join(0);
 }
 
 static void attn_bwd(Run& R, const mb_attn_params& p, const mb_row_graph& g, const AttnInter& it, const float* d_node_out,
@@ -530,14 +641,20 @@ static void refine_fwd(Run& R, const mb_refine_params& p, const mb_row_graph& g,
   it.env = get((size_t)n_bonds * 128);
   it.zn = mode == NONE ? nullptr : get(nodes * 128);
   it.ze = mode == NONE || !want_edge ? nullptr : get(rows * 128);
+  R.side(1, [&] { MB_OP(mb_small_linear_fwd, n_bonds, 7, rbf, p.wenv, it.env); });
   edge_update_fwd(R, p.edge, g, node, edge, g.is_atom ? nullptr : atom_feat, nullptr, nullptr, it.z1, it.z2, it.h, nullptr,
                   nullptr);
   Scope sc(R);
   float* agg = R.ar.bottom(nodes * 128);
-  MB_OP(mb_small_linear_fwd, n_bonds, 7, rbf, p.wenv, it.env);
-  MB_OP(mb_seg_smooth_sum_fwd, (int32_t)g.n_nodes, g.tgt_ptr, g.emap, g.is_atom ? nullptr : g.src, 1, it.env, it.h, agg);
-  ffn_fwd(R, p.nffn, g.n_nodes, agg, it.zn, nullptr, node, p.wn, node_out ? node_out : R.ar.bottom(nodes * 128));
-  if (!want_edge) return;  // the last layer's edge update feeds nothing
+  auto node_update = [&] {
+    MB_OP(mb_seg_smooth_sum_fwd, (int32_t)g.n_nodes, g.tgt_ptr, g.emap, g.is_atom ? nullptr : g.src, 1, it.env, it.h, agg);
+    ffn_fwd(R, p.nffn, g.n_nodes, agg, it.zn, nullptr, node, p.wn, node_out ? node_out : R.ar.bottom(nodes * 128));
+  };
+  R.join(1);
+  if (!want_edge) {  // the last layer's edge update feeds nothing
+    node_update();
+    return;
+  }
   // the edge update reads the unsmoothed rows unless use_smoothed_for_delta_edge (atom graph only,
   // matris/model/interaction_block.py:262-266): then h * s, s = the envelope row of the edge's bond
   const float* x = it.h;
@@ -546,13 +663,17 @@ static void refine_fwd(Run& R, const mb_refine_params& p, const mb_row_graph& g,
     MB_OP(mb_mul_rows_gather, g.n_rows, it.h, it.env, g.emap, t);
     x = t;
   }
-  if (g.is_atom) {
-    float* y = R.ar.bottom(rows * 128);
-    ffn_fwd(R, p.effn, g.n_rows, x, it.ze, y, nullptr, nullptr, nullptr);
-    if (edge_out) MB_OP(mb_pair_mean_res, (int32_t)g.n_edge_rows, g.u2d, g.rev, y, edge, p.we, edge_out);
-  } else {
-    ffn_fwd(R, p.effn, g.n_rows, x, it.ze, nullptr, edge, p.we, edge_out ? edge_out : R.ar.bottom(rows * 128));
-  }
+  float* y = g.is_atom || !edge_out ? R.ar.bottom(rows * 128) : nullptr;
+  R.side(0, [&] {
+    if (g.is_atom) {
+      ffn_fwd(R, p.effn, g.n_rows, x, it.ze, y, nullptr, nullptr, nullptr);
+      if (edge_out) MB_OP(mb_pair_mean_res, (int32_t)g.n_edge_rows, g.u2d, g.rev, y, edge, p.we, edge_out);
+    } else {
+      ffn_fwd(R, p.effn, g.n_rows, x, it.ze, nullptr, edge, p.we, edge_out ? edge_out : y);
+    }
+  });
+  node_update();
+  R.join(0);
 }
 
 static void refine_bwd(Run& R, const mb_refine_params& p, const mb_row_graph& g, int64_t n_bonds, const RefineInter& it,
@@ -563,35 +684,40 @@ static void refine_bwd(Run& R, const mb_refine_params& p, const mb_row_graph& g,
   const bool want_edge = d_edge_out != nullptr, gated = p.edge.kind == MB_UPDATE_GATED;
   // node FFN
   float* dagg = R.ar.bottom(nodes * 128);
-  ffn_bwd(R, p.nffn, g.n_nodes, d_node_out, nullptr, 1.f, it.zn, dagg);
+  auto node_ffn = [&] { ffn_bwd(R, p.nffn, g.n_nodes, d_node_out, nullptr, 1.f, it.zn, dagg); };
   // edge FFN (atom graph: the mean over the two directions is a gather * 0.5)
   float* dh = R.ar.bottom(rows * 128);
   const float* drow = nullptr;
   if (want_edge) {
     float* dx = p.smoothed_edge ? R.ar.bottom(rows * 128) : dh;
+    R.side(0, node_ffn);
     ffn_bwd(R, p.effn, g.n_rows, d_edge_out, g.is_atom ? g.emap : nullptr, g.is_atom ? 0.5f : 1.f, it.ze, dx);
     if (p.smoothed_edge) {  // dx is the gradient of the smoothed rows h * s
       drow = dx;
       MB_OP(mb_mul_rows_gather, g.n_rows, dx, it.env, g.emap, dh);
     }
+    R.join(0);
+  } else {
+    node_ffn();
   }
   // smoothed aggregation; with a gated update dh is finished in registers and leaves as dz2
   const int32_t* src_idx = g.is_atom ? nullptr : g.src;
   float* dz2 = gated ? R.ar.bottom(rows * 256) : nullptr;
-  MB_OP(mb_seg_smooth_sum_bwd_rows, g.n_rows, g.tgt, src_idx, 1, g.emap, it.env, dagg, dh, want_edge ? 1 : 0,
-        gated ? it.z2 : nullptr, gated ? p.edge.nc : nullptr, gated ? p.edge.ng : nullptr, dz2);
-  {
-    Scope s2(R);
-    float* denv = R.ar.bottom((size_t)n_bonds * 128);
+  float* denv = R.ar.bottom((size_t)n_bonds * 128);
+  R.side(1, [&] {
     MB_OP(mb_seg_smooth_sum_bwd_env, (int32_t)n_bonds, g.tgt_ptr, g.is_atom ? nullptr : g.src_ptr, g.src_perm, g.tgt, g.src, 1,
           g.u2d, g.rev, it.env, it.h, dagg, drow, denv);
     MB_OP(mb_small_linear_bwd, n_bonds, 7, denv, p.wenv, d_rbf, 1);
-  }
+  });
+  MB_OP(mb_seg_smooth_sum_bwd_rows, g.n_rows, g.tgt, src_idx, 1, g.emap, it.env, dagg, dh, want_edge ? 1 : 0,
+        gated ? it.z2 : nullptr, gated ? p.edge.nc : nullptr, gated ? p.edge.ng : nullptr, dz2);
   // edge update
   if (gated) {
     edge_update_bwd(R, p.edge, g, it.z1, dz2, nullptr, nullptr, d_edge_out, p.we, d_edge, d_node_out, p.wn, d_node, d_atom);
+    R.join(1);
     return;
   }
+  R.join(1);
   MB_OP(mb_scale_rows, g.n_nodes, d_node_out, p.wn, d_node, 0);
   const Dest to_tgt{d_node, g.tgt, MB_OUT_ATOMIC, nullptr, nullptr}, to_src{d_node, g.src, MB_OUT_ATOMIC, nullptr, nullptr};
   if (g.is_atom) {
@@ -650,6 +776,21 @@ static int evaluate(Run& R, mb_eval& E) {
   float* node = A.bottom(N * 128);
   float* edge = A.bottom(Eu * 128);
   float* trip = line ? A.bottom(T * 128) : nullptr;
+  const int n_basis = M.fourier ? 7 : 16;
+  auto angle_embed = [&](float* basis, float* t1, float* z, int act) {  // z = (act: SiLU of) the triplet embedding's pre-activation
+    if (M.fourier) MB_OP(mb_fourier_basis_fwd, E.n_triplets, E.line_graph, unit, M.t_freq, basis);
+    else MB_OP(mb_angle_basis_fwd, E.n_triplets, E.line_graph, unit, M.sph_factor, M.cut2, basis);
+    MB_OP(mb_small_linear_fwd, E.n_triplets, n_basis, basis, M.t_wa, t1);
+    LinearOpt o;
+    o.out_act = act;
+    linear(R, E.n_triplets, t1, M.t_wb, 128, 128, z, o);
+  };
+  Scope embed(R);
+  if (line) {
+    float* basis = A.bottom(T * n_basis);
+    float* t1 = A.bottom(T * 128);
+    R.side(0, [&] { angle_embed(basis, t1, trip, 1); });
+  }
   {
     Scope sc(R);
     float* t = A.bottom(N * 128);
@@ -676,19 +817,8 @@ static int evaluate(Run& R, mb_eval& E) {
     o.out_act = 1;
     linear(R, E.n_bonds, e3, M.e_w3, 128, 128, edge, o);
   }
-  const int n_basis = M.fourier ? 7 : 16;
-  auto angle_embed = [&](float* z, int act) {  // z = (act: SiLU of) the triplet embedding's pre-activation
-    Scope sc(R);
-    float* basis = A.bottom(T * n_basis);
-    float* t1 = A.bottom(T * 128);
-    if (M.fourier) MB_OP(mb_fourier_basis_fwd, E.n_triplets, E.line_graph, unit, M.t_freq, basis);
-    else MB_OP(mb_angle_basis_fwd, E.n_triplets, E.line_graph, unit, M.sph_factor, M.cut2, basis);
-    MB_OP(mb_small_linear_fwd, E.n_triplets, n_basis, basis, M.t_wa, t1);
-    LinearOpt o;
-    o.out_act = act;
-    linear(R, E.n_triplets, t1, M.t_wb, 128, 128, z, o);
-  };
-  if (line) angle_embed(trip, 1);
+  R.join(0);
+  embed.close();
 
   // ---- interaction blocks.  Without a backward pass the features of a layer live in two sets of buffers used in turn.
   std::vector<AttnInter> ia(L), il(L);
@@ -847,6 +977,20 @@ static int evaluate(Run& R, mb_eval& E) {
   float* dunit = A.bottom(Ed * 3);
   R.zero(dlen, Ed * 4);
   R.zero(dunit, Ed * 12);
+  if (line) {
+    float* z = A.bottom(T * 128);
+    float* t1 = A.bottom(T * 128);
+    float* dz = dT[1];  // free by now
+    float* basis = A.bottom(T * n_basis);
+    R.side(0, [&] {
+      angle_embed(basis, t1, z, 0);
+      MB_OP(mb_silu_bwd, E.n_triplets, dT[0], z, dz);
+      linear(R, E.n_triplets, dz, M.t_wbt, 128, 128, z);
+      MB_OP(mb_small_linear_bwd, E.n_triplets, n_basis, z, M.t_wa, basis, 0);  // its gradient takes the basis's place
+      if (M.fourier) MB_OP(mb_fourier_basis_bwd, E.n_triplets, E.line_graph, unit, M.t_freq, basis, dunit);
+      else MB_OP(mb_angle_basis_bwd, E.n_triplets, E.line_graph, unit, M.sph_factor, M.cut2, basis, dunit);
+    });
+  }
   {
     Scope sc(R);
     float* e2 = A.bottom(Eu * 128);
@@ -863,18 +1007,7 @@ static int evaluate(Run& R, mb_eval& E) {
     if (M.gaussian) MB_OP(mb_gaussian_bwd, nb, E.u2d, len, M.freq2, M.coeff2, M.freq3, M.coeff3, d_rbf2, d_rbf3, dlen);
     else MB_OP(mb_bessel_bwd, nb, E.u2d, len, M.freq2, M.cut2, M.freq3, M.cut3, M.envelope_exponent, d_rbf2, d_rbf3, dlen);
   }
-  if (line) {
-    Scope sc(R);
-    float* z = A.bottom(T * 128);
-    float* dz = dT[1];  // free by now
-    float* dbasis = A.bottom(T * n_basis);
-    angle_embed(z, 0);
-    MB_OP(mb_silu_bwd, E.n_triplets, dT[0], z, dz);
-    linear(R, E.n_triplets, dz, M.t_wbt, 128, 128, z);
-    MB_OP(mb_small_linear_bwd, E.n_triplets, n_basis, z, M.t_wa, dbasis, 0);
-    if (M.fourier) MB_OP(mb_fourier_basis_bwd, E.n_triplets, E.line_graph, unit, M.t_freq, dbasis, dunit);
-    else MB_OP(mb_angle_basis_bwd, E.n_triplets, E.line_graph, unit, M.sph_factor, M.cut2, dbasis, dunit);
-  }
+  R.join(0);
   float* ge = A.bottom(Ed * 3);
   float* dcart = A.bottom(N * 3);
   float* virial = A.bottom(N * 9);
@@ -921,7 +1054,19 @@ extern "C" int mb_evaluate(mb_eval* e, void* stream) {
   R.ar.cap = e->ws_bytes;
   R.ar.alloc = e->alloc;
   R.ar.release = e->release;
-  const int rc = evaluate(R, *e);
+  Side side;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  // not while every launch is timed by itself, nor with the composed contractions (R.scratch), which drop temporaries on the way
+  const bool beside = !R.scratch && !g_times.on && cudaStreamIsCapturing(R.st, &capture) == cudaSuccess &&
+                      capture == cudaStreamCaptureStatusNone && side_take(side);
+  if (beside) R.sides = &side;
+  int rc = evaluate(R, *e);
+  if (beside) {
+    R.join(0);  // (only after an error is anything left)
+    R.join(1);
+    rc = R.rc;
+    side_give(side);
+  }
   e->n_launches = R.launches;
   return rc;
 }
