@@ -128,6 +128,16 @@ typedef struct mb_graph {
 
 size_t mb_graph_scan_tmp_len(int64_t n);
 int mb_graph_build(const mb_graph* g, void* stream);
+/* Host side of a batch.  mb_cell_grid: cells per axis of every structure's neighbour search (each at least `cutoff` wide
+ * where the cell allows it, at most 4 n + 8 in all), the half-width of the search in cells and the first global cell index
+ * -> grid [B,8]; volume [B] and the total number of cells; MB_ERR_INVALID for a singular lattice, MB_ERR_OVERFLOW for more
+ * than 2^31 - 2 cells.  mb_host_batch fills the two staging buffers of a batch: f64 = cart | lattice | inverse lattice, i32 =
+ * atom_struct | atom_ptr | grid | numbers | cart32 | lattice32 | volume32 (float bits), and frac32 [N,3]. */
+int mb_cell_grid(int64_t n_struct, const double* lattice, const int64_t* n_atoms, double cutoff, int32_t* grid,
+                 double* volume, int64_t* n_cells);
+int mb_host_batch(int64_t n_struct, const int32_t* atom_ptr, const int64_t* numbers, const double* cart,
+                  const double* lattice, const double* inv_lattice, const int32_t* grid, double* f64, int32_t* i32,
+                  float* frac32);
 /* status code of a build from the host copy of counts[16]: MB_OK, MB_ERR_ISOLATED, MB_ERR_OVERFLOW (image index or
  * a count beyond int32), MB_ERR_CAPACITY, MB_ERR_UNPAIRED */
 int mb_graph_status(const int32_t* counts_host);

@@ -12,7 +12,7 @@ _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "libmatris_b200.so")
 
 MB_OK = 0
-MB_ERR_CAPACITY = 7
+MB_ERR_INVALID, MB_ERR_OVERFLOW, MB_ERR_CAPACITY = 1, 3, 7
 MB_GRAPH_EDGES_ONLY = 1
 OUT_STORE, OUT_ADD, OUT_ATOMIC = 0, 1, 2
 
@@ -154,6 +154,8 @@ class MbOpRecord(C.Structure):
 
 # name -> argtypes (every function returns int status unless listed in _OTHER)
 _SIGNATURES = {
+    "mb_cell_grid": [_i64, _vp, _vp, C.c_double, _vp, _vp, C.POINTER(_i64)],
+    "mb_host_batch": [_i64] + [_vp] * 9,
     "mb_graph_build": [C.POINTER(MbGraph), _vp],
     "mb_graph_status": [C.POINTER(C.c_int32)],
     "mb_graph_skin_check": [_i32, _vp, _vp, C.c_double, _vp, _vp],

@@ -642,3 +642,77 @@ extern "C" int mb_graph_status(const int32_t* counts_host) {
   if (counts_host[CT_TRIPLETS] != counts_host[CT_TRIPLETS_BY_SOURCE]) return MB_ERR_INVALID;
   return MB_OK;
 }
+
+// ------------------------------------------------------------------ host side of a batch
+// Everything of a batch that is computed before the copy to the device.  In an interpreter's array library the same arithmetic cost
+// 1.0 ms for 256 structures of 36 atoms, half of it in calls and temporaries, and as much again to pin the result; it now writes
+// into the pinned staging buffers.  The float32 positions are rounded step by step (float64 fractional coordinates, rounded, times
+// the rounded lattice), products summed left to right.
+static void host_cross(const double* a, const double* b, double* c) {
+  c[0] = a[1] * b[2] - a[2] * b[1]; c[1] = a[2] * b[0] - a[0] * b[2]; c[2] = a[0] * b[1] - a[1] * b[0];
+}
+
+extern "C" int mb_cell_grid(int64_t n_struct, const double* lattice, const int64_t* n_atoms, double cutoff, int32_t* grid,
+                            double* volume, int64_t* n_cells) {
+  if (!(n_struct >= 0 && lattice && n_atoms && cutoff > 0 && grid && volume && n_cells)) return MB_ERR_INVALID;
+  int64_t base = 0;
+  for (int64_t i = 0; i < n_struct; ++i) {
+    const double *a = lattice + 9 * i, *b = a + 3, *c = a + 6;
+    double n[3][3], width[3];
+    host_cross(b, c, n[0]); host_cross(c, a, n[1]); host_cross(a, b, n[2]);
+    const double vol = fabs(a[0] * n[0][0] + a[1] * n[0][1] + a[2] * n[0][2]);
+    if (!(vol > 0)) return MB_ERR_INVALID;
+    const double cap = 4.0 * (double)n_atoms[i] + 8.0;
+    double g[3];
+    for (int k = 0; k < 3; ++k) {
+      width[k] = vol / sqrt(n[k][0] * n[k][0] + n[k][1] * n[k][1] + n[k][2] * n[k][2]);
+      g[k] = fmax(1.0, floor(width[k] / cutoff));
+    }
+    for (int it = 0; it < 64 && g[0] * g[1] * g[2] > cap; ++it) {  // never more cells than a few per atom: halve the longest axis
+      const int k = g[0] >= g[1] && g[0] >= g[2] ? 0 : (g[1] >= g[2] ? 1 : 2);
+      g[k] = fmax(1.0, floor(g[k] / 2.0));
+    }
+    if ((double)base + g[0] * g[1] * g[2] > 2147483646.0) return MB_ERR_OVERFLOW;
+    int32_t* o = grid + 8 * i;
+    for (int k = 0; k < 3; ++k) {
+      o[k] = (int32_t)g[k];
+      o[3 + k] = (int32_t)fmin(fmax(1.0, ceil(cutoff * g[k] / width[k] - 1e-12)), 2147483647.0);
+    }
+    o[6] = (int32_t)base;
+    o[7] = 0;
+    volume[i] = vol;
+    base += (int64_t)(g[0] * g[1] * g[2]);
+  }
+  *n_cells = base;
+  return MB_OK;
+}
+
+extern "C" int mb_host_batch(int64_t n_struct, const int32_t* atom_ptr, const int64_t* numbers, const double* cart,
+                             const double* lattice, const double* inv_lattice, const int32_t* grid, double* f64, int32_t* i32,
+                             float* frac32) {
+  if (!(n_struct > 0 && atom_ptr && numbers && cart && lattice && inv_lattice && grid && f64 && i32 && frac32)) return MB_ERR_INVALID;
+  const int64_t N = atom_ptr[n_struct], B = n_struct;
+  memcpy(f64, cart, sizeof(double) * 3 * N);
+  memcpy(f64 + 3 * N, lattice, sizeof(double) * 9 * B);
+  memcpy(f64 + 3 * N + 9 * B, inv_lattice, sizeof(double) * 9 * B);
+  int32_t *atom_struct = i32, *ptr = i32 + N, *grid_out = ptr + B + 1, *num = grid_out + 8 * B;
+  float *cart32 = reinterpret_cast<float*>(num + N), *lat32 = cart32 + 3 * N, *vol32 = lat32 + 9 * B;
+  memcpy(ptr, atom_ptr, sizeof(int32_t) * (B + 1));
+  memcpy(grid_out, grid, sizeof(int32_t) * 8 * B);
+  for (int64_t b = 0; b < B; ++b) {
+    const double* inv = inv_lattice + 9 * b;
+    float* L = lat32 + 9 * b;
+    for (int k = 0; k < 9; ++k) L[k] = (float)lattice[9 * b + k];
+    const float c0 = L[4] * L[8] - L[5] * L[7], c1 = L[5] * L[6] - L[3] * L[8], c2 = L[3] * L[7] - L[4] * L[6];
+    vol32[b] = L[0] * c0 + L[1] * c1 + L[2] * c2;
+    for (int64_t i = atom_ptr[b]; i < atom_ptr[b + 1]; ++i) {
+      const double* x = cart + 3 * i;
+      float* f = frac32 + 3 * i;
+      for (int j = 0; j < 3; ++j) f[j] = (float)(x[0] * inv[j] + x[1] * inv[3 + j] + x[2] * inv[6 + j]);
+      for (int j = 0; j < 3; ++j) cart32[3 * i + j] = f[0] * L[j] + f[1] * L[3 + j] + f[2] * L[6 + j];
+      atom_struct[i] = (int32_t)b;
+      num[i] = (int32_t)numbers[i];
+    }
+  }
+  return MB_OK;
+}

@@ -57,35 +57,22 @@ def _formula(numbers: np.ndarray) -> str:
     return " ".join(f"Z{int(a)}:{int(b)}" for a, b in zip(z, n))
 
 
-def cell_grid(lattice: np.ndarray, n_atoms: np.ndarray, cutoff: float) -> tuple[np.ndarray, int]:
+def cell_grid(lattice: np.ndarray, n_atoms: np.ndarray, cutoff: float) -> tuple[np.ndarray, int, np.ndarray]:
     """Per-structure cell grid for the neighbour search: cells per axis (each cell at
     least ``cutoff`` wide where the cell allows it), search half-width in cells, and
-    the first global cell index.  lattice [B,3,3], n_atoms [B] -> int32 [B,8], n_cells."""
-    a, b, c = lattice[:, 0], lattice[:, 1], lattice[:, 2]
-    vol = np.abs(np.einsum("bi,bi->b", a, np.cross(b, c)))
-    if (vol <= 0).any():
+    the first global cell index.  lattice [B,3,3], n_atoms [B] -> int32 [B,8], n_cells, volumes [B]."""
+    lattice = np.ascontiguousarray(lattice, dtype=np.float64)
+    n_atoms = np.ascontiguousarray(n_atoms, dtype=np.int64)
+    grid, volume = np.empty((len(lattice), 8), dtype=np.int32), np.empty(len(lattice))
+    n_cells = C.c_int64(0)
+    status = _lib.load().mb_cell_grid(len(lattice), lattice.ctypes.data, n_atoms.ctypes.data, float(cutoff), grid.ctypes.data,
+                                      volume.ctypes.data, C.byref(n_cells))
+    if status == _lib.MB_ERR_INVALID:
         raise ValueError("singular lattice")
-    width = np.stack([vol / np.linalg.norm(np.cross(b, c), axis=1),
-                      vol / np.linalg.norm(np.cross(c, a), axis=1),
-                      vol / np.linalg.norm(np.cross(a, b), axis=1)], axis=1)
-    g = np.maximum(1, np.floor(width / cutoff)).astype(np.int64)
-    # never more cells than a few per atom (huge vacuum boxes would waste memory)
-    cap = 4 * n_atoms.astype(np.int64) + 8
-    for _ in range(64):
-        over = g.prod(axis=1) > cap
-        if not over.any():
-            break
-        k = g.argmax(axis=1)
-        rows = np.nonzero(over)[0]
-        g[rows, k[rows]] = np.maximum(1, g[rows, k[rows]] // 2)
-    s = np.maximum(1, np.ceil(cutoff * g / width - 1e-12)).astype(np.int64)
-    cells = g.prod(axis=1)
-    base = np.concatenate([[0], np.cumsum(cells)[:-1]])
-    grid = np.zeros((len(lattice), 8), dtype=np.int32)
-    grid[:, 0:3], grid[:, 3:6], grid[:, 6] = g, s, base
-    if cells.sum() > 2**31 - 2:
+    if status == _lib.MB_ERR_OVERFLOW:
         raise ValueError("cell grid too large")
-    return grid, int(cells.sum())
+    _lib.check(status, "mb_cell_grid")
+    return grid, n_cells.value, volume
 
 
 # ------------------------------------------------------------------ batched graph
@@ -122,27 +109,26 @@ class HostBatch:
         n_per = np.asarray([len(z) for z in numbers], dtype=np.int64)
         if len(n_per) == 0 or (n_per <= 0).any():
             raise ValueError("empty structure")
-        self.n_struct, self.n_atoms = len(n_per), int(n_per.sum())
-        self.atoms_per_graph = [int(x) for x in n_per]
-        self.atom_ptr = np.concatenate([[0], np.cumsum(n_per)]).astype(np.int32)
-        self.numbers = np.concatenate(numbers).astype(np.int64)
+        B, N = self.n_struct, self.n_atoms = len(n_per), int(n_per.sum())
+        self.atoms_per_graph = n_per.tolist()
+        self.atom_ptr = np.zeros(B + 1, dtype=np.int32)
+        np.cumsum(n_per, out=self.atom_ptr[1:])
+        self.numbers = np.concatenate(numbers).astype(np.int64, copy=False)
         self.cart = np.ascontiguousarray(np.concatenate(carts), dtype=np.float64)
-        self.lattice = np.ascontiguousarray(np.stack(lattices), dtype=np.float64)
+        self.lattice = np.ascontiguousarray(np.concatenate(lattices).reshape(B, 3, 3), dtype=np.float64)
+        if self.numbers.shape != (N,) or self.cart.shape != (N, 3):
+            raise ValueError("numbers and positions differ in length")
         inv = np.linalg.inv(self.lattice)
-        self.atom_struct = np.repeat(np.arange(self.n_struct, dtype=np.int32), n_per)
-        grid, self.n_cells = cell_grid(self.lattice, n_per, float(cutoff))
+        grid, self.n_cells, self.volume = cell_grid(self.lattice, n_per, cutoff)
         # float32 model inputs exactly as the reference derives them (converter.py:82-83, processgraph.py:87)
-        self.frac32 = np.einsum("ni,nij->nj", self.cart, inv[self.atom_struct]).astype(np.float32)
-        lat32 = self.lattice.astype(np.float32)
-        cart32 = np.einsum("ni,nij->nj", self.frac32, lat32[self.atom_struct]).astype(np.float32)
-        vol32 = np.einsum("bi,bi->b", lat32[:, 0], np.cross(lat32[:, 1], lat32[:, 2])).astype(np.float32)
+        self.frac32 = np.empty((N, 3), dtype=np.float32)
         # two staging buffers (one float64, one 32-bit) so that a batch is two host->device copies
-        f64 = np.concatenate([self.cart.ravel(), self.lattice.ravel(), inv.ravel()])
-        i32 = np.concatenate([self.atom_struct, self.atom_ptr, grid.ravel(), self.numbers.astype(np.int32),
-                              cart32.ravel().view(np.int32), lat32.ravel().view(np.int32), vol32.view(np.int32)])
-        self.f64, self.i32 = torch.from_numpy(f64), torch.from_numpy(i32)
-        if pin and torch.cuda.is_available():
-            self.f64, self.i32 = self.f64.pin_memory(), self.i32.pin_memory()
+        pin = pin and torch.cuda.is_available()
+        self.f64 = torch.empty(3 * N + 18 * B, dtype=torch.float64, pin_memory=pin)
+        self.i32 = torch.empty(5 * N + 19 * B + 1, dtype=torch.int32, pin_memory=pin)
+        _lib.check(_lib.load().mb_host_batch(B, self.atom_ptr.ctypes.data, self.numbers.ctypes.data, self.cart.ctypes.data,
+                                             self.lattice.ctypes.data, inv.ctypes.data, grid.ctypes.data, self.f64.data_ptr(),
+                                             self.i32.data_ptr(), self.frac32.ctypes.data), "mb_host_batch")
         self.h2d_bytes = self.f64.numel() * 8 + self.i32.numel() * 4
 
 
@@ -154,7 +140,7 @@ def upload(hb: HostBatch, cutoff, line_cutoff, device) -> BatchedGraph:
     g.n_atoms, g.n_struct, g.n_cells = N, Bn, hb.n_cells
     g.cutoff, g.line_cutoff = float(cutoff), float(line_cutoff)
     g.atoms_per_graph, g.atom_ptr_host, g.numbers_host = hb.atoms_per_graph, hb.atom_ptr, hb.numbers
-    g.cart64_host, g.lattice64_host, g.frac32_host = hb.cart, hb.lattice, hb.frac32
+    g.cart64_host, g.lattice64_host, g.frac32_host, g.volume64_host = hb.cart, hb.lattice, hb.frac32, hb.volume
     g.cart64, g.lattice64, g.inv_lattice64 = f64[:3 * N].view(N, 3), f64[3 * N:3 * N + 9 * Bn].view(Bn, 3, 3), \
         f64[3 * N + 9 * Bn:].view(Bn, 3, 3)
     o = 0
@@ -178,9 +164,7 @@ def _capacity_estimate(g: BatchedGraph) -> tuple[int, int]:
     sphere; triplets = ordered pairs of short bonds per atom), with a margin.  A guess that turns out too small costs
     one more launch with the exact sizes."""
     n = np.asarray(g.atoms_per_graph, dtype=np.float64)
-    lat = g.lattice64_host
-    vol = np.abs(np.einsum("bi,bi->b", lat[:, 0], np.cross(lat[:, 1], lat[:, 2])))
-    rho = n / vol
+    rho = n / g.volume64_host
     nbr = 4.0 / 3.0 * np.pi * g.cutoff ** 3 * rho
     short = 4.0 / 3.0 * np.pi * g.line_cutoff ** 3 * rho
     edges = float((n * nbr).sum())
@@ -224,7 +208,7 @@ class _Candidates:
         self.skin, self.cap = float(skin), int(cap)
         n_atoms = g.n_atoms
         n_per = np.asarray(g.atoms_per_graph, dtype=np.int64)
-        grid, self.n_cells = cell_grid(g.lattice64_host, n_per, g.cutoff + self.skin)
+        grid, self.n_cells, _ = cell_grid(g.lattice64_host, n_per, g.cutoff + self.skin)
         self.grid = torch.from_numpy(grid).to(device)
         i64 = lambda n: torch.empty(max(int(n), 1), dtype=torch.int64, device=device)  # noqa: E731
         f64 = lambda n: torch.empty(max(int(n), 1), dtype=torch.float64, device=device)  # noqa: E731
@@ -245,9 +229,7 @@ class _Candidates:
 
 def _candidate_capacity(g: BatchedGraph, skin: float) -> int:
     n = np.asarray(g.atoms_per_graph, dtype=np.float64)
-    lat = g.lattice64_host
-    vol = np.abs(np.einsum("bi,bi->b", lat[:, 0], np.cross(lat[:, 1], lat[:, 2])))
-    cap = int(1.25 * float((n * 4.0 / 3.0 * np.pi * (g.cutoff + skin) ** 3 * n / vol).sum())) + 1024
+    cap = int(1.25 * float((n * 4.0 / 3.0 * np.pi * (g.cutoff + skin) ** 3 * n / g.volume64_host).sum())) + 1024
     return cap + (cap & 1)
 
 
