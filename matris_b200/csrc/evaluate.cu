@@ -3,7 +3,7 @@
 //
 // What bounds a small system is the host: an evaluation is 600 - 800 launches, and from an interpreter each costs about
 // 20 us (descriptor packing, foreign-function call, tensor allocation, autograd bookkeeping), 13 ms in all, while the
-// device needs 9 ms.  Queued from here a launch costs 2 - 3 us.
+// device needs 9 ms.  Queued from here a launch costs 2 - 3 us: 4 atoms 13.2 -> 9.2 ms, bound by the device.
 //
 // Memory is handed out from two stacks: inputs of the sub-blocks (always needed by the backward pass) and temporaries on the
 // bottom one, internals of the layers that keep them on the top one.  The backward pass pops both in reverse order.  A small

@@ -443,7 +443,7 @@ class MatRIS(nn.Module):
             raise RuntimeError("matris_b200 runs on a CUDA device only: move the model with .to('cuda')")
         g = self._as_batch(graphs)
         self.last_batch = g
-        with torch.cuda.device(self.device):
+        with torch.cuda.device(g.device):
             # The GEMM kernels bound every wait and raise a status word instead of hanging.  The word of the previous
             # evaluation was copied to pinned memory in stream order; it is read here, so a failure surfaces at the
             # latest one call later and costs no synchronisation.
@@ -482,7 +482,10 @@ class MatRIS(nn.Module):
             free, total = torch.cuda.mem_get_info(self.device)
             st["total"], st["outside"] = total, total - free - torch.cuda.memory_reserved(self.device)
         st["calls"] += 1
-        avail = st["total"] - st["outside"] - torch.cuda.memory_allocated(self.device)
+        # (the one counter: torch.cuda.memory_allocated would flatten all of them on every call, while the device idles)
+        counters = torch.cuda.memory_stats_as_nested_dict(self.device)
+        allocated = counters["allocated_bytes"]["all"]["current"] if counters else 0
+        avail = st["total"] - st["outside"] - allocated
         if self.memory_limit_bytes is not None:
             avail = min(avail, float(self.memory_limit_bytes))
         return avail
@@ -526,7 +529,7 @@ class MatRIS(nn.Module):
         return split_ranges(np.diff(tp), np.diff(ep), lambda t, e: kept_layers_for(n_layers, t, e, avail) == n_layers)
 
     def _evaluate(self, g: BatchedGraph, task: str):
-        dev, n_struct, n_atoms = self.device, g.n_struct, g.n_atoms
+        dev, n_struct, n_atoms = g.device, g.n_struct, g.n_atoms
         P = self.packed(dev)
         want = {"f": 3 * n_atoms if "f" in task else 0, "s": 9 * n_struct if "s" in task else 0,
                 "m": n_atoms if "m" in task else 0}
