@@ -480,7 +480,7 @@ def main():
         # (A rows read + gate / residual rows read + output rows written); scaled here to the average launch of the
         # step by its algorithmic bytes.
         pk = clocks_peak.summary()
-        roofline = {"kernel": "k_gemm_ps + k_gated_fwd (mb_gemm, mb_gated_mlp_fwd)", "bound": "tensor", "achieved": ach,
+        roofline = {"kernel": "k_linear + k_mlp (mb_gemm, mb_gated_mlp_fwd, mb_mlp_bwd_data)", "bound": "tensor", "achieved": ach,
                     "peak": peak_tf, "unit": "TFLOP/s", "frac": ach / peak_tf, "traffic": 0.93 * gemm_bytes / n_gemm,
                     "traffic_note": "bytes per average launch, scaled from ncu captures by the algorithmic bytes",
                     "peak_source": src + " bf16 sustained",
