@@ -44,9 +44,16 @@ def as_arrays(structure) -> tuple[np.ndarray, np.ndarray, np.ndarray]:
         numbers, cart, lattice = structure.numbers, structure.cart, structure.lattice
     else:
         numbers, cart, lattice = structure
-    numbers = np.ascontiguousarray(numbers, dtype=np.int64).reshape(-1)
-    cart = np.ascontiguousarray(cart, dtype=np.float64).reshape(-1, 3)
-    lattice = np.ascontiguousarray(lattice, dtype=np.float64).reshape(3, 3)
+    numbers = np.ascontiguousarray(numbers, dtype=np.int64)
+    cart = np.ascontiguousarray(cart, dtype=np.float64)
+    lattice = np.ascontiguousarray(lattice, dtype=np.float64)
+    # (a list is hundreds of structures, nearly all of these shapes already)
+    if numbers.ndim != 1:
+        numbers = numbers.reshape(-1)
+    if cart.ndim != 2 or cart.shape[1] != 3:
+        cart = cart.reshape(-1, 3)
+    if lattice.shape != (3, 3):
+        lattice = lattice.reshape(3, 3)
     if len(numbers) != len(cart):
         raise ValueError("numbers and positions differ in length")
     return numbers, cart, lattice
@@ -181,14 +188,18 @@ class _GraphBuffers:
         cap_e += cap_e & 1
         n_atoms, n_cells = g.n_atoms, g.n_cells
         self.cap_e, self.cap_t = cap_e, cap_t
-        i64 = lambda n: torch.empty(max(int(n), 1), dtype=torch.int64, device=device)  # noqa: E731
-        self.scratch = dict(
-            cell_ptr=_i32(n_cells + 1, device), cell_fill=_i32(n_cells, device), cell_atoms=_i32(n_atoms, device),
-            atom_cell=_i32(4 * n_atoms, device), atom_wrap=_i32(4 * n_atoms, device),
-            scan_tmp=_i32(lib.mb_graph_scan_tmp_len(max(n_atoms, n_cells, cap_e)), device),
-            key_unsorted=i64(cap_e), dist_unsorted=torch.empty(cap_e, dtype=torch.float64, device=device),
-            key=i64(cap_e), atom_counts=_i32(2 * n_atoms, device), edge_rank=_i32(2 * cap_e + 2, device),
-            bond_counts=_i32(cap_e + 4, device), edge_flag=torch.empty(cap_e, dtype=torch.uint8, device=device))
+        # scratch: bytes of each array, handed to the library as addresses inside one allocation
+        sizes = dict(
+            cell_ptr=4 * (n_cells + 1), cell_fill=4 * n_cells, cell_atoms=4 * n_atoms, atom_cell=16 * n_atoms,
+            atom_wrap=16 * n_atoms, scan_tmp=4 * lib.mb_graph_scan_tmp_len(max(n_atoms, n_cells, cap_e)),
+            key_unsorted=8 * cap_e, dist_unsorted=8 * cap_e, key=8 * cap_e, atom_counts=8 * n_atoms,
+            edge_rank=4 * (2 * cap_e + 2), bond_counts=4 * (cap_e + 4), edge_flag=cap_e)
+        offsets, total = {}, 0
+        for k, n in sizes.items():
+            offsets[k], total = total, total + (int(n) + 255) // 256 * 256
+        self.scratch_bytes = torch.empty(total, dtype=torch.uint8, device=device)
+        base = self.scratch_bytes.data_ptr()
+        self.scratch = {k: base + o for k, o in offsets.items()}
         self.out = dict(
             edge_ptr=_i32(n_atoms + 1, device), center=_i32(cap_e, device), neighbor=_i32(cap_e, device),
             image=_i32(3 * cap_e, device), dist=torch.empty(cap_e, dtype=torch.float64, device=device),
@@ -196,7 +207,7 @@ class _GraphBuffers:
             trip_ptr=_i32(cap_e // 2 + 1, device), trip_src_ptr=_i32(cap_e // 2 + 1, device),
             line_graph=_i32(5 * cap_t, device), trip_src_perm=_i32(cap_t, device))
         self.counts = torch.zeros(64, dtype=torch.int32, device=device)  # 16 used; the rest is spare
-        self.counts_host = torch.zeros(64, dtype=torch.int32).pin_memory()
+        self.counts_host = torch.zeros(64, dtype=torch.int32, pin_memory=True)
 
 
 class _Candidates:
@@ -284,8 +295,8 @@ def build_on_device(g: BatchedGraph, tol: float = 1e-8, stream=None, skin: float
             m = base_desc()
             m.n_cells, m.cap_edges, m.cap_triplets = n_cells, buf.cap_e, buf.cap_t
             m.cutoff, m.line_cutoff, m.grid = g.cutoff, g.line_cutoff, g.grid.data_ptr()
-            for k, v in buf.scratch.items():
-                setattr(m, k, v.data_ptr())
+            for k, address in buf.scratch.items():
+                setattr(m, k, address)
             for k, v in buf.out.items():
                 setattr(m, k, v.data_ptr())
             m.counts = buf.counts.data_ptr()
