@@ -70,6 +70,14 @@ __global__ void k_force_stress_finish(int n_atoms, int n_struct, const float* __
   if (s && i < 9 * (int64_t)n_struct) s[i] = dstrain[i] * (160.21766208f / volume[i / 9]);
 }
 
+// a memset that joins the chain of programmatic launches (the copy engine's would end it before and after): n 4-byte words
+__global__ void k_zero(size_t n, float* __restrict__ p) {
+  pdl_sync();
+  const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  if (i + 4 <= n) *reinterpret_cast<float4*>(p + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+  else for (size_t k = i; k < n; ++k) p[k] = 0.f;
+}
+
 // ------------------------------------------------------------------ instrumentation
 struct OpTimes {
   bool on = false;
@@ -214,7 +222,7 @@ struct Run {
     if (!g_times.on) {
       launch_after_event = behind[on];
       rc = f();
-      behind[on] = launch_after_event;  // (a memset or copy leaves it)
+      behind[on] = launch_after_event;  // (what launches nothing leaves it)
       launch_after_event = false;
       return;
     }
@@ -227,15 +235,11 @@ struct Run {
     cudaEventRecord(rec.b, st);
     g_times.recs.push_back(rec);
   }
-  void zero(void* p, size_t bytes) {
+  void zero(float* p, size_t bytes) {
+    if (bytes == 0) return;
     op("memset", [&] {
-      MB_CUDA_CHECK(cudaMemsetAsync(p, 0, bytes, st));
-      return (int)MB_OK;
-    });
-  }
-  void copy(void* d, const void* s, size_t bytes) {
-    op("memcpy", [&] {
-      MB_CUDA_CHECK(cudaMemcpyAsync(d, s, bytes, cudaMemcpyDeviceToDevice, st));
+      launch(k_zero, (unsigned)((bytes / 16 + 256) / 256), 256, 0, st, bytes / 4, p);
+      MB_LAUNCH_CHECK("k_zero");
       return (int)MB_OK;
     });
   }
