@@ -103,10 +103,11 @@ __global__ void k_gate_bwd(int64_t n_rows, const float* __restrict__ z, const fl
 // walking a segment in two passes, 295 with batches of eight rows, 233 with four (64 registers, twice the warps).  Atom graph of
 // 9372 atoms / 234,096 edges 103 -> 105 us (eight warps: 124), of 32 atoms a third of the time.
 template <int WARPS>
-__global__ void __launch_bounds__(WARPS == 1 ? RW_THREADS : 128, WARPS == 1 ? 4 : 5) k_seg_attn_fwd(int n_nodes, const int32_t* __restrict__ tgt_ptr, const int32_t* __restrict__ src_ptr,
-                               const int32_t* __restrict__ src_perm, const int32_t* __restrict__ emap,
-                               const float* __restrict__ logits, const float* __restrict__ h,
-                               float* __restrict__ agg_t, float* __restrict__ agg_s, float* __restrict__ stats) {
+__global__ void __launch_bounds__(WARPS == 1 ? RW_THREADS : 128, WARPS == 1 ? 4 : 5)
+k_seg_attn_fwd(int n_nodes, const int32_t* __restrict__ tgt_ptr, const int32_t* __restrict__ src_ptr,
+               const int32_t* __restrict__ src_perm, const int32_t* __restrict__ emap,
+               const float* __restrict__ logits, const float* __restrict__ h,
+               float* __restrict__ agg_t, float* __restrict__ agg_s, float* __restrict__ stats) {
   pdl_sync();
   constexpr int NB = WARPS == 1 ? 4 : 8;
   __shared__ float4 part[WARPS > 1 ? 3 : 1][WARPS > 1 ? WARPS : 1][WARPS > 1 ? 32 : 1];
@@ -177,15 +178,16 @@ __global__ void __launch_bounds__(WARPS == 1 ? RW_THREADS : 128, WARPS == 1 ? 4 
 
 // Latency of the gathered rows bounds it (5 TB/s of DRAM traffic at half occupancy): six blocks per SM, even with a few spills, beat
 // what 62 registers allow.  522,844 angles 579 -> 526 us, 234,096 edges 252 -> 229; eight blocks 557 and 242.
-__global__ void __launch_bounds__(RW_THREADS, 6) k_seg_attn_bwd(int64_t n_rows, const int32_t* __restrict__ tgt, const int32_t* __restrict__ src,
-                               int idx_stride, const int32_t* __restrict__ emap, const float* __restrict__ logits,
-                               const float* __restrict__ h, const float* __restrict__ agg_t,
-                               const float* __restrict__ agg_s, const float* __restrict__ stats,
-                               const float* __restrict__ dagg_t, const float* __restrict__ dagg_s,
-                               const float* __restrict__ dh_in, const int32_t* __restrict__ dh_map, float dh_scale,
-                               float* __restrict__ dh, float* __restrict__ dlogits, const float* __restrict__ gate_z,
-                               const float* __restrict__ gate_wc, const float* __restrict__ gate_wg,
-                               float* __restrict__ gate_dz) {
+__global__ void __launch_bounds__(RW_THREADS, 6)
+k_seg_attn_bwd(int64_t n_rows, const int32_t* __restrict__ tgt, const int32_t* __restrict__ src,
+               int idx_stride, const int32_t* __restrict__ emap, const float* __restrict__ logits,
+               const float* __restrict__ h, const float* __restrict__ agg_t,
+               const float* __restrict__ agg_s, const float* __restrict__ stats,
+               const float* __restrict__ dagg_t, const float* __restrict__ dagg_s,
+               const float* __restrict__ dh_in, const int32_t* __restrict__ dh_map, float dh_scale,
+               float* __restrict__ dh, float* __restrict__ dlogits, const float* __restrict__ gate_z,
+               const float* __restrict__ gate_wc, const float* __restrict__ gate_wg,
+               float* __restrict__ gate_dz) {
   pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
   const int64_t nt = tgt[row * idx_stride], ns = src[row * idx_stride];
@@ -250,12 +252,13 @@ __global__ void k_seg_smooth_sum_fwd(int n_nodes, const int32_t* __restrict__ tg
 
 // Bounded by latency like k_seg_attn_bwd; the exponentials of the gate's adjoint come next.  522,844 angles with the adjoint: one
 // sigmoid per branch instead of three in all 351 -> 301 us, eight blocks per SM 274 us; 234,096 edges 156 -> 125.
-__global__ void __launch_bounds__(RW_THREADS, 8) k_seg_smooth_sum_bwd_rows(int64_t n_rows, const int32_t* __restrict__ tgt,
-                                          const int32_t* __restrict__ src, int idx_stride,
-                                          const int32_t* __restrict__ emap, const float* __restrict__ env,
-                                          const float* __restrict__ dagg, float* __restrict__ dh, int accumulate,
-                                          const float* __restrict__ gate_z, const float* __restrict__ gate_wc,
-                                          const float* __restrict__ gate_wg, float* __restrict__ gate_dz) {
+__global__ void __launch_bounds__(RW_THREADS, 8)
+k_seg_smooth_sum_bwd_rows(int64_t n_rows, const int32_t* __restrict__ tgt,
+                          const int32_t* __restrict__ src, int idx_stride,
+                          const int32_t* __restrict__ emap, const float* __restrict__ env,
+                          const float* __restrict__ dagg, float* __restrict__ dh, int accumulate,
+                          const float* __restrict__ gate_z, const float* __restrict__ gate_wc,
+                          const float* __restrict__ gate_wg, float* __restrict__ gate_dz) {
   pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
   const int64_t nt = tgt[row * idx_stride];
@@ -293,11 +296,12 @@ __global__ void k_mul_rows_gather(int64_t n_rows, const float* __restrict__ x, c
 }
 
 // Four rows in flight and six blocks per SM (40 registers): 180 -> 121 us for 117,048 bonds / 522,844 angles (four blocks 156).
-__global__ void __launch_bounds__(RW_THREADS, 6) k_smooth_env_bwd_line(int n_nodes, const int32_t* __restrict__ tgt_ptr,
-                                      const int32_t* __restrict__ src_ptr, const int32_t* __restrict__ src_perm,
-                                      const int32_t* __restrict__ tgt, const int32_t* __restrict__ src,
-                                      int idx_stride, const float* __restrict__ env, const float* __restrict__ h,
-                                      const float* __restrict__ dagg, float* __restrict__ denv) {
+__global__ void __launch_bounds__(RW_THREADS, 6)
+k_smooth_env_bwd_line(int n_nodes, const int32_t* __restrict__ tgt_ptr,
+                      const int32_t* __restrict__ src_ptr, const int32_t* __restrict__ src_perm,
+                      const int32_t* __restrict__ tgt, const int32_t* __restrict__ src,
+                      int idx_stride, const float* __restrict__ env, const float* __restrict__ h,
+                      const float* __restrict__ dagg, float* __restrict__ denv) {
   pdl_sync();
   MB_ROW_PROLOGUE(n_nodes)
   constexpr int NB = 4;  // rows in flight
@@ -348,9 +352,10 @@ __global__ void __launch_bounds__(RW_THREADS, 6) k_smooth_env_bwd_line(int n_nod
 // segments would otherwise be walked by a handful of warps.
 // 117,048 bonds 178 -> 162 us with four blocks per SM (five: 193, spilling), 9372 atoms 73 -> 62 with eight.
 template <int WARPS>
-__global__ void __launch_bounds__(256, WARPS == 1 ? 4 : 8) k_seg_sum(int n_nodes, const int32_t* __restrict__ tgt_ptr, const int32_t* __restrict__ src_ptr,
-                          const int32_t* __restrict__ src_perm, const int32_t* __restrict__ ctr,
-                          const float* __restrict__ x, float* __restrict__ out, float* __restrict__ ctr_out) {
+__global__ void __launch_bounds__(256, WARPS == 1 ? 4 : 8)
+k_seg_sum(int n_nodes, const int32_t* __restrict__ tgt_ptr, const int32_t* __restrict__ src_ptr,
+          const int32_t* __restrict__ src_perm, const int32_t* __restrict__ ctr,
+          const float* __restrict__ x, float* __restrict__ out, float* __restrict__ ctr_out) {
   pdl_sync();
   constexpr int NB = 4;  // rows in flight per warp
   __shared__ float4 part[WARPS > 1 ? WARPS : 1][WARPS > 1 ? 64 : 1];
