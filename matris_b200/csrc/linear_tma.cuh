@@ -287,13 +287,13 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
     bool alive = true;
     uint32_t g = (uint32_t)parity, conv_n = 0;
     auto tile_row = [&](int t) { return (first_rt + t * step_rt) * 128 + quarter * 32; };
-    auto request = [&](int t, int s, int k) {
+    auto request = [&](int t, int s, int k, bool stored) {
       if (lane == 0 && alive) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(my_conv), "r"(ML_PATCH) : "memory");
-        tma_load_2d(patch, &maps.src[shared_a ? s : j0 + s], my_conv, 32 * (parity + 2 * k), tile_row(t));
+        if (stored) to_async_proxy();  // the patch held gathered rows
+        load_patch(&maps.src[shared_a ? s : j0 + s], patch, my_conv, 32 * (parity + 2 * k), tile_row(t));
       }
     };
-    if (segment(0).idx == nullptr) request(0, 0, 0);
+    if (segment(0).idx == nullptr) request(0, 0, 0, false);
     for (int t = 0; t < n_tiles; ++t) {
       const int64_t row0 = tile_row(t);
       auto row_of = [&](int i) { const int64_t r = row0 + lr + 4 * i; return r < n_rows ? r : n_rows - 1; };
@@ -347,7 +347,7 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
           // next chunk overwrite it.  Issued right after the reads it could overtake them.
           __syncwarp();
           const int s2 = k == 0 ? s : (s + 1 < n_seg ? s + 1 : 0), t2 = k == 1 && s + 1 == n_seg ? t + 1 : t;
-          if (t2 < n_tiles && segment(s2).idx == nullptr) request(t2, s2, k ^ 1);
+          if (t2 < n_tiles && segment(s2).idx == nullptr) request(t2, s2, k ^ 1, idx != nullptr);
           asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();

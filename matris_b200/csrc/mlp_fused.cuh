@@ -86,6 +86,9 @@ __device__ __forceinline__ float4 lds4(uint32_t addr) {
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
   return v;
 }
+// Between ordinary accesses of a patch and the copy engine's writes to it: a barrier orders the threads, not the two proxies.
+// Any thread on the path from the last ordinary store to the copy may execute it; here it is the one that issues the copy.
+__device__ __forceinline__ void to_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
 }
@@ -386,8 +389,10 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
     auto request = [&](uint32_t n, int k, int row0) {  // residual patch k (EPI_RES)
       if (!alive) return;
       asked = n + 1;
-      if (lane == 0)
+      if (lane == 0) {
+        to_async_proxy();  // the buffer held addend sums that a producer warp stored
         load_patch(&maps.res, side0 + (n & 1) * ML_PATCH, my_full + 8 * (n & 1), 64 * grp + 32 * k, row0);
+      }
     };
     // finished columns `col`..: h = v and / or out2 = v + res_w * res (the residual rows arrive as a side patch)
     auto finish = [&](float (&v)[32], int col, int row0) {
@@ -592,9 +597,11 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
     };
     auto tile_row = [&](int t) { return (first_rt + t * step_rt) * 128 + quarter * 32; };
     auto is_direct = [&](int s) { return (s < d.n_src ? d.src[s].idx : d.ext[s - d.n_src].idx) == nullptr; };
-    auto request = [&](int t, int s, int k) {  // rows read in place: this warp's chunk k of segment s
-      if (lane == 0 && alive)
+    auto request = [&](int t, int s, int k, bool stored) {  // rows read in place: this warp's chunk k of segment s
+      if (lane == 0 && alive) {
+        if (stored) to_async_proxy();  // the patch held gathered rows
         load_patch(s < d.n_src ? &maps.src[s] : &maps.ext[s - d.n_src], patch, my_conv, 32 * (parity + 2 * k), tile_row(t));
+      }
     };
     auto wait_empty = [&]() {  // the next side patch may be filled
       if (side_n >= 2 && alive) alive = mbar_wait(side_empty + 8 * (2 * pw + (side_n & 1)), ((side_n >> 1) - 1) & 1);
@@ -653,7 +660,7 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
         if (lane == 0) mbar_arrive(side_full + 8 * (2 * pw + (side_n & 1)));
       }
     };
-    if (n_seg > 0 && is_direct(0)) request(0, 0, 0);
+    if (n_seg > 0 && is_direct(0)) request(0, 0, 0, false);
     asm volatile("bar.sync 5, 512;" ::: "memory");  // the constants are there
     for (int t = 0; t < n_tiles; ++t) {
       const int64_t row0 = tile_row(t);
@@ -710,7 +717,7 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
           // next chunk overwrite it.  Issued right after the reads it could overtake them.
           __syncwarp();
           const int s2 = k == 0 ? s : (s + 1 < n_seg ? s + 1 : 0), t2 = k == 1 && s + 1 == n_seg ? t + 1 : t;
-          if (t2 < n_tiles && is_direct(s2)) request(t2, s2, k ^ 1);
+          if (t2 < n_tiles && is_direct(s2)) request(t2, s2, k ^ 1, idx != nullptr);
           asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
