@@ -223,8 +223,8 @@ int mb_set_gemm_mode(int mode);
 int mb_gemm_status(int* status, void* stream);
 int mb_gemm_status_async(int* host_status, void* stream);
 int mb_gemm_status_clear(void* stream);
-/* Self-test of the failure path above: launches one CTA that waits, with a limit of a few polls, on an mbarrier
- * that nothing ever arrives at.  The wait runs out, the kernel sets bit 0 of the status word and returns through
+/* Self-test of the failure path above: launches one CTA that waits, as the tensor-core kernels do, on an
+ * mbarrier that nothing ever arrives at.  The wait runs out after its limit (2 seconds), the kernel sets bit 0 of the status word and returns through
  * its normal exit; nothing faults, traps or hangs.  The next mb_gemm_status* call sees bit 0. */
 int mb_selftest_wait_expiry(void* stream);
 /* Timed issue rate of the tensor-core instruction the kernels above are built on: every SM runs `iters` batches of

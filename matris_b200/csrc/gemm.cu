@@ -215,7 +215,7 @@ constexpr int TC_XPOSE_BYTES = 4 * TC_A_STAGES * 32 * 128;  // per producer warp
 constexpr int TC_SMEM_BYTES = TC_RING_BYTES + TC_XPOSE_BYTES + 128 /*barriers, tmem slot*/;
 constexpr uint32_t TC_TMEM_COLS = 256;
 constexpr uint32_t TC_IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
-constexpr uint32_t TC_WAIT_LIMIT = 1u << 22;     // polls per wait
+constexpr uint32_t WAIT_LIMIT_NS = 2000000000u;  // of one wait on an mbarrier; the longest legitimate one takes milliseconds
 static_assert(128 * TC_STAGE_LD * 4 <= TC_RING_BYTES + TC_XPOSE_BYTES, "staging area must fit in ring + patches");
 static_assert(2 * (TC_SMEM_BYTES + 1024) <= 227 * 1024, "two CTAs per SM");
 
@@ -225,15 +225,32 @@ __device__ int g_gemm_status = 0;  // bit 0: an mbarrier wait expired
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// Bounded wait.  try_wait parks the thread for a while in hardware: against a loop of test_wait polls the waiting warps leave the
-// issue slots to the others (gated MLP forward 0.71 -> 0.67 ms, plain backward 0.24 -> 0.19 ms at 573,894 rows).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit = TC_WAIT_LIMIT) {
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  for (uint32_t it = 0; it < limit; ++it) {
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    if (ok) return true;
-  }
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ uint32_t global_ns() {  // low word: differences of up to 4.29 s
+  uint32_t t;
+  asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
+  return t;
+}
+// Bounded wait: gives up WAIT_LIMIT_NS after its first poll has failed.  The limit is a time and not a number of polls because the
+// hardware chooses how long try_wait parks the thread.  It parks it at all so that the waiting warps leave the issue slots to
+// the others (against a loop of test_wait polls: gated MLP forward 0.71 -> 0.67 ms, plain backward 0.24 -> 0.19 ms at 573,894 rows);
+// reading the clock between polls, which takes longer than counting them, leaves them more (4 atoms 5.37 -> 5.02 ms an evaluation,
+// energies of 96 crystals 11.25 -> 10.57).
+__device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity) {
+  if (mbar_try(bar, parity)) return true;
+  const uint32_t t0 = global_ns();
+  do {
+    if (mbar_try(bar, parity)) return true;
+  } while (global_ns() - t0 < WAIT_LIMIT_NS);
+  return false;
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+  if (mbar_poll(bar, parity)) return true;
   atomicOr(&g_gemm_status, 1);
   return false;
 }
@@ -670,7 +687,7 @@ __global__ void k_add_gathered(int64_t n_rows, int n_add, const AddList adds, in
   *reinterpret_cast<float4*>(z1 + row * ld + c) = v;
 }
 
-// ---- self-test of the bounded wait: a barrier nothing arrives at, a limit of a few polls
+// ---- self-test of the bounded wait: a barrier nothing arrives at
 __global__ void k_selftest_wait_expiry() {
   __shared__ uint64_t bar;
   if (threadIdx.x == 0) {
@@ -678,8 +695,7 @@ __global__ void k_selftest_wait_expiry() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  // same wait, same give-up path as in the GEMM kernels (status bit 0), with 8 polls instead of 2^22
-  if (threadIdx.x == 0) mbar_wait(smem_u32(&bar), 0, 8);
+  if (threadIdx.x == 0) mbar_wait(smem_u32(&bar), 0);  // the wait of the tensor-core kernels, its limit and its give-up path
   __syncthreads();
 }
 
@@ -731,8 +747,10 @@ __global__ void __launch_bounds__(128, 1) k_mma_rate(int iters) {
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                    :: "r"(smem_u32(&bar)) : "memory");
     __syncwarp();
-    // every issued instruction has retired when the commit arrives; bounded like every other wait here
-    mbar_wait(smem_u32(&bar), 0, 1u << 22);
+    // every issued instruction has retired when the commit arrives: 2.6 s for the most iterations a caller may ask for
+    bool retired = false;
+    for (int i = 0; i < 5 && !retired; ++i) retired = mbar_poll(smem_u32(&bar), 0);
+    if (!retired) atomicOr(&g_gemm_status, 1);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
