@@ -262,6 +262,22 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(bar) : "memory");
 }
 
+// One arrival when everything this thread has issued to the tensor cores so far has retired (it retires in order).
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
+}
+// What a role does before the common exit, whatever became of the others: nothing it started may still read or write this CTA's
+// shared or tensor memory when they are given back.  On the normal path its consumers have long waited for the same things.
+__device__ __forceinline__ void drain_mma(uint32_t bar, bool issuer) {  // bar: not used for anything else
+  if (issuer) mma_commit(bar);
+  __syncwarp();
+  mbar_wait(bar, 0);
+}
+// The last of `n` copies that went through the barriers bar, bar + 8, .. (n_slots of them) in turn, one phase each.
+__device__ __forceinline__ void drain_copies(uint32_t bar, uint32_t n_slots, uint32_t n) {
+  for (uint32_t i = n >= n_slots ? n - n_slots : 0; i < n; ++i) mbar_wait(bar + 8 * (i % n_slots), (i / n_slots) & 1);
+}
+
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
   // K-major, SWIZZLE_128B: start address, LBO = 1 (unused), SBO = 1024 B between 8-row groups, version 1
   return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
@@ -319,7 +335,8 @@ k_gemm_tc(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ TcMaps
   const mb_colblock& cb = d.blk[jb];
   extern __shared__ __align__(1024) uint8_t smem[];  // W ring (1024-byte aligned tiles) | transpose patches | barriers
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TC_RING_BYTES + TC_XPOSE_BYTES);
-  // bars[0..1]: A buffer full (4 producer warps); bars[2..3]: W slot landed (TMA); bars[5..6]: MMAs of a chunk done
+  // bars[0..1]: A buffer full (4 producer warps); bars[2..3]: W slot landed (TMA); bars[4]: everything has retired;
+  // bars[5..6]: MMAs of a chunk done
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + TC_RING_BYTES + TC_XPOSE_BYTES + 64);
   if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled tiles need a 1024-byte aligned base
     if (threadIdx.x == 0) atomicOr(&g_gemm_status, 2);
@@ -391,6 +408,7 @@ k_gemm_tc(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ TcMaps
       mbar_init(a_full, 4); mbar_init(a_full + 8, 4);
       mbar_init(w_full, 1); mbar_init(w_full + 8, 1);
       mbar_init(mma_done, 1); mbar_init(mma_done + 8, 1);
+      mbar_init(smem_u32(bars + 4), 1);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       load_w(0);  // the first weight tiles travel while tensor memory is being allocated
@@ -414,7 +432,8 @@ k_gemm_tc(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ TcMaps
     // ------------------------------------------------------------ control thread: TMA + MMA issue
     if (lane == 0) {
       bool alive = true;
-      for (int c = 0; c < n_chunks; ++c) {
+      uint32_t n_loads = n_chunks > 1 ? 2 : 1;
+      for (int c = 0; c < n_chunks && alive; ++c) {
         const int ab = c & 1;  // A buffer, W slot and completion barrier of this chunk
         if (alive) alive = mbar_wait(a_full + 8 * ab, (uint32_t)((c >> 1) & 1));
         if (alive) alive = mbar_wait(w_full + 8 * ab, (uint32_t)((c >> 1) & 1));
@@ -432,11 +451,19 @@ k_gemm_tc(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ TcMaps
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                      :: "r"(mma_done + 8 * ab) : "memory");
         if (c + 2 < n_chunks) {  // this chunk's W slot is refilled as soon as its MMAs have retired
-          if (alive) alive = mbar_wait(mma_done + 8 * ab, (uint32_t)((c >> 1) & 1));
-          load_w(c + 2);
+          alive = alive && mbar_wait(mma_done + 8 * ab, (uint32_t)((c >> 1) & 1));
+          if (alive) {
+            load_w(c + 2);
+            ++n_loads;
+          }
         }
       }
+      mma_commit(smem_u32(bars + 4));
+      mbar_wait(smem_u32(bars + 4), 0);
+      drain_copies(w_full, 2, n_loads);
     }
+    __syncwarp();
+    asm volatile("bar.arrive 1, 160;" ::: "memory");  // tensor memory may go
     return;
   }
 
@@ -499,7 +526,7 @@ k_gemm_tc(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ TcMaps
       *reinterpret_cast<uint4*>(stage + tid * TC_STAGE_LD + cg * 32 + 4 * q) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps only
+  asm volatile("bar.sync 1, 160;" ::: "memory");  // the four epilogue warps, and the control warp has nothing in flight
   if (warp == 0) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"(TC_TMEM_COLS) : "memory");
   }

@@ -188,12 +188,12 @@ k_gemm_ps(const __grid_constant__ mb_gemm_desc d_param, const __grid_constant__ 
   }
   // barriers: a_ready[8] (A chunk stored: 4 producer warps) | a_done[8] (its MMAs retired: the A buffer is free) |
   //           w_ready[4] (W slot landed: the TMA thread's expect_tx arrival + bytes) | w_done[4] (slot free) |
-  //           d_full[2] | d_free[2] (8 epilogue warps).  Chunk g uses A buffer g % NB; W-slot use u = g / CPW uses
+  //           d_full[2] | d_free[2] (8 epilogue warps) | retired.  Chunk g uses A buffer g % NB; W-slot use u = g / CPW uses
   //           ring slot u % w_period.  Every waiter sees every phase of the barriers it waits on (a parity wait can
   //           tell apart only two consecutive phases).
   const uint32_t a_ready = smem_u32(bars), a_done = smem_u32(bars + 8);
   const uint32_t w_ready = smem_u32(bars + 16), w_done = smem_u32(bars + 20);
-  const uint32_t d_full = smem_u32(bars + 24), d_free = smem_u32(bars + 26);
+  const uint32_t d_full = smem_u32(bars + 24), d_free = smem_u32(bars + 26), retired = smem_u32(bars + 28);
   const uint32_t ring = smem_u32(smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // The descriptor is indexed dynamically (column block, K segment) all through the kernel.  From kernel-parameter
@@ -296,6 +296,7 @@ k_gemm_ps(const __grid_constant__ mb_gemm_desc d_param, const __grid_constant__ 
       for (int b = 0; b < 8; ++b) { mbar_init(a_ready + 8 * b, 4); mbar_init(a_done + 8 * b, 1); }
       for (int b = 0; b < 4; ++b) { mbar_init(w_ready + 8 * b, 1); mbar_init(w_done + 8 * b, 1); }
       for (int b = 0; b < 2; ++b) { mbar_init(d_full + 8 * b, 1); mbar_init(d_free + 8 * b, 8); }
+      mbar_init(retired, 1);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -361,6 +362,7 @@ k_gemm_ps(const __grid_constant__ mb_gemm_desc d_param, const __grid_constant__ 
       }
       if (sh && jb == n_blocks - 1) ++t_sh;
     }
+    drain_mma(retired, elected);
   } else if (warp == PS_TMA_WARP) {
     // ---------------------------------------------------------------- TMA warp: W_hi / W_lo tiles, up to 4 chunks ahead
     // (warp-uniform loop, one elected lane issues: same reason as in the MMA warp)
@@ -392,10 +394,7 @@ k_gemm_ps(const __grid_constant__ mb_gemm_desc d_param, const __grid_constant__ 
         __syncwarp();
       }
     }
-    if (!alive) {  // failure path only: no TMA write may still be in flight when the CTA's shared memory is released
-      for (uint32_t i = wu >= w_period ? wu - w_period : 0; i < wu; ++i)
-        mbar_wait(w_ready + 8 * (i % w_period), (i / w_period) & 1);
-    }
+    drain_copies(w_ready, w_period, wu);
   } else if (warp >= PS_EPI_WARP0) {
     // ---------------------------------------------------------------- epilogue warps
     // Epilogue warp e finishes rows 32 (warp & 3).. (its TMEM lane quarter), columns 64 (e >> 2).. of the accumulator

@@ -39,10 +39,11 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
     return;
   }
   // a_ready[4] (4 producer warps) a_done[4] | w_ready[5] w_done[5] | d_full[6] d_free[6] (4 epilogue warps; block number mod 6:
-  // always the same region and the same group) | side_full[8][2] side_empty[8][2] | conv_full[8]
+  // always the same region and the same group) | side_full[8][2] side_empty[8][2] | conv_full[8] | retired
   const uint32_t bar0 = smem_u32(bars);
   const uint32_t a_ready = bar0, a_done = bar0 + 32, w_ready = bar0 + 64, w_done = bar0 + 104, d_full = bar0 + 144,
-                 d_free = bar0 + 192, side_full = bar0 + 256, side_empty = bar0 + 384, conv_full = bar0 + 512;
+                 d_free = bar0 + 192, side_full = bar0 + 256, side_empty = bar0 + 384, conv_full = bar0 + 512,
+                 retired = bar0 + 576;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   float* const cst = reinterpret_cast<float*>(smem + LN_CONST_OFF);
   const int64_t n_rows = d.n_rows;
@@ -63,6 +64,7 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
       for (int b = 0; b < 6; ++b) { mbar_init(d_full + 8 * b, 1); mbar_init(d_free + 8 * b, 4); }
       for (int b = 0; b < 16; ++b) { mbar_init(side_full + 8 * b, 1); mbar_init(side_empty + 8 * b, 1); }
       for (int b = 0; b < 8; ++b) mbar_init(conv_full + 8 * b, 1);
+      mbar_init(retired, 1);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -134,6 +136,7 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
       }
       __syncwarp();
     });
+    drain_mma(retired, elected);
   } else if (warp == ML_TMA_WARP) {
     pdl_sync();
     uint32_t elected;
@@ -158,10 +161,7 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
         if (++slot == ML_W_SLOTS) { slot = 0; ++phase; }
       }
     });
-    if (!alive) {  // failure path only: no TMA write may still be in flight when the CTA's shared memory is released
-      for (uint32_t i = n >= ML_W_SLOTS ? n - ML_W_SLOTS : 0; i < n; ++i)
-        mbar_wait(w_ready + 8 * (i % ML_W_SLOTS), (i / ML_W_SLOTS) & 1);
-    }
+    drain_copies(w_ready, ML_W_SLOTS, n);
   } else if (warp == LN_SIDE_WARP) {
     // ---------------------------------------------------------------- gate / residual patches: lane e serves epilogue warp e
     pdl_sync();
@@ -186,8 +186,7 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
           }
         }
       }
-      if (!alive)
-        for (uint32_t i = n >= 2 ? n - 2 : 0; i < n; ++i) mbar_wait(side_full + 8 * (2 * lane + (i & 1)), (i >> 1) & 1);
+      drain_copies(side_full + 16 * lane, 2, n);
     }
     __syncwarp();
   } else if (warp >= ML_EPI_WARP0) {
@@ -285,10 +284,12 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
     const uint32_t patch = sm0 + ML_CONV_OFF + pw * ML_PATCH, my_conv = conv_full + 8 * pw;
     const uint32_t put_even = lr * 128 + ((lc ^ lr) << 4), put_odd = lr * 128 + ((lc ^ (lr | 4)) << 4);
     bool alive = true;
-    uint32_t g = (uint32_t)parity, conv_n = 0;
+    uint32_t g = (uint32_t)parity, conv_n = 0, conv_asked = 0;
     auto tile_row = [&](int t) { return (first_rt + t * step_rt) * 128 + quarter * 32; };
     auto request = [&](int t, int s, int k, bool stored) {
-      if (lane == 0 && alive) {
+      if (!alive) return;
+      ++conv_asked;
+      if (lane == 0) {
         if (stored) to_async_proxy();  // the patch held gathered rows
         load_patch(&maps.src[shared_a ? s : j0 + s], patch, my_conv, 32 * (parity + 2 * k), tile_row(t));
       }
@@ -355,7 +356,7 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
         }
       }
     }
-    if (!alive) mbar_wait(my_conv, conv_n & 1);  // failure path only: no copy may still be in flight
+    if (!alive) drain_copies(my_conv, 1, conv_asked);  // (otherwise it has used all that it asked for)
   }
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -89,9 +89,6 @@ __device__ __forceinline__ float4 lds4(uint32_t addr) {
 // Between ordinary accesses of a patch and the copy engine's writes to it: a barrier orders the threads, not the two proxies.
 // Any thread on the path from the last ordinary store to the copy may execute it; here it is the one that issues the copy.
 __device__ __forceinline__ void to_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
-}
 // 32 row values (thread = row) <-> the swizzled patch: 16-byte chunk j of row r sits at position j ^ (r & 7)
 __device__ __forceinline__ void patch_put(uint32_t patch, int lane, const float (&x)[32]) {
 #pragma unroll
@@ -146,11 +143,11 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
     return;
   }
   // a_ready[4] (4 producer warps) a_done[4] | w_ready[5] w_done[5] | d1_full[2] (L1 of branch / group) | d2_full[2] (L2) |
-  // mid_ready[2][4] (4 epilogue warps) | epi_done[2] | side_full[8][2] side_empty[8][2] | conv_full[8]
+  // mid_ready[2][4] (4 epilogue warps) | epi_done[2] | side_full[8][2] side_empty[8][2] | conv_full[8] | retired
   const uint32_t bar0 = smem_u32(bars);
   const uint32_t a_ready = bar0, a_done = bar0 + 32, w_ready = bar0 + 64, w_done = bar0 + 104, d1_full = bar0 + 144,
                  d2_full = bar0 + 160, mid_ready = bar0 + 176, epi_done = bar0 + 240, side_full = bar0 + 256,
-                 side_empty = bar0 + 384, conv_full = bar0 + 512;
+                 side_empty = bar0 + 384, conv_full = bar0 + 512, retired = bar0 + 576;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   float* const cst = reinterpret_cast<float*>(smem + ML_CONST_OFF);
   const int64_t n_rows = d.n_rows;
@@ -170,6 +167,7 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
       }
       for (int b = 0; b < 8; ++b) { mbar_init(mid_ready + 8 * b, 4); mbar_init(conv_full + 8 * b, 1); }
       for (int b = 0; b < 16; ++b) { mbar_init(side_full + 8 * b, 1); mbar_init(side_empty + 8 * b, 1); }
+      mbar_init(retired, 1);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -315,6 +313,7 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
       }
       __syncwarp();
     });
+    drain_mma(retired, elected);
   } else if (warp == ML_TMA_WARP) {
     // ---------------------------------------------------------------- TMA warp: weight tiles, up to five ahead
     pdl_sync();
@@ -346,10 +345,7 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
         if (++slot == ML_W_SLOTS) { slot = 0; ++phase; }
       }
     });
-    if (!alive) {  // failure path only: no TMA write may still be in flight when the CTA's shared memory is released
-      for (uint32_t i = n >= ML_W_SLOTS ? n - ML_W_SLOTS : 0; i < n; ++i)
-        mbar_wait(w_ready + 8 * (i % ML_W_SLOTS), (i / ML_W_SLOTS) & 1);
-    }
+    drain_copies(w_ready, ML_W_SLOTS, n);
   } else if (warp >= ML_EPI_WARP0) {
     // ---------------------------------------------------------------- epilogue warps
     pdl_sync();  // (the MMA warp touches nothing but this CTA's own memory)
@@ -575,9 +571,7 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
         }
       }
     }
-    if (EPI_RES && !alive) {  // failure path only: no copy may still be in flight when the CTA's shared memory is released
-      for (uint32_t n = asked >= 2 ? asked - 2 : 0; n < asked; ++n) mbar_wait(my_full + 8 * (n & 1), (n >> 1) & 1);
-    }
+    if (EPI_RES && !alive) drain_copies(my_full, 2, asked);  // (otherwise it has used all that it asked for)
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   } else {
     // ---------------------------------------------------------------- producers
@@ -590,7 +584,8 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
     const uint32_t put_even = lr * 128 + ((lc ^ lr) << 4), put_odd = lr * 128 + ((lc ^ (lr | 4)) << 4);
     const int n_seg = d.n_src + (MODE == MLP_GATED_BWD ? d.n_ext : 0);
     bool alive = true;
-    uint32_t g = (uint32_t)parity, side_n = 0, conv_n = 0;  // number of this warp's next chunk; its copies by TMA so far
+    uint32_t g = (uint32_t)parity, side_n = 0, conv_n = 0;  // number of this warp's next chunk, side patch, chunk by TMA
+    uint32_t conv_asked = 0, side_asked = 0;                // copies asked for: numbers below these
     const uint32_t my_conv = conv_full + 8 * pw;
     auto put = [&](uint32_t p, int i, const float4& v) {  // row lr + 4 i of a patch
       sts4(p + ((i & 1) ? put_odd : put_even) + 512u * i, v.x, v.y, v.z, v.w);
@@ -598,7 +593,9 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
     auto tile_row = [&](int t) { return (first_rt + t * step_rt) * 128 + quarter * 32; };
     auto is_direct = [&](int s) { return (s < d.n_src ? d.src[s].idx : d.ext[s - d.n_src].idx) == nullptr; };
     auto request = [&](int t, int s, int k, bool stored) {  // rows read in place: this warp's chunk k of segment s
-      if (lane == 0 && alive) {
+      if (!alive) return;
+      ++conv_asked;
+      if (lane == 0) {
         if (stored) to_async_proxy();  // the patch held gathered rows
         load_patch(s < d.n_src ? &maps.src[s] : &maps.ext[s - d.n_src], patch, my_conv, 32 * (parity + 2 * k), tile_row(t));
       }
@@ -607,14 +604,17 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
       if (side_n >= 2 && alive) alive = mbar_wait(side_empty + 8 * (2 * pw + (side_n & 1)), ((side_n >> 1) - 1) & 1);
       alive = __all_sync(0xffffffffu, alive);
     };
+    auto request_side = [&](const CUtensorMap* map, int x, int y) {  // the next side patch by TMA
+      wait_empty();
+      if (alive) {
+        side_asked = side_n + 1;
+        if (lane == 0) load_patch(map, side0 + (side_n & 1) * ML_PATCH, side_full + 8 * (2 * pw + (side_n & 1)), x, y);
+      }
+      ++side_n;
+    };
     auto residual = [&](int t) {
       if (!has_res) return;
-      for (int c = 0; c < (GATED ? 2 : 4); ++c, ++side_n) {
-        wait_empty();
-        if (lane == 0 && alive)
-          load_patch(&maps.res, side0 + (side_n & 1) * ML_PATCH, side_full + 8 * (2 * pw + (side_n & 1)),
-                     (GATED ? 64 * parity : 0) + 32 * c, tile_row(t));
-      }
+      for (int c = 0; c < (GATED ? 2 : 4); ++c) request_side(&maps.res, (GATED ? 64 * parity : 0) + 32 * c, tile_row(t));
     };
     // Addend sums of a tile.  The loads are latency bound, so as many as fit in the registers are requested together: three addends
     // half a patch (16 rows) at a time (0.58 -> 0.54 ms for 573,894 rows), fewer one after the other with the whole patch each (two at
@@ -738,22 +738,14 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
           else if (d.n_add == 2) gather(std::integral_constant<int, 2>{}, t, col0);
           else gather(std::integral_constant<int, 3>{}, t, col0);
         } else {
-          for (int c = 0; c < 4; ++c, ++side_n) {
-            wait_empty();
-            if (lane == 0 && alive)
-              load_patch(&maps.side, side0 + (side_n & 1) * ML_PATCH, side_full + 8 * (2 * pw + (side_n & 1)), col0 + 32 * c,
-                         (int)row0);
-          }
+          for (int c = 0; c < 4; ++c) request_side(&maps.side, col0 + 32 * c, (int)row0);
         }
       }
       if (MODE == MLP_GATED_BWD) residual(t);
     }
     if (!GATED && ((n_tiles - 1) & 1) == parity) residual(n_tiles - 1);
-    if (!alive) {  // failure path only: no copy may still be in flight when the CTA's shared memory is released
-      if (n_seg > 0) mbar_wait(my_conv, conv_n & 1);
-      if (!EPI_RES)
-        for (uint32_t n = side_n >= 2 ? side_n - 2 : 0; n < side_n; ++n) mbar_wait(side_full + 8 * (2 * pw + (n & 1)), (n >> 1) & 1);
-    }
+    if (!alive) drain_copies(my_conv, 1, conv_asked);  // (otherwise it has used all that it asked for)
+    drain_copies(side_full + 16 * pw, 2, side_asked);
   }
 
   // ------------------------------------------------------------------ common exit: release tensor memory

@@ -35,3 +35,24 @@ def test_proxy_fence_before_copies_into_patches_that_threads_stored_to(name, n_r
     assert len(requests) == n_requests
     for r in requests:
         assert 0 <= r.find("to_async_proxy()") < r.find("load_patch("), r
+
+
+@pytest.mark.parametrize("name,drains", [
+    ("mlp_fused.cuh", ["drain_mma(retired, elected);", "drain_copies(w_ready, ML_W_SLOTS, n);",
+                       "if (EPI_RES && !alive) drain_copies(my_full, 2, asked);",
+                       "if (!alive) drain_copies(my_conv, 1, conv_asked);", "drain_copies(side_full + 16 * pw, 2, side_asked);"]),
+    ("linear_tma.cuh", ["drain_mma(retired, elected);", "drain_copies(w_ready, ML_W_SLOTS, n);",
+                        "drain_copies(side_full + 16 * lane, 2, n);", "if (!alive) drain_copies(my_conv, 1, conv_asked);"]),
+    ("gemm_persistent.cuh", ["drain_mma(retired, elected);", "drain_copies(w_ready, w_period, wu);"]),
+    ("gemm.cu", ["drain_copies(w_full, 2, n_loads);", '"bar.arrive 1, 160;"', '"bar.sync 1, 160;"'])])
+def test_nothing_is_in_flight_when_a_block_ends(name, drains):
+    """After an expired wait a role may leave copies or matrix instructions behind that nobody has waited for: every role that
+    issues them waits for its last ones, counted where they are issued.  A role that has itself used all it asked for
+    unless its own wait expired may leave the wait out in that case only."""
+    lines = [s.strip() for s in code(name).splitlines()]
+    for d in drains:
+        assert any(s == d or (d.startswith('"') and d in s) for s in lines), d
+    # the counts go up where a copy is issued, and nowhere else
+    for counter, issue in (("++conv_asked;", "load_patch("), ("side_asked = side_n + 1;", "load_patch(")):
+        at = [i for i, s in enumerate(lines) if s == counter]
+        assert all(any(issue in s for s in lines[i:i + 5]) for i in at)
