@@ -267,7 +267,7 @@ class _Node(nn.Module):
 
 
 def kept_layers_for(n_layers: int, n_triplets: int, n_edges: int, avail: float) -> int:
-    """The memory policy of ``MatRIS.kept_layers`` as a function of the available bytes."""
+    """The estimate of ``MatRIS.kept_layers`` as a function of the available bytes."""
     per_layer = 6.7e3 * n_triplets + 6.2e3 * n_edges
     budget = 0.45 * avail
     n_keep = n_layers if per_layer * n_layers < budget else max(0, int(budget // max(per_layer, 1.0)))
@@ -490,6 +490,24 @@ class MatRIS(nn.Module):
             avail = min(avail, float(self.memory_limit_bytes))
         return avail
 
+    def _fixed_layers(self) -> int | None:
+        """The number of layers ``keep_activations`` names (None: it leaves the choice to the memory policy)."""
+        n_layers, keep = int(self.config["num_layers"]), self.keep_activations
+        if keep is None or isinstance(keep, bool):
+            return None if keep is None else n_layers * keep
+        return max(0, min(n_layers, int(keep)))
+
+    def kept_layers(self, n_triplets: int, n_edges: int, avail: float | None = None) -> int:
+        """An estimate, without a graph in hand, of how many (last) layers keep their internals for the backward pass on a
+        batch with that many triplet rows and directed edges, on the safe side of what ``forward`` finds out from the
+        exact need of the evaluation.  ``avail``: bytes to plan with (None: what the device has left); ``keep_activations``
+        overrides."""
+        fixed = self._fixed_layers()
+        if fixed is not None:
+            return fixed
+        return kept_layers_for(int(self.config["num_layers"]), n_triplets, n_edges,
+                               self._available_bytes() if avail is None else avail)
+
     def _plan_memory(self, e: _lib.MbEval) -> int:
         """Decide how many (last) layers keep their internals for the backward pass - as many as fit in memory, or what
         ``keep_activations`` says - and set it in ``e``; returns the bytes the evaluation will use."""
@@ -498,10 +516,9 @@ class MatRIS(nn.Module):
             _lib.check(_lib.load().mb_evaluate_workspace(C.byref(e), C.byref(size)), "mb_evaluate_workspace")
             return size.value
 
-        size, n_layers, keep = C.c_size_t(0), e.model.contents.n_layers, self.keep_activations
-        if keep is not None:
-            n = (n_layers if keep else 0) if isinstance(keep, bool) else max(0, min(n_layers, int(keep)))
-            return need(n)
+        size, n_layers, fixed = C.c_size_t(0), e.model.contents.n_layers, self._fixed_layers()
+        if fixed is not None:
+            return need(fixed)
         budget = 0.9 * self._available_bytes()
         # the need grows with the number of kept layers: the largest that fits, by bisection
         best = need(n_layers)
