@@ -38,6 +38,8 @@ GPA_PER_EV_A3 = 160.21766208  # matris/model/readout.py:215
 # again at the next call.  Larger ones ask for their buffers one by one, so that a block of a large part of the device is
 # never wanted in one piece; their host time is far below their device time.
 WORKSPACE_LIMIT = 4 << 30
+# An evaluation plans with this much of the memory that is left: the rest is for what the allocator cannot place.
+MEMORY_SHARE = 0.9
 
 
 # ------------------------------------------------------------------ packed parameters
@@ -290,22 +292,27 @@ def split_ranges(triplets, edges, fits) -> list[tuple[int, int]]:
     ``fits(sum of triplets, sum of edges)`` true for every range, as few as a greedy walk needs and then balanced
     by triplet + edge rows.  A structure that does not fit alone gets a range of its own."""
     triplets, edges = np.asarray(triplets, dtype=np.int64), np.asarray(edges, dtype=np.int64)
-    n = len(triplets)
-    greedy, a, t, e = [], 0, 0, 0
-    for i in range(n):
-        if i > a and not fits(t + int(triplets[i]), e + int(edges[i])):
-            greedy.append((a, i))
-            a, t, e = i, 0, 0
-        t, e = t + int(triplets[i]), e + int(edges[i])
-    greedy.append((a, n))
+    return _split(triplets + edges, lambda a, b: fits(int(triplets[a:b].sum()), int(edges[a:b].sum())))
+
+
+def _split(rows, fits) -> list[tuple[int, int]]:
+    """``split_ranges`` for a predicate of the range itself, ``fits(a, b)``; whatever is part of a range that fits fits too, so
+    the longest range from a structure on is found by bisection."""
+    n, greedy, a = len(rows), [], 0
+    while a < n:
+        lo, hi = a + 1, n + 1  # the range [a, lo) is taken, [a, hi) is too long
+        while hi - lo > 1:
+            mid = (lo + hi) // 2
+            lo, hi = (mid, hi) if fits(a, mid) else (lo, mid)
+        greedy.append((a, lo))
+        a = lo
     if len(greedy) == 1:
         return greedy
-    cum = np.cumsum(triplets + edges, dtype=np.float64)
+    cum = np.cumsum(rows, dtype=np.float64)
     for parts in range(len(greedy), min(n, len(greedy) + 2) + 1):
         cuts = [0] + [int(np.searchsorted(cum, cum[-1] * k / parts, side="left")) + 1 for k in range(1, parts)] + [n]
         ranges = [(cuts[k], cuts[k + 1]) for k in range(parts)]
-        if all(b > a for a, b in ranges) and all(fits(int(triplets[a:b].sum()), int(edges[a:b].sum())) or b - a == 1
-                                                 for a, b in ranges):
+        if all(b > a for a, b in ranges) and all(b - a == 1 or fits(a, b) for a, b in ranges):
             return ranges
     return greedy
 
@@ -508,27 +515,28 @@ class MatRIS(nn.Module):
         return kept_layers_for(int(self.config["num_layers"]), n_triplets, n_edges,
                                self._available_bytes() if avail is None else avail)
 
+    def _need(self, e: _lib.MbEval, keep: int) -> int:
+        """Bytes the evaluation ``e`` has in use at most when its last ``keep`` layers keep their internals."""
+        size, e.keep_layers = C.c_size_t(0), keep
+        _lib.check(_lib.load().mb_evaluate_workspace(C.byref(e), C.byref(size)), "mb_evaluate_workspace")
+        return size.value
+
     def _plan_memory(self, e: _lib.MbEval) -> int:
         """Decide how many (last) layers keep their internals for the backward pass - as many as fit in memory, or what
         ``keep_activations`` says - and set it in ``e``; returns the bytes the evaluation will use."""
-        def need(n):
-            e.keep_layers = n
-            _lib.check(_lib.load().mb_evaluate_workspace(C.byref(e), C.byref(size)), "mb_evaluate_workspace")
-            return size.value
-
-        size, n_layers, fixed = C.c_size_t(0), e.model.contents.n_layers, self._fixed_layers()
+        n_layers, fixed = e.model.contents.n_layers, self._fixed_layers()
         if fixed is not None:
-            return need(fixed)
-        budget = 0.9 * self._available_bytes()
+            return self._need(e, fixed)
+        budget = MEMORY_SHARE * self._available_bytes()
         # the need grows with the number of kept layers: the largest that fits, by bisection
-        best = need(n_layers)
+        best = self._need(e, n_layers)
         if best <= budget:
             return best
         lo, hi = 0, n_layers
         while hi - lo > 1:
             mid = (lo + hi) // 2
-            lo, hi = (mid, hi) if need(mid) <= budget else (lo, mid)
-        return need(lo)
+            lo, hi = (mid, hi) if self._need(e, mid) <= budget else (lo, mid)
+        return self._need(e, lo)
 
     def split_for_memory(self, g: BatchedGraph, headroom: float = 0.93) -> list[tuple[int, int]]:
         """Contiguous ranges of the structures of batch ``g`` such that every range, evaluated as a batch of its own,
@@ -538,12 +546,21 @@ class MatRIS(nn.Module):
         available memory the plan may count on (the ranges' own graphs and results take some)."""
         if g.n_struct <= 1 or self.keep_activations is not None:
             return [(0, g.n_struct)]
-        n_layers = int(self.config["num_layers"])
-        avail = headroom * self._available_bytes()
-        if kept_layers_for(n_layers, g.n_triplets, g.n_edges, avail / headroom) == n_layers:
+        P, n_layers = self.packed(g.device), int(self.config["num_layers"])
+        budget = MEMORY_SHARE * self._available_bytes()
+        e = _lib.MbEval()
+        e.model = C.pointer(P.model)
+        e.f = e.s = e.m = 256  # all outputs (the counts alone matter to a dry run; nothing is read)
+
+        def need(n_atoms, n_struct, n_edges, n_triplets):
+            e.n_atoms, e.n_struct, e.n_edges, e.n_bonds, e.n_triplets = n_atoms, n_struct, n_edges, n_edges // 2, n_triplets
+            return self._need(e, n_layers)
+
+        if need(g.n_atoms, g.n_struct, g.n_edges, g.n_triplets) <= budget:
             return [(0, g.n_struct)]
-        _, ep, _, tp = g.structure_slices()
-        return split_ranges(np.diff(tp), np.diff(ep), lambda t, e: kept_layers_for(n_layers, t, e, avail) == n_layers)
+        ap, ep, _, tp = (np.asarray(p, dtype=np.int64) for p in g.structure_slices())
+        return _split(np.diff(tp) + np.diff(ep), lambda a, b: need(int(ap[b] - ap[a]), b - a, int(ep[b] - ep[a]),
+                                                                   int(tp[b] - tp[a])) <= headroom * budget)
 
     def _evaluate(self, g: BatchedGraph, task: str):
         dev, n_struct, n_atoms = g.device, g.n_struct, g.n_atoms

@@ -1,7 +1,11 @@
 """CPU: how many layers keep their internals - the estimate from two counts against the library's dry run of the same evaluation."""
 import ctypes as C
+import math
+from types import SimpleNamespace
 
+import numpy as np
 import pytest
+import torch
 
 from matris_b200 import MatRIS, _lib
 
@@ -39,3 +43,35 @@ def test_keep_activations_overrides_the_estimate():
     for keep, want in ((True, 4), (False, 0), (2, 2), (9, 4), (-1, 0)):
         model.keep_activations = keep
         assert model.kept_layers(10 ** 9, 4 * 10 ** 8, 1e9) == want
+
+
+def batch_of(n_per, edges_per_atom, triplets_per_atom):
+    """The parts of a batch's graph that a memory plan reads."""
+    ap = np.concatenate([[0], np.cumsum(n_per)])
+    ep, tp = 2 * (np.asarray(ap * edges_per_atom, dtype=np.int64) // 2), np.asarray(ap * triplets_per_atom, dtype=np.int64)
+    return SimpleNamespace(device=torch.device("cpu"), n_struct=len(n_per), n_atoms=int(ap[-1]), n_edges=int(ep[-1]),
+                           n_triplets=int(tp[-1]), structure_slices=lambda: (ap, ep, ep // 2, tp))
+
+
+@pytest.mark.parametrize("shape", list(SHAPES))
+@pytest.mark.parametrize("gigabytes", [4.0, 20.0, 120.0])
+def test_sub_batches_and_evaluation_plan_with_the_same_need(shape, gigabytes):
+    """A list is cut exactly when the dry run of its batch does not fit with all layers kept, and every part does fit then."""
+    model = MatRIS(num_layers=10)
+    model._available_bytes = lambda: gigabytes * 1e9
+    rng = np.random.default_rng(0)
+    per_atom, one = SHAPES[shape], dry_run(10, 4000, 100, int(SHAPES[shape][0] * 4000) // 2 * 2, int(SHAPES[shape][1] * 4000)) / 4000
+    for share in (0.8, 0.97, 1.1, 2.5):  # of what fits at once
+        n_per = rng.integers(8, 65, max(2, int(share * 0.9 * gigabytes * 1e9 / one / 36.5)))
+        g = batch_of(n_per, *per_atom)
+        ranges = model.split_for_memory(g)
+        fits = dry_run(10, g.n_atoms, g.n_struct, g.n_edges, g.n_triplets) <= 0.9 * gigabytes * 1e9
+        assert (ranges == [(0, g.n_struct)]) == fits, (share, ranges)
+        ap, ep, _, tp = g.structure_slices()
+        assert ranges[0][0] == 0 and ranges[-1][1] == g.n_struct and all(x[1] == y[0] for x, y in zip(ranges, ranges[1:]))
+        for a, b in ranges:
+            need = dry_run(10, int(ap[b] - ap[a]), b - a, int(ep[b] - ep[a]), int(tp[b] - tp[a]))
+            assert need <= 0.9 * gigabytes * 1e9 * (1.0 if fits else 0.93)
+        # no more parts than the memory asks for, but for the balancing
+        whole = dry_run(10, g.n_atoms, g.n_struct, g.n_edges, g.n_triplets)
+        assert fits or len(ranges) <= math.ceil(whole / (0.93 * 0.9 * gigabytes * 1e9)) + 2
