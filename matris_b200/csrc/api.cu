@@ -1,11 +1,24 @@
 // Version, status strings and the per-thread CUDA error record of the C ABI.
 #include <stdio.h>
+#include <atomic>
 #include "common.cuh"
 
 namespace mb {
 static thread_local char g_cuda_error[512] = "";
 void set_cuda_error(cudaError_t e, const char* where) {
   snprintf(g_cuda_error, sizeof(g_cuda_error), "%s: %s (%s)", where, cudaGetErrorString(e), cudaGetErrorName(e));
+}
+
+int sm_count(int* n) {
+  static std::atomic<int> of_device[64];
+  int dev = 0;
+  MB_CUDA_CHECK(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return MB_ERR_INVALID;
+  if ((*n = of_device[dev]) == 0) {
+    MB_CUDA_CHECK(cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, dev));
+    of_device[dev] = *n;
+  }
+  return MB_OK;
 }
 }  // namespace mb
 

@@ -52,6 +52,7 @@ __device__ __forceinline__ void pdl_sync() {
 
 static inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 
+int sm_count(int* n);  // multiprocessors of the current device, asked for once per device; a status code
 int gemm_mode();  // the contraction core selected with mb_set_gemm_mode
 
 // exclusive scan of n int32 values into out[0..n] (out[n] = total); tmp holds

@@ -793,16 +793,18 @@ extern "C" int mb_scale_rows(int64_t n_rows, const float* x, const float* a, flo
 }
 
 // a warp loads its weights once: no more blocks than are resident at a time, which walk the rows
-static inline unsigned small_linear_grid(int64_t n_rows, int rows_per_warp, int blocks_per_sm) {
+static inline unsigned small_linear_grid(int64_t n_rows, int rows_per_warp, int resident) {
   const int64_t blocks = (n_rows + rows_per_warp * (RW_THREADS / 32) - 1) / (rows_per_warp * (RW_THREADS / 32));
-  return (unsigned)(blocks < 148 * blocks_per_sm ? blocks : 148 * blocks_per_sm);
+  return (unsigned)(blocks < resident ? blocks : resident);
 }
 
 extern "C" int mb_small_linear_fwd(int64_t n_rows, int32_t k, const float* x, const float* w, float* y, void* stream) {
   MB_REQUIRE(n_rows >= 0 && k >= 1 && k <= 16 && x && w && y);
   if (n_rows == 0) return MB_OK;
-  if (k <= 8) launch(k_small_linear_fwd<8>, small_linear_grid(n_rows, 4, 4), RW_THREADS, 0, STREAM, n_rows, k, x, w, y);
-  else launch(k_small_linear_fwd<16>, small_linear_grid(n_rows, 2, 2), RW_THREADS, 0, STREAM, n_rows, k, x, w, y);
+  int n_sm = 0;
+  if (const int rc = sm_count(&n_sm)) return rc;
+  if (k <= 8) launch(k_small_linear_fwd<8>, small_linear_grid(n_rows, 4, 4 * n_sm), RW_THREADS, 0, STREAM, n_rows, k, x, w, y);
+  else launch(k_small_linear_fwd<16>, small_linear_grid(n_rows, 2, 2 * n_sm), RW_THREADS, 0, STREAM, n_rows, k, x, w, y);
   MB_LAUNCH_CHECK("k_small_linear_fwd");
   return MB_OK;
 }
@@ -811,8 +813,12 @@ extern "C" int mb_small_linear_bwd(int64_t n_rows, int32_t k, const float* dy, c
                                    int32_t accumulate, void* stream) {
   MB_REQUIRE(n_rows >= 0 && k >= 1 && k <= 16 && dy && w && dx);
   if (n_rows == 0) return MB_OK;
-  if (k <= 8) launch(k_small_linear_bwd<8>, small_linear_grid(n_rows, 4, 3), RW_THREADS, 0, STREAM, n_rows, k, dy, w, dx, accumulate);
-  else launch(k_small_linear_bwd<16>, small_linear_grid(n_rows, 2, 2), RW_THREADS, 0, STREAM, n_rows, k, dy, w, dx, accumulate);
+  int n_sm = 0;
+  if (const int rc = sm_count(&n_sm)) return rc;
+  if (k <= 8)
+    launch(k_small_linear_bwd<8>, small_linear_grid(n_rows, 4, 3 * n_sm), RW_THREADS, 0, STREAM, n_rows, k, dy, w, dx, accumulate);
+  else
+    launch(k_small_linear_bwd<16>, small_linear_grid(n_rows, 2, 2 * n_sm), RW_THREADS, 0, STREAM, n_rows, k, dy, w, dx, accumulate);
   MB_LAUNCH_CHECK("k_small_linear_bwd");
   return MB_OK;
 }

@@ -56,3 +56,9 @@ def test_nothing_is_in_flight_when_a_block_ends(name, drains):
     for counter, issue in (("++conv_asked;", "load_patch("), ("side_asked = side_n + 1;", "load_patch(")):
         at = [i for i, s in enumerate(lines) if s == counter]
         assert all(any(issue in s for s in lines[i:i + 5]) for i in at)
+
+
+def test_no_launch_assumes_a_number_of_multiprocessors():
+    """Grids are sized by what the device says; the number of this card's multiprocessors appears in comments only."""
+    for name in sorted(os.listdir(CSRC)):
+        assert not re.search(r"\b148\b", code(name)), name
