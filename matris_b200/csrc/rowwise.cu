@@ -119,7 +119,8 @@ k_seg_attn_fwd(int n_nodes, const int32_t* __restrict__ tgt_ptr, const int32_t* 
   const int32_t* ptr = side == 0 ? tgt_ptr : src_ptr;
   const int q0 = ptr[row], q1 = ptr[row + 1];
   const int lcol = side == 0 ? 128 : 0;
-  float4 mx = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+  // (not -inf: a batch whose logits are all -inf would rescale by exp(-inf + inf))
+  float4 mx = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX);
   float4 s = zero4(), acc = zero4();
   for (int q = q0 + (WARPS > 1 ? w * NB : 0); q < q1; q += NB * WARPS) {
     int64_t r[NB], er[NB];

@@ -51,3 +51,26 @@ def test_segment_lengths(lengths, with_emap):
         denv = ops.seg_smooth_sum_bwd_env(n, dev(tptr, i32), dev(sptr, i32), dev(perm, i32), dev(tgt, i32), dev(src, i32), None, None,
                                           dev(env), dev(h), dev(dagg))
         report("smooth segment sum: gradient of the envelope", denv, de[:n], 1e-6, scaled=True)
+
+
+@pytest.mark.parametrize("value", [float("-inf"), -3.4028234663852886e38])
+@pytest.mark.parametrize("with_emap", [False, True])
+@pytest.mark.parametrize("lengths", [[3, 9], [40, 70, 5]])
+def test_rows_masked_with_the_lowest_logits(lengths, with_emap, value):
+    """Rows whose logit is -inf or the lowest float drop out of the softmax, also where they fill a whole batch of rows of a warp
+    (the first four or eight of a segment, or a later one)."""
+    from matris_b200 import ops
+    n, rows, i32 = len(lengths), sum(lengths), torch.int32
+    tgt = torch.repeat_interleave(torch.arange(n), torch.tensor(lengths))
+    (perm, tptr) = _csr(tgt, n)
+    emap = torch.arange(rows) if with_emap else None
+    logits, h = 4 * rnd(rows, 256, seed=1), rnd(rows, 128, seed=2)
+    start = torch.repeat_interleave(tptr[:-1], torch.tensor(lengths))
+    at = torch.arange(rows) - start  # position in the segment; its last row always stays
+    masked = ((at < 16) | ((at >= 24) & (at < 48))) & (at < torch.tensor(lengths)[tgt] - 1)
+    logits[masked, ::2] = value
+    agg = ops.seg_attn_fwd(n, dev(tptr, i32), dev(tptr, i32), dev(perm, i32), dev(emap, i32) if with_emap else None, dev(logits),
+                           dev(h))[:2]
+    for cols, out in ((logits[:, 128:], agg[0]), (logits[:, :128], agg[1])):
+        ref = torch.stack([(torch.softmax(cols[tgt == k].double(), 0) * h[tgt == k].double()).sum(0) for k in range(n)])
+        report(f"segment softmax, rows masked with {value}", out, ref, 5e-6)
