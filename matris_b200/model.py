@@ -440,6 +440,13 @@ class MatRIS(nn.Module):
         return build_batched_graph([a[0] for a in arrays], [a[1] for a in arrays], [a[2] for a in arrays],
                                    self.config["pairwise_cutoff"], self.config["three_body_cutoff"], self.device)
 
+    def _check_elements(self, g: BatchedGraph) -> None:
+        """The kernels look atoms up in tables by their number without a test of their own."""
+        n = self.atom_embedding.embedding.weight.shape[0]
+        lo, hi = g.number_range
+        if lo < 1 or hi > n:
+            raise IndexError(f"atomic numbers from {lo} to {hi}: the model knows the elements 1 to {n}")
+
     def forward(self, graphs: Sequence[RadiusGraph] | BatchedGraph, task: str = "ef", is_training: bool = False):
         """Same result dictionary as the reference's ``MatRIS.forward`` (model.py:183-250): ``e`` [B] energy per
         atom including the reference energy, ``f`` tuple of [n_i,3], ``s`` list of [3,3] in GPa, ``m`` list of
@@ -449,6 +456,7 @@ class MatRIS(nn.Module):
         if self.device.type != "cuda":
             raise RuntimeError("matris_b200 runs on a CUDA device only: move the model with .to('cuda')")
         g = self._as_batch(graphs)
+        self._check_elements(g)
         self.last_batch = g
         with torch.cuda.device(g.device):
             # The GEMM kernels bound every wait and raise a status word instead of hanging.  The word of the previous

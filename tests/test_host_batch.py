@@ -46,3 +46,18 @@ def test_host_batch(count, cutoff):
 def test_singular_lattice():
     with pytest.raises((ValueError, np.linalg.LinAlgError)):
         cell_grid(np.zeros((1, 3, 3)), np.array([2]), 6.0)
+
+
+@pytest.mark.parametrize("numbers,ok", [([1, 94], True), ([29, 0], False), ([-3, 29], False), ([95, 8], False), ([2 ** 32 + 8, 8], False)])
+def test_elements_outside_the_tables_are_refused(numbers, ok):
+    """Graphs take any atomic number; a model refuses the ones its tables have no row for (the kernels do not look)."""
+    from matris_b200 import MatRIS
+    from matris_b200.graph import HostBatch, upload
+    model = MatRIS(num_layers=1)
+    hb = HostBatch([np.array([6]), np.array(numbers)], [np.zeros((1, 3)), np.eye(2, 3)], [5 * np.eye(3)] * 2, 6.0, pin=False)
+    g = upload(hb, 6.0, 4.0, "cpu")
+    if ok:
+        model._check_elements(g)
+    else:
+        with pytest.raises(IndexError, match="the model knows the elements 1 to 94"):
+            model._check_elements(g)
