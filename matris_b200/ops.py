@@ -19,30 +19,8 @@ D = 128
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
-_pinned_stream = None
-
-
-class pinned_stream:
-    """Within the block every entry point launches on the stream that is current at entry (looked up once instead
-    of once per launch).  The autograd engine runs backward functions on that same stream, from its own thread,
-    so the handle is shared process-wide for the duration of the block; blocks do not nest across devices."""
-
-    def __enter__(self):
-        global _pinned_stream
-        self.outer, _pinned_stream = _pinned_stream, None
-        _pinned_stream = _stream()
-        return self
-
-    def __exit__(self, *exc):
-        global _pinned_stream
-        _pinned_stream = self.outer
-        return False
-
-
 def _stream():
     """Raw handle of torch's current stream on the current device (the stream every entry point launches on)."""
-    if _pinned_stream is not None:
-        return _pinned_stream
     if _raw_stream is not None:
         return _raw_stream(torch.cuda.current_device())
     return torch.cuda.current_stream().cuda_stream
