@@ -62,13 +62,14 @@ _split_cache: dict = {}
 def as_split(W) -> SplitWeight:
     if isinstance(W, SplitWeight):
         return W
-    key = (W.data_ptr(), tuple(W.shape), W._version)
-    sw = _split_cache.get(key)
-    if sw is None:
+    # an entry keeps W, so that its address is not handed out again; views of one storage differ in shape or strides
+    key = (W.data_ptr(), tuple(W.shape), W.stride(), W._version)
+    entry = _split_cache.get(key)
+    if entry is None:
         if len(_split_cache) > 256:
             _split_cache.clear()
-        sw = _split_cache[key] = SplitWeight(W)
-    return sw
+        entry = _split_cache[key] = (W.detach(), SplitWeight(W))
+    return entry[1]
 
 
 def S(t, idx=None, col=0, act=0):
