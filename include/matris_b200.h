@@ -587,7 +587,8 @@ int mb_refine_layer(const mb_refine_params* p, const mb_row_graph* g, const floa
 /* MatRIS.forward (matris/model/model.py:183-250) on a batch graph: energies, and forces / virial through the backward
  * pass when f or s is given, as one call that queues every kernel.  mb_evaluate_workspace gives the most memory that is in
  * use at any time for a number of layers whose internals are kept for the backward pass (the earlier layers' are
- * recomputed), which is also the size of a workspace.  All outputs but e are optional. */
+ * recomputed), which is also the size of a workspace.  All outputs but e are optional.  MB_ERR_CAPACITY: the workspace
+ * is too small, alloc returned NULL, or the host has no memory for the bookkeeping. */
 typedef void* (*mb_alloc_fn)(size_t bytes);     /* device memory, 256-byte aligned, NULL when there is none */
 typedef void (*mb_free_fn)(void* p);            /* may be called while work that uses p is still queued on the stream */
 typedef struct mb_eval {

@@ -14,6 +14,7 @@
 #include <stdio.h>
 #include <string.h>
 #include <array>
+#include <exception>
 #include <initializer_list>
 #include <mutex>
 #include <vector>
@@ -105,6 +106,7 @@ struct Arena {
     size_t step = 256;
     while (step * 64 <= floats * 4) step *= 2;
     const size_t bytes = (floats * 4 + step - 1) / step * step;
+    stack.push_back({nullptr, bytes});  // (may throw: before anything is taken)
     used += bytes;
     if (lo + hi > peak) peak = lo + hi;
     void* p = nullptr;
@@ -112,7 +114,7 @@ struct Arena {
     else if (mode == BUFFER) p = lo + hi > cap ? nullptr : base + (from_top ? cap - hi : lo - bytes);
     else if (!failed) p = bytes ? alloc(bytes) : reinterpret_cast<void*>(256);
     if (!p) failed = true;
-    stack.push_back({p, bytes});
+    stack.back() = {p, bytes};
     return static_cast<float*>(p);
   }
   void drop(std::vector<Piece>& stack, size_t& used, size_t count) {
@@ -1037,14 +1039,25 @@ static bool valid(const mb_eval* E) {
 
 using namespace mb;
 
+// The callers are C: host memory that runs out (the lists of buffers, the layers' bookkeeping) comes back as a status.
+template <typename F> static int guarded(F f) {
+  try {
+    return f();
+  } catch (const std::exception&) {
+    return MB_ERR_CAPACITY;
+  }
+}
+
 extern "C" int mb_evaluate_workspace(const mb_eval* e, size_t* bytes) {
   if (!valid(e) || !bytes) return MB_ERR_INVALID;
-  Run R;
-  R.scratch = gemm_mode() != 0;
-  mb_eval copy = *e;
-  const int rc = evaluate(R, copy);
-  *bytes = R.ar.peak;
-  return rc;
+  return guarded([&] {
+    Run R;
+    R.scratch = gemm_mode() != 0;
+    mb_eval copy = *e;
+    const int rc = evaluate(R, copy);
+    *bytes = R.ar.peak;
+    return rc;
+  });
 }
 
 extern "C" int mb_evaluate(mb_eval* e, void* stream) {
@@ -1064,12 +1077,18 @@ extern "C" int mb_evaluate(mb_eval* e, void* stream) {
   const bool beside = !R.scratch && !g_times.on && cudaStreamIsCapturing(R.st, &capture) == cudaSuccess &&
                       capture == cudaStreamCaptureStatusNone && side_take(side);
   if (beside) R.sides = &side;
-  int rc = evaluate(R, *e);
+  int rc = guarded([&] { return evaluate(R, *e); });
+  if (rc != MB_OK && R.rc == MB_OK) {  // left in the middle of something, perhaps of a branch
+    R.rc = rc;
+    R.st = (cudaStream_t)stream;
+    R.on = 0;
+    R.pending[0] = R.pending[1] = beside;
+  }
   if (beside) {
     R.join(0);  // (only after an error is anything left)
     R.join(1);
     rc = R.rc;
-    side_give(side);
+    if (guarded([&] { side_give(side); return (int)MB_OK; }) != MB_OK) side_free(side);
   }
   e->n_launches = R.launches;
   return rc;
@@ -1092,11 +1111,13 @@ extern "C" int mb_attention_layer(const mb_attn_params* p, const mb_row_graph* g
   if (!p || !g || start_layer(R, ws, ws_bytes, stream)) return MB_ERR_INVALID;
   const bool bwd = d_node_out != nullptr;
   if (ws && (!node || !edge || (bwd && (!d_edge_out || !d_node || !d_edge)))) return MB_ERR_INVALID;
-  AttnInter it;
-  attn_fwd(R, *p, *g, node, edge, node_out, edge_out, bwd ? TEMP : NONE, it);
-  if (bwd) attn_bwd(R, *p, *g, it, d_node_out, d_edge_out, d_node, d_edge);
-  if (!ws) *ws_bytes = R.ar.peak;
-  return R.rc;
+  return guarded([&] {
+    AttnInter it;
+    attn_fwd(R, *p, *g, node, edge, node_out, edge_out, bwd ? TEMP : NONE, it);
+    if (bwd) attn_bwd(R, *p, *g, it, d_node_out, d_edge_out, d_node, d_edge);
+    if (!ws) *ws_bytes = R.ar.peak;
+    return R.rc;
+  });
 }
 
 extern "C" int mb_refine_layer(const mb_refine_params* p, const mb_row_graph* g, const float* node, const float* edge,
@@ -1108,11 +1129,13 @@ extern "C" int mb_refine_layer(const mb_refine_params* p, const mb_row_graph* g,
   const bool bwd = d_node_out != nullptr, want_edge = bwd ? d_edge_out != nullptr : edge_out != nullptr;
   if (ws && (!node || !edge || !rbf || (bwd && (!d_node || !d_edge || !d_rbf)))) return MB_ERR_INVALID;
   const int64_t n_bonds = g->is_atom ? g->n_edge_rows : g->n_nodes;
-  RefineInter it;
-  refine_fwd(R, *p, *g, n_bonds, node, edge, rbf, atom_feat, node_out, edge_out, want_edge, bwd ? TEMP : NONE, it);
-  if (bwd) refine_bwd(R, *p, *g, n_bonds, it, d_node_out, d_edge_out, d_node, d_edge, d_rbf, d_atom);
-  if (!ws) *ws_bytes = R.ar.peak;
-  return R.rc;
+  return guarded([&] {
+    RefineInter it;
+    refine_fwd(R, *p, *g, n_bonds, node, edge, rbf, atom_feat, node_out, edge_out, want_edge, bwd ? TEMP : NONE, it);
+    if (bwd) refine_bwd(R, *p, *g, n_bonds, it, d_node_out, d_edge_out, d_node, d_edge, d_rbf, d_atom);
+    if (!ws) *ws_bytes = R.ar.peak;
+    return R.rc;
+  });
 }
 
 extern "C" int mb_profile_enable(int on) {
