@@ -200,6 +200,8 @@ static int gemm_validate(const mb_gemm_desc* desc) {
 // finishes normally (TMEM is always released).
 #include <cuda.h>
 #include <stdio.h>
+#include <memory>
+#include <new>
 #include <type_traits>
 
 namespace mb {
@@ -632,8 +634,9 @@ static int weight_map(const void* w, int64_t ldw, int k, CUtensorMap* out, int r
   struct Key { const void* w; int64_t ld; int k, rows, bf16, box; };
   struct Entry { Key key; CUtensorMap map; };
   constexpr int SLOTS = 1024;
-  static thread_local Entry* cache = nullptr;
-  if (!cache) cache = new Entry[SLOTS]();
+  static thread_local std::unique_ptr<Entry[]> cache;  // given back when the thread ends
+  if (!cache) cache.reset(new (std::nothrow) Entry[SLOTS]());
+  if (!cache) return MB_ERR_CAPACITY;
   const size_t hsh = ((reinterpret_cast<uintptr_t>(w) >> 4) * 0x9E3779B97F4A7C15ull + (uint64_t)(k + rows)) >> 54;  // 10 bits
   Entry& e = cache[hsh % SLOTS];
   if (e.key.w == w && e.key.ld == ldw && e.key.k == k && e.key.rows == rows && e.key.bf16 == (int)bf16 && e.key.box == box_rows) {
