@@ -242,19 +242,22 @@ __device__ __forceinline__ uint32_t global_ns() {  // low word: differences of u
 // hardware chooses how long try_wait parks the thread.  It parks it at all so that the waiting warps leave the issue slots to
 // the others (against a loop of test_wait polls: gated MLP forward 0.71 -> 0.67 ms, plain backward 0.24 -> 0.19 ms at 573,894 rows);
 // reading the clock between polls, which takes longer than counting them, leaves them more (4 atoms 5.37 -> 5.02 ms an evaluation,
-// energies of 96 crystals 11.25 -> 10.57).
+// energies of 96 crystals 11.25 -> 10.5).  Out of line, because the clock's registers inside every role's loops were spills there:
+// gated forward of 573,894 rows with K = 384 gathered 0.67 ms with counted polls, 0.69 inlined, 0.63 out of line.
 __device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity) {
-  if (mbar_try(bar, parity)) return true;
   const uint32_t t0 = global_ns();
   do {
     if (mbar_try(bar, parity)) return true;
   } while (global_ns() - t0 < WAIT_LIMIT_NS);
   return false;
 }
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity) {
   if (mbar_poll(bar, parity)) return true;
   atomicOr(&g_gemm_status, 1);
   return false;
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+  return mbar_try(bar, parity) || mbar_wait_slow(bar, parity);
 }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
