@@ -162,9 +162,14 @@ static bool side_take(Side& s) {
       }
   }
   s.device = dev;
+  auto failed = [&] {  // the evaluation goes on without: its first launch must not find this error as its own
+    side_free(s);
+    cudaGetLastError();
+    return false;
+  };
   for (cudaStream_t& t : s.st)
-    if (cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking) != cudaSuccess) { side_free(s); return false; }
-  if (cudaEventCreateWithFlags(&s.ev, cudaEventDisableTiming) != cudaSuccess) { side_free(s); return false; }
+    if (cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking) != cudaSuccess) return failed();
+  if (cudaEventCreateWithFlags(&s.ev, cudaEventDisableTiming) != cudaSuccess) return failed();
   return true;
 }
 static void side_give(Side& s) {

@@ -62,3 +62,13 @@ def test_no_launch_assumes_a_number_of_multiprocessors():
     """Grids are sized by what the device says; the number of this card's multiprocessors appears in comments only."""
     for name in sorted(os.listdir(CSRC)):
         assert not re.search(r"\b148\b", code(name)), name
+
+
+def test_side_streams_that_cannot_be_made_leave_no_error_behind():
+    """An evaluation runs without side streams when they cannot be created; the error is taken off the thread's record, where
+    the check after the first launch would find it."""
+    text = code("evaluate.cu")
+    taken = body(text, text.index("static bool side_take("))
+    assert "cudaGetLastError();" in body(taken, taken.index("auto failed"))
+    for call in re.findall(r"cuda(?:Stream|Event)CreateWithFlags[^;]*;", taken):
+        assert call.rstrip("; ").endswith("return failed()"), call
