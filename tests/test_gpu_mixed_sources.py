@@ -72,3 +72,25 @@ def test_gated_forward_with_residual(ops, order, n_rows):
     assert ops.gemm_status() == 0
     for name, v, w in zip(("z1", "z2", "h", "out2"), got, (z1, z2, h, h + rw.double() * res.double())):
         report(f"gated forward {name} {order} R={n_rows}", v, w, TOL, scaled=True)
+
+
+@pytest.mark.parametrize("stride", [0, 64])
+@pytest.mark.parametrize("n_rows", [1, 300, 148 * 128 + 77])
+def test_rows_that_share_memory(ops, n_rows, stride):
+    """Row strides shorter than a row: one row for all (0) and overlapping windows (64), as operand, gate and residual."""
+    def rows(seed):
+        return rnd(64 * n_rows + 128, seed=seed).cuda().as_strided((n_rows, 128), (stride, 1))
+    x, z, r = rows(1), rows(2), rows(3)
+    full = [t.cpu().double() for t in (x, z, r)]
+    W, rw = rnd(128, 128, seed=4, scale=0.09), rnd(128, seed=5)
+    zz = full[1].clone().requires_grad_(True)
+    (sg,) = torch.autograd.grad(F.silu(zz).sum(), zz)
+    y = ops.linear(x, dev(W), gate=z, res=r, res_w=dev(rw))
+    report(f"row GEMM stride {stride} R={n_rows}", y, F.linear(full[0], W.double()) * sg + rw.double() * full[2], TOL, scaled=True)
+    w1, w2 = rnd(128, 128, seed=6, scale=0.09), rnd(128, 128, seed=7, scale=0.09)
+    p = SimpleNamespace(w1=dev(w1), b1=None, w2=dev(w2), b2=None)
+    _, got, out2 = ops.ffn_fwd(p, x, res=r, res_w=dev(rw))
+    want = F.linear(F.silu(F.linear(full[0], w1.double())), w2.double())
+    report(f"FFN stride {stride} R={n_rows}", got, want, TOL, scaled=True)
+    report(f"FFN + residual stride {stride} R={n_rows}", out2, want + rw.double() * full[2], TOL, scaled=True)
+    assert ops.gemm_status() == 0
