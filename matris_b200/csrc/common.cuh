@@ -29,8 +29,9 @@ void set_cuda_error(cudaError_t e, const char* where);
 
 // Kernels of an evaluation are launched with programmatic stream serialization: a kernel may be scheduled, and set itself up,
 // while its predecessor is still running, and waits in pdl_sync() before it touches anything a predecessor wrote (or read).
-// Launch gaps and prologues (tensor-memory allocation, barriers, weight tiles) then overlap; on small systems, where a kernel
-// lasts a few microseconds, they are most of the time (4 atoms: 8.6 -> 7.2 ms an evaluation).  Every kernel so launched must call
+// Launch gaps and prologues (tensor-memory allocation, barriers) then overlap; on small systems, where a kernel lasts a few
+// microseconds, they are most of the time (4 atoms: 8.6 -> 7.2 ms an evaluation).  Weights and constants are read behind the wait
+// like everything else: a caller of the C ABI may have written them in the launch before.  Every kernel so launched must call
 // pdl_sync().  The first launch behind an event of another stream does without: what it waits for is more than its predecessor.
 inline thread_local bool launch_after_event = false;
 template <typename... P, typename... A>

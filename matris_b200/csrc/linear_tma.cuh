@@ -12,8 +12,8 @@
 // blocks of all of them fit the SMs at once): one CTA per (tile, column block), which shortens the chain where only latency
 // counts.
 //
-// HBM bounds the large launches: 573,894 rows take 0.175 ms for 128 -> 256 (k_gemm_ps 0.214), 0.30 for two gated 128 -> 128 blocks
-// (0.345), 0.37 for 512 -> 128, 0.29 for 128 -> 512.  One tile takes 12 us (15), with K = 512 19 us: the chain of its 16 chunks.
+// HBM bounds the large launches: 573,894 rows take 0.171 ms for 128 -> 256 (k_gemm_ps 0.214), 0.25 with a gate, 0.36 for
+// 512 -> 128, 0.275 for 128 -> 512.  One tile takes 12 us (15), with K = 512 19 us: the chain of its 16 chunks.
 
 struct alignas(64) LinMaps {
   CUtensorMap w[4][2];                       // weights of a column block: hi, lo

@@ -31,9 +31,10 @@
 // r+1 as soon as L2 gate(t) is done, under the epilogue of t.  GATED_BWD: 0, 1 and 2.  PLAIN_*: tiles alternate between the
 // two epilogue groups, L1(t) -> 2t mod 3, L2(t) -> 2t+1 mod 3, issued L1(t+1) before L2(t).
 //
-// Measured, 573,894 rows with z1 and z2 kept: two addends and a residual 0.57 ms, three addends 0.54 (nothing kept: 0.43), no
-// contraction and three addends 0.48, K = 384 gathered with a residual 0.64; GATED_BWD with a residual 0.43, with E too 0.61; FFN
-// forward 0.22, backward 0.19.  One tile alone takes 30 us forward, 22 us backward: the chain of its stages.
+// Measured behind an L2 flush (bench_gemm.py; addend tables of a fifth of the rows), 573,894 rows with z1 and z2 kept: two addends
+// and a residual 0.53 ms, three addends 0.65 (nothing kept: 0.54), no contraction and three addends 0.58, K = 384 gathered with a
+// residual 0.64; GATED_BWD with a residual 0.42, with E too 0.59; FFN forward 0.23, backward 0.18.  One tile alone takes 28 us
+// forward, 21 us backward: the chain of its stages.
 //
 // Warps: 0 MMA, 1 TMA (weights, 16 KB tiles of 64 K values, five slots), 2-9 producers, 10-17 epilogue (two groups of four; the
 // group's branch or tile parity, the warp's lane quarter).  Every mbarrier wait is bounded; on expiry the status word is set, the

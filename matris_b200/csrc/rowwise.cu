@@ -4,8 +4,9 @@
 // owns one row (or one segment); lane l holds channels 4l..4l+3 as a float4, so a
 // row is one coalesced 512-byte access and row reductions are warp shuffles.
 // Segment reductions walk CSR ranges (rows are stored grouped by target node;
-// the source-side grouping is a permutation), so there are no atomics and the
-// summation order is fixed.
+// the source-side grouping is a permutation), so they need no atomics and their
+// summation order is fixed.  The one exception is k_seg_sum's third sum, over
+// the rows of a centre atom, which adds finished pieces with atomics.
 #include <float.h>
 #include "common.cuh"
 
