@@ -93,6 +93,13 @@ class BatchedGraph:
     def device(self):
         return self.cart32.device
 
+    @property
+    def number_range(self) -> tuple[int, int]:
+        """Smallest and largest atomic number (found when a model first asks: graphs alone do without)."""
+        if getattr(self, "_number_range", None) is None:
+            self._number_range = int(self.numbers_host.min()), int(self.numbers_host.max())
+        return self._number_range
+
     def structure_slices(self):
         """Host index ranges of every structure: atoms, directed edges, bonds, triplets."""
         if getattr(self, "_slices", None) is None:
@@ -125,7 +132,6 @@ class HostBatch:
         self.lattice = np.ascontiguousarray(np.concatenate(lattices).reshape(B, 3, 3), dtype=np.float64)
         if self.numbers.shape != (N,) or self.cart.shape != (N, 3):
             raise ValueError("numbers and positions differ in length")
-        self.number_range = int(self.numbers.min()), int(self.numbers.max())
         inv = np.linalg.inv(self.lattice)
         grid, self.n_cells, self.volume = cell_grid(self.lattice, n_per, cutoff)
         # float32 model inputs exactly as the reference derives them (converter.py:82-83, processgraph.py:87)
@@ -148,7 +154,6 @@ def upload(hb: HostBatch, cutoff, line_cutoff, device) -> BatchedGraph:
     g.n_atoms, g.n_struct, g.n_cells = N, Bn, hb.n_cells
     g.cutoff, g.line_cutoff = float(cutoff), float(line_cutoff)
     g.atoms_per_graph, g.atom_ptr_host, g.numbers_host = hb.atoms_per_graph, hb.atom_ptr, hb.numbers
-    g.number_range = hb.number_range
     g.cart64_host, g.lattice64_host, g.frac32_host, g.volume64_host = hb.cart, hb.lattice, hb.frac32, hb.volume
     g.cart64, g.lattice64, g.inv_lattice64 = f64[:3 * N].view(N, 3), f64[3 * N:3 * N + 9 * Bn].view(Bn, 3, 3), \
         f64[3 * N + 9 * Bn:].view(Bn, 3, 3)
