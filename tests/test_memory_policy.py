@@ -7,7 +7,12 @@ import numpy as np
 import pytest
 import torch
 
-from matris_b200 import MatRIS, _lib
+from matris_b200 import MatRIS, _lib, build
+
+@pytest.fixture(scope="module", autouse=True)
+def library():
+    build.build()
+
 
 # per atom: directed edges within 6 A, triplets (sparse and dense crystals, close-packed metals)
 SHAPES = {"crystals": (28.0, 72.0), "glass": (50.0, 215.0), "bcc": (64.0, 260.0), "perovskite": (69.0, 322.0), "fcc": (78.0, 306.0)}
