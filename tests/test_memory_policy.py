@@ -9,6 +9,7 @@ import torch
 
 from matris_b200 import MatRIS, _lib, build
 
+
 @pytest.fixture(scope="module", autouse=True)
 def library():
     build.build()
