@@ -34,6 +34,9 @@ void set_cuda_error(cudaError_t e, const char* where);
 // like everything else: a caller of the C ABI may have written them in the launch before.  Every kernel so launched must call
 // pdl_sync().  The first launch behind an event of another stream does without: what it waits for is more than its predecessor.
 inline thread_local bool launch_after_event = false;
+// Set while an evaluation queues a launch that is not the first on its stream: the weights have not been written since before the
+// launch ahead of it (whose blocks passed their own wait before this one's were scheduled), so they may be read before pdl_sync().
+inline thread_local bool weights_settled = false;
 template <typename... P, typename... A>
 static inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
   cudaLaunchConfig_t cfg = {};

@@ -190,6 +190,7 @@ struct Run {
   bool pending[2] = {};
   int on = 0;             // 0: the caller's stream, 1 + k: side stream k
   bool behind[3] = {};    // the last thing queued there is a wait for another stream's event
+  bool queued[3] = {};    // this evaluation has launched something there
 
   // f's launches on side stream k, after everything queued on the caller's stream so far.  The buffers they touch must live, and
   // must not be written or (where f writes) read on the caller's stream, until join(k).
@@ -228,7 +229,10 @@ struct Run {
     ++launches;
     if (!g_times.on) {
       launch_after_event = behind[on];
+      weights_settled = behind[on] || queued[on];
       rc = f();
+      weights_settled = false;
+      queued[on] = true;
       behind[on] = launch_after_event;  // (what launches nothing leaves it)
       launch_after_event = false;
       return;

@@ -1,0 +1,420 @@
+// Dense layers and two-layer MLPs of few rows (included by gemm.cu inside namespace mb, after linear_tma.cuh).
+//
+// What bounds a small call is the chain of one tile, not a rate: k_mlp and k_linear walk 128-row tiles through seven or eight
+// hand-overs between warp roles, a thread works through a whole row, and all but a few multiprocessors idle (back to back, one tile
+// of the gated forward 17.7 us, of its backward 13, a dense layer 6 - 11; here 8.2, 6.9 and 3.5 - 7.6; an evaluation of 4 atoms
+// 5.1 -> 3.45 ms).  Here a block takes R = 16 or 32 rows and the product is TRANSPOSED, features x rows:
+//
+//   D^T [128 features, R rows] = W [128, K] x X^T       M = 128 weight rows (A, by TMA), N = rows (B, K-major, converted by threads)
+//
+// so that the matrix instruction's M is always full, however few the rows, and its time shrinks with them.  With thread = feature
+// (tensor-memory lane) and registers = rows, bias and weights of an epilogue are one register, a row of an addend table, gate,
+// residual or output is one 128-byte access of a warp straight from or to global memory (no staging, no hand-over), and the hidden
+// layer goes back to shared memory as the MN-major B operand of layer 2.  A feature's rows are spread over 16 warps.
+//
+// The products of a K step are accumulated in the order of the persistent kernels, so that a row's sums do not depend on how many rows
+// a call has.  (w_hi x [x_hi ; x_lo] as one instruction of N = 2 R, the small terms in columns of their own, would save a third of the
+// matrix instructions' time, but rounds differently.)
+//
+// One tile per block and every barrier used once, but for the ring of weight slots (32 KB: hi and lo of 64 K values).  Inside an
+// evaluation the weights are asked for before the wait for the preceding kernel (`early`, see common.cuh): by the time its
+// results are there, up to 128 KB of them are on chip.
+//
+// Warps 0 - 15: rows in, epilogues; 16: matrix instructions; 17: weights.
+
+enum FewMode { FEW_GATED_FWD = MLP_GATED_FWD, FEW_PLAIN_FWD = MLP_PLAIN_FWD, FEW_GATED_BWD = MLP_GATED_BWD,
+               FEW_PLAIN_BWD = MLP_PLAIN_BWD, FEW_LINEAR = 4 };
+template <int MODE> struct FewArgs { typedef MlpArgs T; };
+template <> struct FewArgs<FEW_LINEAR> { typedef mb_gemm_desc T; };
+struct alignas(64) FewMaps { CUtensorMap w[4][2]; };  // hi, lo; MLPs: layer 1, layer 2, E's weights; LINEAR: column blocks
+
+constexpr int FW_WORKERS = 16, FW_MMA_WARP = 16, FW_TMA_WARP = 17, FW_THREADS = 576;
+constexpr uint32_t FW_SMEM_LIMIT = 227 * 1024;
+constexpr uint32_t FW_SLOT_BYTES = 2 * TC_TILE_BYTES, FW_MAX_SLOTS = 6;
+constexpr uint32_t FW_GROUP = 2048;  // bytes of 8 rows x 128 K of an operand part: 16-byte cores of 8 rows x 8 K or 8 K x 8 rows
+
+// shared memory: weight ring | X segments | hidden layer | sums of squares | barriers
+__host__ __device__ constexpr uint32_t few_operand_bytes(int r) { return (uint32_t)r * 512u; }  // hi and lo of R rows x 128 K
+__host__ __device__ constexpr int few_branches(int mode) { return mode == FEW_GATED_FWD || mode == FEW_GATED_BWD ? 2 : mode == FEW_LINEAR ? 0 : 1; }
+__host__ __device__ constexpr uint32_t few_tail_bytes(int r) { return (uint32_t)r * 32u + 256u; }
+__host__ __device__ constexpr uint32_t few_columns(int mode, int r) {
+  const uint32_t need = (uint32_t)r * (mode == FEW_GATED_FWD ? 4 : mode == FEW_GATED_BWD ? 3 : mode == FEW_LINEAR ? 1 : 2);
+  return need <= 32 ? 32 : need <= 64 ? 64 : 128;
+}
+
+// no swizzle: LBO 128 bytes between cores along K, SBO 2048 between groups of 8 rows (both majors, see FW_GROUP)
+__device__ __forceinline__ uint64_t few_desc(uint32_t saddr) {
+  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (uint64_t)(128u >> 4) << 16 | (uint64_t)(FW_GROUP >> 4) << 32 | 1ull << 46;
+}
+__device__ __forceinline__ void umma_bf16_ss(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+               :: "r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+}
+template <int N> __device__ __forceinline__ void few_tmem_ld(uint32_t addr, uint32_t (&v)[N]) {
+  static_assert(N == 4 || N == 8, "rows of a thread");
+  if constexpr (N == 8)
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(addr) : "memory");
+  else
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr) : "memory");
+}
+template <int RT> __device__ __forceinline__ void few_result(uint32_t addr, float (&y)[RT]) {
+  uint32_t a[RT];
+  few_tmem_ld(addr, a);
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < RT; ++i) y[i] = __uint_as_float(a[i]);
+}
+// V sums of squares over the 32 lanes at once: lane l ends with that of value l / (32 / V) (V - 1 + log2(32 / V) shuffles).  The order
+// of the additions is that of sum_of_squares() in mlp_fused.cuh.
+template <int V> __device__ __forceinline__ float few_sums_of_squares(float (&v)[V], int lane) {
+  int o = 16;
+#pragma unroll
+  for (int n = V / 2; n > 0; n >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float own = up ? v[i + n] : v[i], other = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + n], o);
+      if (2 * n == V) {
+        const float lower = up ? other : own, upper = up ? own : other;
+        v[i] = fmaf(upper, upper, __fmul_rn(lower, lower));
+      } else {
+        v[i] = own + other;
+      }
+    }
+  }
+  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
+}
+
+template <int MODE, int R>
+__global__ void __launch_bounds__(FW_THREADS, MODE == FEW_LINEAR ? 2 : 1)
+k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant__ FewMaps maps, const int n_slots, const int early) {
+  constexpr bool LINEAR = MODE == FEW_LINEAR, GATED = MODE == FEW_GATED_FWD || MODE == FEW_GATED_BWD;
+  constexpr bool FWD = MODE == FEW_GATED_FWD || MODE == FEW_PLAIN_FWD, BWD = MODE == FEW_GATED_BWD || MODE == FEW_PLAIN_BWD;
+  constexpr int NB = GATED ? 2 : 1, RT = R / 4, JOBS = R / 2;  // rows of a thread; (8 rows x 32 values) pieces of a segment
+  constexpr uint32_t OPERAND = few_operand_bytes(R), LO = (R / 8) * FW_GROUP;
+  constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)R >> 3) << 17 | ((128u >> 4) << 24), MN_MAJOR_B = 1u << 16;
+  constexpr uint32_t COLUMNS = few_columns(MODE, R);
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t sm0 = smem_u32(smem);
+  if ((sm0 & 1023u) != 0) {
+    if (threadIdx.x == 0) atomicOr(&g_gemm_status, 2);
+    return;
+  }
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int64_t row0 = (int64_t)blockIdx.x * R, n_rows = d.n_rows;
+  int n_src, n_ext = 0;  // segments of layer 1 (GATED_BWD: core and gate half of dz2); of E
+  if constexpr (LINEAR) n_src = d.blk[blockIdx.y].n_src;
+  else n_src = d.n_src;
+  if constexpr (MODE == FEW_GATED_BWD) n_ext = d.n_ext;
+  const int n_seg = n_src + n_ext;
+
+  const uint32_t x_sm = sm0 + n_slots * FW_SLOT_BYTES, act_sm = x_sm + n_seg * OPERAND, ss_off = act_sm + few_branches(MODE) * OPERAND - sm0;
+  float* const sums = reinterpret_cast<float*>(smem + ss_off);  // [row quarter][value][lane quarter]
+  const uint32_t bar0 = sm0 + ss_off + R * 32;
+  // w_full[6] w_empty[6] | x_ready[6] (per segment) | act_ready[2] d1_full[2] | d2_full[2] | retired | tensor-memory address
+  const uint32_t w_full = bar0, w_empty = bar0 + 48, x_ready = bar0 + 96, act_ready = bar0 + 144, d1_full = bar0 + 160,
+                 d2_full = bar0 + 176, retired = bar0 + 192, slot_at = bar0 + 200;
+  if (warp == FW_MMA_WARP) {
+    if (lane == 0) {
+      for (uint32_t b = 0; b < FW_MAX_SLOTS; ++b) { mbar_init(w_full + 8 * b, 1); mbar_init(w_empty + 8 * b, 1); mbar_init(x_ready + 8 * b, JOBS); }
+      for (int b = 0; b < 2; ++b) { mbar_init(act_ready + 8 * b, FW_WORKERS); mbar_init(d1_full + 8 * b, 1); mbar_init(d2_full + 8 * b, 1); }
+      mbar_init(retired, 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncwarp();
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(slot_at), "r"(COLUMNS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  uint32_t tmem_base;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(slot_at) : "memory");
+
+  // The sequence of 64-value K pieces both issuing warps walk: step(number, layer, branch, piece).  Layer 2 stands for E.
+  auto walk = [&](auto step) {
+    int n = 0;
+    for (int br = 0; br < NB; ++br)
+      for (int kp = 0; kp < (MODE == FEW_GATED_BWD ? 2 : 2 * n_src); ++kp) step(n++, 0, br, kp);
+    for (int kp = 0; kp < 2 * n_ext; ++kp) step(n++, 2, 0, kp);
+    if constexpr (!LINEAR)
+      for (int br = 0; br < NB; ++br)
+        for (int kp = 0; kp < 2; ++kp) step(n++, 1, br, kp);
+  };
+
+  if (warp == FW_MMA_WARP) {
+    uint32_t elected;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
+    const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0), sm_u = __shfl_sync(0xffffffffu, sm0, 0);
+    const uint32_t x_u = sm_u + n_slots * FW_SLOT_BYTES, act_u = x_u + n_seg * OPERAND;
+    bool alive = true;
+    auto wait = [&](uint32_t bar, uint32_t parity) { if (alive) alive = mbar_wait(bar, parity & 1); };
+    walk([&](int n, int layer, int br, int kp) {
+      const int slot = n % n_slots;
+      uint32_t operand, d_col, idesc = IDESC;
+      bool fresh = kp == 0, last;
+      if (layer == 1) {
+        if (kp == 0) wait(act_ready + 8 * br, 0);
+        operand = act_u + br * OPERAND + kp * 1024u;
+        idesc |= MN_MAJOR_B;
+        d_col = (uint32_t)R * (MODE == FEW_GATED_FWD ? 2 + br : NB);
+        if (MODE == FEW_GATED_BWD && (br == 1 || n_ext > 0)) fresh = false;
+        last = kp == 1 && (MODE != FEW_GATED_BWD || br == 1);
+      } else {
+        const int seg = layer == 2 ? n_src + (kp >> 1) : MODE == FEW_GATED_BWD ? br : kp >> 1;
+        if ((kp & 1) == 0) wait(x_ready + 8 * seg, 0);
+        operand = x_u + seg * OPERAND + (kp & 1) * 1024u;
+        d_col = layer == 2 ? 2u * R : (uint32_t)R * br;
+        last = layer == 0 && kp == (MODE == FEW_GATED_BWD ? 2 : 2 * n_src) - 1;
+      }
+      wait(w_full + 8 * slot, (uint32_t)(n / n_slots));
+      alive = __all_sync(0xffffffffu, alive);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (elected) {
+        const uint64_t wh = umma_desc(sm_u + slot * FW_SLOT_BYTES), wl = umma_desc(sm_u + slot * FW_SLOT_BYTES + TC_TILE_BYTES);
+        const uint64_t xh = few_desc(operand), xl = few_desc(operand + LO);
+        const uint32_t dt = tmem_u + d_col;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {  // K steps of 16: 32 bytes of the weight rows, two cores of the rows
+          umma_bf16_ss(dt, wh + 2 * kk, xl + 16 * kk, idesc, (!fresh || kk > 0) ? 1u : 0u);
+          umma_bf16_ss(dt, wl + 2 * kk, xh + 16 * kk, idesc, 1u);
+          umma_bf16_ss(dt, wh + 2 * kk, xh + 16 * kk, idesc, 1u);
+        }
+        mma_commit(w_empty + 8 * slot);
+        if (last) mma_commit(layer == 1 ? d2_full + (MODE == FEW_GATED_FWD ? 8 * br : 0) : LINEAR ? d2_full : d1_full + 8 * br);
+      }
+      __syncwarp();
+    });
+    drain_mma(retired, elected);
+  } else if (warp == FW_TMA_WARP) {
+    if (!early) pdl_sync();
+    uint32_t elected;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
+    const uint32_t sm_u = __shfl_sync(0xffffffffu, sm0, 0);
+    bool alive = true;
+    uint32_t asked = 0;
+    walk([&](int n, int layer, int br, int kp) {
+      const int slot = n % n_slots;
+      if (n >= n_slots && alive) alive = mbar_wait(w_empty + 8 * slot, (uint32_t)(n / n_slots - 1) & 1);
+      alive = __all_sync(0xffffffffu, alive);
+      if (!alive) return;
+      // the rows of a branch's weights, but W1t of GATED_BWD has its branches side by side
+      const bool beside = MODE == FEW_GATED_BWD && layer == 1;
+      const int x = 64 * kp + (beside ? 128 * br : 0), y = beside ? 0 : 128 * br;
+      if (elected) {
+        const CUtensorMap* const m = maps.w[LINEAR ? (int)blockIdx.y : layer];
+        const uint32_t bar = w_full + 8 * slot, dst = sm_u + slot * FW_SLOT_BYTES;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(FW_SLOT_BYTES) : "memory");
+        tma_load_2d(dst, m, bar, x, y);
+        tma_load_2d(dst + TC_TILE_BYTES, m + 1, bar, x, y);
+      }
+      __syncwarp();
+      ++asked;
+    });
+    drain_copies(w_full, (uint32_t)n_slots, asked);
+  } else {
+    // ---------------------------------------------------------------- workers
+    const int q = warp & 3, rg = warp >> 2, f = 32 * q + lane, r0 = rg * RT;
+    const uint32_t lane_q = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)r0;
+    bool alive = true;
+    auto wait = [&](uint32_t bar) {
+      if (alive) alive = mbar_wait(bar, 0);
+      alive = __all_sync(0xffffffffu, alive);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    };
+    auto row_of = [&](int i) { const int64_t r = row0 + r0 + i; return r < n_rows ? r : n_rows - 1; };  // (past the end: the last row)
+    const int n_own = (int)(n_rows - row0 - r0 < RT ? n_rows - row0 - r0 : RT);                       // rows to be written (may be < 0)
+    auto store = [&](float* p, int64_t ld, const float (&v)[RT]) {
+#pragma unroll
+      for (int i = 0; i < RT; ++i)
+        if (i < n_own && alive) p[(row0 + r0 + i) * ld] = v[i];
+    };
+    pdl_sync();
+    // ---------------------------------------------- X: 8 rows x 32 values per warp and turn, lane = (row, 8 values)
+    for (int j = warp; j < n_seg * JOBS; j += FW_WORKERS) {
+      const int seg = j / JOBS, piece = j % JOBS, n = 8 * (piece >> 2) + (lane & 7), c8 = 4 * (piece & 3) + (lane >> 3);
+      const mb_src* sr;
+      if constexpr (LINEAR) sr = &d.blk[blockIdx.y].src[seg];
+      else sr = seg < n_src ? &d.src[seg] : &d.ext[seg - n_src];
+      int64_t r = row0 + n < n_rows ? row0 + n : n_rows - 1;
+      if (sr->idx) r = sr->idx[r];
+      const float* const p = sr->ptr + r * sr->ld + sr->col + 8 * c8;
+      const float4 u = ld4(p), v = ld4(p + 4);
+      float x[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+      if (sr->act) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = silu_fast_f(x[i]);
+      }
+      uint32_t hi[4], lo[4];
+      split_bf16(x, hi, lo);
+      const uint32_t at = x_sm + seg * OPERAND + (n >> 3) * FW_GROUP + c8 * 128u + (n & 7) * 16u;
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" :: "r"(at), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]) : "memory");
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" :: "r"(at + LO), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]) : "memory");
+      to_async_proxy();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(x_ready + 8 * seg);
+    }
+    if constexpr (LINEAR) {
+      const mb_colblock& cb = d.blk[blockIdx.y];
+      const float bias = cb.bias ? cb.bias[f] : 0.f, rw = cb.res && cb.res_w ? cb.res_w[f] : 1.f, sc = cb.out_scale;
+      float g[RT], x[RT], y[RT];
+      if (cb.gate) {
+#pragma unroll
+        for (int i = 0; i < RT; ++i) g[i] = cb.gate[row_of(i) * cb.ld_gate + cb.col_gate + f];
+      }
+      if (cb.res) {
+#pragma unroll
+        for (int i = 0; i < RT; ++i) x[i] = cb.res[row_of(i) * cb.ld_res + cb.col_res + f];
+      }
+      wait(d2_full);
+      few_result(lane_q, y);
+#pragma unroll
+      for (int i = 0; i < RT; ++i) {
+        y[i] += bias;
+        if (cb.gate) y[i] *= silu_grad_fast_f(g[i]);
+        if (cb.out_act) y[i] = silu_fast_f(y[i]);
+        if (cb.res) y[i] = fmaf(rw, x[i], y[i]);
+        y[i] *= sc;
+      }
+      float* const out = cb.out + cb.col_out + f;
+      if (cb.mode == MB_OUT_STORE) {
+        store(out, cb.ld_out, y);
+      } else {  // one addition per element at the memory side; every row has one writer
+#pragma unroll
+        for (int i = 0; i < RT; ++i)
+          if (i < n_own && alive) atomicAdd(out + (row0 + r0 + i) * cb.ld_out, y[i]);
+      }
+    } else {
+      // -------------------------------------------- what the epilogues add, on its way while the first products are formed
+      float side[NB][RT], res[RT];
+      const bool has_res = d.out2 != nullptr;
+      if constexpr (FWD) {
+#pragma unroll
+        for (int br = 0; br < NB; ++br) {
+          const float b = d.b1 ? d.b1[128 * br + f] : 0.f;
+#pragma unroll
+          for (int i = 0; i < RT; ++i) side[br][i] = b;
+        }
+        if constexpr (GATED)
+          for (int a = 0; a < d.n_add; ++a) {
+            const mb_add& t = d.add[a];
+            int64_t at[RT];
+#pragma unroll
+            for (int i = 0; i < RT; ++i) at[i] = (t.idx ? (int64_t)t.idx[row_of(i)] : row_of(i)) * t.ld + f;
+            float v[NB][RT];
+#pragma unroll
+            for (int br = 0; br < NB; ++br)
+#pragma unroll
+              for (int i = 0; i < RT; ++i) v[br][i] = t.ptr[at[i] + 128 * br];
+#pragma unroll
+            for (int br = 0; br < NB; ++br)
+#pragma unroll
+              for (int i = 0; i < RT; ++i) side[br][i] += v[br][i];
+          }
+      } else {
+#pragma unroll
+        for (int br = 0; br < NB; ++br)
+#pragma unroll
+          for (int i = 0; i < RT; ++i) side[br][i] = d.side[row_of(i) * d.ld_side + 128 * br + f];
+      }
+      if (has_res) {
+#pragma unroll
+        for (int i = 0; i < RT; ++i) res[i] = d.res[row_of(i) * d.ld_res + f];
+      }
+      // -------------------------------------------- layer 1 out, hidden layer back as the operand of layer 2
+#pragma unroll
+      for (int br = 0; br < NB; ++br) {
+        float x[RT];
+        if (!FWD || n_src > 0) {
+          wait(d1_full + 8 * br);
+          few_result(lane_q + (uint32_t)R * br, x);
+        } else {
+#pragma unroll
+          for (int i = 0; i < RT; ++i) x[i] = 0.f;
+        }
+        float a[RT];
+#pragma unroll
+        for (int i = 0; i < RT; ++i) {
+          if constexpr (FWD) {
+            x[i] += side[br][i];
+            a[i] = silu_fast_f(x[i]);
+          } else {
+            x[i] *= (MODE == FEW_PLAIN_BWD ? d.scale : 1.f) * silu_grad_fast_f(side[br][i]);
+            a[i] = x[i];
+          }
+        }
+        uint32_t hi[RT / 2], lo[RT / 2];
+        split_bf16(a, hi, lo);
+        const uint32_t at = act_sm + br * OPERAND + (r0 >> 3) * FW_GROUP + f * 16u + (r0 & 7) * 2u;
+        if constexpr (RT == 8) {
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" :: "r"(at), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]) : "memory");
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" :: "r"(at + LO), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]) : "memory");
+        } else {
+          asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(at), "r"(hi[0]), "r"(hi[1]) : "memory");
+          asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(at + LO), "r"(lo[0]), "r"(lo[1]) : "memory");
+        }
+        to_async_proxy();
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(act_ready + 8 * br);
+        if (d.z1) store(d.z1 + 128 * br + f, d.ld_z1, x);
+      }
+      // -------------------------------------------- layer 2 out
+      float y[RT];
+      if constexpr (MODE == FEW_GATED_FWD) {
+        float z[2][RT], v[2 * RT];
+#pragma unroll
+        for (int br = 0; br < 2; ++br) {
+          const float b = d.b2 ? d.b2[128 * br + f] : 0.f;
+          wait(d2_full + 8 * br);
+          few_result(lane_q + (uint32_t)R * (2 + br), z[br]);
+#pragma unroll
+          for (int i = 0; i < RT; ++i) {
+            z[br][i] += b;
+            v[RT * br + i] = z[br][i];
+          }
+          if (d.z2) store(d.z2 + 128 * br + f, d.ld_z2, z[br]);
+        }
+        constexpr int PER = 32 / (2 * RT);  // lanes that end with the same sum
+        const float s = few_sums_of_squares(v, lane);
+        if (lane % PER == 0) sums[(rg * 2 * RT + lane / PER) * 4 + q] = s;
+        asm volatile("bar.sync %0, 128;" :: "r"(1 + rg) : "memory");  // the four lane quarters of these rows
+        const float nc = d.norm_core[f], ng = d.norm_gate[f];
+#pragma unroll
+        for (int i = 0; i < RT; ++i) {
+          const float4 c = *reinterpret_cast<const float4*>(sums + (rg * 2 * RT + i) * 4);
+          const float4 g = *reinterpret_cast<const float4*>(sums + (rg * 2 * RT + RT + i) * 4);
+          const float rc = rsqrtf(((c.x + c.y) + (c.z + c.w)) * (1.0f / 128.0f) + ML_RMS_EPS);
+          const float rr = rsqrtf(((g.x + g.y) + (g.z + g.w)) * (1.0f / 128.0f) + ML_RMS_EPS);
+          y[i] = gated_value(z[0][i] * (rc * nc), z[1][i] * (rr * ng));
+        }
+      } else {
+        const float b = FWD && d.b2 ? d.b2[f] : 0.f;
+        wait(d2_full);
+        few_result(lane_q + (uint32_t)R * NB, y);
+#pragma unroll
+        for (int i = 0; i < RT; ++i) y[i] += b;
+      }
+      if (d.h) store(d.h + f, d.ld_h, y);
+      if (has_res) {
+        const float rw = d.res_w ? d.res_w[f] : 1.f;
+#pragma unroll
+        for (int i = 0; i < RT; ++i) y[i] = fmaf(rw, res[i], y[i]);
+        store(d.out2 + f, d.ld_out2, y);
+      }
+    }
+  }
+
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == FW_MMA_WARP) {
+    __syncwarp();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"(COLUMNS) : "memory");
+  }
+}

@@ -609,6 +609,7 @@ k_gemm_tc(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ TcMaps
 #include "gemm_persistent.cuh"
 #include "mlp_fused.cuh"
 #include "linear_tma.cuh"
+#include "few_rows.cuh"
 
 // 0: persistent tcgen05 3xBF16 (default), 1: fp32 SIMT, 2: one-tile-per-CTA tcgen05 3xTF32, 3: persistent tcgen05 3xTF32
 static int g_gemm_mode = 0;
@@ -676,6 +677,44 @@ static int row_map(const float* p, int64_t ld, int cols, int64_t rows, CUtensorM
 // Per-device set-up of the tensor-core kernels: the dynamic shared-memory attribute belongs to the (function, device)
 // pair and the persistent grids are sized by the device's SM count.  One slot per device ordinal; two host threads
 // that race on a device's first call write the same values.
+template <int MODE> static int few_config_mode() {
+  MB_CUDA_CHECK(cudaFuncSetAttribute(k_few<MODE, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, FW_SMEM_LIMIT));
+  MB_CUDA_CHECK(cudaFuncSetAttribute(k_few<MODE, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, FW_SMEM_LIMIT));
+  return MB_OK;
+}
+static int few_config() {
+  int rc = few_config_mode<FEW_LINEAR>();
+  if (!rc) rc = few_config_mode<FEW_GATED_FWD>();
+  if (!rc) rc = few_config_mode<FEW_PLAIN_FWD>();
+  if (!rc) rc = few_config_mode<FEW_GATED_BWD>();
+  if (!rc) rc = few_config_mode<FEW_PLAIN_BWD>();
+  return rc;
+}
+// R of k_few for a launch, 0: the persistent kernels.  A block of k_few takes one tile, so the line lies where its tiles no longer run
+// side by side: 16 rows a block while a multiprocessor gets one at most, then 32 while all are resident (dense layers with K = 128:
+// two on a multiprocessor).  Back to back, weights in L2, us (persistent kernel / 16 / 32 rows a block): gated forward with two
+// addends, 2300 rows 17.8 / 8.5 / 10.1, 4700 rows 17.9 / 16.7 / 10.6, 9400 rows 18.7 / 33 / 20.5; its backward, 2300 rows 13.1 / 7.2 /
+// 7.9, 9400 rows 14.2 / 29 / 16.1; dense 128 -> 128, 2300 rows 6.1 / 3.6 / 4.3, 4700 rows 6.1 / 4.9 / 4.4, 9400 rows 6.9 / 9.6 / 6.1;
+// dense 128 -> 512, 2300 rows 6.7 / 9.6 / 6.1, 4700 rows 7.5 / 17.7 / 11.8; dense 512 -> 128, 2300 rows 10.9 / 7.8 / 8.1.
+static int few_choice(int mode, int64_t n_rows, int n_src, int n_blocks, int n_sm) {
+  const int64_t t16 = (n_rows + 15) / 16 * n_blocks, t32 = (n_rows + 31) / 32 * n_blocks;
+  if (t16 <= n_sm) return 16;
+  return t32 <= (mode == FEW_LINEAR && n_src == 1 ? 2 : 1) * (int64_t)n_sm ? 32 : 0;
+}
+// n_seg: A segments of a block, n_kp: weight slots it uses
+template <int MODE> static void few_launch(const typename FewArgs<MODE>::T& args, const FewMaps& maps, int r, int n_seg, int n_kp,
+                                           int n_blocks, cudaStream_t st) {
+  const uint32_t rest = (n_seg + few_branches(MODE)) * few_operand_bytes(r) + few_tail_bytes(r);
+  uint32_t slots = (FW_SMEM_LIMIT - rest) / FW_SLOT_BYTES;
+  if (slots > FW_MAX_SLOTS) slots = FW_MAX_SLOTS;
+  if (slots > (uint32_t)n_kp) slots = (uint32_t)n_kp;
+  const dim3 grid((unsigned)((args.n_rows + r - 1) / r), (unsigned)n_blocks);
+  const size_t smem = slots * FW_SLOT_BYTES + rest;
+  const int early = weights_settled ? 1 : 0;
+  if (r == 16) launch(k_few<MODE, 16>, grid, FW_THREADS, smem, st, args, maps, (int)slots, early);
+  else launch(k_few<MODE, 32>, grid, FW_THREADS, smem, st, args, maps, (int)slots, early);
+}
+
 struct DeviceConfig { bool ready; int n_sm; };
 static DeviceConfig g_device_config[64];
 
@@ -693,6 +732,7 @@ static int device_config(int* n_sm) {
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_PLAIN_FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_GATED_BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_PLAIN_BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
+    if (int rc = few_config()) return rc;
     int n = 0;
     MB_CUDA_CHECK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
     c.n_sm = n;
@@ -922,6 +962,18 @@ extern "C" int mb_gemm(const mb_gemm_desc* desc, void* stream_) {
           same_a = a.src[s].ptr == b.src[s].ptr && a.src[s].idx == b.src[s].idx && a.src[s].ld == b.src[s].ld &&
                    a.src[s].col == b.src[s].col && a.src[s].act == b.src[s].act;
       }
+      if (direct) {
+        int n_src = 1;
+        for (int j = 0; j < desc->n_blocks; ++j) n_src = desc->blk[j].n_src > n_src ? desc->blk[j].n_src : n_src;
+        if (const int r = mb::few_choice(mb::FEW_LINEAR, desc->n_rows, n_src, desc->n_blocks, n_sm)) {
+          mb::FewMaps fm;
+          for (int j = 0; j < desc->n_blocks; ++j)
+            for (int part = 0; part < 2; ++part) fm.w[j][part] = maps.m[j][part];
+          mb::few_launch<mb::FEW_LINEAR>(*desc, fm, r, n_src, 2 * n_src, desc->n_blocks, (cudaStream_t)stream_);
+          MB_LAUNCH_CHECK("k_few");
+          return MB_OK;
+        }
+      }
       direct = direct && (same_a ? desc->blk[0].n_src == 1 || desc->n_blocks <= 3 : one_seg) && desc->n_rows <= 0x7fffff00LL;
       if (direct) {
         mb::LinMaps lm;
@@ -1082,10 +1134,21 @@ extern "C" int mb_gated_mlp_fwd(const mb_gated_mlp* g, void* stream_) {
   a.z1 = g->z1; a.ld_z1 = g->ld_z1; a.z2 = g->z2; a.ld_z2 = g->ld_z2; a.h = g->h; a.ld_h = g->ld_h;
   a.res = g->res; a.res_w = g->res_w; a.ld_res = g->ld_res; a.out2 = g->out2; a.ld_out2 = g->ld_out2;
   const int width = plain ? 128 : 256;
+  if (plain) a.z2 = nullptr;
+  if (const int r = mb::few_choice(plain ? mb::FEW_PLAIN_FWD : mb::FEW_GATED_FWD, g->n_rows, 1, 1, n_sm)) {
+    mb::FewMaps fm;
+    for (int part = 0; part < 2; ++part) {
+      if (g->n_src > 0) fm.w[0][part] = maps.w1[part];
+      fm.w[1][part] = maps.w2[part];
+    }
+    if (plain) mb::few_launch<mb::FEW_PLAIN_FWD>(a, fm, r, g->n_src, 2 * g->n_src + 2, 1, (cudaStream_t)stream_);
+    else mb::few_launch<mb::FEW_GATED_FWD>(a, fm, r, g->n_src, 4 * g->n_src + 4, 1, (cudaStream_t)stream_);
+    MB_LAUNCH_CHECK("k_few");
+    return MB_OK;
+  }
   for (int s = 0; s < g->n_src; ++s)
     if (!a.src[s].idx && (rc = mb::row_map(a.src[s].ptr + a.src[s].col, a.src[s].ld, 128, g->n_rows, &maps.src[s]))) return rc;
   if (a.z1 && (rc = mb::row_map(a.z1, a.ld_z1, width, g->n_rows, &maps.z1))) return rc;
-  if (plain) a.z2 = nullptr;
   if (a.z2 && (rc = mb::row_map(a.z2, a.ld_z2, width, g->n_rows, &maps.z2))) return rc;
   if (a.h && (rc = mb::row_map(a.h, a.ld_h, 128, g->n_rows, &maps.h))) return rc;
   if (a.out2 && ((rc = mb::row_map(a.out2, a.ld_out2, 128, g->n_rows, &maps.out2)) ||
@@ -1186,6 +1249,18 @@ extern "C" int mb_mlp_bwd_data(const mb_mlp_bwd* g, void* stream_) {
     a.h = g->dx; a.ld_h = g->ld_dx;
   }
   const int width = plain ? 128 : 256;
+  if (const int r = mb::few_choice(plain ? mb::FEW_PLAIN_BWD : mb::FEW_GATED_BWD, g->n_rows, 1, 1, n_sm)) {
+    mb::FewMaps fm;
+    for (int part = 0; part < 2; ++part) {
+      fm.w[0][part] = maps.w1[part];
+      fm.w[1][part] = maps.w2[part];
+      if (g->n_ext > 0) fm.w[2][part] = maps.w3[part];
+    }
+    if (plain) mb::few_launch<mb::FEW_PLAIN_BWD>(a, fm, r, 1, 4, 1, (cudaStream_t)stream_);
+    else mb::few_launch<mb::FEW_GATED_BWD>(a, fm, r, 2 + a.n_ext, 8 + 2 * a.n_ext, 1, (cudaStream_t)stream_);
+    MB_LAUNCH_CHECK("k_few");
+    return MB_OK;
+  }
   for (int s = 0; s < a.n_src; ++s)
     if (!a.src[s].idx && (rc = mb::row_map(a.src[s].ptr + a.src[s].col, a.src[s].ld, 128, g->n_rows, &maps.src[s]))) return rc;
   for (int s = 0; s < a.n_ext; ++s)

@@ -58,7 +58,6 @@ __device__ __forceinline__ void st8(float* p, const float (&v)[8]) {
                :: "r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]),      \
                   "r"(v[7]) : "memory")
 
-// two floats -> one 32-bit word of two bf16 (round to nearest even): `first` in the low half (the lower K index)
 // Two floats -> one word of two bf16 (round to nearest even), the first value in the low half.
 __device__ __forceinline__ uint32_t pack_bf16x2(float first, float second) {
   uint32_t r;
@@ -66,10 +65,10 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float first, float second) {
   return r;
 }
 
-// hi / lo split of 16 consecutive K values into 8 + 8 packed words (BF16): hi = bf16(x), lo = bf16(x - hi) ...
-__device__ __forceinline__ void split_bf16(const float (&x)[16], uint32_t (&hi)[8], uint32_t (&lo)[8]) {
+// hi / lo split of 2 H consecutive values into H + H packed words (BF16): hi = bf16(x), lo = bf16(x - hi) ...
+template <int H> __device__ __forceinline__ void split_bf16(const float (&x)[2 * H], uint32_t (&hi)[H], uint32_t (&lo)[H]) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
+  for (int i = 0; i < H; ++i) {
     hi[i] = pack_bf16x2(x[2 * i], x[2 * i + 1]);
     const float r0 = x[2 * i] - __uint_as_float(hi[i] << 16);
     const float r1 = x[2 * i + 1] - __uint_as_float(hi[i] & 0xFFFF0000u);

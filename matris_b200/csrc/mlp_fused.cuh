@@ -125,6 +125,19 @@ __device__ __forceinline__ float gated_value(float a, float b) {
   return a * r;
 }
 
+// Sum of squares of 32 values of a row, halves added to halves: the order in which k_few adds them across its lanes, so that a row's
+// norm does not depend on which kernel a launch of its size takes.
+__device__ __forceinline__ float sum_of_squares(const float (&y)[32]) {
+  float v[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = fmaf(y[i + 16], y[i + 16], __fmul_rn(y[i], y[i]));
+#pragma unroll
+  for (int n = 8; n > 0; n >>= 1)
+#pragma unroll
+    for (int i = 0; i < n; ++i) v[i] += v[i + n];
+  return v[0];
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(ML_THREADS, 1)
 k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
@@ -495,7 +508,7 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
         wait(d2_full + 8 * grp, par);
         const float4* const b2s = reinterpret_cast<const float4*>(cst + 256);
         const uint32_t own = lane_q + 128u * reg_d;
-        float ss = 0.f;
+        float s01 = 0.f, s23 = 0.f;
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
           float y[32];
@@ -504,12 +517,13 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
           for (int j = 0; j < 8; ++j) {
             const float4 v = b2s[32 * grp + 8 * c + j];
             y[4 * j] += v.x; y[4 * j + 1] += v.y; y[4 * j + 2] += v.z; y[4 * j + 3] += v.w;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) ss = fmaf(y[4 * j + i], y[4 * j + i], ss);
           }
+          const float s = sum_of_squares(y);
+          if (c < 2) s01 += s;
+          else s23 += s;
           if (d.z2) write(&maps.z2, y, 128 * grp + 32 * c, row0);
         }
-        rinvs[((t & 1) * 2 + grp) * 128 + q * 32 + lane] = rsqrtf(ss * (1.0f / 128.0f) + ML_RMS_EPS);
+        rinvs[((t & 1) * 2 + grp) * 128 + q * 32 + lane] = rsqrtf((s01 + s23) * (1.0f / 128.0f) + ML_RMS_EPS);
         wait(d2_full + 8 * (grp ^ 1), par);
         asm volatile("bar.sync %0, 64;" :: "r"(1 + q) : "memory");  // the two groups' warps of this lane quarter
         const float rc = rinvs[((t & 1) * 2) * 128 + q * 32 + lane], rg = rinvs[((t & 1) * 2 + 1) * 128 + q * 32 + lane];
