@@ -2,8 +2,8 @@
 //
 // What bounds a small call is the chain of one tile, not a rate: k_mlp and k_linear walk 128-row tiles through seven or eight
 // hand-overs between warp roles, a thread works through a whole row, and all but a few multiprocessors idle (back to back, one tile
-// of the gated forward 17.7 us, of its backward 13, a dense layer 6 - 11; here 8.2, 6.9 and 3.5 - 7.6; an evaluation of 4 atoms
-// 5.1 -> 3.45 ms).  Here a block takes R = 16 or 32 rows and the product is TRANSPOSED, features x rows:
+// of the gated forward 17.7 us, of its backward 13, a dense layer 6 - 11; here 7.2, 6.5 and 3.3 - 6.2; an evaluation of 4 atoms
+// 5.1 -> 3.4 ms).  Here a block takes R = 16 or 32 rows and the product is TRANSPOSED, features x rows:
 //
 //   D^T [128 features, R rows] = W [128, K] x X^T       M = 128 weight rows (A, by TMA), N = rows (B, K-major, converted by threads)
 //
@@ -136,7 +136,7 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant
   uint32_t tmem_base;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(slot_at) : "memory");
 
-  // The sequence of 64-value K pieces both issuing warps walk: step(number, layer, branch, piece).  Layer 2 stands for E.
+  // The sequence of 64-value K pieces of weights: step(number, layer, branch, piece).  Layer 2 stands for E.
   auto walk = [&](auto step) {
     int n = 0;
     for (int br = 0; br < NB; ++br)
@@ -148,37 +148,22 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant
   };
 
   if (warp == FW_MMA_WARP) {
+    // The chain's longest part: 12 instructions a piece of 64 K values, 40 cycles each for N <= 32 (A is read from shared memory), if
+    // the loop around them stays short (slots counted up, no division, descriptors stepped): 1100 -> 720 cycles a piece.
     uint32_t elected;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
     const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0), sm_u = __shfl_sync(0xffffffffu, sm0, 0);
     const uint32_t x_u = sm_u + n_slots * FW_SLOT_BYTES, act_u = x_u + n_seg * OPERAND;
+    const uint64_t w_first = umma_desc(sm_u);
     bool alive = true;
-    auto wait = [&](uint32_t bar, uint32_t parity) { if (alive) alive = mbar_wait(bar, parity & 1); };
-    walk([&](int n, int layer, int br, int kp) {
-      const int slot = n % n_slots;
-      uint32_t operand, d_col, idesc = IDESC;
-      bool fresh = kp == 0, last;
-      if (layer == 1) {
-        if (kp == 0) wait(act_ready + 8 * br, 0);
-        operand = act_u + br * OPERAND + kp * 1024u;
-        idesc |= MN_MAJOR_B;
-        d_col = (uint32_t)R * (MODE == FEW_GATED_FWD ? 2 + br : NB);
-        if (MODE == FEW_GATED_BWD && (br == 1 || n_ext > 0)) fresh = false;
-        last = kp == 1 && (MODE != FEW_GATED_BWD || br == 1);
-      } else {
-        const int seg = layer == 2 ? n_src + (kp >> 1) : MODE == FEW_GATED_BWD ? br : kp >> 1;
-        if ((kp & 1) == 0) wait(x_ready + 8 * seg, 0);
-        operand = x_u + seg * OPERAND + (kp & 1) * 1024u;
-        d_col = layer == 2 ? 2u * R : (uint32_t)R * br;
-        last = layer == 0 && kp == (MODE == FEW_GATED_BWD ? 2 : 2 * n_src) - 1;
-      }
-      wait(w_full + 8 * slot, (uint32_t)(n / n_slots));
-      alive = __all_sync(0xffffffffu, alive);
+    uint32_t slot = 0, phase = 0;  // of the next piece
+    auto wait = [&](uint32_t bar, uint32_t parity) { if (alive) alive = mbar_wait(bar, parity); };
+    // one piece; xh: descriptor of the rows' hi part
+    auto piece = [&](uint32_t dt, uint64_t xh, uint32_t idesc, bool fresh) {
+      wait(w_full + 8 * slot, phase);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (elected) {
-        const uint64_t wh = umma_desc(sm_u + slot * FW_SLOT_BYTES), wl = umma_desc(sm_u + slot * FW_SLOT_BYTES + TC_TILE_BYTES);
-        const uint64_t xh = few_desc(operand), xl = few_desc(operand + LO);
-        const uint32_t dt = tmem_u + d_col;
+        const uint64_t wh = w_first + slot * (FW_SLOT_BYTES >> 4), wl = wh + (TC_TILE_BYTES >> 4), xl = xh + (LO >> 4);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {  // K steps of 16: 32 bytes of the weight rows, two cores of the rows
           umma_bf16_ss(dt, wh + 2 * kk, xl + 16 * kk, idesc, (!fresh || kk > 0) ? 1u : 0u);
@@ -186,10 +171,40 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant
           umma_bf16_ss(dt, wh + 2 * kk, xh + 16 * kk, idesc, 1u);
         }
         mma_commit(w_empty + 8 * slot);
-        if (last) mma_commit(layer == 1 ? d2_full + (MODE == FEW_GATED_FWD ? 8 * br : 0) : LINEAR ? d2_full : d1_full + 8 * br);
       }
       __syncwarp();
-    });
+      if (++slot == (uint32_t)n_slots) { slot = 0; phase ^= 1; }
+    };
+    auto segment = [&](int seg, uint32_t dt, bool fresh) {  // both pieces of an X segment
+      wait(x_ready + 8 * seg, 0);
+      const uint64_t xh = few_desc(x_u + seg * OPERAND);
+#pragma unroll 1
+      for (int kp = 0; kp < 2; ++kp) piece(dt, xh + kp * (1024 / 16), IDESC, fresh && kp == 0);
+    };
+    auto full = [&](uint32_t bar) {
+      if (elected) mma_commit(bar);
+      __syncwarp();
+    };
+#pragma unroll 1
+    for (int br = 0; br < NB; ++br) {
+#pragma unroll 1
+      for (int s = 0; s < (MODE == FEW_GATED_BWD ? 1 : n_src); ++s) segment(MODE == FEW_GATED_BWD ? br : s, tmem_u + R * br, s == 0);
+      if (n_src > 0) full(LINEAR ? d2_full : d1_full + 8 * br);
+    }
+#pragma unroll 1
+    for (int s = 0; s < n_ext; ++s) segment(n_src + s, tmem_u + 2 * R, s == 0);
+    if (!LINEAR) {
+#pragma unroll 1
+      for (int br = 0; br < NB; ++br) {
+        wait(act_ready + 8 * br, 0);
+        const uint32_t dt = tmem_u + R * (MODE == FEW_GATED_FWD ? 2 + br : NB);
+        const uint64_t ah = few_desc(act_u + br * OPERAND);
+#pragma unroll 1
+        for (int kp = 0; kp < 2; ++kp)
+          piece(dt, ah + kp * (1024 / 16), IDESC | MN_MAJOR_B, kp == 0 && !(MODE == FEW_GATED_BWD && (br == 1 || n_ext > 0)));
+        if (MODE != FEW_GATED_BWD || br == 1) full(d2_full + (MODE == FEW_GATED_FWD ? 8 * br : 0));
+      }
+    }
     drain_mma(retired, elected);
   } else if (warp == FW_TMA_WARP) {
     if (!early) pdl_sync();

@@ -692,10 +692,9 @@ static int few_config() {
 }
 // R of k_few for a launch, 0: the persistent kernels.  A block of k_few takes one tile, so the line lies where its tiles no longer run
 // side by side: 16 rows a block while a multiprocessor gets one at most, then 32 while all are resident (dense layers with K = 128:
-// two on a multiprocessor).  Back to back, weights in L2, us (persistent kernel / 16 / 32 rows a block): gated forward with two
-// addends, 2300 rows 17.8 / 8.5 / 10.1, 4700 rows 17.9 / 16.7 / 10.6, 9400 rows 18.7 / 33 / 20.5; its backward, 2300 rows 13.1 / 7.2 /
-// 7.9, 9400 rows 14.2 / 29 / 16.1; dense 128 -> 128, 2300 rows 6.1 / 3.6 / 4.3, 4700 rows 6.1 / 4.9 / 4.4, 9400 rows 6.9 / 9.6 / 6.1;
-// dense 128 -> 512, 2300 rows 6.7 / 9.6 / 6.1, 4700 rows 7.5 / 17.7 / 11.8; dense 512 -> 128, 2300 rows 10.9 / 7.8 / 8.1.
+// two on a multiprocessor).  Back to back, weights in L2, us (persistent kernel / here): gated forward with two addends, 2300 rows 17.8 /
+// 7.5, 4700 rows 17.9 / 9.3; its backward 13.1 / 6.9 and 13.3 / 7.7; dense 128 -> 128 6.1 / 3.4 and 6.1 / 4.2; dense 128 -> 512, 1180
+// rows 6.2 / 4.1, 2300 rows 6.7 / 5.7; dense 512 -> 128 10.9 / 6.6 and 11 / 7.2.
 static int few_choice(int mode, int64_t n_rows, int n_src, int n_blocks, int n_sm) {
   const int64_t t16 = (n_rows + 15) / 16 * n_blocks, t32 = (n_rows + 31) / 32 * n_blocks;
   if (t16 <= n_sm) return 16;
