@@ -87,6 +87,44 @@ __device__ __forceinline__ float silu_grad_fast_f(float x) {
   return s * fmaf(x, 1.0f - s, 1.0f);
 }
 
+// What the gradient of a row ahead of a gated MLP's tail consists of (row_math.cuh has the expressions)
+struct RowGrad {
+  int32_t kind;        // 0: dh_in, 1: attention rows, 2: smoothed rows
+  int32_t idx_stride;  // of tgt and src
+  const float* dh_in; const int32_t* dh_map; float dh_scale;  // given part (kinds 1 and 2: may be NULL)
+  const int32_t *tgt, *src, *emap;
+  const float *logits, *h, *agg_t, *agg_s, *stats, *dagg_t, *dagg_s;  // kind 1
+  float* dlogits;                                                     // kind 1, optional in the few-row product
+  const float *env, *dagg;                                            // kind 2
+  const float *z2, *norm_core, *norm_gate;                            // the tail: z2 [rows, 256]
+};
+// The backward pass of a gated MLP from a row's gradient on, for few rows, as one launch: dz2 = tail'(RowGrad) in registers,
+// dz1 = (dz2 W2t) SiLU'(z1), and, with n_out > 0, out[j] = dz1 W1t_j (+ dlogits W3t) (+ res_w res, j = 0).  W1t has 128 rows for
+// every output.  `zero`: n_zero floats to be cleared on the way (a multiple of 4).
+struct RowBwd {
+  int64_t n_rows;
+  RowGrad g;
+  mb_weight w2t, w1t, w3t;  // w3t.W NULL: no logits' share
+  const float* z1; float* dz1;
+  int32_t n_out;
+  float* out[3];
+  const float *res, *res_w;
+  float* zero; int64_t n_zero;
+};
+bool few_rows_fit(int64_t n_rows, int n_out);  // whether few_row_bwd (few_pair_linear) takes so many rows
+int few_row_bwd(const RowBwd& a, cudaStream_t stream);
+// n independent mb_gemm problems of few rows as one launch; with `pair` an operand row is the sum of rows i and pair[i], i = idx[r]
+bool few_linears_fit(const mb_gemm_desc* const* g, int n);
+int few_linears(const mb_gemm_desc* const* g, int n, const int32_t* pair, cudaStream_t stream);
+int few_ffn_bwd(const mb_mlp_bwd* const* g, cudaStream_t stream);  // two plain data gradients (dx only, no residual) of few rows
+// y[i] = x[i] w[i]^T, [n_rows, 7] x [7, 128], for up to MANY_LINEARS problems as one launch
+constexpr int MANY_LINEARS = 40;
+struct ManyLinears { const float *x[MANY_LINEARS], *w[MANY_LINEARS]; float* y[MANY_LINEARS]; };
+int many_small_linears(int64_t n_rows, int n, const ManyLinears& a, cudaStream_t stream);
+// d_rbf[b] += denv[b] w for the envelopes' gradient denv, which stays in registers (mb_seg_smooth_sum_bwd_env, then mb_small_linear_bwd)
+int smooth_env_bwd_rbf(int32_t n_bonds, const mb_row_graph& g, const float* env, const float* h, const float* dagg, const float* drow,
+                       const float* w, float* d_rbf, cudaStream_t stream);
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

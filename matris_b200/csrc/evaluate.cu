@@ -291,24 +291,41 @@ struct Gemm {
     b.out = out; b.ld_out = ld_out; b.col_out = col_out; b.out_idx = out_idx; b.mode = mode; b.out_scale = 1.f;
     return b;
   }
-  void run(Run& R) {
+  void run(Run& R, const int32_t* pair = nullptr) {
     if (d.n_rows == 0 || d.n_blocks == 0) return;
     double flops = 0, bytes = 4.0 * d.n_rows * 128 * (d.blk[0].n_src + d.n_blocks);
     for (int j = 0; j < d.n_blocks; ++j) {
       flops += 2.0 * d.n_rows * 128 * 128 * d.blk[j].n_src;
       bytes += 4.0 * d.n_rows * 128 * ((d.blk[j].gate != nullptr) + (d.blk[j].res != nullptr));
     }
-    R.op("mb_gemm", [&] { return mb_gemm(&d, R.st); }, flops, bytes, d.n_rows, 128 * d.blk[0].n_src, 128 * d.n_blocks);
+    const mb_gemm_desc* const one[1] = {&d};
+    R.op("mb_gemm", [&] { return pair ? few_linears(one, 1, pair, R.st) : mb_gemm(&d, R.st); }, flops, bytes, d.n_rows, 128 * d.blk[0].n_src, 128 * d.n_blocks);
   }
 };
+
+// Independent contractions of few rows as one launch, without the 4 - 9 us that a side stream's fork and join add to the chain;
+// false: nothing done, they do not all run side by side in one
+static bool together(Run& R, std::initializer_list<Gemm*> all) {
+  const mb_gemm_desc* d[4];
+  int n = 0;
+  double flops = 0, bytes = 0;
+  for (Gemm* g : all) {
+    if (g->d.n_rows == 0 || g->d.n_blocks == 0) continue;
+    d[n++] = &g->d;
+    for (int j = 0; j < g->d.n_blocks; ++j) flops += 2.0 * g->d.n_rows * 128 * 128 * g->d.blk[j].n_src;
+    bytes += 4.0 * g->d.n_rows * 128 * (g->d.blk[0].n_src + g->d.n_blocks);
+  }
+  if (!R.go() || n < 2 || !few_linears_fit(d, n)) return false;
+  R.op("mb_gemm", [&] { return few_linears(d, n, nullptr, R.st); }, flops, bytes, d[0]->n_rows, 128 * d[0]->blk[0].n_src, 128 * d[0]->n_blocks);
+  return true;
+}
 
 // y [rows, 128 nb] = epilogue(x [rows, 128 ns] W^T), ns = k / 128, nb = n_out / 128
 struct LinearOpt {
   const float* bias = nullptr; int out_act = 0, in_act = 0; const float* gate = nullptr; float scale = 1.f;
   const int32_t* idx = nullptr;
 };
-static void linear(Run& R, int64_t rows, const float* x, const mb_weight& w, int n_out, int k, float* out,
-                   const LinearOpt& o = LinearOpt()) {
+static Gemm dense(int64_t rows, const float* x, const mb_weight& w, int n_out, int k, float* out, const LinearOpt& o = LinearOpt()) {
   const int ns = k / 128, nb = n_out / 128;
   Gemm g(rows);
   for (int j = 0; j < nb; ++j) {
@@ -319,7 +336,11 @@ static void linear(Run& R, int64_t rows, const float* x, const mb_weight& w, int
     if (o.gate) { b.gate = o.gate; b.ld_gate = n_out; b.col_gate = 128 * j; }
     b.out_scale = o.scale;
   }
-  g.run(R);
+  return g;
+}
+static void linear(Run& R, int64_t rows, const float* x, const mb_weight& w, int n_out, int k, float* out,
+                   const LinearOpt& o = LinearOpt()) {
+  dense(rows, x, w, n_out, k, out, o).run(R);
 }
 
 static void fill_mlp(mb_gated_mlp& m, int64_t rows, std::initializer_list<mb_src> srcs, const mb_weight& w1,
@@ -398,21 +419,24 @@ static void edge_update_fwd(Run& R, const mb_update& p, const mb_row_graph& g, c
     if (!z1) z1 = R.ar.bottom((size_t)g.n_rows * 256);
     if (!z2) z2 = R.ar.bottom((size_t)g.n_rows * 256);
   }
-  if (Pc) R.side(0, [&] { linear(R, g.n_ctr, ctr_feat, p.wc, 256, 128, Pc); });
-  auto node_table = [&] { linear(R, g.n_nodes, node, p.wts, 512, 128, P); };
+  Gemm nodes = dense(g.n_nodes, node, p.wts, 512, 128, P), centres(0);
+  if (Pc) centres = dense(g.n_ctr, ctr_feat, p.wc, 256, 128, Pc);
   Gemm e(g.n_edge_rows);
   if (Pe)
     for (int j = 0; j < 2; ++j) e.block({src(edge)}, p.we, 128 * j, Pe, 256, 128 * j);
   if (logits)
     for (int j = 0; j < 2; ++j) e.block({src(edge)}, *wst, 128 * j, logits, 256, 128 * j);
-  if (g.is_atom) {
-    R.side(0, node_table);
-    e.run(R);
-    R.join(0);
-  } else {  // e holds the logits at most, which the caller waits for
-    if (e.d.n_blocks) R.side(0, [&] { e.run(R); });
-    node_table();
-    if (Pc) R.join(0);
+  if (!together(R, {&e, &nodes, &centres})) {
+    if (Pc) R.side(0, [&] { centres.run(R); });
+    if (g.is_atom) {
+      R.side(0, [&] { nodes.run(R); });
+      e.run(R);
+      R.join(0);
+    } else {  // e holds the logits at most, which the caller waits for
+      if (e.d.n_blocks) R.side(0, [&] { e.run(R); });
+      nodes.run(R);
+      if (Pc) R.join(0);
+    }
   }
   mb_gated_mlp m;
   if (g.is_atom) fill_mlp(m, g.n_rows, {}, p.we, p.w2, p.b1, p.b2);
@@ -428,49 +452,81 @@ static void edge_update_fwd(Run& R, const mb_update& p, const mb_row_graph& g, c
   run_mlp(R, m);
 }
 
-// Backward of the same from dz2 (and dlogits): d_edge = ... + edge_w * edge_res, d_node (+)= ... + node_w * node_res, the centre
+// The row gradient's launch where the few-row product does not form it itself (same expressions): dz2 from rg.
+static int row_grad(const RowGrad& g, int64_t rows, float* dz2, cudaStream_t st) {
+  if (g.kind == 1)
+    return mb_seg_attn_bwd(rows, g.tgt, g.src, g.idx_stride, g.emap, g.logits, g.h, g.agg_t, g.agg_s, g.stats, g.dagg_t, g.dagg_s,
+                           g.dh_in, g.dh_map, g.dh_scale, nullptr, g.dlogits, g.z2, g.norm_core, g.norm_gate, dz2, st);
+  return mb_seg_smooth_sum_bwd_rows(rows, g.tgt, g.src, g.idx_stride, g.emap, g.env, g.dagg, const_cast<float*>(g.dh_in),
+                                    g.dh_in ? 1 : 0, g.z2, g.norm_core, g.norm_gate, dz2, st);
+}
+
+// Backward of the same from the rows' gradient rg on (its dlogits where given): d_edge = ... + edge_w * edge_res, d_node (+)= ... + node_w * node_res, the centre
 // atoms' gradient is accumulated into d_ctr.
-static void edge_update_bwd(Run& R, const mb_update& p, const mb_row_graph& g, const float* z1, const float* dz2,
-                            const float* dlogits, const mb_weight* w_log, const float* edge_res, const float* edge_w,
+static void edge_update_bwd(Run& R, const mb_update& p, const mb_row_graph& g, const float* z1, const RowGrad& rg, float* dz2,
+                            const mb_weight* w_log, const float* edge_res, const float* edge_w,
                             float* d_edge, const float* node_res, const float* node_w, float* d_node, float* d_ctr) {
   Scope sc(R);
   float* dz1 = R.ar.bottom((size_t)g.n_rows * 256);
   float* dP = R.ar.bottom((size_t)g.n_nodes * 512);
   float* dPc = d_ctr ? R.ar.bottom((size_t)g.n_ctr * 256) : nullptr;
-  if (dPc) R.zero(dPc, (size_t)g.n_ctr * 1024);
+  float* const dlogits = rg.dlogits;
+  const bool few = R.go() && few_rows_fit(g.n_rows, 1);
+  RowBwd b{};
+  if (few) {
+    b.n_rows = g.n_rows; b.g = rg; b.w2t = p.w2t; b.z1 = z1; b.dz1 = dz1;
+    if (!g.is_atom) {
+      b.g.dlogits = nullptr;  // used on the way
+      b.w1t = p.wet; b.n_out = 1; b.out[0] = d_edge; b.res = edge_res; b.res_w = edge_w;
+      if (dlogits) b.w3t = *w_log;
+      b.zero = dPc; b.n_zero = dPc ? (int64_t)g.n_ctr * 256 : 0;
+    }
+    const double k = b.n_out ? (dlogits ? 768 : 512) : 256;
+    R.op(dlogits ? "mb_attn_mlp_bwd" : "mb_smooth_mlp_bwd", [&] { return few_row_bwd(b, R.st); }, 2.0 * g.n_rows * 128 * k,
+         4.0 * g.n_rows * 128 * 8, g.n_rows, 256, 256, 1);
+  } else {
+    R.op(rg.kind == 1 ? "mb_seg_attn_bwd" : "mb_seg_smooth_sum_bwd_rows", [&] { return row_grad(rg, g.n_rows, dz2, R.st); });
+    if (dPc) R.zero(dPc, (size_t)g.n_ctr * 1024);
+  }
   auto node_sums = [&] {
     MB_OP(mb_seg_sum, (int32_t)g.n_nodes, g.n_rows, g.tgt_ptr, g.src_ptr, g.src_perm, d_ctr ? g.ctr : nullptr, dz1, dP, dPc);
   };
-  auto node_grad = [&] {
-    Gemm n(g.n_nodes);
+  Gemm n(g.n_nodes);
+  {
     mb_colblock& b = n.block({src(dP, nullptr, 0, 512), src(dP, nullptr, 128, 512), src(dP, nullptr, 256, 512),
                               src(dP, nullptr, 384, 512)}, p.wtst, 0, d_node, 128, 0, nullptr, node_res ? MB_OUT_STORE : MB_OUT_ADD);
     b.res = node_res; b.res_w = node_w; b.ld_res = 128;
-    n.run(R);
-  };
+  }
   if (g.is_atom) {
-    Gemm a(g.n_rows);
-    for (int j = 0; j < 2; ++j) {
-      mb_colblock& b = a.block({src(dz2, nullptr, 128 * j, 256)}, p.w2t, 128 * j, dz1, 256, 128 * j);
-      b.gate = z1; b.ld_gate = 256; b.col_gate = 128 * j;
+    if (!few) {
+      Gemm a(g.n_rows);
+      for (int j = 0; j < 2; ++j) {
+        mb_colblock& b = a.block({src(dz2, nullptr, 128 * j, 256)}, p.w2t, 128 * j, dz1, 256, 128 * j);
+        b.gate = z1; b.ld_gate = 256; b.col_gate = 128 * j;
+      }
+      a.run(R);
     }
-    a.run(R);
     R.side(0, [&] {
       node_sums();
-      node_grad();
+      n.run(R);
     });
     const int ld = dlogits ? 512 : 256;
     float* pair = R.ar.bottom((size_t)g.n_edge_rows * ld);
-    MB_OP(mb_pair_sum, (int32_t)g.n_edge_rows, g.u2d, g.rev, dz1, dlogits, pair);
+    const bool pairs = R.go() && few_rows_fit(g.n_edge_rows, 1);  // the pair's sum is formed on the way
+    if (!pairs) MB_OP(mb_pair_sum, (int32_t)g.n_edge_rows, g.u2d, g.rev, dz1, dlogits, pair);
     Gemm e(g.n_edge_rows);
-    mb_colblock& b = e.block({src(pair, nullptr, 0, ld), src(pair, nullptr, 128, ld)}, dlogits ? *w_log : p.wet, 0, d_edge, 128);
+    auto half = [&](int j) {  // 128 columns of the sums: dz1 core and gate, dlogits
+      if (!pairs) return src(pair, nullptr, 128 * j, ld);
+      return src(j < 2 ? dz1 : dlogits, g.u2d, 128 * (j & 1), 256);
+    };
+    mb_colblock& b = e.block({half(0), half(1)}, dlogits ? *w_log : p.wet, 0, d_edge, 128);
     if (dlogits) {
-      b.src[b.n_src++] = src(pair, nullptr, 256, ld);
-      b.src[b.n_src++] = src(pair, nullptr, 384, ld);
+      b.src[b.n_src++] = half(2);
+      b.src[b.n_src++] = half(3);
     }
     b.res = edge_res; b.res_w = edge_w; b.ld_res = 128;
-    e.run(R);
-  } else {
+    e.run(R, pairs ? g.rev : nullptr);
+  } else if (!few) {
     mb_mlp_bwd m;
     memset(&m, 0, sizeof(m));
     m.n_rows = g.n_rows; m.kind = MB_MLP_GATED;
@@ -489,13 +545,12 @@ static void edge_update_bwd(Run& R, const mb_update& p, const mb_row_graph& g, c
   }
   if (!g.is_atom) {
     node_sums();
-    if (dPc)
-      R.side(0, [&] {
-        Gemm c(g.n_ctr);
-        c.block({src(dPc, nullptr, 0, 256), src(dPc, nullptr, 128, 256)}, p.wct, 0, d_ctr, 128, 0, nullptr, MB_OUT_ADD);
-        c.run(R);
-      });
-    node_grad();
+    Gemm c(g.n_ctr);
+    if (dPc) c.block({src(dPc, nullptr, 0, 256), src(dPc, nullptr, 128, 256)}, p.wct, 0, d_ctr, 128, 0, nullptr, MB_OUT_ADD);
+    if (!together(R, {&n, &c})) {
+      if (dPc) R.side(0, [&] { c.run(R); });
+      n.run(R);
+    }
   }
   R.join(0);
 }
@@ -523,12 +578,24 @@ static void update_bwd(Run& R, const mb_update& p, int64_t rows, const float* z1
     out.run(R);
     return;
   }
+  float* const t = dz2 ? nullptr : R.ar.bottom(rows * 256);
+  float* dz1 = R.ar.bottom(rows * 256);
+  bool plain = dests.size() <= 3;  // outputs at their own rows, a residual on the first at most
+  for (const Dest& d : dests) plain = plain && !d.idx && d.mode == MB_OUT_STORE && (!d.res || &d == dests.begin());
+  if (!dz2 && plain && R.go() && few_rows_fit(rows, (int)dests.size())) {
+    RowBwd b{};
+    b.n_rows = rows; b.w2t = p.w2t; b.w1t = p.w1t; b.z1 = z1;
+    b.g.dh_in = dh; b.g.z2 = z2; b.g.norm_core = p.nc; b.g.norm_gate = p.ng;
+    for (const Dest& d : dests) b.out[b.n_out++] = d.t;
+    b.res = dests.begin()->res; b.res_w = dests.begin()->res_w;
+    R.op("mb_node_mlp_bwd", [&] { return few_row_bwd(b, R.st); }, 2.0 * rows * 256 * (128 + 128 * b.n_out), 4.0 * rows * 128 * (6 + b.n_out),
+         rows, 256, 128 * b.n_out, 1);
+    return;
+  }
   if (!dz2) {
-    float* t = R.ar.bottom(rows * 256);
     MB_OP(mb_gate_bwd, rows, z2, p.nc, p.ng, dh, t);
     dz2 = t;
   }
-  float* dz1 = R.ar.bottom(rows * 256);
   Gemm g(rows);
   for (int j = 0; j < 2; ++j) {
     mb_colblock& b = g.block({src(dz2, nullptr, 128 * j, 256)}, p.w2t, 128 * j, dz1, 256, 128 * j);
@@ -557,10 +624,7 @@ static void ffn_fwd(Run& R, const mb_ffn& p, int64_t rows, const float* x, float
 }
 
 // dx = scale * ((dy W2) * silu'(z1)) W1 ; dy optionally gathered
-static void ffn_bwd(Run& R, const mb_ffn& p, int64_t rows, const float* dy, const int32_t* idx, float scale, const float* z1,
-                    float* dx) {
-  if (rows == 0) return;
-  Scope sc(R);
+static mb_mlp_bwd ffn_grad(const mb_ffn& p, int64_t rows, const float* dy, const int32_t* idx, float scale, const float* z1, float* dx) {
   mb_mlp_bwd m;
   memset(&m, 0, sizeof(m));
   m.n_rows = rows; m.kind = MB_MLP_PLAIN;
@@ -568,6 +632,13 @@ static void ffn_bwd(Run& R, const mb_ffn& p, int64_t rows, const float* dy, cons
   m.scale = scale;
   m.W2t = p.w2t; m.W1t = p.w1t;
   m.z1 = z1; m.ld_z1 = 128; m.dx = dx; m.ld_dx = 128;
+  return m;
+}
+static void ffn_bwd(Run& R, const mb_ffn& p, int64_t rows, const float* dy, const int32_t* idx, float scale, const float* z1,
+                    float* dx) {
+  if (rows == 0) return;
+  Scope sc(R);
+  mb_mlp_bwd m = ffn_grad(p, rows, dy, idx, scale, z1, dx);
   if (R.scratch) { m.dz1 = R.ar.bottom(rows * 128); m.ld_dz1 = 128; }
   R.op("mb_mlp_bwd_data", [&] { return mb_mlp_bwd_data(&m, R.st); }, 4.0 * rows * 128 * 128, 4.0 * rows * 128 * 3, rows, 128,
        128, 1);
@@ -619,11 +690,17 @@ static void attn_bwd(Run& R, const mb_attn_params& p, const mb_row_graph& g, con
   float* dz2 = gated ? R.ar.bottom(rows * 256) : nullptr;
   float* dh = gated ? nullptr : R.ar.bottom(rows * 128);
   float* dlogits = R.ar.bottom(rows * 256);
-  MB_OP(mb_seg_attn_bwd, g.n_rows, g.tgt, g.src, 1, g.emap, it.logits, it.h, it.agg_t, it.agg_s, it.stats, dagg_t, dagg_s,
-        d_edge_out, g.emap, g.is_atom ? 0.5f : 1.f, dh, dlogits, gated ? it.z2 : nullptr, gated ? p.edge.nc : nullptr,
-        gated ? p.edge.ng : nullptr, dz2);
+  RowGrad rg{};
+  rg.kind = 1; rg.idx_stride = 1;
+  rg.dh_in = d_edge_out; rg.dh_map = g.emap; rg.dh_scale = g.is_atom ? 0.5f : 1.f;
+  rg.tgt = g.tgt; rg.src = g.src; rg.emap = g.emap;
+  rg.logits = it.logits; rg.h = it.h; rg.agg_t = it.agg_t; rg.agg_s = it.agg_s; rg.stats = it.stats; rg.dagg_t = dagg_t;
+  rg.dagg_s = dagg_s; rg.dlogits = dlogits; rg.z2 = it.z2; rg.norm_core = p.edge.nc; rg.norm_gate = p.edge.ng;
+  if (!gated)
+    MB_OP(mb_seg_attn_bwd, g.n_rows, g.tgt, g.src, 1, g.emap, it.logits, it.h, it.agg_t, it.agg_s, it.stats, dagg_t, dagg_s,
+          d_edge_out, g.emap, rg.dh_scale, dh, dlogits, nullptr, nullptr, nullptr, nullptr);
   if (gated) {
-    edge_update_bwd(R, p.edge, g, it.z1, dz2, dlogits, g.is_atom ? &p.welt : &p.wstt, d_edge_out, p.we, d_edge, nullptr,
+    edge_update_bwd(R, p.edge, g, it.z1, rg, dz2, g.is_atom ? &p.welt : &p.wstt, d_edge_out, p.we, d_edge, nullptr,
                     nullptr, d_node, nullptr);
     return;
   }
@@ -643,20 +720,25 @@ static void attn_bwd(Run& R, const mb_attn_params& p, const mb_row_graph& g, con
 }
 
 // ------------------------------------------------------------------ refinement layer
+// Up to so many bonds (whatever the device: the memory plan depends on it) the envelopes of all layers come from one launch at the
+// start (84 MB for ten layers at the most), and their gradients go on into the radial basis's in the kernel that forms them: 40 launches
+// less.  More bonds fill the device with a launch of their own.
+constexpr int64_t FEW_BONDS = 8192;
+
 struct RefineInter { float *z1, *z2, *h, *env, *zn, *ze; };
 
 static void refine_fwd(Run& R, const mb_refine_params& p, const mb_row_graph& g, int64_t n_bonds, const float* node,
                        const float* edge, const float* rbf, const float* atom_feat, float* node_out, float* edge_out,
-                       bool want_edge, Internals mode, RefineInter& it) {
+                       bool want_edge, Internals mode, RefineInter& it, float* env = nullptr) {
   auto get = [&](size_t n) { return mode == KEEP ? R.ar.top(n) : R.ar.bottom(n); };
   const size_t rows = (size_t)g.n_rows, nodes = (size_t)g.n_nodes;
   it.z1 = mode == NONE ? nullptr : get(rows * update_width(p.edge));
   it.z2 = mode == NONE ? nullptr : get(rows * update_width(p.edge));
   it.h = get(rows * 128);
-  it.env = get((size_t)n_bonds * 128);
+  it.env = env ? env : get((size_t)n_bonds * 128);
   it.zn = mode == NONE ? nullptr : get(nodes * 128);
   it.ze = mode == NONE || !want_edge ? nullptr : get(rows * 128);
-  R.side(1, [&] { MB_OP(mb_small_linear_fwd, n_bonds, 7, rbf, p.wenv, it.env); });
+  if (!env) R.side(1, [&] { MB_OP(mb_small_linear_fwd, n_bonds, 7, rbf, p.wenv, it.env); });
   edge_update_fwd(R, p.edge, g, node, edge, g.is_atom ? nullptr : atom_feat, nullptr, nullptr, it.z1, it.z2, it.h, nullptr,
                   nullptr);
   Scope sc(R);
@@ -700,13 +782,23 @@ static void refine_bwd(Run& R, const mb_refine_params& p, const mb_row_graph& g,
   // node FFN
   float* dagg = R.ar.bottom(nodes * 128);
   auto node_ffn = [&] { ffn_bwd(R, p.nffn, g.n_nodes, d_node_out, nullptr, 1.f, it.zn, dagg); };
-  // edge FFN (atom graph: the mean over the two directions is a gather * 0.5)
+  // edge FFN
   float* dh = R.ar.bottom(rows * 128);
   const float* drow = nullptr;
   if (want_edge) {
     float* dx = p.smoothed_edge ? R.ar.bottom(rows * 128) : dh;
-    R.side(0, node_ffn);
-    ffn_bwd(R, p.effn, g.n_rows, d_edge_out, g.is_atom ? g.emap : nullptr, g.is_atom ? 0.5f : 1.f, it.ze, dx);
+    const int32_t* const idx = g.is_atom ? g.emap : nullptr;  // (atom graph: the mean over the two directions is a gather * 0.5)
+    const float scale = g.is_atom ? 0.5f : 1.f;
+    if (R.go() && nodes > 0 && rows > 0 && few_rows_fit((g.n_nodes + 31) / 32 * 32 + g.n_rows, 1)) {
+      const mb_mlp_bwd a = ffn_grad(p.nffn, g.n_nodes, d_node_out, nullptr, 1.f, it.zn, dagg);
+      const mb_mlp_bwd b = ffn_grad(p.effn, g.n_rows, d_edge_out, idx, scale, it.ze, dx);
+      const mb_mlp_bwd* const both[2] = {&a, &b};
+      R.op("mb_mlp_bwd_data", [&] { return few_ffn_bwd(both, R.st); }, 4.0 * (rows + nodes) * 128 * 128, 4.0 * (rows + nodes) * 128 * 3,
+           g.n_rows, 128, 128, 1);
+    } else {
+      R.side(0, node_ffn);
+      ffn_bwd(R, p.effn, g.n_rows, d_edge_out, idx, scale, it.ze, dx);
+    }
     if (p.smoothed_edge) {  // dx is the gradient of the smoothed rows h * s
       drow = dx;
       MB_OP(mb_mul_rows_gather, g.n_rows, dx, it.env, g.emap, dh);
@@ -720,18 +812,28 @@ static void refine_bwd(Run& R, const mb_refine_params& p, const mb_row_graph& g,
   float* dz2 = gated ? R.ar.bottom(rows * 256) : nullptr;
   float* denv = R.ar.bottom((size_t)n_bonds * 128);
   R.side(1, [&] {
+    if (R.go() && n_bonds <= FEW_BONDS) {
+      R.op("mb_seg_smooth_sum_bwd_env", [&] {
+        return smooth_env_bwd_rbf((int32_t)n_bonds, g, it.env, it.h, dagg, drow, p.wenv, d_rbf, R.st);
+      });
+      return;
+    }
     MB_OP(mb_seg_smooth_sum_bwd_env, (int32_t)n_bonds, g.tgt_ptr, g.is_atom ? nullptr : g.src_ptr, g.src_perm, g.tgt, g.src, 1,
           g.u2d, g.rev, it.env, it.h, dagg, drow, denv);
     MB_OP(mb_small_linear_bwd, n_bonds, 7, denv, p.wenv, d_rbf, 1);
   });
-  MB_OP(mb_seg_smooth_sum_bwd_rows, g.n_rows, g.tgt, src_idx, 1, g.emap, it.env, dagg, dh, want_edge ? 1 : 0,
-        gated ? it.z2 : nullptr, gated ? p.edge.nc : nullptr, gated ? p.edge.ng : nullptr, dz2);
   // edge update
   if (gated) {
-    edge_update_bwd(R, p.edge, g, it.z1, dz2, nullptr, nullptr, d_edge_out, p.we, d_edge, d_node_out, p.wn, d_node, d_atom);
+    RowGrad rg{};
+    rg.kind = 2; rg.idx_stride = 1;
+    rg.dh_in = want_edge ? dh : nullptr; rg.tgt = g.tgt; rg.src = src_idx; rg.emap = g.emap; rg.env = it.env; rg.dagg = dagg;
+    rg.z2 = it.z2; rg.norm_core = p.edge.nc; rg.norm_gate = p.edge.ng;
+    edge_update_bwd(R, p.edge, g, it.z1, rg, dz2, nullptr, d_edge_out, p.we, d_edge, d_node_out, p.wn, d_node, d_atom);
     R.join(1);
     return;
   }
+  MB_OP(mb_seg_smooth_sum_bwd_rows, g.n_rows, g.tgt, src_idx, 1, g.emap, it.env, dagg, dh, want_edge ? 1 : 0, nullptr, nullptr, nullptr,
+        nullptr);
   R.join(1);
   MB_OP(mb_scale_rows, g.n_nodes, d_node_out, p.wn, d_node, 0);
   const Dest to_tgt{d_node, g.tgt, MB_OUT_ATOMIC, nullptr, nullptr}, to_src{d_node, g.src, MB_OUT_ATOMIC, nullptr, nullptr};
@@ -845,6 +947,18 @@ static int evaluate(Run& R, mb_eval& E) {
       for (int i = 2; i < 5; ++i) r[i] = A.bottom(Eu * 128);
       if (line) for (int i = 5; i < 7; ++i) r[i] = A.bottom(T * 128);
     }
+  std::vector<float*> envs(2 * (size_t)L, nullptr);  // line, atom refinement of each layer
+  if (E.n_bonds <= FEW_BONDS && 2 * L <= MANY_LINEARS) {
+    ManyLinears many{};
+    int n = 0;
+    for (int i = 0; i < L; ++i)
+      for (int k = line ? 0 : 1; k < 2; ++k, ++n) {
+        many.y[n] = envs[2 * i + k] = A.bottom(Eu * 128);
+        many.x[n] = k == 0 ? rbf3 : rbf2;
+        many.w[n] = k == 0 ? M.layers[i].refine_line.wenv : M.layers[i].refine_atom.wenv;
+      }
+    R.op("mb_small_linear_fwd", [&] { return many_small_linears(E.n_bonds, n, many, R.st); });
+  }
   for (int i = 0; i < L; ++i) {
     const mb_layer_params& P = M.layers[i];
     const Internals mode = !grad ? NONE : (i >= first_kept ? KEEP : NONE);
@@ -881,13 +995,14 @@ static int evaluate(Run& R, mb_eval& E) {
     high_mark[i][2] = A.high.size();
     if (line) {
       Scope sc(R);
-      refine_fwd(R, P.refine_line, gl, E.n_bonds, e_at2, t_att, rbf3, n_att, e_ref, t_new, !last, mode, rl[i]);
+      refine_fwd(R, P.refine_line, gl, E.n_bonds, e_at2, t_att, rbf3, n_att, e_ref, t_new, !last, mode, rl[i], envs[2 * i]);
     }
     high_mark[i][3] = A.high.size();
     {
       Scope sc(R);
       // (without gradients e_new may share e_at2's buffer: the line refinement has read it by now)
-      refine_fwd(R, P.refine_atom, ga, E.n_bonds, n_att, e_ref, rbf2, nullptr, n_new, e_new, !last, mode, ra[i]);
+      refine_fwd(R, P.refine_atom, ga, E.n_bonds, n_att, e_ref, rbf2, nullptr, n_new, e_new, !last, mode, ra[i],
+                 envs[2 * i + 1]);
     }
     if (line) half[i].trip = e_att;
     node = n_new;
@@ -946,7 +1061,8 @@ static int evaluate(Run& R, mb_eval& E) {
     {
       Scope sc(R);
       if (!kept)
-        refine_fwd(R, P.refine_atom, ga, E.n_bonds, n_att, e_ref, rbf2, nullptr, nullptr, nullptr, !last, TEMP, ra[i]);
+        refine_fwd(R, P.refine_atom, ga, E.n_bonds, n_att, e_ref, rbf2, nullptr, nullptr, nullptr, !last, TEMP, ra[i],
+                   envs[2 * i + 1]);
       refine_bwd(R, P.refine_atom, ga, E.n_bonds, ra[i], dN[0], have_edge ? dE[0] : nullptr, dN[1], dE[1], d_rbf2, nullptr);
       pop(3);
     }
@@ -955,7 +1071,8 @@ static int evaluate(Run& R, mb_eval& E) {
       {
         Scope sc(R);
         if (!kept)
-          refine_fwd(R, P.refine_line, gl, E.n_bonds, e_at2, t_att, rbf3, n_att, nullptr, nullptr, !last, TEMP, rl[i]);
+          refine_fwd(R, P.refine_line, gl, E.n_bonds, e_at2, t_att, rbf3, n_att, nullptr, nullptr, !last, TEMP, rl[i],
+                     envs[2 * i]);
         refine_bwd(R, P.refine_line, gl, E.n_bonds, rl[i], dE[1], have_edge ? dT[0] : nullptr, dE[0], dT[1], d_rbf3, dN[1]);
         pop(2);
       }

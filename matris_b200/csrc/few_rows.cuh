@@ -22,29 +22,55 @@
 //
 // Warps 0 - 15: rows in, epilogues; 16: matrix instructions; 17: weights.
 
+// A small evaluation is also bound by its launches, 2.5 us of the host's time each and 3 - 4 of the chain, so a launch takes on more:
+// ROW_BWD is the backward pass from a row's own gradient on (RowBwd, common.cuh), a warp forming the row's dz2 (and the logits'
+// gradients) in registers as the row kernels do; LINEAR takes the column blocks of independent problems, and sums of a bond's two
+// directed rows as operand; PLAIN_BWD two problems.  550 -> 430 launches an evaluation: 4 atoms 3.37 -> 2.91 ms, 32 atoms through the
+// calculator 5.02 -> 4.84.
+
 enum FewMode { FEW_GATED_FWD = MLP_GATED_FWD, FEW_PLAIN_FWD = MLP_PLAIN_FWD, FEW_GATED_BWD = MLP_GATED_BWD,
-               FEW_PLAIN_BWD = MLP_PLAIN_BWD, FEW_LINEAR = 4 };
+               FEW_PLAIN_BWD = MLP_PLAIN_BWD, FEW_LINEAR = 4, FEW_ROW_BWD = 5 };
+constexpr int FW_MAX_BLOCKS = 8;
+struct FewLinear { mb_colblock blk[FW_MAX_BLOCKS]; int64_t n_rows[FW_MAX_BLOCKS]; const int32_t* pair; };  // independent problems' column blocks
+struct FewPlainBwd { MlpArgs of[2]; };                                                                     // two independent problems
+struct FewRowBwd : MlpArgs { RowGrad g; float* out[3]; float* zero; int64_t n_zero; };
 template <int MODE> struct FewArgs { typedef MlpArgs T; };
-template <> struct FewArgs<FEW_LINEAR> { typedef mb_gemm_desc T; };
-struct alignas(64) FewMaps { CUtensorMap w[4][2]; };  // hi, lo; MLPs: layer 1, layer 2, E's weights; LINEAR: column blocks
+template <> struct FewArgs<FEW_LINEAR> { typedef FewLinear T; };
+template <> struct FewArgs<FEW_PLAIN_BWD> { typedef FewPlainBwd T; };
+template <> struct FewArgs<FEW_ROW_BWD> { typedef FewRowBwd T; };
+// hi, lo; MLPs: layer 1, layer 2, E's weights (PLAIN_BWD: two of each problem); LINEAR: column blocks
+struct alignas(64) FewMaps { CUtensorMap w[FW_MAX_BLOCKS][2]; };
 
 constexpr int FW_WORKERS = 16, FW_MMA_WARP = 16, FW_TMA_WARP = 17, FW_THREADS = 576;
 constexpr uint32_t FW_SMEM_LIMIT = 227 * 1024;
 constexpr uint32_t FW_SLOT_BYTES = 2 * TC_TILE_BYTES, FW_MAX_SLOTS = 6;
-constexpr uint32_t FW_GROUP = 2048;  // bytes of 8 rows x 128 K of an operand part: 16-byte cores of 8 rows x 8 K or 8 K x 8 rows
+// Operands are 128-byte cores (8 rows x 8 K, or 8 K x 8 rows) in the order of K; bytes of 8 rows x 128 K of an operand part:
+constexpr uint32_t FW_GROUP = 2048;
+constexpr uint32_t FW_ROW_CORE = 144, FW_ROW_GROUP = 16 * FW_ROW_CORE;  // ROW_BWD, whose warps write along K: 16 bytes between cores
 
 // shared memory: weight ring | X segments | hidden layer | sums of squares | barriers
 __host__ __device__ constexpr uint32_t few_operand_bytes(int r) { return (uint32_t)r * 512u; }  // hi and lo of R rows x 128 K
-__host__ __device__ constexpr int few_branches(int mode) { return mode == FEW_GATED_FWD || mode == FEW_GATED_BWD ? 2 : mode == FEW_LINEAR ? 0 : 1; }
+__host__ __device__ constexpr uint32_t few_x_bytes(int mode, int r) { return (uint32_t)(r / 4) * (mode == FEW_ROW_BWD ? FW_ROW_GROUP : FW_GROUP); }
+__host__ __device__ constexpr int few_branches(int mode) {
+  return mode == FEW_GATED_FWD || mode == FEW_GATED_BWD || mode == FEW_ROW_BWD ? 2 : mode == FEW_LINEAR ? 0 : 1;
+}
 __host__ __device__ constexpr uint32_t few_tail_bytes(int r) { return (uint32_t)r * 32u + 256u; }
 __host__ __device__ constexpr uint32_t few_columns(int mode, int r) {
-  const uint32_t need = (uint32_t)r * (mode == FEW_GATED_FWD ? 4 : mode == FEW_GATED_BWD ? 3 : mode == FEW_LINEAR ? 1 : 2);
+  const uint32_t need = (uint32_t)r * (mode == FEW_GATED_FWD ? 4 : mode == FEW_GATED_BWD || mode == FEW_ROW_BWD ? 3 : mode == FEW_LINEAR ? 1 : 2);
   return need <= 32 ? 32 : need <= 64 ? 64 : 128;
 }
 
-// no swizzle: LBO 128 bytes between cores along K, SBO 2048 between groups of 8 rows (both majors, see FW_GROUP)
-__device__ __forceinline__ uint64_t few_desc(uint32_t saddr) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (uint64_t)(128u >> 4) << 16 | (uint64_t)(FW_GROUP >> 4) << 32 | 1ull << 46;
+// no swizzle: LBO = bytes between cores along K, SBO = between groups of 8 rows (both majors)
+__device__ __forceinline__ uint64_t few_desc(uint32_t saddr, uint32_t core = 128, uint32_t group = FW_GROUP) {
+  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (uint64_t)(core >> 4) << 16 | (uint64_t)(group >> 4) << 32 | 1ull << 46;
+}
+// four consecutive K values of a row (c8: their core, second half of it or not) into an operand's hi and lo part
+__device__ __forceinline__ void few_put4(uint32_t at, uint32_t lo_off, const float4& v) {
+  const float x[4] = {v.x, v.y, v.z, v.w};
+  uint32_t hi[2], lo[2];
+  split_bf16(x, hi, lo);
+  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(at), "r"(hi[0]), "r"(hi[1]) : "memory");
+  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(at + lo_off), "r"(lo[0]), "r"(lo[1]) : "memory");
 }
 __device__ __forceinline__ void umma_bf16_ss(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -91,13 +117,20 @@ template <int V> __device__ __forceinline__ float few_sums_of_squares(float (&v)
 
 template <int MODE, int R>
 __global__ void __launch_bounds__(FW_THREADS, MODE == FEW_LINEAR ? 2 : 1)
-k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant__ FewMaps maps, const int n_slots, const int early) {
-  constexpr bool LINEAR = MODE == FEW_LINEAR, GATED = MODE == FEW_GATED_FWD || MODE == FEW_GATED_BWD;
-  constexpr bool FWD = MODE == FEW_GATED_FWD || MODE == FEW_PLAIN_FWD, BWD = MODE == FEW_GATED_BWD || MODE == FEW_PLAIN_BWD;
+k_few(const __grid_constant__ typename FewArgs<MODE>::T args, const __grid_constant__ FewMaps maps, const int n_slots, const int early) {
+  constexpr bool LINEAR = MODE == FEW_LINEAR, ROW_BWD = MODE == FEW_ROW_BWD;
+  constexpr bool GATED_BWD = MODE == FEW_GATED_BWD || ROW_BWD, GATED = MODE == FEW_GATED_FWD || GATED_BWD;
+  constexpr bool FWD = MODE == FEW_GATED_FWD || MODE == FEW_PLAIN_FWD;
   constexpr int NB = GATED ? 2 : 1, RT = R / 4, JOBS = R / 2;  // rows of a thread; (8 rows x 32 values) pieces of a segment
-  constexpr uint32_t OPERAND = few_operand_bytes(R), LO = (R / 8) * FW_GROUP;
+  constexpr uint32_t OPERAND = few_operand_bytes(R), LO = (R / 8) * FW_GROUP;  // of the hidden layer
+  constexpr uint32_t X_CORE = ROW_BWD ? FW_ROW_CORE : 128, X_GROUP = ROW_BWD ? FW_ROW_GROUP : FW_GROUP;
+  constexpr uint32_t X_OPERAND = few_x_bytes(MODE, R), X_LO = X_OPERAND / 2;
   constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)R >> 3) << 17 | ((128u >> 4) << 24), MN_MAJOR_B = 1u << 16;
   constexpr uint32_t COLUMNS = few_columns(MODE, R);
+  const auto& d = [&]() -> const auto& {
+    if constexpr (MODE == FEW_PLAIN_BWD) return args.of[blockIdx.y];
+    else return args;
+  }();
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sm0 = smem_u32(smem);
   if ((sm0 & 1023u) != 0) {
@@ -105,22 +138,29 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant
     return;
   }
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int64_t row0 = (int64_t)blockIdx.x * R, n_rows = d.n_rows;
+  int64_t n_rows;
+  if constexpr (LINEAR) n_rows = d.n_rows[blockIdx.y];
+  else n_rows = d.n_rows;
+  const int64_t row0 = (int64_t)blockIdx.x * R;
+  if (row0 >= n_rows) return;  // (another problem of the launch has more rows)
   int n_src, n_ext = 0;  // segments of layer 1 (GATED_BWD: core and gate half of dz2); of E
   if constexpr (LINEAR) n_src = d.blk[blockIdx.y].n_src;
   else n_src = d.n_src;
-  if constexpr (MODE == FEW_GATED_BWD) n_ext = d.n_ext;
+  if constexpr (GATED_BWD) n_ext = d.n_ext;
+  bool two_layers = !LINEAR;
+  if constexpr (ROW_BWD) two_layers = d.out[0] != nullptr;
   const int n_seg = n_src + n_ext;
 
-  const uint32_t x_sm = sm0 + n_slots * FW_SLOT_BYTES, act_sm = x_sm + n_seg * OPERAND, ss_off = act_sm + few_branches(MODE) * OPERAND - sm0;
+  const uint32_t x_sm = sm0 + n_slots * FW_SLOT_BYTES, act_sm = x_sm + n_seg * X_OPERAND, ss_off = act_sm + few_branches(MODE) * OPERAND - sm0;
   float* const sums = reinterpret_cast<float*>(smem + ss_off);  // [row quarter][value][lane quarter]
   const uint32_t bar0 = sm0 + ss_off + R * 32;
-  // w_full[6] w_empty[6] | x_ready[6] (per segment) | act_ready[2] d1_full[2] | d2_full[2] | retired | tensor-memory address
-  const uint32_t w_full = bar0, w_empty = bar0 + 48, x_ready = bar0 + 96, act_ready = bar0 + 144, d1_full = bar0 + 160,
-                 d2_full = bar0 + 176, retired = bar0 + 192, slot_at = bar0 + 200;
+  // w_full[6] w_empty[6] | x_ready[4] (per segment) | act_ready[2] d1_full[2] d2_full[2] | retired | tensor-memory address
+  const uint32_t w_full = bar0, w_empty = bar0 + 48, x_ready = bar0 + 96, act_ready = bar0 + 128, d1_full = bar0 + 144,
+                 d2_full = bar0 + 160, retired = bar0 + 176, slot_at = bar0 + 184;
   if (warp == FW_MMA_WARP) {
     if (lane == 0) {
-      for (uint32_t b = 0; b < FW_MAX_SLOTS; ++b) { mbar_init(w_full + 8 * b, 1); mbar_init(w_empty + 8 * b, 1); mbar_init(x_ready + 8 * b, JOBS); }
+      for (uint32_t b = 0; b < FW_MAX_SLOTS; ++b) { mbar_init(w_full + 8 * b, 1); mbar_init(w_empty + 8 * b, 1); }
+      for (int b = 0; b < 4; ++b) mbar_init(x_ready + 8 * b, ROW_BWD ? FW_WORKERS : JOBS);
       for (int b = 0; b < 2; ++b) { mbar_init(act_ready + 8 * b, FW_WORKERS); mbar_init(d1_full + 8 * b, 1); mbar_init(d2_full + 8 * b, 1); }
       mbar_init(retired, 1);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -140,9 +180,9 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant
   auto walk = [&](auto step) {
     int n = 0;
     for (int br = 0; br < NB; ++br)
-      for (int kp = 0; kp < (MODE == FEW_GATED_BWD ? 2 : 2 * n_src); ++kp) step(n++, 0, br, kp);
+      for (int kp = 0; kp < (GATED_BWD ? 2 : 2 * n_src); ++kp) step(n++, 0, br, kp);
     for (int kp = 0; kp < 2 * n_ext; ++kp) step(n++, 2, 0, kp);
-    if constexpr (!LINEAR)
+    if (two_layers)
       for (int br = 0; br < NB; ++br)
         for (int kp = 0; kp < 2; ++kp) step(n++, 1, br, kp);
   };
@@ -153,22 +193,22 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant
     uint32_t elected;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
     const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0), sm_u = __shfl_sync(0xffffffffu, sm0, 0);
-    const uint32_t x_u = sm_u + n_slots * FW_SLOT_BYTES, act_u = x_u + n_seg * OPERAND;
+    const uint32_t x_u = sm_u + n_slots * FW_SLOT_BYTES, act_u = x_u + n_seg * X_OPERAND;
     const uint64_t w_first = umma_desc(sm_u);
     bool alive = true;
     uint32_t slot = 0, phase = 0;  // of the next piece
     auto wait = [&](uint32_t bar, uint32_t parity) { if (alive) alive = mbar_wait(bar, parity); };
-    // one piece; xh: descriptor of the rows' hi part
-    auto piece = [&](uint32_t dt, uint64_t xh, uint32_t idesc, bool fresh) {
+    // one piece: rows' descriptors (hi; lo is `lo` further on), step of 16 K values
+    auto piece = [&](uint32_t dt, uint64_t xh, uint32_t lo, uint32_t adv, uint32_t idesc, bool fresh) {
       wait(w_full + 8 * slot, phase);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (elected) {
-        const uint64_t wh = w_first + slot * (FW_SLOT_BYTES >> 4), wl = wh + (TC_TILE_BYTES >> 4), xl = xh + (LO >> 4);
+        const uint64_t wh = w_first + slot * (FW_SLOT_BYTES >> 4), wl = wh + (TC_TILE_BYTES >> 4), xl = xh + (lo >> 4);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {  // K steps of 16: 32 bytes of the weight rows, two cores of the rows
-          umma_bf16_ss(dt, wh + 2 * kk, xl + 16 * kk, idesc, (!fresh || kk > 0) ? 1u : 0u);
-          umma_bf16_ss(dt, wl + 2 * kk, xh + 16 * kk, idesc, 1u);
-          umma_bf16_ss(dt, wh + 2 * kk, xh + 16 * kk, idesc, 1u);
+          umma_bf16_ss(dt, wh + 2 * kk, xl + adv * kk, idesc, (!fresh || kk > 0) ? 1u : 0u);
+          umma_bf16_ss(dt, wl + 2 * kk, xh + adv * kk, idesc, 1u);
+          umma_bf16_ss(dt, wh + 2 * kk, xh + adv * kk, idesc, 1u);
         }
         mma_commit(w_empty + 8 * slot);
       }
@@ -177,9 +217,9 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant
     };
     auto segment = [&](int seg, uint32_t dt, bool fresh) {  // both pieces of an X segment
       wait(x_ready + 8 * seg, 0);
-      const uint64_t xh = few_desc(x_u + seg * OPERAND);
+      const uint64_t xh = few_desc(x_u + seg * X_OPERAND, X_CORE, X_GROUP);
 #pragma unroll 1
-      for (int kp = 0; kp < 2; ++kp) piece(dt, xh + kp * (1024 / 16), IDESC, fresh && kp == 0);
+      for (int kp = 0; kp < 2; ++kp) piece(dt, xh + kp * (8 * X_CORE / 16), X_LO, 2 * X_CORE / 16, IDESC, fresh && kp == 0);
     };
     auto full = [&](uint32_t bar) {
       if (elected) mma_commit(bar);
@@ -188,12 +228,12 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant
 #pragma unroll 1
     for (int br = 0; br < NB; ++br) {
 #pragma unroll 1
-      for (int s = 0; s < (MODE == FEW_GATED_BWD ? 1 : n_src); ++s) segment(MODE == FEW_GATED_BWD ? br : s, tmem_u + R * br, s == 0);
+      for (int s = 0; s < (GATED_BWD ? 1 : n_src); ++s) segment(GATED_BWD ? br : s, tmem_u + R * br, s == 0);
       if (n_src > 0) full(LINEAR ? d2_full : d1_full + 8 * br);
     }
 #pragma unroll 1
     for (int s = 0; s < n_ext; ++s) segment(n_src + s, tmem_u + 2 * R, s == 0);
-    if (!LINEAR) {
+    if (two_layers) {
 #pragma unroll 1
       for (int br = 0; br < NB; ++br) {
         wait(act_ready + 8 * br, 0);
@@ -201,8 +241,8 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant
         const uint64_t ah = few_desc(act_u + br * OPERAND);
 #pragma unroll 1
         for (int kp = 0; kp < 2; ++kp)
-          piece(dt, ah + kp * (1024 / 16), IDESC | MN_MAJOR_B, kp == 0 && !(MODE == FEW_GATED_BWD && (br == 1 || n_ext > 0)));
-        if (MODE != FEW_GATED_BWD || br == 1) full(d2_full + (MODE == FEW_GATED_FWD ? 8 * br : 0));
+          piece(dt, ah + kp * (1024 / 16), LO, 16, IDESC | MN_MAJOR_B, kp == 0 && !(GATED_BWD && (br == 1 || n_ext > 0)));
+        if (!GATED_BWD || br == 1) full(d2_full + (MODE == FEW_GATED_FWD ? 8 * br : 0));
       }
     }
     drain_mma(retired, elected);
@@ -218,11 +258,11 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant
       if (n >= n_slots && alive) alive = mbar_wait(w_empty + 8 * slot, (uint32_t)(n / n_slots - 1) & 1);
       alive = __all_sync(0xffffffffu, alive);
       if (!alive) return;
-      // the rows of a branch's weights, but W1t of GATED_BWD has its branches side by side
-      const bool beside = MODE == FEW_GATED_BWD && layer == 1;
-      const int x = 64 * kp + (beside ? 128 * br : 0), y = beside ? 0 : 128 * br;
+      // the rows of a branch's weights, but W1t of the gated backward has its branches side by side (and 128 rows for every output)
+      const bool beside = GATED_BWD && layer == 1;
+      const int x = 64 * kp + (beside ? 128 * br : 0), y = beside ? 128 * (int)blockIdx.y : 128 * br;
       if (elected) {
-        const CUtensorMap* const m = maps.w[LINEAR ? (int)blockIdx.y : layer];
+        const CUtensorMap* const m = maps.w[LINEAR ? (int)blockIdx.y : MODE == FEW_PLAIN_BWD ? 2 * (int)blockIdx.y + layer : layer];
         const uint32_t bar = w_full + 8 * slot, dst = sm_u + slot * FW_SLOT_BYTES;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(FW_SLOT_BYTES) : "memory");
         tma_load_2d(dst, m, bar, x, y);
@@ -250,6 +290,59 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant
         if (i < n_own && alive) p[(row0 + r0 + i) * ld] = v[i];
     };
     pdl_sync();
+    float side[NB][RT], res[RT];  // what the epilogues add or multiply with
+    bool has_res = false;
+    if constexpr (!LINEAR) has_res = ROW_BWD ? d.res != nullptr && blockIdx.y == 0 : d.out2 != nullptr;
+    auto ask_side = [&]() {
+      if constexpr (!LINEAR && !FWD) {
+#pragma unroll
+        for (int br = 0; br < NB; ++br)
+#pragma unroll
+          for (int i = 0; i < RT; ++i) side[br][i] = d.side[row_of(i) * d.ld_side + 128 * br + f];
+      }
+      if constexpr (!LINEAR) {
+        if (has_res) {
+#pragma unroll
+          for (int i = 0; i < RT; ++i) res[i] = d.res[row_of(i) * d.ld_res + f];
+        }
+      }
+    };
+    if constexpr (ROW_BWD) {
+      // -------------------------------------------- X: a row per warp and turn, lane = 4 channels
+      ask_side();
+#pragma unroll
+      for (int n0 = 0; n0 < R; n0 += FW_WORKERS) {
+        const int n = n0 + warp, c = 4 * lane;
+        const bool mine = row0 + n < n_rows;
+        const int64_t row = mine ? row0 + n : n_rows - 1;
+        const uint32_t at = x_sm + (n >> 3) * FW_ROW_GROUP + (lane >> 1) * FW_ROW_CORE + (n & 7) * 16u + (lane & 1) * 8u;
+        float4 o, ds, dt;
+        if (d.g.kind == 1) {
+          attn_bwd_row(d.g, row, c, o, ds, dt);
+          if (n_ext > 0) {
+            few_put4(at + 2 * X_OPERAND, X_LO, ds);
+            few_put4(at + 3 * X_OPERAND, X_LO, dt);
+          }
+          if (d.g.dlogits && mine) {
+            st4(d.g.dlogits + row * 256 + c, ds);
+            st4(d.g.dlogits + row * 256 + 128 + c, dt);
+          }
+        } else if (d.g.kind == 2) {
+          o = smooth_bwd_row(d.g, row, c);
+        } else {
+          o = ld4(d.g.dh_in + row * 128 + c);
+        }
+        gate_bwd_row(d.g.z2 + row * 256, c, d.g.norm_core, d.g.norm_gate, o, ds, dt);
+        few_put4(at, X_LO, ds);
+        few_put4(at + X_OPERAND, X_LO, dt);
+      }
+      to_async_proxy();
+      __syncwarp();
+      if (lane < n_seg) mbar_arrive(x_ready + 8 * lane);
+      if (blockIdx.y == 0)
+        for (int64_t i = 4 * ((int64_t)blockIdx.x * (32 * FW_WORKERS) + tid); i < d.n_zero; i += 4 * (int64_t)gridDim.x * (32 * FW_WORKERS))
+          st4(d.zero + i, make_float4(0.f, 0.f, 0.f, 0.f));
+    } else
     // ---------------------------------------------- X: 8 rows x 32 values per warp and turn, lane = (row, 8 values)
     for (int j = warp; j < n_seg * JOBS; j += FW_WORKERS) {
       const int seg = j / JOBS, piece = j % JOBS, n = 8 * (piece >> 2) + (lane & 7), c8 = 4 * (piece & 3) + (lane >> 3);
@@ -259,7 +352,14 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant
       int64_t r = row0 + n < n_rows ? row0 + n : n_rows - 1;
       if (sr->idx) r = sr->idx[r];
       const float* const p = sr->ptr + r * sr->ld + sr->col + 8 * c8;
-      const float4 u = ld4(p), v = ld4(p + 4);
+      float4 u = ld4(p), v = ld4(p + 4);
+      if constexpr (LINEAR) {
+        if (d.pair) {
+          const float* const p2 = sr->ptr + (int64_t)d.pair[r] * sr->ld + sr->col + 8 * c8;
+          u = add4(u, ld4(p2));
+          v = add4(v, ld4(p2 + 4));
+        }
+      }
       float x[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
       if (sr->act) {
 #pragma unroll
@@ -306,8 +406,6 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant
       }
     } else {
       // -------------------------------------------- what the epilogues add, on its way while the first products are formed
-      float side[NB][RT], res[RT];
-      const bool has_res = d.out2 != nullptr;
       if constexpr (FWD) {
 #pragma unroll
         for (int br = 0; br < NB; ++br) {
@@ -331,16 +429,8 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant
 #pragma unroll
               for (int i = 0; i < RT; ++i) side[br][i] += v[br][i];
           }
-      } else {
-#pragma unroll
-        for (int br = 0; br < NB; ++br)
-#pragma unroll
-          for (int i = 0; i < RT; ++i) side[br][i] = d.side[row_of(i) * d.ld_side + 128 * br + f];
       }
-      if (has_res) {
-#pragma unroll
-        for (int i = 0; i < RT; ++i) res[i] = d.res[row_of(i) * d.ld_res + f];
-      }
+      if constexpr (!ROW_BWD) ask_side();
       // -------------------------------------------- layer 1 out, hidden layer back as the operand of layer 2
 #pragma unroll
       for (int br = 0; br < NB; ++br) {
@@ -363,6 +453,10 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant
             a[i] = x[i];
           }
         }
+        if (!two_layers) {
+          store(d.z1 + 128 * br + f, d.ld_z1, x);
+          continue;
+        }
         uint32_t hi[RT / 2], lo[RT / 2];
         split_bf16(a, hi, lo);
         const uint32_t at = act_sm + br * OPERAND + (r0 >> 3) * FW_GROUP + f * 16u + (r0 & 7) * 2u;
@@ -381,46 +475,51 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T d, const __grid_constant
       }
       // -------------------------------------------- layer 2 out
       float y[RT];
-      if constexpr (MODE == FEW_GATED_FWD) {
-        float z[2][RT], v[2 * RT];
+      if (two_layers) {
+        if constexpr (MODE == FEW_GATED_FWD) {
+          float z[2][RT], v[2 * RT];
 #pragma unroll
-        for (int br = 0; br < 2; ++br) {
-          const float b = d.b2 ? d.b2[128 * br + f] : 0.f;
-          wait(d2_full + 8 * br);
-          few_result(lane_q + (uint32_t)R * (2 + br), z[br]);
+          for (int br = 0; br < 2; ++br) {
+            const float b = d.b2 ? d.b2[128 * br + f] : 0.f;
+            wait(d2_full + 8 * br);
+            few_result(lane_q + (uint32_t)R * (2 + br), z[br]);
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
+              z[br][i] += b;
+              v[RT * br + i] = z[br][i];
+            }
+            if (d.z2) store(d.z2 + 128 * br + f, d.ld_z2, z[br]);
+          }
+          constexpr int PER = 32 / (2 * RT);  // lanes that end with the same sum
+          const float s = few_sums_of_squares(v, lane);
+          if (lane % PER == 0) sums[(rg * 2 * RT + lane / PER) * 4 + q] = s;
+          asm volatile("bar.sync %0, 128;" :: "r"(1 + rg) : "memory");  // the four lane quarters of these rows
+          const float nc = d.norm_core[f], ng = d.norm_gate[f];
 #pragma unroll
           for (int i = 0; i < RT; ++i) {
-            z[br][i] += b;
-            v[RT * br + i] = z[br][i];
+            const float4 c = *reinterpret_cast<const float4*>(sums + (rg * 2 * RT + i) * 4);
+            const float4 g = *reinterpret_cast<const float4*>(sums + (rg * 2 * RT + RT + i) * 4);
+            const float rc = rsqrtf(((c.x + c.y) + (c.z + c.w)) * (1.0f / 128.0f) + ML_RMS_EPS);
+            const float rr = rsqrtf(((g.x + g.y) + (g.z + g.w)) * (1.0f / 128.0f) + ML_RMS_EPS);
+            y[i] = gated_value(z[0][i] * (rc * nc), z[1][i] * (rr * ng));
           }
-          if (d.z2) store(d.z2 + 128 * br + f, d.ld_z2, z[br]);
+        } else {
+          const float b = FWD && d.b2 ? d.b2[f] : 0.f;
+          wait(d2_full);
+          few_result(lane_q + (uint32_t)R * NB, y);
+#pragma unroll
+          for (int i = 0; i < RT; ++i) y[i] += b;
         }
-        constexpr int PER = 32 / (2 * RT);  // lanes that end with the same sum
-        const float s = few_sums_of_squares(v, lane);
-        if (lane % PER == 0) sums[(rg * 2 * RT + lane / PER) * 4 + q] = s;
-        asm volatile("bar.sync %0, 128;" :: "r"(1 + rg) : "memory");  // the four lane quarters of these rows
-        const float nc = d.norm_core[f], ng = d.norm_gate[f];
-#pragma unroll
-        for (int i = 0; i < RT; ++i) {
-          const float4 c = *reinterpret_cast<const float4*>(sums + (rg * 2 * RT + i) * 4);
-          const float4 g = *reinterpret_cast<const float4*>(sums + (rg * 2 * RT + RT + i) * 4);
-          const float rc = rsqrtf(((c.x + c.y) + (c.z + c.w)) * (1.0f / 128.0f) + ML_RMS_EPS);
-          const float rr = rsqrtf(((g.x + g.y) + (g.z + g.w)) * (1.0f / 128.0f) + ML_RMS_EPS);
-          y[i] = gated_value(z[0][i] * (rc * nc), z[1][i] * (rr * ng));
+        if constexpr (!ROW_BWD) {
+          if (d.h) store(d.h + f, d.ld_h, y);
         }
-      } else {
-        const float b = FWD && d.b2 ? d.b2[f] : 0.f;
-        wait(d2_full);
-        few_result(lane_q + (uint32_t)R * NB, y);
+        if (has_res) {
+          const float rw = d.res_w ? d.res_w[f] : 1.f;
 #pragma unroll
-        for (int i = 0; i < RT; ++i) y[i] += b;
-      }
-      if (d.h) store(d.h + f, d.ld_h, y);
-      if (has_res) {
-        const float rw = d.res_w ? d.res_w[f] : 1.f;
-#pragma unroll
-        for (int i = 0; i < RT; ++i) y[i] = fmaf(rw, res[i], y[i]);
-        store(d.out2 + f, d.ld_out2, y);
+          for (int i = 0; i < RT; ++i) y[i] = fmaf(rw, res[i], y[i]);
+          if constexpr (!ROW_BWD) store(d.out2 + f, d.ld_out2, y);
+        }
+        if constexpr (ROW_BWD) store(d.out[blockIdx.y] + f, 128, y);
       }
     }
   }

@@ -9,13 +9,11 @@
 // (the whole weight set of a layer is ~1 MB and stays L2 resident).  Register
 // tile 8x8 per thread, K staged through shared memory in chunks of 16 with a
 // register-prefetched double buffer.
-#include "common.cuh"
+#include "row_math.cuh"
 
 namespace mb {
 
 constexpr int BM = 128, BN = 128, BK = 16, GEMM_THREADS = 256, LDS = BM + 4;
-
-__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
 __global__ void __launch_bounds__(GEMM_THREADS, 2) k_gemm(const __grid_constant__ mb_gemm_desc d) {
   const mb_colblock& cb = d.blk[blockIdx.y];
@@ -688,6 +686,7 @@ static int few_config() {
   if (!rc) rc = few_config_mode<FEW_PLAIN_FWD>();
   if (!rc) rc = few_config_mode<FEW_GATED_BWD>();
   if (!rc) rc = few_config_mode<FEW_PLAIN_BWD>();
+  if (!rc) rc = few_config_mode<FEW_ROW_BWD>();
   return rc;
 }
 // R of k_few for a launch, 0: the persistent kernels.  A block of k_few takes one tile, so the line lies where its tiles no longer run
@@ -701,13 +700,13 @@ static int few_choice(int mode, int64_t n_rows, int n_src, int n_blocks, int n_s
   return t32 <= (mode == FEW_LINEAR && n_src == 1 ? 2 : 1) * (int64_t)n_sm ? 32 : 0;
 }
 // n_seg: A segments of a block, n_kp: weight slots it uses
-template <int MODE> static void few_launch(const typename FewArgs<MODE>::T& args, const FewMaps& maps, int r, int n_seg, int n_kp,
-                                           int n_blocks, cudaStream_t st) {
-  const uint32_t rest = (n_seg + few_branches(MODE)) * few_operand_bytes(r) + few_tail_bytes(r);
+template <int MODE> static void few_launch(const typename FewArgs<MODE>::T& args, const FewMaps& maps, int64_t n_rows, int r, int n_seg,
+                                           int n_kp, int n_blocks, cudaStream_t st) {
+  const uint32_t rest = n_seg * few_x_bytes(MODE, r) + few_branches(MODE) * few_operand_bytes(r) + few_tail_bytes(r);
   uint32_t slots = (FW_SMEM_LIMIT - rest) / FW_SLOT_BYTES;
   if (slots > FW_MAX_SLOTS) slots = FW_MAX_SLOTS;
   if (slots > (uint32_t)n_kp) slots = (uint32_t)n_kp;
-  const dim3 grid((unsigned)((args.n_rows + r - 1) / r), (unsigned)n_blocks);
+  const dim3 grid((unsigned)((n_rows + r - 1) / r), (unsigned)n_blocks);
   const size_t smem = slots * FW_SLOT_BYTES + rest;
   const int early = weights_settled ? 1 : 0;
   if (r == 16) launch(k_few<MODE, 16>, grid, FW_THREADS, smem, st, args, maps, (int)slots, early);
@@ -738,6 +737,92 @@ static int device_config(int* n_sm) {
     c.ready = true;
   }
   *n_sm = c.n_sm;
+  return MB_OK;
+}
+
+bool few_rows_fit(int64_t n_rows, int n_out) {
+  int n_sm = 0;
+  return g_gemm_mode == 0 && sm_count(&n_sm) == MB_OK && (n_rows + 31) / 32 * n_out <= n_sm;
+}
+static int split_map(const mb_weight& w, int k, int rows, CUtensorMap* maps) {
+  if (!w.W_hi16 || !w.W_lo16 || !aligned16(w.W_hi16) || !aligned16(w.W_lo16) || (w.ldw & 7)) return MB_ERR_INVALID;
+  const int rc = weight_map(w.W_hi16, w.ldw, k, maps, rows, true);
+  return rc ? rc : weight_map(w.W_lo16, w.ldw, k, maps + 1, rows, true);
+}
+int few_row_bwd(const RowBwd& a, cudaStream_t st) {
+  int n_sm = 0, rc = device_config(&n_sm);
+  if (rc) return rc;
+  const bool logits = a.w3t.W != nullptr;
+  FewMaps maps;
+  if ((rc = split_map(a.w2t, 128, 256, maps.w[0]))) return rc;
+  if (a.n_out > 0 && (rc = split_map(a.w1t, 256, 128 * a.n_out, maps.w[1]))) return rc;
+  if (logits && (rc = split_map(a.w3t, 256, 128, maps.w[2]))) return rc;
+  FewRowBwd k = {};
+  k.n_rows = a.n_rows;
+  k.n_src = 2; k.n_ext = logits ? 2 : 0;
+  k.side = a.z1; k.ld_side = 256;
+  k.z1 = a.dz1; k.ld_z1 = 256;
+  k.res = a.res; k.res_w = a.res_w; k.ld_res = 128;
+  k.g = a.g;
+  for (int j = 0; j < 3; ++j) k.out[j] = j < a.n_out ? a.out[j] : nullptr;
+  k.zero = a.zero; k.n_zero = a.n_zero;
+  const int blocks = a.n_out > 1 ? a.n_out : 1, r = (a.n_rows + 15) / 16 * blocks <= n_sm ? 16 : 32;
+  few_launch<FEW_ROW_BWD>(k, maps, k.n_rows, r, 2 + k.n_ext, 4 + 2 * k.n_ext + (a.n_out > 0 ? 4 : 0), blocks, st);
+  MB_LAUNCH_CHECK("k_few");
+  return MB_OK;
+}
+// Blocks of 32 rows that run side by side: two on a multiprocessor where only dense layers with K = 128 are among them.
+bool few_linears_fit(const mb_gemm_desc* const* g, int n) {
+  int n_sm = 0, per_sm = 2, blocks = 0;
+  if (g_gemm_mode != 0 || sm_count(&n_sm) != MB_OK) return false;
+  int64_t tiles = 0;
+  for (int i = 0; i < n; ++i)
+    for (int j = 0; j < g[i]->n_blocks; ++j, ++blocks) {
+      tiles += (g[i]->n_rows + 31) / 32;
+      if (g[i]->blk[j].n_src > 1) per_sm = 1;
+    }
+  return blocks <= FW_MAX_BLOCKS && tiles <= per_sm * (int64_t)n_sm;
+}
+int few_linears(const mb_gemm_desc* const* g, int n, const int32_t* pair, cudaStream_t st) {
+  int n_sm = 0, rc = device_config(&n_sm);
+  if (rc) return rc;
+  FewMaps maps;
+  FewLinear f;
+  f.pair = pair;
+  int n_src = 1, k = 0;
+  int64_t most = 0, tiles = 0;
+  for (int i = 0; i < n; ++i)
+    for (int j = 0; j < g[i]->n_blocks; ++j, ++k) {
+      const mb_colblock& b = f.blk[k] = g[i]->blk[j];
+      const mb_weight w = {b.W, b.W_hi, b.W_lo, b.W_hi16, b.W_lo16, b.ldw};
+      if ((rc = split_map(w, 128 * b.n_src, 128, maps.w[k]))) return rc;
+      f.n_rows[k] = g[i]->n_rows;
+      n_src = b.n_src > n_src ? b.n_src : n_src;
+      most = g[i]->n_rows > most ? g[i]->n_rows : most;
+      tiles += (g[i]->n_rows + 15) / 16;
+    }
+  if (most == 0) return MB_OK;
+  few_launch<FEW_LINEAR>(f, maps, most, tiles <= n_sm ? 16 : 32, n_src, 2 * n_src, k, st);
+  MB_LAUNCH_CHECK("k_few");
+  return MB_OK;
+}
+int few_ffn_bwd(const mb_mlp_bwd* const* g, cudaStream_t st) {
+  int n_sm = 0, rc = device_config(&n_sm);
+  if (rc) return rc;
+  FewMaps maps;
+  FewPlainBwd f = {};
+  int64_t most = 0, tiles = 0;
+  for (int i = 0; i < 2; ++i) {
+    const mb_mlp_bwd& m = *g[i];
+    if ((rc = split_map(m.W2t, 128, 128, maps.w[2 * i])) || (rc = split_map(m.W1t, 128, 128, maps.w[2 * i + 1]))) return rc;
+    MlpArgs& a = f.of[i];
+    a.n_rows = m.n_rows; a.n_src = 1; a.src[0] = m.dy;
+    a.side = m.z1; a.ld_side = m.ld_z1; a.scale = m.scale; a.h = m.dx; a.ld_h = m.ld_dx;
+    most = m.n_rows > most ? m.n_rows : most;
+    tiles += (m.n_rows + 15) / 16;
+  }
+  few_launch<FEW_PLAIN_BWD>(f, maps, most, tiles <= n_sm ? 16 : 32, 1, 4, 2, st);
+  MB_LAUNCH_CHECK("k_few");
   return MB_OK;
 }
 
@@ -966,9 +1051,14 @@ extern "C" int mb_gemm(const mb_gemm_desc* desc, void* stream_) {
         for (int j = 0; j < desc->n_blocks; ++j) n_src = desc->blk[j].n_src > n_src ? desc->blk[j].n_src : n_src;
         if (const int r = mb::few_choice(mb::FEW_LINEAR, desc->n_rows, n_src, desc->n_blocks, n_sm)) {
           mb::FewMaps fm;
-          for (int j = 0; j < desc->n_blocks; ++j)
+          mb::FewLinear fl;
+          fl.pair = nullptr;
+          for (int j = 0; j < desc->n_blocks; ++j) {
+            fl.blk[j] = desc->blk[j];
+            fl.n_rows[j] = desc->n_rows;
             for (int part = 0; part < 2; ++part) fm.w[j][part] = maps.m[j][part];
-          mb::few_launch<mb::FEW_LINEAR>(*desc, fm, r, n_src, 2 * n_src, desc->n_blocks, (cudaStream_t)stream_);
+          }
+          mb::few_launch<mb::FEW_LINEAR>(fl, fm, desc->n_rows, r, n_src, 2 * n_src, desc->n_blocks, (cudaStream_t)stream_);
           MB_LAUNCH_CHECK("k_few");
           return MB_OK;
         }
@@ -1140,8 +1230,8 @@ extern "C" int mb_gated_mlp_fwd(const mb_gated_mlp* g, void* stream_) {
       if (g->n_src > 0) fm.w[0][part] = maps.w1[part];
       fm.w[1][part] = maps.w2[part];
     }
-    if (plain) mb::few_launch<mb::FEW_PLAIN_FWD>(a, fm, r, g->n_src, 2 * g->n_src + 2, 1, (cudaStream_t)stream_);
-    else mb::few_launch<mb::FEW_GATED_FWD>(a, fm, r, g->n_src, 4 * g->n_src + 4, 1, (cudaStream_t)stream_);
+    if (plain) mb::few_launch<mb::FEW_PLAIN_FWD>(a, fm, a.n_rows, r, g->n_src, 2 * g->n_src + 2, 1, (cudaStream_t)stream_);
+    else mb::few_launch<mb::FEW_GATED_FWD>(a, fm, a.n_rows, r, g->n_src, 4 * g->n_src + 4, 1, (cudaStream_t)stream_);
     MB_LAUNCH_CHECK("k_few");
     return MB_OK;
   }
@@ -1255,8 +1345,8 @@ extern "C" int mb_mlp_bwd_data(const mb_mlp_bwd* g, void* stream_) {
       fm.w[1][part] = maps.w2[part];
       if (g->n_ext > 0) fm.w[2][part] = maps.w3[part];
     }
-    if (plain) mb::few_launch<mb::FEW_PLAIN_BWD>(a, fm, r, 1, 4, 1, (cudaStream_t)stream_);
-    else mb::few_launch<mb::FEW_GATED_BWD>(a, fm, r, 2 + a.n_ext, 8 + 2 * a.n_ext, 1, (cudaStream_t)stream_);
+    if (plain) mb::few_launch<mb::FEW_PLAIN_BWD>({{a, {}}}, fm, a.n_rows, r, 1, 4, 1, (cudaStream_t)stream_);
+    else mb::few_launch<mb::FEW_GATED_BWD>(a, fm, a.n_rows, r, 2 + a.n_ext, 8 + 2 * a.n_ext, 1, (cudaStream_t)stream_);
     MB_LAUNCH_CHECK("k_few");
     return MB_OK;
   }

@@ -7,28 +7,17 @@
 // the source-side grouping is a permutation), so they need no atomics and their
 // summation order is fixed.  The one exception is k_seg_sum's third sum, over
 // the rows of a centre atom, which adds finished pieces with atomics.
-#include <float.h>
-#include "common.cuh"
+#include "row_math.cuh"
 
 namespace mb {
 
 constexpr int RW_THREADS = 256;
-constexpr float RMS_EPS = FLT_EPSILON;  // nn.RMSNorm(eps=None) uses the dtype's machine epsilon
-
-__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ float dot4(float4 a, float4 b) { return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
-__device__ __forceinline__ float4 mul4(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
-__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
-__device__ __forceinline__ float4 sub4(float4 a, float4 b) { return make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w); }
-__device__ __forceinline__ float4 scl4(float4 a, float s) { return make_float4(a.x * s, a.y * s, a.z * s, a.w * s); }
 __device__ __forceinline__ float4 fma4(float4 a, float4 b, float4 c) {
   return make_float4(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y), fmaf(a.z, b.z, c.z), fmaf(a.w, b.w, c.w));
 }
 __device__ __forceinline__ float4 max4(float4 a, float4 b) {
   return make_float4(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z), fmaxf(a.w, b.w));
 }
-__device__ __forceinline__ float4 exp4(float4 a) { return make_float4(expf(a.x), expf(a.y), expf(a.z), expf(a.w)); }
 __device__ __forceinline__ float4 zero4() { return make_float4(0.f, 0.f, 0.f, 0.f); }
 
 #define MB_ROW_PROLOGUE(n_rows)                                                       \
@@ -60,39 +49,14 @@ __global__ void k_gate_fwd(int64_t n_rows, const float* __restrict__ z, const fl
   }
 }
 
-// Adjoint of  h = SiLU(RMSNorm(z_core) w_core) * sigmoid(RMSNorm(z_gate) w_gate)  for one row held by a warp (lane =
-// four channels at c): g = dh of the row, result written to dz[row, 0:128 | 128:256].  Shared by k_gate_bwd and by the
-// kernels that produce dh and can hand it over in registers.
-__device__ __forceinline__ void gate_bwd_row(int64_t row, int c, const float* __restrict__ z,
-                                             const float* __restrict__ wc, const float* __restrict__ wg, float4 g,
-                                             float* __restrict__ dz) {
-  const float4 xc = ld4(z + row * 256 + c), xg = ld4(z + row * 256 + 128 + c);
-  const float rc = rsqrtf(warp_sum(dot4(xc, xc)) * (1.f / 128.f) + RMS_EPS);
-  const float rg = rsqrtf(warp_sum(dot4(xg, xg)) * (1.f / 128.f) + RMS_EPS);
-  const float4 gwc = ld4(wc + c), gwg = ld4(wg + c);
-  const float4 nc = scl4(xc, rc), ng = scl4(xg, rg);
-  const float4 yc = mul4(nc, gwc), yg = mul4(ng, gwg);
-  float dnc[4], dng[4];
-  const float ycv[4] = {yc.x, yc.y, yc.z, yc.w}, ygv[4] = {yg.x, yg.y, yg.z, yg.w};
-  const float gv[4] = {g.x, g.y, g.z, g.w}, wcv[4] = {gwc.x, gwc.y, gwc.z, gwc.w}, wgv[4] = {gwg.x, gwg.y, gwg.z, gwg.w};
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const float s = sigmoid_f(ycv[k]), gate = sigmoid_f(ygv[k]);
-    const float core = ycv[k] * s, gg = gv[k] * gate;
-    dnc[k] = gg * (s * (1.f + ycv[k] * (1.f - s))) * wcv[k];
-    dng[k] = gg * core * (1.f - gate) * wgv[k];
-  }
-  const float4 dn_c = make_float4(dnc[0], dnc[1], dnc[2], dnc[3]), dn_g = make_float4(dng[0], dng[1], dng[2], dng[3]);
-  const float mc = warp_sum(dot4(dn_c, nc)) * (1.f / 128.f), mg = warp_sum(dot4(dn_g, ng)) * (1.f / 128.f);
-  st4(dz + row * 256 + c, scl4(sub4(dn_c, scl4(nc, mc)), rc));
-  st4(dz + row * 256 + 128 + c, scl4(sub4(dn_g, scl4(ng, mg)), rg));
-}
-
 __global__ void k_gate_bwd(int64_t n_rows, const float* __restrict__ z, const float* __restrict__ wc,
                            const float* __restrict__ wg, const float* __restrict__ dh, float* __restrict__ dz) {
   pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
-  gate_bwd_row(row, c, z, wc, wg, ld4(dh + row * 128 + c), dz);
+  float4 dc, dg;
+  gate_bwd_row(z + row * 256, c, wc, wg, ld4(dh + row * 128 + c), dc, dg);
+  st4(dz + row * 256 + c, dc);
+  st4(dz + row * 256 + 128 + c, dg);
 }
 
 // ------------------------------------------------------------------ attention aggregation
@@ -181,33 +145,21 @@ k_seg_attn_fwd(int n_nodes, const int32_t* __restrict__ tgt_ptr, const int32_t* 
 // Latency of the gathered rows bounds it (5 TB/s of DRAM traffic at half occupancy): six blocks per SM, even with a few spills, beat
 // what 62 registers allow.  522,844 angles 579 -> 526 us, 234,096 edges 252 -> 229; eight blocks 557 and 242.
 __global__ void __launch_bounds__(RW_THREADS, 6)
-k_seg_attn_bwd(int64_t n_rows, const int32_t* __restrict__ tgt, const int32_t* __restrict__ src,
-               int idx_stride, const int32_t* __restrict__ emap, const float* __restrict__ logits,
-               const float* __restrict__ h, const float* __restrict__ agg_t,
-               const float* __restrict__ agg_s, const float* __restrict__ stats,
-               const float* __restrict__ dagg_t, const float* __restrict__ dagg_s,
-               const float* __restrict__ dh_in, const int32_t* __restrict__ dh_map, float dh_scale,
-               float* __restrict__ dh, float* __restrict__ dlogits, const float* __restrict__ gate_z,
-               const float* __restrict__ gate_wc, const float* __restrict__ gate_wg,
-               float* __restrict__ gate_dz) {
+k_seg_attn_bwd(int64_t n_rows, const RowGrad a, float* __restrict__ dh, float* __restrict__ gate_dz) {
   pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
-  const int64_t nt = tgt[row * idx_stride], ns = src[row * idx_stride];
-  const int64_t er = emap ? emap[row] : row;
-  const float4 xs = ld4(logits + er * 256 + c), xt = ld4(logits + er * 256 + 128 + c);
-  const float4 at = mul4(exp4(sub4(xt, ld4(stats + nt * 512 + c))), ld4(stats + nt * 512 + 128 + c));
-  const float4 as = mul4(exp4(sub4(xs, ld4(stats + ns * 512 + 256 + c))), ld4(stats + ns * 512 + 384 + c));
-  const float4 hv = ld4(h + row * 128 + c);
-  const float4 gt = mul4(at, ld4(dagg_t + nt * 128 + c)), gs = mul4(as, ld4(dagg_s + ns * 128 + c));
-  float4 o = add4(gt, gs);
-  if (dh_in) {
-    const int64_t mr = dh_map ? dh_map[row] : row;
-    o = add4(o, scl4(ld4(dh_in + mr * 128 + c), dh_scale));
+  float4 o, ds, dt;
+  attn_bwd_row(a, row, c, o, ds, dt);
+  if (gate_dz) {  // dh goes on in registers
+    float4 dc, dg;
+    gate_bwd_row(a.z2 + row * 256, c, a.norm_core, a.norm_gate, o, dc, dg);
+    st4(gate_dz + row * 256 + c, dc);
+    st4(gate_dz + row * 256 + 128 + c, dg);
+  } else {
+    st4(dh + row * 128 + c, o);
   }
-  if (gate_dz) gate_bwd_row(row, c, gate_z, gate_wc, gate_wg, o, gate_dz);  // dh goes on in registers
-  else st4(dh + row * 128 + c, o);
-  st4(dlogits + row * 256 + c, mul4(gs, sub4(hv, ld4(agg_s + ns * 128 + c))));
-  st4(dlogits + row * 256 + 128 + c, mul4(gt, sub4(hv, ld4(agg_t + nt * 128 + c))));
+  st4(a.dlogits + row * 256 + c, ds);
+  st4(a.dlogits + row * 256 + 128 + c, dt);
 }
 
 // ------------------------------------------------------------------ refinement aggregation
@@ -255,37 +207,70 @@ __global__ void k_seg_smooth_sum_fwd(int n_nodes, const int32_t* __restrict__ tg
 // Bounded by latency like k_seg_attn_bwd; the exponentials of the gate's adjoint come next.  522,844 angles with the adjoint: one
 // sigmoid per branch instead of three in all 351 -> 301 us, eight blocks per SM 274 us; 234,096 edges 156 -> 125.
 __global__ void __launch_bounds__(RW_THREADS, 8)
-k_seg_smooth_sum_bwd_rows(int64_t n_rows, const int32_t* __restrict__ tgt,
-                          const int32_t* __restrict__ src, int idx_stride,
-                          const int32_t* __restrict__ emap, const float* __restrict__ env,
-                          const float* __restrict__ dagg, float* __restrict__ dh, int accumulate,
-                          const float* __restrict__ gate_z, const float* __restrict__ gate_wc,
-                          const float* __restrict__ gate_wg, float* __restrict__ gate_dz) {
+k_seg_smooth_sum_bwd_rows(int64_t n_rows, const RowGrad a, float* __restrict__ dh, float* __restrict__ gate_dz) {
   pdl_sync();
   MB_ROW_PROLOGUE(n_rows)
-  const int64_t nt = tgt[row * idx_stride];
-  float4 s;
-  if (src) s = mul4(ld4(env + (int64_t)src[row * idx_stride] * 128 + c), ld4(env + nt * 128 + c));
-  else s = ld4(env + (int64_t)emap[row] * 128 + c);
-  float4 o = mul4(ld4(dagg + nt * 128 + c), s);
-  if (accumulate) o = add4(o, ld4(dh + row * 128 + c));
-  if (gate_dz) gate_bwd_row(row, c, gate_z, gate_wc, gate_wg, o, gate_dz);  // dh goes on in registers
-  else st4(dh + row * 128 + c, o);
+  const float4 o = smooth_bwd_row(a, row, c);
+  if (gate_dz) {  // dh goes on in registers
+    float4 dc, dg;
+    gate_bwd_row(a.z2 + row * 256, c, a.norm_core, a.norm_gate, o, dc, dg);
+    st4(gate_dz + row * 256 + c, dc);
+    st4(gate_dz + row * 256 + 128 + c, dg);
+  } else {
+    st4(dh + row * 128 + c, o);
+  }
 }
 
-__global__ void k_smooth_env_bwd_atom(int n_bonds, const int32_t* __restrict__ u2d, const int32_t* __restrict__ rev,
-                                      const int32_t* __restrict__ tgt, const float* __restrict__ h,
-                                      const float* __restrict__ dagg, const float* __restrict__ drow,
-                                      float* __restrict__ denv) {
-  pdl_sync();
-  MB_ROW_PROLOGUE(n_bonds)
+__device__ __forceinline__ float4 smooth_env_bwd_atom(int64_t row, int c, const int32_t* __restrict__ u2d, const int32_t* __restrict__ rev,
+                                                      const int32_t* __restrict__ tgt, const float* __restrict__ h,
+                                                      const float* __restrict__ dagg, const float* __restrict__ drow) {
   const int64_t e1 = u2d[row], e2 = rev[e1];
   float4 g1 = ld4(dagg + (int64_t)tgt[e1] * 128 + c), g2 = ld4(dagg + (int64_t)tgt[e2] * 128 + c);
   if (drow) {  // gradient that reached the smoothed rows directly (edge FFN fed with h * s)
     g1 = add4(g1, ld4(drow + e1 * 128 + c));
     g2 = add4(g2, ld4(drow + e2 * 128 + c));
   }
-  st4(denv + row * 128 + c, add4(mul4(g1, ld4(h + e1 * 128 + c)), mul4(g2, ld4(h + e2 * 128 + c))));
+  return add4(mul4(g1, ld4(h + e1 * 128 + c)), mul4(g2, ld4(h + e2 * 128 + c)));
+}
+__global__ void k_smooth_env_bwd_atom(int n_bonds, const int32_t* __restrict__ u2d, const int32_t* __restrict__ rev,
+                                      const int32_t* __restrict__ tgt, const float* __restrict__ h,
+                                      const float* __restrict__ dagg, const float* __restrict__ drow,
+                                      float* __restrict__ denv) {
+  pdl_sync();
+  MB_ROW_PROLOGUE(n_bonds)
+  st4(denv + row * 128 + c, smooth_env_bwd_atom(row, c, u2d, rev, tgt, h, dagg, drow));
+}
+// dx[row, 0:7] += v w for a row v held by a warp (w [128, 7]), products and additions in the order of k_small_linear_bwd
+__device__ __forceinline__ void row_times_small(int64_t row, int lane, float4 v, const float* __restrict__ w, float* __restrict__ dx) {
+  float wr[28];  // of this lane's four channels
+#pragma unroll
+  for (int i = 0; i < 7; ++i) *reinterpret_cast<float4*>(wr + 4 * i) = ld4(w + 28 * lane + 4 * i);
+  float p[8];
+#pragma unroll
+  for (int j = 0; j < 7; ++j) p[j] = dot4(v, make_float4(wr[j], wr[7 + j], wr[14 + j], wr[21 + j]));
+  p[7] = 0.f;
+  int o = 16;
+#pragma unroll
+  for (int n = 4; n > 0; n >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float keep = up ? p[i + n] : p[i], give = up ? p[i] : p[i + n];
+      p[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  for (; o > 0; o >>= 1) p[0] += __shfl_xor_sync(0xffffffffu, p[0], o);
+  const int j = lane >> 2;
+  if ((lane & 3) == 0 && j < 7) dx[row * 7 + j] = p[0] + dx[row * 7 + j];
+}
+// The envelopes' gradient straight on into the radial basis's: for few bonds one launch and no denv instead of two.
+__global__ void __launch_bounds__(RW_THREADS) k_smooth_env_bwd_atom_rbf(int n_bonds, const int32_t* __restrict__ u2d, const int32_t* __restrict__ rev,
+                                          const int32_t* __restrict__ tgt, const float* __restrict__ h,
+                                          const float* __restrict__ dagg, const float* __restrict__ drow,
+                                          const float* __restrict__ w, float* __restrict__ d_rbf) {
+  pdl_sync();
+  MB_ROW_PROLOGUE(n_bonds)
+  row_times_small(row, lane, smooth_env_bwd_atom(row, c, u2d, rev, tgt, h, dagg, drow), w, d_rbf);
 }
 
 // y[r] = x[r] * s[idx[r]]  (rows scaled channel-wise by a gathered row)
@@ -297,16 +282,12 @@ __global__ void k_mul_rows_gather(int64_t n_rows, const float* __restrict__ x, c
   st4(y + row * 128 + c, mul4(ld4(x + row * 128 + c), ld4(s + sr * 128 + c)));
 }
 
-// Four rows in flight and six blocks per SM (40 registers): 180 -> 121 us for 117,048 bonds / 522,844 angles (four blocks 156).
-__global__ void __launch_bounds__(RW_THREADS, 6)
-k_smooth_env_bwd_line(int n_nodes, const int32_t* __restrict__ tgt_ptr,
-                      const int32_t* __restrict__ src_ptr, const int32_t* __restrict__ src_perm,
-                      const int32_t* __restrict__ tgt, const int32_t* __restrict__ src,
-                      int idx_stride, const float* __restrict__ env, const float* __restrict__ h,
-                      const float* __restrict__ dagg, float* __restrict__ denv) {
-  pdl_sync();
-  MB_ROW_PROLOGUE(n_nodes)
-  constexpr int NB = 4;  // rows in flight
+template <int NB>  // rows in flight
+__device__ __forceinline__ float4 smooth_env_bwd_line(int64_t row, int c, const int32_t* __restrict__ tgt_ptr,
+                                                      const int32_t* __restrict__ src_ptr, const int32_t* __restrict__ src_perm,
+                                                      const int32_t* __restrict__ tgt, const int32_t* __restrict__ src,
+                                                      int idx_stride, const float* __restrict__ env, const float* __restrict__ h,
+                                                      const float* __restrict__ dagg) {
   float4 acc = zero4();
   const int q0 = tgt_ptr[row], q1 = tgt_ptr[row + 1];
   for (int q = q0; q < q1; q += NB) {
@@ -342,7 +323,28 @@ k_smooth_env_bwd_line(int n_nodes, const int32_t* __restrict__ tgt_ptr,
     for (int i = 0; i < NB; ++i)
       if (q + i < s1) acc = fma4(mul4(gv[i], hv[i]), ev[i], acc);
   }
-  st4(denv + row * 128 + c, acc);
+  return acc;
+}
+// Four rows in flight and six blocks per SM (40 registers): 180 -> 121 us for 117,048 bonds / 522,844 angles (four blocks 156).
+__global__ void __launch_bounds__(RW_THREADS, 6)
+k_smooth_env_bwd_line(int n_nodes, const int32_t* __restrict__ tgt_ptr,
+                      const int32_t* __restrict__ src_ptr, const int32_t* __restrict__ src_perm,
+                      const int32_t* __restrict__ tgt, const int32_t* __restrict__ src,
+                      int idx_stride, const float* __restrict__ env, const float* __restrict__ h,
+                      const float* __restrict__ dagg, float* __restrict__ denv) {
+  pdl_sync();
+  MB_ROW_PROLOGUE(n_nodes)
+  st4(denv + row * 128 + c, smooth_env_bwd_line<4>(row, c, tgt_ptr, src_ptr, src_perm, tgt, src, idx_stride, env, h, dagg));
+}
+// For few bonds (see k_smooth_env_bwd_atom_rbf) a warp's chain counts, not the rows in flight on a multiprocessor: eight of them.
+__global__ void __launch_bounds__(RW_THREADS, 2)
+k_smooth_env_bwd_line_rbf(int n_nodes, const int32_t* __restrict__ tgt_ptr, const int32_t* __restrict__ src_ptr,
+                          const int32_t* __restrict__ src_perm, const int32_t* __restrict__ tgt, const int32_t* __restrict__ src,
+                          const float* __restrict__ env, const float* __restrict__ h, const float* __restrict__ dagg,
+                          const float* __restrict__ w, float* __restrict__ d_rbf) {
+  pdl_sync();
+  MB_ROW_PROLOGUE(n_nodes)
+  row_times_small(row, lane, smooth_env_bwd_line<8>(row, c, tgt_ptr, src_ptr, src_perm, tgt, src, 1, env, h, dagg), w, d_rbf);
 }
 
 // ------------------------------------------------------------------ sums of row gradients over a node's rows
@@ -478,13 +480,12 @@ __device__ __forceinline__ void small_linear_weights(const float* __restrict__ w
 }
 
 template <int KP>
-__global__ void __launch_bounds__(RW_THREADS, KP == 8 ? 4 : 2)
-k_small_linear_fwd(int64_t n_rows, int k, const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y) {
+__device__ __forceinline__ void small_linear_fwd(int64_t n_rows, int k, const float* __restrict__ x, const float* __restrict__ w,
+                                                 float* __restrict__ y) {
   constexpr int ROWS = 32 / KP;
   const int lane = threadIdx.x & 31, c = lane * 4, ri = lane / KP, rj = lane % KP;
   const int64_t step = ((int64_t)gridDim.x * blockDim.x >> 5) * ROWS;
   float4 wr[KP];
-  pdl_sync();
   small_linear_weights<KP>(w, k, c, wr);
   for (int64_t r0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * ROWS; r0 < n_rows; r0 += step) {
     const float xv = rj < k && r0 + ri < n_rows ? x[(r0 + ri) * k + rj] : 0.f;
@@ -499,6 +500,17 @@ k_small_linear_fwd(int64_t n_rows, int k, const float* __restrict__ x, const flo
       if (r0 + r < n_rows) st4(y + (r0 + r) * 128 + c, acc);
     }
   }
+}
+
+template <int KP>
+__global__ void __launch_bounds__(RW_THREADS, KP == 8 ? 4 : 2)
+k_small_linear_fwd(int64_t n_rows, int k, const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y) {
+  pdl_sync();
+  small_linear_fwd<KP>(n_rows, k, x, w, y);
+}
+__global__ void __launch_bounds__(RW_THREADS, 4) k_many_small_linears(int64_t n_rows, const __grid_constant__ ManyLinears a) {
+  pdl_sync();
+  small_linear_fwd<8>(n_rows, 7, a.x[blockIdx.y], a.w[blockIdx.y], a.y[blockIdx.y]);
 }
 
 // dx = dy W: every lane's 32 partial sums (32 / KP rows x KP) are reduced across the warp by halving, 31 shuffles in all, which leaves
@@ -689,9 +701,11 @@ extern "C" int mb_seg_attn_bwd(int64_t n_rows, const int32_t* tgt, const int32_t
   MB_REQUIRE(n_rows >= 0 && tgt && src && idx_stride > 0 && logits && h && agg_t && agg_s && stats && dagg_t &&
              dagg_s && dlogits && (gate_dz ? (gate_z && gate_wc && gate_wg) : dh != nullptr));
   if (n_rows == 0) return MB_OK;
-  launch(k_seg_attn_bwd, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, tgt, src, idx_stride, emap, logits, h, agg_t,
-                                                             agg_s, stats, dagg_t, dagg_s, dh_in, dh_map, dh_scale,
-                                                             dh, dlogits, gate_z, gate_wc, gate_wg, gate_dz);
+  RowGrad a = {};
+  a.idx_stride = idx_stride; a.dh_in = dh_in; a.dh_map = dh_map; a.dh_scale = dh_scale; a.tgt = tgt; a.src = src; a.emap = emap;
+  a.logits = logits; a.h = h; a.agg_t = agg_t; a.agg_s = agg_s; a.stats = stats; a.dagg_t = dagg_t; a.dagg_s = dagg_s;
+  a.dlogits = dlogits; a.z2 = gate_z; a.norm_core = gate_wc; a.norm_gate = gate_wg;
+  launch(k_seg_attn_bwd, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, a, dh, gate_dz);
   MB_LAUNCH_CHECK("k_seg_attn_bwd");
   return MB_OK;
 }
@@ -717,9 +731,10 @@ extern "C" int mb_seg_smooth_sum_bwd_rows(int64_t n_rows, const int32_t* tgt, co
   MB_REQUIRE(n_rows >= 0 && tgt && (emap || src) && env && dagg && idx_stride > 0 && (dh || (gate_dz && !accumulate)) &&
              (!gate_dz || (gate_z && gate_wc && gate_wg)));
   if (n_rows == 0) return MB_OK;
-  launch(k_seg_smooth_sum_bwd_rows, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, tgt, src, idx_stride, emap, env,
-                                                                        dagg, dh, accumulate, gate_z, gate_wc, gate_wg,
-                                                                        gate_dz);
+  RowGrad a = {};
+  a.idx_stride = idx_stride; a.dh_in = accumulate ? dh : nullptr; a.tgt = tgt; a.src = src; a.emap = emap; a.env = env; a.dagg = dagg;
+  a.z2 = gate_z; a.norm_core = gate_wc; a.norm_gate = gate_wg;
+  launch(k_seg_smooth_sum_bwd_rows, row_grid(n_rows), RW_THREADS, 0, STREAM, n_rows, a, dh, gate_dz);
   MB_LAUNCH_CHECK("k_seg_smooth_sum_bwd_rows");
   return MB_OK;
 }
@@ -903,3 +918,25 @@ extern "C" int mb_segment_sum_scalar(int32_t n_seg, const int32_t* seg_ptr, cons
   MB_LAUNCH_CHECK("k_segment_sum_scalar");
   return MB_OK;
 }
+
+namespace mb {
+int many_small_linears(int64_t n_rows, int n, const ManyLinears& a, cudaStream_t stream) {
+  if (n_rows == 0 || n == 0) return MB_OK;
+  int n_sm = 0;
+  if (const int rc = sm_count(&n_sm)) return rc;
+  launch(k_many_small_linears, dim3(small_linear_grid(n_rows, 4, 4 * n_sm), (unsigned)n), RW_THREADS, 0, stream, n_rows, a);
+  MB_LAUNCH_CHECK("k_many_small_linears");
+  return MB_OK;
+}
+int smooth_env_bwd_rbf(int32_t n_bonds, const mb_row_graph& g, const float* env, const float* h, const float* dagg, const float* drow,
+                       const float* w, float* d_rbf, cudaStream_t stream) {
+  if (n_bonds == 0) return MB_OK;
+  if (g.is_atom)
+    launch(k_smooth_env_bwd_atom_rbf, row_grid(n_bonds), RW_THREADS, 0, stream, n_bonds, g.u2d, g.rev, g.tgt, h, dagg, drow, w, d_rbf);
+  else
+    launch(k_smooth_env_bwd_line_rbf, row_grid(n_bonds), RW_THREADS, 0, stream, n_bonds, g.tgt_ptr, g.src_ptr, g.src_perm, g.tgt,
+           g.src, env, h, dagg, w, d_rbf);
+  MB_LAUNCH_CHECK("k_smooth_env_bwd_rbf");
+  return MB_OK;
+}
+}  // namespace mb

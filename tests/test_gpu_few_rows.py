@@ -96,3 +96,23 @@ def test_mlps(ops, at):
     h = F.silu(rms(y[:, :128], nc.double())) * torch.sigmoid(rms(y[:, 128:], ng.double()))
     for name, got, want in zip(("z1", "z2", "h"), small["gated, K = 384"], (z, y, h)):
         report(f"few rows gated K=384 {name} R={rows}", got, want, TOL, scaled=True)
+
+
+@pytest.mark.parametrize("options", [{}, dict(use_bias=True, use_smoothed_for_delta_edge=True)])
+def test_small_structures_equal_their_batch(options):
+    """Alone, a small structure takes the few-row kernels, merged launches and gradients formed on the way; in a large batch its rows
+    take the row kernels and the persistent contractions.  The expressions are the same; sums over atoms' rows may meet in another
+    order (rounding of float32 sums of order one)."""
+    from matris_b200 import MatRIS, workloads
+    from matris_b200.weights import random_checkpoint
+    from conftest import GPA
+    small = [workloads.cu_fcc((1, 1, 1), sigma=0.05), workloads.demo_pu4si6(), workloads.cu_fcc((2, 2, 2), sigma=0.05),
+             workloads.random_crystals(1, seed=3)[0]]
+    model = MatRIS.from_dict(random_checkpoint(dict(num_layers=2, reference_energy="mpa", **options), seed=1, jitter=0.1)).to("cuda")
+    many = model.predict(small * 40, "efsm")
+    for i, c in enumerate(small):
+        one = model.predict([c], "efsm")
+        report(f"alone vs in a batch {i}: E", one["e"][0], many["e"][i], 1e-6, scaled=True)
+        report(f"alone vs in a batch {i}: F", one["f"][0], many["f"][i], 2e-6)
+        report(f"alone vs in a batch {i}: S", one["s"][0] / GPA, many["s"][i] / GPA, 2e-7)
+        report(f"alone vs in a batch {i}: M", one["m"][0], many["m"][i], 2e-6)
