@@ -964,6 +964,9 @@ extern "C" int mb_bench_mma_rate(int kind, int iters, float* elapsed_ms, int* n_
   cudaEvent_t e0, e1;
   MB_CUDA_CHECK(cudaEventCreate(&e0));
   MB_CUDA_CHECK(cudaEventCreate(&e1));
+  // an untimed launch first: the kernel's code is loaded with it
+  if (kind == 0) mb::k_mma_rate<0><<<n_sm, 128, smem, st>>>(1);
+  else mb::k_mma_rate<1><<<n_sm, 128, smem, st>>>(1);
   cudaError_t err = cudaEventRecord(e0, st);
   if (err == cudaSuccess) {
     if (kind == 0) mb::k_mma_rate<0><<<n_sm, 128, smem, st>>>(iters);
