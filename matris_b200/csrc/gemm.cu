@@ -726,7 +726,10 @@ static int device_config(int* n_sm) {
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_gemm_ps<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PS_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_gemm_ps<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PS_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_linear, cudaFuncAttributeMaxDynamicSharedMemorySize, LN_SMEM_BYTES));
-    MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_GATED_FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
+    MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_GATED_FWD, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
+    MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_GATED_FWD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
+    MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_GATED_FWD, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
+    MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_GATED_FWD, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_PLAIN_FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_GATED_BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_PLAIN_BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
@@ -1250,7 +1253,10 @@ extern "C" int mb_gated_mlp_fwd(const mb_gated_mlp* g, void* stream_) {
   const unsigned grid = (unsigned)(n_tiles < n_sm ? n_tiles : n_sm);
   cudaStream_t st = (cudaStream_t)stream_;
   if (plain) mb::launch(mb::k_mlp<mb::MLP_PLAIN_FWD>, grid, mb::ML_THREADS, mb::ML_SMEM_BYTES, st, a, maps);
-  else mb::launch(mb::k_mlp<mb::MLP_GATED_FWD>, grid, mb::ML_THREADS, mb::ML_SMEM_BYTES, st, a, maps);
+  else if (a.n_add == 0) mb::launch(mb::k_mlp<mb::MLP_GATED_FWD, 0>, grid, mb::ML_THREADS, mb::ML_SMEM_BYTES, st, a, maps);
+  else if (a.n_add == 1) mb::launch(mb::k_mlp<mb::MLP_GATED_FWD, 1>, grid, mb::ML_THREADS, mb::ML_SMEM_BYTES, st, a, maps);
+  else if (a.n_add == 2) mb::launch(mb::k_mlp<mb::MLP_GATED_FWD, 2>, grid, mb::ML_THREADS, mb::ML_SMEM_BYTES, st, a, maps);
+  else mb::launch(mb::k_mlp<mb::MLP_GATED_FWD, 3>, grid, mb::ML_THREADS, mb::ML_SMEM_BYTES, st, a, maps);
   MB_LAUNCH_CHECK("k_mlp forward");
   return MB_OK;
 }

@@ -32,8 +32,8 @@
 // two epilogue groups, L1(t) -> 2t mod 3, L2(t) -> 2t+1 mod 3, issued L1(t+1) before L2(t).
 //
 // Measured behind an L2 flush (bench_gemm.py; addend tables of a fifth of the rows), 573,894 rows with z1 and z2 kept: two addends
-// and a residual 0.53 ms, three addends 0.65 (nothing kept: 0.54), no contraction and three addends 0.58, K = 384 gathered with a
-// residual 0.64; GATED_BWD with a residual 0.42, with E too 0.59; FFN forward 0.23, backward 0.18.  One tile alone takes 28 us
+// and a residual 0.50 ms, three addends 0.58 (nothing kept: 0.42), no contraction and three addends 0.48, K = 384 gathered with a
+// residual 0.63; GATED_BWD with a residual 0.42, with E too 0.59; FFN forward 0.23, backward 0.18.  One tile alone takes 28 us
 // forward, 21 us backward: the chain of its stages.
 //
 // Warps: 0 MMA, 1 TMA (weights, 16 KB tiles of 64 K values, five slots), 2-9 producers, 10-17 epilogue (two groups of four; the
@@ -138,7 +138,8 @@ __device__ __forceinline__ float sum_of_squares(const float (&y)[32]) {
   return v[0];
 }
 
-template <int MODE>
+// N_ADD: GATED_FWD's number of addends (a launch without any keeps the registers of their gather)
+template <int MODE, int N_ADD = 0>
 __global__ void __launch_bounds__(ML_THREADS, 1)
 k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
   constexpr bool GATED = MODE == MLP_GATED_FWD || MODE == MLP_GATED_BWD;
@@ -170,7 +171,8 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
   const int n_tiles = (n_row_tiles - first_rt + step_rt - 1) / step_rt;  // the grid never exceeds the tile count
   const int n_kp1 = 2 * d.n_src, n_kpx = MODE == MLP_GATED_BWD ? 2 * d.n_ext : 0;  // pairs of 32-float K chunks
   const int n_kpa = n_kp1 + n_kpx;
-  const bool has_side = MODE == MLP_GATED_FWD ? d.n_add > 0 : !FWD, has_res = d.out2 != nullptr;
+  constexpr bool has_side = MODE == MLP_GATED_FWD ? N_ADD > 0 : !FWD;
+  const bool has_res = d.out2 != nullptr;
 
   if (warp == ML_MMA_WARP) {
     if (lane == 0) {
@@ -631,51 +633,49 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
       if (!has_res) return;
       for (int c = 0; c < (GATED ? 2 : 4); ++c) request_side(&maps.res, (GATED ? 64 * parity : 0) + 32 * c, tile_row(t));
     };
-    // Addend sums of a tile.  The loads are latency bound, so as many as fit in the registers are requested together: three addends
-    // half a patch (16 rows) at a time (0.58 -> 0.54 ms for 573,894 rows), fewer one after the other with the whole patch each (two at
-    // once by halves: 0.68 instead of 0.60 ms).
-    auto gather = [&](auto count, int t, int col0) {
-      constexpr int N = decltype(count)::value, ROWS = N == 3 ? 4 : 8, AT_ONCE = N == 3 ? 3 : 1;
-      const int64_t row0 = tile_row(t);
-      int32_t ix[N][8];
+    // Addend sums of a tile.  The loads are latency bound (2 k cycles a batch in the running kernel), so as many as fit in the registers
+    // are requested together: up to two addends a patch (32 rows), three half a patch at a time.  The row numbers take one register
+    // of a lane (= row) for each addend and are shuffled; they are asked for a tile ahead.  573,894 rows, z1 and z2 kept: three addends 0.665 ->
+    // 0.576 ms (nothing kept 0.543 -> 0.42), two and a residual 0.534 -> 0.50, no contraction and three addends 0.580 -> 0.484.
+    int32_t nx[N_ADD > 0 ? N_ADD : 1];  // row numbers of the next tile
+    auto ask_rows = [&](int t) {
+      const int64_t at = tile_row(t) + lane, row = at < n_rows ? at : n_rows - 1;
 #pragma unroll
-      for (int a = 0; a < N; ++a)
+      for (int a = 0; a < N_ADD; ++a) nx[a] = d.add[a].idx ? d.add[a].idx[row] : (int32_t)row;
+    };
+    auto gather = [&](int t, int col0) {
+      constexpr int N = N_ADD, ROWS = N == 3 ? 4 : 8;
+      int32_t ix[N > 0 ? N : 1];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int64_t r = row0 + lr + 4 * i < n_rows ? row0 + lr + 4 * i : n_rows - 1;
-          ix[a][i] = d.add[a].idx ? d.add[a].idx[r] : (int32_t)r;
-        }
+      for (int a = 0; a < N; ++a) ix[a] = nx[a];
+      if (t + 1 < n_tiles) ask_rows(t + 1);
 #pragma unroll 1
       for (int c = 0; c < 4; ++c, ++side_n) {
         const int col = col0 + 32 * c + lc * 4;
         const float4 b = reinterpret_cast<const float4*>(cst)[col >> 2];
 #pragma unroll
         for (int i0 = 0; i0 < 8; i0 += ROWS) {
-          float4 sum[ROWS];
+          float4 v[N > 0 ? N : 1][ROWS];
 #pragma unroll
-          for (int a0 = 0; a0 < N; a0 += AT_ONCE) {
-            float4 v[AT_ONCE][ROWS];
+          for (int a = 0; a < N; ++a)
 #pragma unroll
-            for (int a = 0; a < AT_ONCE; ++a)
-#pragma unroll
-              for (int i = 0; i < ROWS; ++i) v[a][i] = ld4(d.add[a0 + a].ptr + (int64_t)ix[a0 + a][i0 + i] * d.add[a0 + a].ld + col);
-#pragma unroll
-            for (int a = 0; a < AT_ONCE; ++a)
-#pragma unroll
-              for (int i = 0; i < ROWS; ++i) {
-                const float4 o = a0 + a == 0 ? b : sum[i];
-                sum[i] = make_float4(o.x + v[a][i].x, o.y + v[a][i].y, o.z + v[a][i].z, o.w + v[a][i].w);
-              }
-          }
+            for (int i = 0; i < ROWS; ++i)
+              v[a][i] = ld4(d.add[a].ptr + (int64_t)__shfl_sync(0xffffffffu, ix[a], lr + 4 * (i0 + i)) * d.add[a].ld + col);
           if (i0 == 0) wait_empty();
 #pragma unroll
-          for (int i = 0; i < ROWS; ++i) put(side0 + (side_n & 1) * ML_PATCH, i0 + i, sum[i]);
+          for (int i = 0; i < ROWS; ++i) {
+            float4 s = b;
+#pragma unroll
+            for (int a = 0; a < N; ++a) s = make_float4(s.x + v[a][i].x, s.y + v[a][i].y, s.z + v[a][i].z, s.w + v[a][i].w);
+            put(side0 + (side_n & 1) * ML_PATCH, i0 + i, s);
+          }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(side_full + 8 * (2 * pw + (side_n & 1)));
       }
     };
     if (n_seg > 0 && is_direct(0)) request(0, 0, 0, false);
+    if constexpr (N_ADD > 0) ask_rows(0);
     asm volatile("bar.sync 5, 512;" ::: "memory");  // the constants are there
     for (int t = 0; t < n_tiles; ++t) {
       const int64_t row0 = tile_row(t);
@@ -746,15 +746,11 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
         if (t > 0) residual(t - 1);
         continue;
       }
-      if (has_side) {
-        const int col0 = GATED ? 128 * parity : 0;
-        if constexpr (FWD) {
-          if (d.n_add == 1) gather(std::integral_constant<int, 1>{}, t, col0);
-          else if (d.n_add == 2) gather(std::integral_constant<int, 2>{}, t, col0);
-          else gather(std::integral_constant<int, 3>{}, t, col0);
-        } else {
-          for (int c = 0; c < 4; ++c) request_side(&maps.side, col0 + 32 * c, (int)row0);
-        }
+      const int col0 = GATED ? 128 * parity : 0;
+      if constexpr (N_ADD > 0) {
+        gather(t, col0);
+      } else if constexpr (!FWD) {
+        for (int c = 0; c < 4; ++c) request_side(&maps.side, col0 + 32 * c, (int)row0);
       }
       if (MODE == MLP_GATED_BWD) residual(t);
     }
