@@ -471,7 +471,7 @@ static void edge_update_bwd(Run& R, const mb_update& p, const mb_row_graph& g, c
   float* dP = R.ar.bottom((size_t)g.n_nodes * 512);
   float* dPc = d_ctr ? R.ar.bottom((size_t)g.n_ctr * 256) : nullptr;
   float* const dlogits = rg.dlogits;
-  const bool few = R.go() && few_rows_fit(g.n_rows, 1);
+  const bool few = R.go() && few_row_bwd_fits(g.n_rows, 1, !g.is_atom && dlogits);
   RowBwd b{};
   if (few) {
     b.n_rows = g.n_rows; b.g = rg; b.w2t = p.w2t; b.z1 = z1; b.dz1 = dz1;
@@ -512,19 +512,17 @@ static void edge_update_bwd(Run& R, const mb_update& p, const mb_row_graph& g, c
     });
     const int ld = dlogits ? 512 : 256;
     float* pair = R.ar.bottom((size_t)g.n_edge_rows * ld);
-    const bool pairs = R.go() && few_rows_fit(g.n_edge_rows, 1);  // the pair's sum is formed on the way
-    if (!pairs) MB_OP(mb_pair_sum, (int32_t)g.n_edge_rows, g.u2d, g.rev, dz1, dlogits, pair);
     Gemm e(g.n_edge_rows);
-    auto half = [&](int j) {  // 128 columns of the sums: dz1 core and gate, dlogits
-      if (!pairs) return src(pair, nullptr, 128 * j, ld);
-      return src(j < 2 ? dz1 : dlogits, g.u2d, 128 * (j & 1), 256);
-    };
-    mb_colblock& b = e.block({half(0), half(1)}, dlogits ? *w_log : p.wet, 0, d_edge, 128);
-    if (dlogits) {
-      b.src[b.n_src++] = half(2);
-      b.src[b.n_src++] = half(3);
-    }
+    mb_colblock& b = e.block({}, dlogits ? *w_log : p.wet, 0, d_edge, 128);
     b.res = edge_res; b.res_w = edge_w; b.ld_res = 128;
+    b.n_src = dlogits ? 4 : 2;  // the sums of dz1 (core, gate) and of dlogits, formed on the way where the rows are few
+    for (int j = 0; j < b.n_src; ++j) b.src[j] = src(j < 2 ? dz1 : dlogits, g.u2d, 128 * (j & 1), 256);
+    const mb_gemm_desc* const one[1] = {&e.d};
+    const bool pairs = R.go() && few_linears_fit(one, 1);
+    if (!pairs) {
+      MB_OP(mb_pair_sum, (int32_t)g.n_edge_rows, g.u2d, g.rev, dz1, dlogits, pair);
+      for (int j = 0; j < b.n_src; ++j) b.src[j] = src(pair, nullptr, 128 * j, ld);
+    }
     e.run(R, pairs ? g.rev : nullptr);
   } else if (!few) {
     mb_mlp_bwd m;
@@ -582,7 +580,7 @@ static void update_bwd(Run& R, const mb_update& p, int64_t rows, const float* z1
   float* dz1 = R.ar.bottom(rows * 256);
   bool plain = dests.size() <= 3;  // outputs at their own rows, a residual on the first at most
   for (const Dest& d : dests) plain = plain && !d.idx && d.mode == MB_OUT_STORE && (!d.res || &d == dests.begin());
-  if (!dz2 && plain && R.go() && few_rows_fit(rows, (int)dests.size())) {
+  if (!dz2 && plain && R.go() && few_row_bwd_fits(rows, (int)dests.size(), false)) {
     RowBwd b{};
     b.n_rows = rows; b.w2t = p.w2t; b.w1t = p.w1t; b.z1 = z1;
     b.g.dh_in = dh; b.g.z2 = z2; b.g.norm_core = p.nc; b.g.norm_gate = p.ng;
@@ -789,7 +787,7 @@ static void refine_bwd(Run& R, const mb_refine_params& p, const mb_row_graph& g,
     float* dx = p.smoothed_edge ? R.ar.bottom(rows * 128) : dh;
     const int32_t* const idx = g.is_atom ? g.emap : nullptr;  // (atom graph: the mean over the two directions is a gather * 0.5)
     const float scale = g.is_atom ? 0.5f : 1.f;
-    if (R.go() && nodes > 0 && rows > 0 && few_rows_fit((g.n_nodes + 31) / 32 * 32 + g.n_rows, 1)) {
+    if (R.go() && nodes > 0 && rows > 0 && few_ffn_bwd_fits(g.n_nodes, g.n_rows)) {
       const mb_mlp_bwd a = ffn_grad(p.nffn, g.n_nodes, d_node_out, nullptr, 1.f, it.zn, dagg);
       const mb_mlp_bwd b = ffn_grad(p.effn, g.n_rows, d_edge_out, idx, scale, it.ze, dx);
       const mb_mlp_bwd* const both[2] = {&a, &b};

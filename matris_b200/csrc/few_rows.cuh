@@ -3,14 +3,16 @@
 // What bounds a small call is the chain of one tile, not a rate: k_mlp and k_linear walk 128-row tiles through seven or eight
 // hand-overs between warp roles, a thread works through a whole row, and all but a few multiprocessors idle (back to back, one tile
 // of the gated forward 17.7 us, of its backward 13, a dense layer 6 - 11; here 7.2, 6.5 and 3.3 - 6.2; an evaluation of 4 atoms
-// 5.1 -> 3.4 ms).  Here a block takes R = 16 or 32 rows and the product is TRANSPOSED, features x rows:
+// 5.1 -> 3.4 ms).  Here a block takes R = 16, 32 or 64 rows and the product is TRANSPOSED, features x
+// rows:
 //
 //   D^T [128 features, R rows] = W [128, K] x X^T       M = 128 weight rows (A, by TMA), N = rows (B, K-major, converted by threads)
 //
 // so that the matrix instruction's M is always full, however few the rows, and its time shrinks with them.  With thread = feature
 // (tensor-memory lane) and registers = rows, bias and weights of an epilogue are one register, a row of an addend table, gate,
 // residual or output is one 128-byte access of a warp straight from or to global memory (no staging, no hand-over), and the hidden
-// layer goes back to shared memory as the MN-major B operand of layer 2.  A feature's rows are spread over 16 warps.
+// layer goes back to shared memory as the MN-major B operand of layer 2.  A feature's rows are spread over 16 warps.  A table's row
+// numbers are asked for first of all, in one register of a lane each, and shuffled.
 //
 // The products of a K step are accumulated in the order of the persistent kernels, so that a row's sums do not depend on how many rows
 // a call has.  (w_hi x [x_hi ; x_lo] as one instruction of N = 2 R, the small terms in columns of their own, would save a third of the
@@ -48,16 +50,15 @@ constexpr uint32_t FW_SLOT_BYTES = 2 * TC_TILE_BYTES, FW_MAX_SLOTS = 6;
 constexpr uint32_t FW_GROUP = 2048;
 constexpr uint32_t FW_ROW_CORE = 144, FW_ROW_GROUP = 16 * FW_ROW_CORE;  // ROW_BWD, whose warps write along K: 16 bytes between cores
 
-// shared memory: weight ring | X segments | hidden layer | sums of squares | barriers
+// shared memory: weight ring | X segments | hidden layer | sums of squares | barriers.  A branch's hidden layer takes the place of an X
+// segment whose products are done by then (GATED_FWD: the gate's, whose segments serve the core as well).
 __host__ __device__ constexpr uint32_t few_operand_bytes(int r) { return (uint32_t)r * 512u; }  // hi and lo of R rows x 128 K
 __host__ __device__ constexpr uint32_t few_x_bytes(int mode, int r) { return (uint32_t)(r / 4) * (mode == FEW_ROW_BWD ? FW_ROW_GROUP : FW_GROUP); }
-__host__ __device__ constexpr int few_branches(int mode) {
-  return mode == FEW_GATED_FWD || mode == FEW_GATED_BWD || mode == FEW_ROW_BWD ? 2 : mode == FEW_LINEAR ? 0 : 1;
-}
+__host__ __device__ constexpr int few_hidden(int mode, int n_src) { return mode != FEW_GATED_FWD ? 0 : n_src > 0 ? 1 : 2; }  // of its own
 __host__ __device__ constexpr uint32_t few_tail_bytes(int r) { return (uint32_t)r * 32u + 256u; }
 __host__ __device__ constexpr uint32_t few_columns(int mode, int r) {
   const uint32_t need = (uint32_t)r * (mode == FEW_GATED_FWD ? 4 : mode == FEW_GATED_BWD || mode == FEW_ROW_BWD ? 3 : mode == FEW_LINEAR ? 1 : 2);
-  return need <= 32 ? 32 : need <= 64 ? 64 : 128;
+  return need <= 32 ? 32 : need <= 64 ? 64 : need <= 128 ? 128 : need <= 256 ? 256 : 512;
 }
 
 // no swizzle: LBO = bytes between cores along K, SBO = between groups of 8 rows (both majors)
@@ -121,7 +122,8 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T args, const __grid_const
   constexpr bool LINEAR = MODE == FEW_LINEAR, ROW_BWD = MODE == FEW_ROW_BWD;
   constexpr bool GATED_BWD = MODE == FEW_GATED_BWD || ROW_BWD, GATED = MODE == FEW_GATED_FWD || GATED_BWD;
   constexpr bool FWD = MODE == FEW_GATED_FWD || MODE == FEW_PLAIN_FWD;
-  constexpr int NB = GATED ? 2 : 1, RT = R / 4, JOBS = R / 2;  // rows of a thread; (8 rows x 32 values) pieces of a segment
+  constexpr int NB = GATED ? 2 : 1, RT = R < 32 ? R / 4 : 8, NCH = R < 32 ? 1 : R / 32;  // rows of a thread: NCH times RT
+  constexpr int JOBS = R / 2;                                                           // (8 rows x 32 values) pieces of a segment
   constexpr uint32_t OPERAND = few_operand_bytes(R), LO = (R / 8) * FW_GROUP;  // of the hidden layer
   constexpr uint32_t X_CORE = ROW_BWD ? FW_ROW_CORE : 128, X_GROUP = ROW_BWD ? FW_ROW_GROUP : FW_GROUP;
   constexpr uint32_t X_OPERAND = few_x_bytes(MODE, R), X_LO = X_OPERAND / 2;
@@ -151,8 +153,12 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T args, const __grid_const
   if constexpr (ROW_BWD) two_layers = d.out[0] != nullptr;
   const int n_seg = n_src + n_ext;
 
-  const uint32_t x_sm = sm0 + n_slots * FW_SLOT_BYTES, act_sm = x_sm + n_seg * X_OPERAND, ss_off = act_sm + few_branches(MODE) * OPERAND - sm0;
-  float* const sums = reinterpret_cast<float*>(smem + ss_off);  // [row quarter][value][lane quarter]
+  const uint32_t x_sm = sm0 + n_slots * FW_SLOT_BYTES, own_sm = x_sm + n_seg * X_OPERAND, ss_off = own_sm + few_hidden(MODE, n_src) * OPERAND - sm0;
+  auto hidden_at = [&](uint32_t x, uint32_t own, int br) {  // a branch's hidden layer
+    if constexpr (MODE == FEW_GATED_FWD) return br == 0 ? own : n_src > 0 ? x : own + OPERAND;
+    else return x + br * X_OPERAND;
+  };
+  float* const sums = reinterpret_cast<float*>(smem + ss_off);  // [8 rows x 4][row quarter][value][lane quarter]
   const uint32_t bar0 = sm0 + ss_off + R * 32;
   // w_full[6] w_empty[6] | x_ready[4] (per segment) | act_ready[2] d1_full[2] d2_full[2] | retired | tensor-memory address
   const uint32_t w_full = bar0, w_empty = bar0 + 48, x_ready = bar0 + 96, act_ready = bar0 + 128, d1_full = bar0 + 144,
@@ -193,7 +199,7 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T args, const __grid_const
     uint32_t elected;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
     const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0), sm_u = __shfl_sync(0xffffffffu, sm0, 0);
-    const uint32_t x_u = sm_u + n_slots * FW_SLOT_BYTES, act_u = x_u + n_seg * X_OPERAND;
+    const uint32_t x_u = sm_u + n_slots * FW_SLOT_BYTES, own_u = x_u + n_seg * X_OPERAND;
     const uint64_t w_first = umma_desc(sm_u);
     bool alive = true;
     uint32_t slot = 0, phase = 0;  // of the next piece
@@ -238,7 +244,7 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T args, const __grid_const
       for (int br = 0; br < NB; ++br) {
         wait(act_ready + 8 * br, 0);
         const uint32_t dt = tmem_u + R * (MODE == FEW_GATED_FWD ? 2 + br : NB);
-        const uint64_t ah = few_desc(act_u + br * OPERAND);
+        const uint64_t ah = few_desc(hidden_at(x_u, own_u, br));
 #pragma unroll 1
         for (int kp = 0; kp < 2; ++kp)
           piece(dt, ah + kp * (1024 / 16), LO, 16, IDESC | MN_MAJOR_B, kp == 0 && !(GATED_BWD && (br == 1 || n_ext > 0)));
@@ -274,7 +280,7 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T args, const __grid_const
     drain_copies(w_full, (uint32_t)n_slots, asked);
   } else {
     // ---------------------------------------------------------------- workers
-    const int q = warp & 3, rg = warp >> 2, f = 32 * q + lane, r0 = rg * RT;
+    const int q = warp & 3, rg = warp >> 2, f = 32 * q + lane, r0 = rg * RT;  // first row of chunk 0; chunk c: 32 c further on
     const uint32_t lane_q = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)r0;
     bool alive = true;
     auto wait = [&](uint32_t bar) {
@@ -282,31 +288,43 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T args, const __grid_const
       alive = __all_sync(0xffffffffu, alive);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     };
-    auto row_of = [&](int i) { const int64_t r = row0 + r0 + i; return r < n_rows ? r : n_rows - 1; };  // (past the end: the last row)
-    const int n_own = (int)(n_rows - row0 - r0 < RT ? n_rows - row0 - r0 : RT);                       // rows to be written (may be < 0)
-    auto store = [&](float* p, int64_t ld, const float (&v)[RT]) {
+    auto row_of = [&](int c, int i) { const int64_t r = row0 + 32 * c + r0 + i; return r < n_rows ? r : n_rows - 1; };  // (past the end: the last)
+    auto store = [&](float* p, int64_t ld, int c, const float (&v)[RT]) {
+      const int64_t first = row0 + 32 * c + r0, n = alive ? n_rows - first : 0;
 #pragma unroll
       for (int i = 0; i < RT; ++i)
-        if (i < n_own && alive) p[(row0 + r0 + i) * ld] = v[i];
+        if (i < n) p[(first + i) * ld] = v[i];
     };
     pdl_sync();
-    float side[NB][RT], res[RT];  // what the epilogues add or multiply with
+    float side[NCH][NB][RT], res[RT];  // what the epilogues add or multiply with; the residual's rows of a chunk
     bool has_res = false;
     if constexpr (!LINEAR) has_res = ROW_BWD ? d.res != nullptr && blockIdx.y == 0 : d.out2 != nullptr;
+    auto ask_res = [&](int c) {
+      if constexpr (!LINEAR) {
+#pragma unroll
+        for (int i = 0; i < RT; ++i) res[i] = d.res[row_of(c, i) * d.ld_res + f];
+      }
+    };
     auto ask_side = [&]() {
       if constexpr (!LINEAR && !FWD) {
 #pragma unroll
-        for (int br = 0; br < NB; ++br)
+        for (int c = 0; c < NCH; ++c)
 #pragma unroll
-          for (int i = 0; i < RT; ++i) side[br][i] = d.side[row_of(i) * d.ld_side + 128 * br + f];
+          for (int br = 0; br < NB; ++br)
+#pragma unroll
+            for (int i = 0; i < RT; ++i) side[c][br][i] = d.side[row_of(c, i) * d.ld_side + 128 * br + f];
       }
       if constexpr (!LINEAR) {
-        if (has_res) {
-#pragma unroll
-          for (int i = 0; i < RT; ++i) res[i] = d.res[row_of(i) * d.ld_res + f];
-        }
+        if (has_res && NCH == 1) ask_res(0);
       }
     };
+    int32_t ix[3] = {0, 0, 0};  // row numbers of the addends: lane RT c + i has row i of chunk c
+    if constexpr (MODE == FEW_GATED_FWD) {
+      const int64_t at = row0 + 32 * (lane / RT) + r0 + lane % RT, r = at < n_rows ? at : n_rows - 1;
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+        if (a < d.n_add) ix[a] = d.add[a].idx ? d.add[a].idx[r] : (int32_t)r;
+    }
     if constexpr (ROW_BWD) {
       // -------------------------------------------- X: a row per warp and turn, lane = 4 channels
       ask_side();
@@ -377,32 +395,36 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T args, const __grid_const
     if constexpr (LINEAR) {
       const mb_colblock& cb = d.blk[blockIdx.y];
       const float bias = cb.bias ? cb.bias[f] : 0.f, rw = cb.res && cb.res_w ? cb.res_w[f] : 1.f, sc = cb.out_scale;
-      float g[RT], x[RT], y[RT];
-      if (cb.gate) {
-#pragma unroll
-        for (int i = 0; i < RT; ++i) g[i] = cb.gate[row_of(i) * cb.ld_gate + cb.col_gate + f];
-      }
-      if (cb.res) {
-#pragma unroll
-        for (int i = 0; i < RT; ++i) x[i] = cb.res[row_of(i) * cb.ld_res + cb.col_res + f];
-      }
-      wait(d2_full);
-      few_result(lane_q, y);
-#pragma unroll
-      for (int i = 0; i < RT; ++i) {
-        y[i] += bias;
-        if (cb.gate) y[i] *= silu_grad_fast_f(g[i]);
-        if (cb.out_act) y[i] = silu_fast_f(y[i]);
-        if (cb.res) y[i] = fmaf(rw, x[i], y[i]);
-        y[i] *= sc;
-      }
       float* const out = cb.out + cb.col_out + f;
-      if (cb.mode == MB_OUT_STORE) {
-        store(out, cb.ld_out, y);
-      } else {  // one addition per element at the memory side; every row has one writer
 #pragma unroll
-        for (int i = 0; i < RT; ++i)
-          if (i < n_own && alive) atomicAdd(out + (row0 + r0 + i) * cb.ld_out, y[i]);
+      for (int c = 0; c < NCH; ++c) {
+        float g[RT], x[RT], y[RT];
+        if (cb.gate) {
+#pragma unroll
+          for (int i = 0; i < RT; ++i) g[i] = cb.gate[row_of(c, i) * cb.ld_gate + cb.col_gate + f];
+        }
+        if (cb.res) {
+#pragma unroll
+          for (int i = 0; i < RT; ++i) x[i] = cb.res[row_of(c, i) * cb.ld_res + cb.col_res + f];
+        }
+        if (c == 0) wait(d2_full);
+        few_result(lane_q + 32u * c, y);
+#pragma unroll
+        for (int i = 0; i < RT; ++i) {
+          y[i] += bias;
+          if (cb.gate) y[i] *= silu_grad_fast_f(g[i]);
+          if (cb.out_act) y[i] = silu_fast_f(y[i]);
+          if (cb.res) y[i] = fmaf(rw, x[i], y[i]);
+          y[i] *= sc;
+        }
+        if (cb.mode == MB_OUT_STORE) {
+          store(out, cb.ld_out, c, y);
+        } else {  // one addition per element at the memory side; every row has one writer
+          const int64_t first = row0 + 32 * c + r0, n = alive ? n_rows - first : 0;
+#pragma unroll
+          for (int i = 0; i < RT; ++i)
+            if (i < n) atomicAdd(out + (first + i) * cb.ld_out, y[i]);
+        }
       }
     } else {
       // -------------------------------------------- what the epilogues add, on its way while the first products are formed
@@ -411,115 +433,134 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T args, const __grid_const
         for (int br = 0; br < NB; ++br) {
           const float b = d.b1 ? d.b1[128 * br + f] : 0.f;
 #pragma unroll
-          for (int i = 0; i < RT; ++i) side[br][i] = b;
+          for (int c = 0; c < NCH; ++c)
+#pragma unroll
+            for (int i = 0; i < RT; ++i) side[c][br][i] = b;
         }
-        if constexpr (GATED)
-          for (int a = 0; a < d.n_add; ++a) {
-            const mb_add& t = d.add[a];
-            int64_t at[RT];
+        if constexpr (GATED) {
 #pragma unroll
-            for (int i = 0; i < RT; ++i) at[i] = (t.idx ? (int64_t)t.idx[row_of(i)] : row_of(i)) * t.ld + f;
-            float v[NB][RT];
+          for (int a = 0; a < 3; ++a)
+            if (a < d.n_add) {
+              const mb_add& t = d.add[a];
+              float v[NCH][NB][RT];
 #pragma unroll
-            for (int br = 0; br < NB; ++br)
+              for (int c = 0; c < NCH; ++c)
 #pragma unroll
-              for (int i = 0; i < RT; ++i) v[br][i] = t.ptr[at[i] + 128 * br];
+                for (int i = 0; i < RT; ++i) {
+                  const float* const p = t.ptr + (int64_t)__shfl_sync(0xffffffffu, ix[a], RT * c + i) * t.ld + f;
 #pragma unroll
-            for (int br = 0; br < NB; ++br)
+                  for (int br = 0; br < NB; ++br) v[c][br][i] = p[128 * br];
+                }
 #pragma unroll
-              for (int i = 0; i < RT; ++i) side[br][i] += v[br][i];
-          }
+              for (int c = 0; c < NCH; ++c)
+#pragma unroll
+                for (int br = 0; br < NB; ++br)
+#pragma unroll
+                  for (int i = 0; i < RT; ++i) side[c][br][i] += v[c][br][i];
+            }
+        }
       }
       if constexpr (!ROW_BWD) ask_side();
       // -------------------------------------------- layer 1 out, hidden layer back as the operand of layer 2
 #pragma unroll
       for (int br = 0; br < NB; ++br) {
-        float x[RT];
-        if (!FWD || n_src > 0) {
-          wait(d1_full + 8 * br);
-          few_result(lane_q + (uint32_t)R * br, x);
-        } else {
+        float x[NCH][RT];
+        if (!FWD || n_src > 0) wait(d1_full + 8 * br);
 #pragma unroll
-          for (int i = 0; i < RT; ++i) x[i] = 0.f;
-        }
-        float a[RT];
-#pragma unroll
-        for (int i = 0; i < RT; ++i) {
-          if constexpr (FWD) {
-            x[i] += side[br][i];
-            a[i] = silu_fast_f(x[i]);
+        for (int c = 0; c < NCH; ++c) {
+          if (!FWD || n_src > 0) {
+            few_result(lane_q + (uint32_t)R * br + 32u * c, x[c]);
           } else {
-            x[i] *= (MODE == FEW_PLAIN_BWD ? d.scale : 1.f) * silu_grad_fast_f(side[br][i]);
-            a[i] = x[i];
-          }
-        }
-        if (!two_layers) {
-          store(d.z1 + 128 * br + f, d.ld_z1, x);
-          continue;
-        }
-        uint32_t hi[RT / 2], lo[RT / 2];
-        split_bf16(a, hi, lo);
-        const uint32_t at = act_sm + br * OPERAND + (r0 >> 3) * FW_GROUP + f * 16u + (r0 & 7) * 2u;
-        if constexpr (RT == 8) {
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" :: "r"(at), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]) : "memory");
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" :: "r"(at + LO), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]) : "memory");
-        } else {
-          asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(at), "r"(hi[0]), "r"(hi[1]) : "memory");
-          asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(at + LO), "r"(lo[0]), "r"(lo[1]) : "memory");
-        }
-        to_async_proxy();
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(act_ready + 8 * br);
-        if (d.z1) store(d.z1 + 128 * br + f, d.ld_z1, x);
-      }
-      // -------------------------------------------- layer 2 out
-      float y[RT];
-      if (two_layers) {
-        if constexpr (MODE == FEW_GATED_FWD) {
-          float z[2][RT], v[2 * RT];
 #pragma unroll
-          for (int br = 0; br < 2; ++br) {
-            const float b = d.b2 ? d.b2[128 * br + f] : 0.f;
-            wait(d2_full + 8 * br);
-            few_result(lane_q + (uint32_t)R * (2 + br), z[br]);
-#pragma unroll
-            for (int i = 0; i < RT; ++i) {
-              z[br][i] += b;
-              v[RT * br + i] = z[br][i];
-            }
-            if (d.z2) store(d.z2 + 128 * br + f, d.ld_z2, z[br]);
+            for (int i = 0; i < RT; ++i) x[c][i] = 0.f;
           }
-          constexpr int PER = 32 / (2 * RT);  // lanes that end with the same sum
-          const float s = few_sums_of_squares(v, lane);
-          if (lane % PER == 0) sums[(rg * 2 * RT + lane / PER) * 4 + q] = s;
-          asm volatile("bar.sync %0, 128;" :: "r"(1 + rg) : "memory");  // the four lane quarters of these rows
-          const float nc = d.norm_core[f], ng = d.norm_gate[f];
+          float a[RT];
 #pragma unroll
           for (int i = 0; i < RT; ++i) {
-            const float4 c = *reinterpret_cast<const float4*>(sums + (rg * 2 * RT + i) * 4);
-            const float4 g = *reinterpret_cast<const float4*>(sums + (rg * 2 * RT + RT + i) * 4);
-            const float rc = rsqrtf(((c.x + c.y) + (c.z + c.w)) * (1.0f / 128.0f) + ML_RMS_EPS);
-            const float rr = rsqrtf(((g.x + g.y) + (g.z + g.w)) * (1.0f / 128.0f) + ML_RMS_EPS);
-            y[i] = gated_value(z[0][i] * (rc * nc), z[1][i] * (rr * ng));
+            if constexpr (FWD) {
+              x[c][i] += side[c][br][i];
+              a[i] = silu_fast_f(x[c][i]);
+            } else {
+              x[c][i] *= (MODE == FEW_PLAIN_BWD ? d.scale : 1.f) * silu_grad_fast_f(side[c][br][i]);
+              a[i] = x[c][i];
+            }
           }
-        } else {
-          const float b = FWD && d.b2 ? d.b2[f] : 0.f;
-          wait(d2_full);
-          few_result(lane_q + (uint32_t)R * NB, y);
+          if (!two_layers) continue;
+          uint32_t hi[RT / 2], lo[RT / 2];
+          split_bf16(a, hi, lo);
+          const int n = 32 * c + r0;
+          const uint32_t at = hidden_at(x_sm, own_sm, br) + (n >> 3) * FW_GROUP + f * 16u + (n & 7) * 2u;
+          if constexpr (RT == 8) {
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" :: "r"(at), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]) : "memory");
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" :: "r"(at + LO), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]) : "memory");
+          } else {
+            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(at), "r"(hi[0]), "r"(hi[1]) : "memory");
+            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(at + LO), "r"(lo[0]), "r"(lo[1]) : "memory");
+          }
+        }
+        if (two_layers) {
+          to_async_proxy();
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(act_ready + 8 * br);
+        }
+        if (d.z1) {
 #pragma unroll
-          for (int i = 0; i < RT; ++i) y[i] += b;
+          for (int c = 0; c < NCH; ++c) store(d.z1 + 128 * br + f, d.ld_z1, c, x[c]);
         }
-        if constexpr (!ROW_BWD) {
-          if (d.h) store(d.h + f, d.ld_h, y);
-        }
-        if (has_res) {
-          const float rw = d.res_w ? d.res_w[f] : 1.f;
+      }
+      // -------------------------------------------- layer 2 out
+      if (two_layers) {
 #pragma unroll
-          for (int i = 0; i < RT; ++i) y[i] = fmaf(rw, res[i], y[i]);
-          if constexpr (!ROW_BWD) store(d.out2 + f, d.ld_out2, y);
+        for (int c = 0; c < NCH; ++c) {
+          float y[RT];
+          if (has_res && NCH > 1) ask_res(c);
+          if constexpr (MODE == FEW_GATED_FWD) {
+            float z[2][RT], v[2 * RT];
+#pragma unroll
+            for (int br = 0; br < 2; ++br) {
+              const float b = d.b2 ? d.b2[128 * br + f] : 0.f;
+              if (c == 0) wait(d2_full + 8 * br);
+              few_result(lane_q + (uint32_t)R * (2 + br) + 32u * c, z[br]);
+#pragma unroll
+              for (int i = 0; i < RT; ++i) {
+                z[br][i] += b;
+                v[RT * br + i] = z[br][i];
+              }
+              if (d.z2) store(d.z2 + 128 * br + f, d.ld_z2, c, z[br]);
+            }
+            constexpr int PER = 32 / (2 * RT);  // lanes that end with the same sum
+            const float s = few_sums_of_squares(v, lane);
+            float* const mine = sums + (c * 4 + rg) * 8 * RT;
+            if (lane % PER == 0) mine[(lane / PER) * 4 + q] = s;
+            asm volatile("bar.sync %0, 128;" :: "r"(1 + rg) : "memory");  // the four lane quarters of these rows
+            const float nc = d.norm_core[f], ng = d.norm_gate[f];
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
+              const float4 sc = *reinterpret_cast<const float4*>(mine + 4 * i);
+              const float4 sg = *reinterpret_cast<const float4*>(mine + 4 * (RT + i));
+              const float rc = rsqrtf(((sc.x + sc.y) + (sc.z + sc.w)) * (1.0f / 128.0f) + ML_RMS_EPS);
+              const float rr = rsqrtf(((sg.x + sg.y) + (sg.z + sg.w)) * (1.0f / 128.0f) + ML_RMS_EPS);
+              y[i] = gated_value(z[0][i] * (rc * nc), z[1][i] * (rr * ng));
+            }
+          } else {
+            const float b = FWD && d.b2 ? d.b2[f] : 0.f;
+            if (c == 0) wait(d2_full);
+            few_result(lane_q + (uint32_t)R * NB + 32u * c, y);
+#pragma unroll
+            for (int i = 0; i < RT; ++i) y[i] += b;
+          }
+          if constexpr (!ROW_BWD) {
+            if (d.h) store(d.h + f, d.ld_h, c, y);
+          }
+          if (has_res) {
+            const float rw = d.res_w ? d.res_w[f] : 1.f;
+#pragma unroll
+            for (int i = 0; i < RT; ++i) y[i] = fmaf(rw, res[i], y[i]);
+            if constexpr (!ROW_BWD) store(d.out2 + f, d.ld_out2, c, y);
+          }
+          if constexpr (ROW_BWD) store(d.out[blockIdx.y] + f, 128, c, y);
         }
-        if constexpr (ROW_BWD) store(d.out[blockIdx.y] + f, 128, y);
       }
     }
   }

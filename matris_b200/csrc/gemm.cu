@@ -672,12 +672,12 @@ static int row_map(const float* p, int64_t ld, int cols, int64_t rows, CUtensorM
   return weight_map(p, ld, cols, out, (int)rows, false, 32);
 }
 
-// Per-device set-up of the tensor-core kernels: the dynamic shared-memory attribute belongs to the (function, device)
-// pair and the persistent grids are sized by the device's SM count.  One slot per device ordinal; two host threads
-// that race on a device's first call write the same values.
+// rows of a block at the most: dense layers and the products that form their operand themselves gain nothing from 64
+static constexpr int few_most(int mode) { return mode == FEW_LINEAR || mode == FEW_ROW_BWD ? 32 : 64; }
 template <int MODE> static int few_config_mode() {
   MB_CUDA_CHECK(cudaFuncSetAttribute(k_few<MODE, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, FW_SMEM_LIMIT));
   MB_CUDA_CHECK(cudaFuncSetAttribute(k_few<MODE, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, FW_SMEM_LIMIT));
+  if constexpr (few_most(MODE) >= 64) MB_CUDA_CHECK(cudaFuncSetAttribute(k_few<MODE, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, FW_SMEM_LIMIT));
   return MB_OK;
 }
 static int few_config() {
@@ -690,19 +690,32 @@ static int few_config() {
   return rc;
 }
 // R of k_few for a launch, 0: the persistent kernels.  A block of k_few takes one tile, so the line lies where its tiles no longer run
-// side by side: 16 rows a block while a multiprocessor gets one at most, then 32 while all are resident (dense layers with K = 128:
-// two on a multiprocessor).  Back to back, weights in L2, us (persistent kernel / here): gated forward with two addends, 2300 rows 17.8 /
-// 7.5, 4700 rows 17.9 / 9.3; its backward 13.1 / 6.9 and 13.3 / 7.7; dense 128 -> 128 6.1 / 3.4 and 6.1 / 4.2; dense 128 -> 512, 1180
-// rows 6.2 / 4.1, 2300 rows 6.7 / 5.7; dense 512 -> 128 10.9 / 6.6 and 11 / 7.2.
-static int few_choice(int mode, int64_t n_rows, int n_src, int n_blocks, int n_sm) {
-  const int64_t t16 = (n_rows + 15) / 16 * n_blocks, t32 = (n_rows + 31) / 32 * n_blocks;
-  if (t16 <= n_sm) return 16;
-  return t32 <= (mode == FEW_LINEAR && n_src == 1 ? 2 : 1) * (int64_t)n_sm ? 32 : 0;
+// side by side: 16 rows a block while a multiprocessor gets one at most, then 32 (dense layers with K = 128: two blocks on a
+// multiprocessor), the MLPs then 64.  Back to back, weights in L2, us (persistent kernel / here): gated forward with two addends, 2300
+// rows 17.8 / 7.5, 4700 rows 17.9 / 9.2, 9400 rows 18.2 / 14.3; its backward 13.1 / 6.9, 13.3 / 7.8, 13.6 / 11.4; feed-forward block, 4700
+// rows 10.4 / 5.7, 9400 rows 10.7 / 8.2; dense 128 -> 128 6.1 / 3.4 and 6.1 / 4.1; dense 128 -> 512, 1180 rows 6.2 / 4.1, 2300 rows
+// 6.7 / 5.7; dense 512 -> 128 10.9 / 6.6 and 11 / 7.2.  With 96 rows (14,200) the gated forward spills: 18.9 / 25.
+static uint32_t few_rest(int mode, int r, int n_src, int n_ext) {  // shared memory beside the weight ring
+  return (n_src + n_ext) * few_x_bytes(mode, r) + few_hidden(mode, n_src) * few_operand_bytes(r) + few_tail_bytes(r);
+}
+// tiles(r): blocks of r rows the launch takes
+template <typename F> static int few_choose(int mode, int n_src, int n_ext, F tiles) {
+  int n_sm = 0;
+  if (g_gemm_mode != 0 || sm_count(&n_sm) != MB_OK) return 0;
+  for (int r = 16; r <= few_most(mode); r *= 2) {
+    const bool two = mode == FEW_LINEAR && n_src == 1 && r == 32;  // blocks on a multiprocessor
+    if (FW_SMEM_LIMIT < few_rest(mode, r, n_src, n_ext) + 2 * FW_SLOT_BYTES) return 0;
+    if (tiles(r) <= (two ? 2 : 1) * (int64_t)n_sm) return r;
+  }
+  return 0;
+}
+static int few_choice(int mode, int64_t n_rows, int n_src, int n_ext, int n_blocks) {
+  return few_choose(mode, n_src, n_ext, [&](int r) { return (n_rows + r - 1) / r * n_blocks; });
 }
 // n_seg: A segments of a block, n_kp: weight slots it uses
-template <int MODE> static void few_launch(const typename FewArgs<MODE>::T& args, const FewMaps& maps, int64_t n_rows, int r, int n_seg,
-                                           int n_kp, int n_blocks, cudaStream_t st) {
-  const uint32_t rest = n_seg * few_x_bytes(MODE, r) + few_branches(MODE) * few_operand_bytes(r) + few_tail_bytes(r);
+template <int MODE> static void few_launch(const typename FewArgs<MODE>::T& args, const FewMaps& maps, int64_t n_rows, int r, int n_src,
+                                           int n_ext, int n_kp, int n_blocks, cudaStream_t st) {
+  const uint32_t rest = few_rest(MODE, r, n_src, n_ext);
   uint32_t slots = (FW_SMEM_LIMIT - rest) / FW_SLOT_BYTES;
   if (slots > FW_MAX_SLOTS) slots = FW_MAX_SLOTS;
   if (slots > (uint32_t)n_kp) slots = (uint32_t)n_kp;
@@ -710,9 +723,13 @@ template <int MODE> static void few_launch(const typename FewArgs<MODE>::T& args
   const size_t smem = slots * FW_SLOT_BYTES + rest;
   const int early = weights_settled ? 1 : 0;
   if (r == 16) launch(k_few<MODE, 16>, grid, FW_THREADS, smem, st, args, maps, (int)slots, early);
-  else launch(k_few<MODE, 32>, grid, FW_THREADS, smem, st, args, maps, (int)slots, early);
+  else if (r == 32) launch(k_few<MODE, 32>, grid, FW_THREADS, smem, st, args, maps, (int)slots, early);
+  else if constexpr (few_most(MODE) >= 64) launch(k_few<MODE, 64>, grid, FW_THREADS, smem, st, args, maps, (int)slots, early);
 }
 
+// Per-device set-up of the tensor-core kernels: the dynamic shared-memory attribute belongs to the (function, device)
+// pair and the persistent grids are sized by the device's SM count.  One slot per device ordinal; two host threads
+// that race on a device's first call write the same values.
 struct DeviceConfig { bool ready; int n_sm; };
 static DeviceConfig g_device_config[64];
 
@@ -743,9 +760,8 @@ static int device_config(int* n_sm) {
   return MB_OK;
 }
 
-bool few_rows_fit(int64_t n_rows, int n_out) {
-  int n_sm = 0;
-  return g_gemm_mode == 0 && sm_count(&n_sm) == MB_OK && (n_rows + 31) / 32 * n_out <= n_sm;
+bool few_row_bwd_fits(int64_t n_rows, int n_out, bool logits) {
+  return few_choice(FEW_ROW_BWD, n_rows, 2, logits ? 2 : 0, n_out) != 0;
 }
 static int split_map(const mb_weight& w, int k, int rows, CUtensorMap* maps) {
   if (!w.W_hi16 || !w.W_lo16 || !aligned16(w.W_hi16) || !aligned16(w.W_lo16) || (w.ldw & 7)) return MB_ERR_INVALID;
@@ -769,23 +785,24 @@ int few_row_bwd(const RowBwd& a, cudaStream_t st) {
   k.g = a.g;
   for (int j = 0; j < 3; ++j) k.out[j] = j < a.n_out ? a.out[j] : nullptr;
   k.zero = a.zero; k.n_zero = a.n_zero;
-  const int blocks = a.n_out > 1 ? a.n_out : 1, r = (a.n_rows + 15) / 16 * blocks <= n_sm ? 16 : 32;
-  few_launch<FEW_ROW_BWD>(k, maps, k.n_rows, r, 2 + k.n_ext, 4 + 2 * k.n_ext + (a.n_out > 0 ? 4 : 0), blocks, st);
+  const int blocks = a.n_out > 1 ? a.n_out : 1, r = few_choice(FEW_ROW_BWD, a.n_rows, 2, k.n_ext, blocks);
+  if (r == 0) return MB_ERR_INVALID;
+  few_launch<FEW_ROW_BWD>(k, maps, k.n_rows, r, 2, k.n_ext, 4 + 2 * k.n_ext + (a.n_out > 0 ? 4 : 0), blocks, st);
   MB_LAUNCH_CHECK("k_few");
   return MB_OK;
 }
-// Blocks of 32 rows that run side by side: two on a multiprocessor where only dense layers with K = 128 are among them.
-bool few_linears_fit(const mb_gemm_desc* const* g, int n) {
-  int n_sm = 0, per_sm = 2, blocks = 0;
-  if (g_gemm_mode != 0 || sm_count(&n_sm) != MB_OK) return false;
-  int64_t tiles = 0;
+static int few_linears_choice(const mb_gemm_desc* const* g, int n) {
+  int n_src = 1, blocks = 0;
   for (int i = 0; i < n; ++i)
-    for (int j = 0; j < g[i]->n_blocks; ++j, ++blocks) {
-      tiles += (g[i]->n_rows + 31) / 32;
-      if (g[i]->blk[j].n_src > 1) per_sm = 1;
-    }
-  return blocks <= FW_MAX_BLOCKS && tiles <= per_sm * (int64_t)n_sm;
+    for (int j = 0; j < g[i]->n_blocks; ++j, ++blocks) n_src = g[i]->blk[j].n_src > n_src ? g[i]->blk[j].n_src : n_src;
+  if (blocks > FW_MAX_BLOCKS) return 0;
+  return few_choose(FEW_LINEAR, n_src, 0, [&](int r) {
+    int64_t tiles = 0;
+    for (int i = 0; i < n; ++i) tiles += (g[i]->n_rows + r - 1) / r * g[i]->n_blocks;
+    return tiles;
+  });
 }
+bool few_linears_fit(const mb_gemm_desc* const* g, int n) { return few_linears_choice(g, n) != 0; }
 int few_linears(const mb_gemm_desc* const* g, int n, const int32_t* pair, cudaStream_t st) {
   int n_sm = 0, rc = device_config(&n_sm);
   if (rc) return rc;
@@ -793,7 +810,9 @@ int few_linears(const mb_gemm_desc* const* g, int n, const int32_t* pair, cudaSt
   FewLinear f;
   f.pair = pair;
   int n_src = 1, k = 0;
-  int64_t most = 0, tiles = 0;
+  int64_t most = 0;
+  const int r = few_linears_choice(g, n);
+  if (r == 0) return MB_ERR_INVALID;
   for (int i = 0; i < n; ++i)
     for (int j = 0; j < g[i]->n_blocks; ++j, ++k) {
       const mb_colblock& b = f.blk[k] = g[i]->blk[j];
@@ -802,19 +821,24 @@ int few_linears(const mb_gemm_desc* const* g, int n, const int32_t* pair, cudaSt
       f.n_rows[k] = g[i]->n_rows;
       n_src = b.n_src > n_src ? b.n_src : n_src;
       most = g[i]->n_rows > most ? g[i]->n_rows : most;
-      tiles += (g[i]->n_rows + 15) / 16;
     }
   if (most == 0) return MB_OK;
-  few_launch<FEW_LINEAR>(f, maps, most, tiles <= n_sm ? 16 : 32, n_src, 2 * n_src, k, st);
+  few_launch<FEW_LINEAR>(f, maps, most, r, n_src, 0, 2 * n_src, k, st);
   MB_LAUNCH_CHECK("k_few");
   return MB_OK;
 }
+static int few_ffn_bwd_choice(int64_t a, int64_t b) {
+  return few_choose(FEW_PLAIN_BWD, 1, 0, [&](int r) { return (a + r - 1) / r + (b + r - 1) / r; });
+}
+bool few_ffn_bwd_fits(int64_t n_rows_a, int64_t n_rows_b) { return few_ffn_bwd_choice(n_rows_a, n_rows_b) != 0; }
 int few_ffn_bwd(const mb_mlp_bwd* const* g, cudaStream_t st) {
   int n_sm = 0, rc = device_config(&n_sm);
   if (rc) return rc;
+  const int r = few_ffn_bwd_choice(g[0]->n_rows, g[1]->n_rows);
+  if (r == 0) return MB_ERR_INVALID;
   FewMaps maps;
   FewPlainBwd f = {};
-  int64_t most = 0, tiles = 0;
+  int64_t most = 0;
   for (int i = 0; i < 2; ++i) {
     const mb_mlp_bwd& m = *g[i];
     if ((rc = split_map(m.W2t, 128, 128, maps.w[2 * i])) || (rc = split_map(m.W1t, 128, 128, maps.w[2 * i + 1]))) return rc;
@@ -822,9 +846,8 @@ int few_ffn_bwd(const mb_mlp_bwd* const* g, cudaStream_t st) {
     a.n_rows = m.n_rows; a.n_src = 1; a.src[0] = m.dy;
     a.side = m.z1; a.ld_side = m.ld_z1; a.scale = m.scale; a.h = m.dx; a.ld_h = m.ld_dx;
     most = m.n_rows > most ? m.n_rows : most;
-    tiles += (m.n_rows + 15) / 16;
   }
-  few_launch<FEW_PLAIN_BWD>(f, maps, most, tiles <= n_sm ? 16 : 32, 1, 4, 2, st);
+  few_launch<FEW_PLAIN_BWD>(f, maps, most, r, 1, 0, 4, 2, st);
   MB_LAUNCH_CHECK("k_few");
   return MB_OK;
 }
@@ -1055,7 +1078,7 @@ extern "C" int mb_gemm(const mb_gemm_desc* desc, void* stream_) {
       if (direct) {
         int n_src = 1;
         for (int j = 0; j < desc->n_blocks; ++j) n_src = desc->blk[j].n_src > n_src ? desc->blk[j].n_src : n_src;
-        if (const int r = mb::few_choice(mb::FEW_LINEAR, desc->n_rows, n_src, desc->n_blocks, n_sm)) {
+        if (const int r = mb::few_choice(mb::FEW_LINEAR, desc->n_rows, n_src, 0, desc->n_blocks)) {
           mb::FewMaps fm;
           mb::FewLinear fl;
           fl.pair = nullptr;
@@ -1064,7 +1087,7 @@ extern "C" int mb_gemm(const mb_gemm_desc* desc, void* stream_) {
             fl.n_rows[j] = desc->n_rows;
             for (int part = 0; part < 2; ++part) fm.w[j][part] = maps.m[j][part];
           }
-          mb::few_launch<mb::FEW_LINEAR>(fl, fm, desc->n_rows, r, n_src, 2 * n_src, desc->n_blocks, (cudaStream_t)stream_);
+          mb::few_launch<mb::FEW_LINEAR>(fl, fm, desc->n_rows, r, n_src, 0, 2 * n_src, desc->n_blocks, (cudaStream_t)stream_);
           MB_LAUNCH_CHECK("k_few");
           return MB_OK;
         }
@@ -1230,14 +1253,14 @@ extern "C" int mb_gated_mlp_fwd(const mb_gated_mlp* g, void* stream_) {
   a.res = g->res; a.res_w = g->res_w; a.ld_res = g->ld_res; a.out2 = g->out2; a.ld_out2 = g->ld_out2;
   const int width = plain ? 128 : 256;
   if (plain) a.z2 = nullptr;
-  if (const int r = mb::few_choice(plain ? mb::FEW_PLAIN_FWD : mb::FEW_GATED_FWD, g->n_rows, 1, 1, n_sm)) {
+  if (const int r = mb::few_choice(plain ? mb::FEW_PLAIN_FWD : mb::FEW_GATED_FWD, g->n_rows, g->n_src, 0, 1)) {
     mb::FewMaps fm;
     for (int part = 0; part < 2; ++part) {
       if (g->n_src > 0) fm.w[0][part] = maps.w1[part];
       fm.w[1][part] = maps.w2[part];
     }
-    if (plain) mb::few_launch<mb::FEW_PLAIN_FWD>(a, fm, a.n_rows, r, g->n_src, 2 * g->n_src + 2, 1, (cudaStream_t)stream_);
-    else mb::few_launch<mb::FEW_GATED_FWD>(a, fm, a.n_rows, r, g->n_src, 4 * g->n_src + 4, 1, (cudaStream_t)stream_);
+    if (plain) mb::few_launch<mb::FEW_PLAIN_FWD>(a, fm, a.n_rows, r, g->n_src, 0, 2 * g->n_src + 2, 1, (cudaStream_t)stream_);
+    else mb::few_launch<mb::FEW_GATED_FWD>(a, fm, a.n_rows, r, g->n_src, 0, 4 * g->n_src + 4, 1, (cudaStream_t)stream_);
     MB_LAUNCH_CHECK("k_few");
     return MB_OK;
   }
@@ -1347,15 +1370,15 @@ extern "C" int mb_mlp_bwd_data(const mb_mlp_bwd* g, void* stream_) {
     a.h = g->dx; a.ld_h = g->ld_dx;
   }
   const int width = plain ? 128 : 256;
-  if (const int r = mb::few_choice(plain ? mb::FEW_PLAIN_BWD : mb::FEW_GATED_BWD, g->n_rows, 1, 1, n_sm)) {
+  if (const int r = mb::few_choice(plain ? mb::FEW_PLAIN_BWD : mb::FEW_GATED_BWD, g->n_rows, plain ? 1 : 2, a.n_ext, 1)) {
     mb::FewMaps fm;
     for (int part = 0; part < 2; ++part) {
       fm.w[0][part] = maps.w1[part];
       fm.w[1][part] = maps.w2[part];
       if (g->n_ext > 0) fm.w[2][part] = maps.w3[part];
     }
-    if (plain) mb::few_launch<mb::FEW_PLAIN_BWD>({{a, {}}}, fm, a.n_rows, r, 1, 4, 1, (cudaStream_t)stream_);
-    else mb::few_launch<mb::FEW_GATED_BWD>(a, fm, a.n_rows, r, 2 + a.n_ext, 8 + 2 * a.n_ext, 1, (cudaStream_t)stream_);
+    if (plain) mb::few_launch<mb::FEW_PLAIN_BWD>({{a, {}}}, fm, a.n_rows, r, 1, 0, 4, 1, (cudaStream_t)stream_);
+    else mb::few_launch<mb::FEW_GATED_BWD>(a, fm, a.n_rows, r, 2, a.n_ext, 8 + 2 * a.n_ext, 1, (cudaStream_t)stream_);
     MB_LAUNCH_CHECK("k_few");
     return MB_OK;
   }

@@ -19,15 +19,15 @@ def ops():
 
 
 def sizes():
-    """One row, edges of the 16- and 32-row tiles, the last launch of each kind and the first of the next."""
+    """One row, edges of the tiles, the last launch of each tile height and the first of the next (the last one: persistent kernels)."""
     n = torch.cuda.get_device_properties(0).multi_processor_count if torch.cuda.is_available() else 1
-    return [1, 15, 17, 33, 16 * n, 16 * n + 1, 32 * n - 1, 32 * n + 1]
+    return [1, 15, 17, 33, 16 * n, 16 * n + 1, 32 * n - 1, 32 * n + 1, 64 * n, 64 * n + 1]
 
 
 BIG = 40_000
 
 
-@pytest.mark.parametrize("at", range(8))
+@pytest.mark.parametrize("at", range(10))
 @pytest.mark.parametrize("k,n,mode", [(128, 128, "plain"), (512, 128, "res"), (128, 512, "gate"), (256, 256, "add")])
 def test_dense(ops, k, n, mode, at):
     rows = sizes()[at]
@@ -58,7 +58,7 @@ def test_dense(ops, k, n, mode, at):
     assert torch.equal(got, run(BIG)[:rows])
 
 
-@pytest.mark.parametrize("at", range(8))
+@pytest.mark.parametrize("at", range(10))
 def test_mlps(ops, at):
     rows = sizes()[at]
     n_nodes = 61
