@@ -113,9 +113,12 @@ struct RowBwd {
 };
 bool few_row_bwd_fits(int64_t n_rows, int n_out, bool logits);  // whether it takes so many rows
 int few_row_bwd(const RowBwd& a, cudaStream_t stream);
-// n independent mb_gemm problems of few rows as one launch; with `pair` an operand row is the sum of rows i and pair[i], i = idx[r]
+// n independent mb_gemm problems of few rows as one launch
 bool few_linears_fit(const mb_gemm_desc* const* g, int n);
-int few_linears(const mb_gemm_desc* const* g, int n, const int32_t* pair, cudaStream_t stream);
+int few_linears(const mb_gemm_desc* const* g, int n, cudaStream_t stream);
+// mb_gemm with an operand row that is the sum of rows i and pair[i], i = idx[r]
+bool pair_linear_fits(const mb_gemm_desc* g);
+int pair_linear(const mb_gemm_desc* g, const int32_t* pair, cudaStream_t stream);
 bool few_ffn_bwd_fits(int64_t n_rows_a, int64_t n_rows_b);
 int few_ffn_bwd(const mb_mlp_bwd* const* g, cudaStream_t stream);  // two plain data gradients (dx only, no residual) of few rows
 // y[i] = x[i] w[i]^T, [n_rows, 7] x [7, 128], for up to MANY_LINEARS problems as one launch

@@ -298,8 +298,7 @@ struct Gemm {
       flops += 2.0 * d.n_rows * 128 * 128 * d.blk[j].n_src;
       bytes += 4.0 * d.n_rows * 128 * ((d.blk[j].gate != nullptr) + (d.blk[j].res != nullptr));
     }
-    const mb_gemm_desc* const one[1] = {&d};
-    R.op("mb_gemm", [&] { return pair ? few_linears(one, 1, pair, R.st) : mb_gemm(&d, R.st); }, flops, bytes, d.n_rows, 128 * d.blk[0].n_src, 128 * d.n_blocks);
+    R.op("mb_gemm", [&] { return pair ? pair_linear(&d, pair, R.st) : mb_gemm(&d, R.st); }, flops, bytes, d.n_rows, 128 * d.blk[0].n_src, 128 * d.n_blocks);
   }
 };
 
@@ -316,7 +315,7 @@ static bool together(Run& R, std::initializer_list<Gemm*> all) {
     bytes += 4.0 * g->d.n_rows * 128 * (g->d.blk[0].n_src + g->d.n_blocks);
   }
   if (!R.go() || n < 2 || !few_linears_fit(d, n)) return false;
-  R.op("mb_gemm", [&] { return few_linears(d, n, nullptr, R.st); }, flops, bytes, d[0]->n_rows, 128 * d[0]->blk[0].n_src, 128 * d[0]->n_blocks);
+  R.op("mb_gemm", [&] { return few_linears(d, n, R.st); }, flops, bytes, d[0]->n_rows, 128 * d[0]->blk[0].n_src, 128 * d[0]->n_blocks);
   return true;
 }
 
@@ -515,11 +514,10 @@ static void edge_update_bwd(Run& R, const mb_update& p, const mb_row_graph& g, c
     Gemm e(g.n_edge_rows);
     mb_colblock& b = e.block({}, dlogits ? *w_log : p.wet, 0, d_edge, 128);
     b.res = edge_res; b.res_w = edge_w; b.ld_res = 128;
-    b.n_src = dlogits ? 4 : 2;  // the sums of dz1 (core, gate) and of dlogits, formed on the way where the rows are few
+    b.n_src = dlogits ? 4 : 2;  // the sums of dz1 (core, gate) and of dlogits, formed on the way
     for (int j = 0; j < b.n_src; ++j) b.src[j] = src(j < 2 ? dz1 : dlogits, g.u2d, 128 * (j & 1), 256);
-    const mb_gemm_desc* const one[1] = {&e.d};
-    const bool pairs = R.go() && few_linears_fit(one, 1);
-    if (!pairs) {
+    const bool pairs = pair_linear_fits(&e.d);
+    if (!pairs) {  // contraction modes other than the default, weights that are not aligned to 32 bytes
       MB_OP(mb_pair_sum, (int32_t)g.n_edge_rows, g.u2d, g.rev, dz1, dlogits, pair);
       for (int j = 0; j < b.n_src; ++j) b.src[j] = src(pair, nullptr, 128 * j, ld);
     }

@@ -742,7 +742,8 @@ static int device_config(int* n_sm) {
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_gemm_ps<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PS_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_gemm_ps<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PS_SMEM_BYTES));
-    MB_CUDA_CHECK(cudaFuncSetAttribute(k_linear, cudaFuncAttributeMaxDynamicSharedMemorySize, LN_SMEM_BYTES));
+    MB_CUDA_CHECK(cudaFuncSetAttribute(k_linear<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, LN_SMEM_BYTES));
+    MB_CUDA_CHECK(cudaFuncSetAttribute(k_linear<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, LN_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_GATED_FWD, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_GATED_FWD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
     MB_CUDA_CHECK(cudaFuncSetAttribute(k_mlp<MLP_GATED_FWD, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ML_SMEM_BYTES));
@@ -803,12 +804,12 @@ static int few_linears_choice(const mb_gemm_desc* const* g, int n) {
   });
 }
 bool few_linears_fit(const mb_gemm_desc* const* g, int n) { return few_linears_choice(g, n) != 0; }
-int few_linears(const mb_gemm_desc* const* g, int n, const int32_t* pair, cudaStream_t st) {
+int few_linears(const mb_gemm_desc* const* g, int n, cudaStream_t st) {
   int n_sm = 0, rc = device_config(&n_sm);
   if (rc) return rc;
   FewMaps maps;
   FewLinear f;
-  f.pair = pair;
+  f.pair = nullptr;
   int n_src = 1, k = 0;
   int64_t most = 0;
   const int r = few_linears_choice(g, n);
@@ -1012,9 +1013,32 @@ extern "C" int mb_bench_mma_rate(int kind, int iters, float* elapsed_ms, int* n_
   return MB_OK;
 }
 
-extern "C" int mb_gemm(const mb_gemm_desc* desc, void* stream_) {
+namespace mb {
+// The persistent kernels' epilogue uses 32-byte accesses.  Operands aligned to 16 bytes only (a caller of the C ABI that passes views
+// at odd column offsets; the Python host side never does) take the one-tile kernel.
+static bool wide_operands(const mb_gemm_desc* desc) {
+  auto ok32 = [](const void* p, int64_t ld, int col) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0 && (ld & 7) == 0 && (col & 7) == 0; };
+  for (int j = 0; j < desc->n_blocks; ++j) {
+    const mb_colblock& cb = desc->blk[j];
+    if (!ok32(cb.out, cb.ld_out, cb.col_out) || (cb.gate && !ok32(cb.gate, cb.ld_gate, cb.col_gate)) ||
+        (cb.res && !ok32(cb.res, cb.ld_res, cb.col_res)) || (cb.bias && !ok32(cb.bias, 0, 0)) || (cb.res_w && !ok32(cb.res_w, 0, 0)))
+      return false;
+  }
+  return true;
+}
+bool pair_linear_fits(const mb_gemm_desc* g) {
+  const mb_colblock& b = g->blk[0];
+  bool ok = g_gemm_mode == 0 && g->n_blocks == 1 && !b.out_idx && b.mode != MB_OUT_ATOMIC && g->n_rows <= 0x7fffff00LL && wide_operands(g);
+  for (int s = 0; s < b.n_src; ++s) ok = ok && b.src[s].idx && b.src[s].idx == b.src[0].idx && !b.src[s].act;
+  return ok;
+}
+}  // namespace mb
+
+// pair: see pair_linear in common.cuh
+static int gemm_run(const mb_gemm_desc* desc, const int32_t* pair, void* stream_) {
   int rc = gemm_validate(desc);
   if (rc) return rc;
+  if (pair && !mb::pair_linear_fits(desc)) return MB_ERR_INVALID;
   if (desc->n_rows == 0) return MB_OK;
   const long long gx = (desc->n_rows + 127) / 128;
   if (gx * desc->n_blocks > 0x7fffffffLL) return MB_ERR_OVERFLOW;
@@ -1025,18 +1049,7 @@ extern "C" int mb_gemm(const mb_gemm_desc* desc, void* stream_) {
     int n_sm = 0;
     rc = mb::device_config(&n_sm);
     if (rc) return rc;
-    // The persistent kernels' epilogue uses 32-byte accesses.  Operands aligned to 16 bytes only (a caller of the C
-    // ABI that passes views at odd column offsets; the Python host side never does) take the one-tile kernel.
-    bool wide_ok = true;
-    for (int j = 0; j < desc->n_blocks; ++j) {
-      const mb_colblock& cb = desc->blk[j];
-      auto ok32 = [](const void* p, int64_t ld, int col) {
-        return (reinterpret_cast<uintptr_t>(p) & 31) == 0 && (ld & 7) == 0 && (col & 7) == 0;
-      };
-      wide_ok = wide_ok && ok32(cb.out, cb.ld_out, cb.col_out) && (!cb.gate || ok32(cb.gate, cb.ld_gate, cb.col_gate)) &&
-                (!cb.res || ok32(cb.res, cb.ld_res, cb.col_res)) && (!cb.bias || ok32(cb.bias, 0, 0)) &&
-                (!cb.res_w || ok32(cb.res_w, 0, 0));
-    }
+    const bool wide_ok = mb::wide_operands(desc);
     const bool persistent = (mb::g_gemm_mode == 0 || mb::g_gemm_mode == 3) && wide_ok;
     const bool bf16 = persistent && mb::g_gemm_mode == 0;
     mb::TcMaps maps;
@@ -1081,7 +1094,7 @@ extern "C" int mb_gemm(const mb_gemm_desc* desc, void* stream_) {
         if (const int r = mb::few_choice(mb::FEW_LINEAR, desc->n_rows, n_src, 0, desc->n_blocks)) {
           mb::FewMaps fm;
           mb::FewLinear fl;
-          fl.pair = nullptr;
+          fl.pair = pair;
           for (int j = 0; j < desc->n_blocks; ++j) {
             fl.blk[j] = desc->blk[j];
             fl.n_rows[j] = desc->n_rows;
@@ -1111,8 +1124,8 @@ extern "C" int mb_gemm(const mb_gemm_desc* desc, void* stream_) {
         }
         const int split = n_tiles <= n_sm ? 1 : 0;
         const long long items = split ? n_tiles : gx;
-        mb::launch(mb::k_linear, (unsigned)(items < n_sm ? items : n_sm), mb::LN_THREADS, mb::LN_SMEM_BYTES,
-                   (cudaStream_t)stream_, *desc, lm, same_a ? 1 : 0, split);
+        mb::launch(pair ? mb::k_linear<true> : mb::k_linear<false>, (unsigned)(items < n_sm ? items : n_sm), mb::LN_THREADS,
+                   mb::LN_SMEM_BYTES, (cudaStream_t)stream_, *desc, lm, same_a ? 1 : 0, split, pair);
         MB_LAUNCH_CHECK("k_linear");
         return MB_OK;
       }
@@ -1128,6 +1141,12 @@ extern "C" int mb_gemm(const mb_gemm_desc* desc, void* stream_) {
   MB_LAUNCH_CHECK("k_gemm");
   return MB_OK;
 }
+
+extern "C" int mb_gemm(const mb_gemm_desc* desc, void* stream_) { return gemm_run(desc, nullptr, stream_); }
+
+namespace mb {
+int pair_linear(const mb_gemm_desc* g, const int32_t* pair, cudaStream_t st) { return gemm_run(g, pair, st); }
+}  // namespace mb
 
 // The same result as the fused kernel from the separate kernels (the GEMM modes other than 0): two mb_gemm launches and the row-wise gate kernel, with z1 / z2 as scratch.
 static int gated_mlp_composed(const mb_gated_mlp* g, void* stream_) {

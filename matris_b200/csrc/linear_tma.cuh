@@ -14,6 +14,11 @@
 //
 // HBM bounds the large launches: 573,894 rows take 0.171 ms for 128 -> 256 (k_gemm_ps 0.214), 0.25 with a gate, 0.36 for
 // 512 -> 128, 0.275 for 128 -> 512.  One tile takes 12 us (15), with K = 512 19 us: the chain of its 16 chunks.
+//
+// PAIR sums the two directed rows of a bond on the way in, instead of a pass that writes the sums and one that reads them back: with
+// K = 512, 117,048 bonds 98 + 87 -> 115 us (92 at the copy rate), with K = 256 49 + 49 -> 62.  The rows are gathered by cp.async
+// into two patches of a producer warp, the next chunk's while this one is converted.  (Through registers 153 and 82 us: beside this
+// kernel's shared memory the L1 keeps 28 KB, which is less than the lines the loads of eight warps wait for.)
 
 struct alignas(64) LinMaps {
   CUtensorMap w[4][2];                       // weights of a column block: hi, lo
@@ -28,8 +33,15 @@ constexpr int LN_BAR_OFF = LN_CONST_OFF + 1024 * 4;
 constexpr int LN_SMEM_BYTES = LN_BAR_OFF + 640;
 static_assert(LN_SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
 
+__device__ __forceinline__ void copy16(uint32_t to, const float* from) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(to), "l"(from) : "memory");
+}
+// PAIR: an operand row is the sum of rows i and pair[i], i = idx[r], one idx for all segments
+template <bool PAIR>
 __global__ void __launch_bounds__(LN_THREADS, 1)
-k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps maps, const int shared_a, const int split) {
+k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps maps, const int shared_a, const int split,
+         const int32_t* const pair) {
+  constexpr uint32_t SLOTS = PAIR ? 1 : 2;  // gate / residual patches of an epilogue warp; PAIR: the other one holds its producer's second rows
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + LN_BAR_OFF);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + LN_BAR_OFF + 632);
@@ -176,8 +188,8 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
 #pragma unroll
           for (int what = 0; what < 2; ++what) {
             if (!(what == 0 ? (const void*)cb.gate : (const void*)cb.res) || !alive) continue;
-            const uint32_t sl = n & 1;
-            if (n >= 2) alive = mbar_wait(side_empty + 8 * (2 * lane + sl), ((n >> 1) - 1) & 1);
+            const uint32_t sl = n % SLOTS;
+            if (n >= SLOTS) alive = mbar_wait(side_empty + 8 * (2 * lane + sl), (n / SLOTS - 1) & 1);
             if (!alive) continue;
             const uint32_t bar = side_full + 8 * (2 * lane + sl);
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(ML_PATCH) : "memory");
@@ -186,7 +198,10 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
           }
         }
       }
-      drain_copies(side_full + 16 * lane, 2, n);
+      if constexpr (PAIR)
+        drain_copies(side_full + 16 * lane, 1, n);
+      else
+        drain_copies(side_full + 16 * lane, 2, n);
     }
     __syncwarp();
   } else if (warp >= ML_EPI_WARP0) {
@@ -210,12 +225,12 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     };
     auto with_patch = [&](auto f) {  // f(j, the row's 16-byte piece j) for the next side patch, which then goes back
-      const uint32_t patch = side0 + (side_n & 1) * ML_PATCH;
-      wait(my_full + 8 * (side_n & 1), side_n >> 1);
+      const uint32_t patch = side0 + side_n % SLOTS * ML_PATCH;
+      wait(my_full + 8 * (side_n % SLOTS), side_n / SLOTS);
 #pragma unroll
       for (int j = 0; j < 8; ++j) f(j, lds4(patch + lane * 128 + ((j ^ (lane & 7)) << 4)));
       __syncwarp();
-      if (lane == 0) mbar_arrive(my_empty + 8 * (side_n & 1));
+      if (lane == 0) mbar_arrive(my_empty + 8 * (side_n % SLOTS));
       ++side_n;
     };
     for (int b = grp; b < n_tiles * nb; b += 2) {
@@ -294,8 +309,35 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
         load_patch(&maps.src[shared_a ? s : j0 + s], patch, my_conv, 32 * (parity + 2 * k), tile_row(t));
       }
     };
-    if (segment(0).idx == nullptr) request(0, 0, 0, false);
+    // PAIR: rows first and second of this lane's row in the current and the next tile, row numbers asked for two tiles ahead
+    const uint32_t patch2 = sm0 + ML_SIDE_OFF + (2 * pw + 1) * ML_PATCH;
+    int32_t first = 0, second = 0, first1 = 0, second1 = 0, first2 = 0;
+    auto pair_row = [&](int t) {
+      const int64_t r = t < n_tiles ? (int64_t)tile_row(t) + lane : 0;
+      return d.blk[0].src[0].idx[r < n_rows ? r : n_rows - 1];
+    };
+    auto ask_pair = [&](int s, int k, int32_t r1, int32_t r2) {  // chunk k of segment s of both rows
+      const mb_src& sr = segment(s);
+      const float* const base = sr.ptr + sr.col + lc * 4 + 32 * (parity + 2 * k);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t at = ((i & 1) ? put_odd : put_even) + 512u * i;
+        copy16(patch + at, base + (int64_t)__shfl_sync(0xffffffffu, r1, lr + 4 * i) * sr.ld);
+        copy16(patch2 + at, base + (int64_t)__shfl_sync(0xffffffffu, r2, lr + 4 * i) * sr.ld);
+      }
+    };
+    if constexpr (PAIR) {
+      first = pair_row(0);
+      first1 = pair_row(1);
+      second = pair[first];
+      ask_pair(0, 0, first, second);
+    }
+    if (!PAIR && segment(0).idx == nullptr) request(0, 0, 0, false);
     for (int t = 0; t < n_tiles; ++t) {
+      if constexpr (PAIR) {
+        second1 = pair[first1];
+        first2 = pair_row(t + 2);
+      }
       const int64_t row0 = tile_row(t);
       auto row_of = [&](int i) { const int64_t r = row0 + lr + 4 * i; return r < n_rows ? r : n_rows - 1; };
       for (int s = 0; s < n_seg; ++s) {
@@ -304,7 +346,10 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
         const bool act = sr.act != 0;
 #pragma unroll 1
         for (int k = 0; k < 2; ++k, g += 2) {
-          if (!idx) {
+          if constexpr (PAIR) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncwarp();
+          } else if (!idx) {
             if (alive) alive = mbar_wait(my_conv, conv_n & 1);
             alive = __all_sync(0xffffffffu, alive);
             ++conv_n;
@@ -322,6 +367,16 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
           for (int i = 0; i < 8; ++i) {
             const float4 v = lds4(patch + lane * 128 + ((i ^ (lane & 7)) << 4));
             x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
+          }
+          const int s2 = k == 0 ? s : (s + 1 < n_seg ? s + 1 : 0), t2 = k == 1 && s + 1 == n_seg ? t + 1 : t;  // the chunk after this one
+          if constexpr (PAIR) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float4 v = lds4(patch2 + lane * 128 + ((i ^ (lane & 7)) << 4));
+              x[4 * i] += v.x; x[4 * i + 1] += v.y; x[4 * i + 2] += v.z; x[4 * i + 3] += v.w;
+            }
+            __syncwarp();  // every lane has read: the next chunk's copies may be asked for
+            if (t2 < n_tiles) ask_pair(s2, k ^ 1, t2 == t ? first : first1, t2 == t ? second : second1);
           }
           if (act) {
 #pragma unroll
@@ -347,14 +402,14 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
           // Every lane has used the values it read from the patch (the stores above depend on them): only now may the copy of the
           // next chunk overwrite it.  Issued right after the reads it could overtake them.
           __syncwarp();
-          const int s2 = k == 0 ? s : (s + 1 < n_seg ? s + 1 : 0), t2 = k == 1 && s + 1 == n_seg ? t + 1 : t;
-          if (t2 < n_tiles && segment(s2).idx == nullptr) request(t2, s2, k ^ 1, idx != nullptr);
+          if (!PAIR && t2 < n_tiles && segment(s2).idx == nullptr) request(t2, s2, k ^ 1, idx != nullptr);
           asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
           if (lane == 0) mbar_arrive(a_ready + 8 * ab);
         }
       }
+      if constexpr (PAIR) { first = first1; second = second1; first1 = first2; }
     }
     if (!alive) drain_copies(my_conv, 1, conv_asked);  // (otherwise it has used all that it asked for)
   }

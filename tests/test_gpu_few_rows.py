@@ -116,3 +116,18 @@ def test_small_structures_equal_their_batch(options):
         report(f"alone vs in a batch {i}: F", one["f"][0], many["f"][i], 2e-6)
         report(f"alone vs in a batch {i}: S", one["s"][0] / GPA, many["s"][i] / GPA, 2e-7)
         report(f"alone vs in a batch {i}: M", one["m"][0], many["m"][i], 2e-6)
+
+
+@pytest.mark.parametrize("count", [61, 125])
+def test_sums_of_a_bonds_two_rows_as_operand(count):
+    """A bond's gradient contracts the sums of its two directed rows.  156 bonds a structure: 75 row tiles, the last of 44 rows, one
+    for each column block a multiprocessor; and 153, more than one for some.  Alone, a structure takes the few-row kernel."""
+    from matris_b200 import MatRIS, workloads
+    from matris_b200.weights import random_checkpoint
+    from conftest import GPA
+    c = workloads.cu_fcc((1, 1, 1), sigma=0.05)
+    model = MatRIS.from_dict(random_checkpoint(dict(num_layers=2, reference_energy="mpa"), seed=1, jitter=0.1)).to("cuda")
+    one, many = model.predict([c], "efs"), model.predict([c] * count, "efs")
+    for i in range(count):  # tolerances as above: the same expressions, float32 sums of order one in another order
+        report(f"bond sums {count}/{i}: F", one["f"][0], many["f"][i], 2e-6)
+        report(f"bond sums {count}/{i}: S", one["s"][0] / GPA, many["s"][i] / GPA, 2e-7)
