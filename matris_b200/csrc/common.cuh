@@ -87,6 +87,64 @@ __device__ __forceinline__ float silu_grad_fast_f(float x) {
   return s * fmaf(x, 1.0f - s, 1.0f);
 }
 
+// Two float32 values at a time: one instruction where the scalar forms take two, each half rounded as the scalar form rounds it.  The
+// warps of the contraction kernels' prologues and epilogues wait for instruction slots as much as for anything else (k_mlp: 13 k
+// a scheduler for a tile of 30 k cycles, a third of them float32 additions and products).
+struct f2 { unsigned long long v; };
+__device__ __forceinline__ f2 two(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void apart(f2 x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v)); }
+__device__ __forceinline__ f2 operator+(f2 a, f2 b) {
+  asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a.v) : "l"(b.v));
+  return a;
+}
+__device__ __forceinline__ f2 operator*(f2 a, f2 b) {
+  asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(a.v) : "l"(b.v));
+  return a;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(a.v) : "l"(b.v), "l"(c.v));
+  return a;
+}
+__device__ __forceinline__ f2 less(f2 a, f2 b) { return fma2(b, two(-1.f, -1.f), a); }  // a - b
+__device__ __forceinline__ f2 low(const float4& v) { return two(v.x, v.y); }
+__device__ __forceinline__ f2 high(const float4& v) { return two(v.z, v.w); }
+__device__ __forceinline__ f2 sigmoid_fast_2(f2 x) {
+  float e0, e1;
+  apart(x * two(-1.442695041f, -1.442695041f), e0, e1);
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(e0));
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(e1));
+  apart(two(1.f, 1.f) + two(e0, e1), e0, e1);
+  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(e0));
+  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(e1));
+  return two(e0, e1);
+}
+__device__ __forceinline__ f2 silu_fast_2(f2 x) { return x * sigmoid_fast_2(x); }
+__device__ __forceinline__ f2 silu_grad_fast_2(f2 x) {
+  const f2 s = sigmoid_fast_2(x), one = two(1.f, 1.f);
+  return s * fma2(x, less(one, s), one);
+}
+// x[0..3] += v, *= SiLU'(v), = v w + x, = SiLU(x)
+__device__ __forceinline__ void add4_to(float* x, const float4& v) {
+  apart(two(x[0], x[1]) + low(v), x[0], x[1]);
+  apart(two(x[2], x[3]) + high(v), x[2], x[3]);
+}
+__device__ __forceinline__ void silu_grad4_to(float* x, const float4& v) {
+  apart(two(x[0], x[1]) * silu_grad_fast_2(low(v)), x[0], x[1]);
+  apart(two(x[2], x[3]) * silu_grad_fast_2(high(v)), x[2], x[3]);
+}
+__device__ __forceinline__ void fma4_to(float* x, const float4& v, const float4& w) {
+  apart(fma2(low(w), low(v), two(x[0], x[1])), x[0], x[1]);
+  apart(fma2(high(w), high(v), two(x[2], x[3])), x[2], x[3]);
+}
+template <int N> __device__ __forceinline__ void silu_fast_all(const float* x, float (&y)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; i += 2) apart(silu_fast_2(two(x[i], x[i + 1])), y[i], y[i + 1]);
+}
+
 // What the gradient of a row ahead of a gated MLP's tail consists of (row_math.cuh has the expressions)
 struct RowGrad {
   int32_t kind;        // 0: dh_in, 1: attention rows, 2: smoothed rows

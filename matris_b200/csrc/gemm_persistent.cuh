@@ -70,8 +70,8 @@ template <int H> __device__ __forceinline__ void split_bf16(const float (&x)[2 *
 #pragma unroll
   for (int i = 0; i < H; ++i) {
     hi[i] = pack_bf16x2(x[2 * i], x[2 * i + 1]);
-    const float r0 = x[2 * i] - __uint_as_float(hi[i] << 16);
-    const float r1 = x[2 * i + 1] - __uint_as_float(hi[i] & 0xFFFF0000u);
+    float r0, r1;
+    apart(less(two(x[2 * i], x[2 * i + 1]), two(__uint_as_float(hi[i] << 16), __uint_as_float(hi[i] & 0xFFFF0000u))), r0, r1);
     lo[i] = pack_bf16x2(r0, r1);
   }
 }

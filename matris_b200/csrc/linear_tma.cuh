@@ -252,27 +252,24 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const float4 v = bias[i];
-          y[4 * i] += v.x; y[4 * i + 1] += v.y; y[4 * i + 2] += v.z; y[4 * i + 3] += v.w;
+          add4_to(y + 4 * i, v);
         }
         if (has_gate)
           with_patch([&](int i, const float4& v) {
-            y[4 * i] *= silu_grad_fast_f(v.x); y[4 * i + 1] *= silu_grad_fast_f(v.y);
-            y[4 * i + 2] *= silu_grad_fast_f(v.z); y[4 * i + 3] *= silu_grad_fast_f(v.w);
+            silu_grad4_to(y + 4 * i, v);
           });
         if (act) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) y[i] = silu_fast_f(y[i]);
+          silu_fast_all(y, y);
         }
         if (has_res) {
           const float4* const rw = reinterpret_cast<const float4*>(cst + 512 + 128 * j + 32 * c);
           with_patch([&](int i, const float4& v) {
             const float4 w = rw[i];
-            y[4 * i] = fmaf(w.x, v.x, y[4 * i]); y[4 * i + 1] = fmaf(w.y, v.y, y[4 * i + 1]);
-            y[4 * i + 2] = fmaf(w.z, v.z, y[4 * i + 2]); y[4 * i + 3] = fmaf(w.w, v.w, y[4 * i + 3]);
+            fma4_to(y + 4 * i, v, w);
           });
         }
 #pragma unroll
-        for (int i = 0; i < 32; ++i) y[i] *= sc;
+        for (int i = 0; i < 32; i += 2) apart(two(y[i], y[i + 1]) * two(sc, sc), y[i], y[i + 1]);
         if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the previous copy has left the patch
         __syncwarp();
         patch_put(stage, lane, y);
@@ -373,7 +370,7 @@ k_linear(const __grid_constant__ mb_gemm_desc d, const __grid_constant__ LinMaps
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const float4 v = lds4(patch2 + lane * 128 + ((i ^ (lane & 7)) << 4));
-              x[4 * i] += v.x; x[4 * i + 1] += v.y; x[4 * i + 2] += v.z; x[4 * i + 3] += v.w;
+              add4_to(x + 4 * i, v);
             }
             __syncwarp();  // every lane has read: the next chunk's copies may be asked for
             if (t2 < n_tiles) ask_pair(s2, k ^ 1, t2 == t ? first : first1, t2 == t ? second : second1);

@@ -34,7 +34,10 @@
 // Measured behind an L2 flush (bench_gemm.py; addend tables of a fifth of the rows), 573,894 rows with z1 and z2 kept: two addends
 // and a residual 0.50 ms, three addends 0.58 (nothing kept: 0.42), no contraction and three addends 0.48, K = 384 gathered with a
 // residual 0.63; GATED_BWD with a residual 0.42, with E too 0.59; FFN forward 0.23, backward 0.18.  One tile alone takes 28 us
-// forward, 21 us backward: the chain of its stages.
+// forward, 21 us backward: the chain of its stages.  With the epilogues' arithmetic two values at a time (f2, common.cuh), 523,000 rows:
+// three addends 0.497 -> 0.483 (nothing kept 0.382 -> 0.364), no contraction 0.439 -> 0.433, FFN forward 0.208 -> 0.202, backward 0.169 -> 0.156.
+// (The addends' own sums that way: 0.523.)  Of the cycles 44 % issue an instruction, the load / store data pipe is busy in 44 %, the
+// tensor pipe in 20 %: 4.5 warps a scheduler that wait for their own chains.
 //
 // Warps: 0 MMA, 1 TMA (weights, 16 KB tiles of 64 K values, five slots), 2-9 producers, 10-17 epilogue (two groups of four; the
 // group's branch or tile parity, the warp's lane quarter).  Every mbarrier wait is bounded; on expiry the status word is set, the
@@ -124,18 +127,35 @@ __device__ __forceinline__ float gated_value(float a, float b) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((1.0f + ea) * (1.0f + eb)));
   return a * r;
 }
+__device__ __forceinline__ f2 gated_value(f2 a, f2 b) {
+  const f2 c = two(-1.442695041f, -1.442695041f), one = two(1.f, 1.f);
+  float a0, a1, b0, b1;
+  apart(a * c, a0, a1);
+  apart(b * c, b0, b1);
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(a0));
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(a1));
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(b0));
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(b1));
+  apart((one + two(a0, a1)) * (one + two(b0, b1)), a0, a1);
+  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(a0));
+  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(a1));
+  return a * two(a0, a1);
+}
 
 // Sum of squares of 32 values of a row, halves added to halves: the order in which k_few adds them across its lanes, so that a row's
 // norm does not depend on which kernel a launch of its size takes.
 __device__ __forceinline__ float sum_of_squares(const float (&y)[32]) {
   float v[16];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = fmaf(y[i + 16], y[i + 16], __fmul_rn(y[i], y[i]));
+  for (int i = 0; i < 16; i += 2) {
+    const f2 lower = two(y[i], y[i + 1]), upper = two(y[i + 16], y[i + 17]);
+    apart(fma2(upper, upper, lower * lower), v[i], v[i + 1]);
+  }
 #pragma unroll
-  for (int n = 8; n > 0; n >>= 1)
+  for (int n = 8; n > 1; n >>= 1)
 #pragma unroll
-    for (int i = 0; i < n; ++i) v[i] += v[i + n];
-  return v[0];
+    for (int i = 0; i < n; i += 2) apart(two(v[i], v[i + 1]) + two(v[i + n], v[i + n + 1]), v[i], v[i + 1]);
+  return v[0] + v[1];
 }
 
 // N_ADD: GATED_FWD's number of addends (a launch without any keeps the registers of their gather)
@@ -416,8 +436,7 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const float4 x = lds4(patch + lane * 128 + ((j ^ (lane & 7)) << 4)), w = rws[j];
-          v[4 * j] = fmaf(w.x, x.x, v[4 * j]); v[4 * j + 1] = fmaf(w.y, x.y, v[4 * j + 1]);
-          v[4 * j + 2] = fmaf(w.z, x.z, v[4 * j + 2]); v[4 * j + 3] = fmaf(w.w, x.w, v[4 * j + 3]);
+          fma4_to(v + 4 * j, x, w);
         }
         __syncwarp();
         if ((has_side || !EPI_RES) && lane == 0) mbar_arrive(my_empty + 8 * (side_n & 1));
@@ -463,22 +482,26 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
               const float4 v = lds4(patch + lane * 128 + ((j ^ (lane & 7)) << 4));
-              x[4 * j] += v.x; x[4 * j + 1] += v.y; x[4 * j + 2] += v.z; x[4 * j + 3] += v.w;
+              add4_to(x + 4 * j, v);
             }
           } else {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
               const float4 v = b1s[8 * c + j];
-              x[4 * j] += v.x; x[4 * j + 1] += v.y; x[4 * j + 2] += v.z; x[4 * j + 3] += v.w;
+              add4_to(x + 4 * j, v);
             }
           }
         } else {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const float4 v = lds4(patch + lane * 128 + ((j ^ (lane & 7)) << 4));
-            const float s = MODE == MLP_PLAIN_BWD ? d.scale : 1.f;
-            x[4 * j] *= s * silu_grad_fast_f(v.x); x[4 * j + 1] *= s * silu_grad_fast_f(v.y);
-            x[4 * j + 2] *= s * silu_grad_fast_f(v.z); x[4 * j + 3] *= s * silu_grad_fast_f(v.w);
+            if constexpr (MODE == MLP_PLAIN_BWD) {
+              const f2 s = two(d.scale, d.scale);
+              apart(two(x[4 * j], x[4 * j + 1]) * (s * silu_grad_fast_2(low(v))), x[4 * j], x[4 * j + 1]);
+              apart(two(x[4 * j + 2], x[4 * j + 3]) * (s * silu_grad_fast_2(high(v))), x[4 * j + 2], x[4 * j + 3]);
+            } else {
+              silu_grad4_to(x + 4 * j, v);
+            }
           }
         }
         if (has_side) {
@@ -491,8 +514,12 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
           float sx[16];
+          if constexpr (FWD) {
+            silu_fast_all(x + 16 * hh, sx);
+          } else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) sx[i] = FWD ? silu_fast_f(x[16 * hh + i]) : x[16 * hh + i];
+            for (int i = 0; i < 16; ++i) sx[i] = x[16 * hh + i];
+          }
           uint32_t hi[8], lo[8];
           split_bf16(sx, hi, lo);
           MB_TMEM_ST8(ta + 8 * hh, hi);
@@ -518,7 +545,7 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const float4 v = b2s[32 * grp + 8 * c + j];
-            y[4 * j] += v.x; y[4 * j + 1] += v.y; y[4 * j + 2] += v.z; y[4 * j + 3] += v.w;
+            add4_to(y + 4 * j, v);
           }
           const float s = sum_of_squares(y);
           if (c < 2) s01 += s;
@@ -530,6 +557,7 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
         asm volatile("bar.sync %0, 64;" :: "r"(1 + q) : "memory");  // the two groups' warps of this lane quarter
         const float rc = rinvs[((t & 1) * 2) * 128 + q * 32 + lane], rg = rinvs[((t & 1) * 2 + 1) * 128 + q * 32 + lane];
         // ---------------------------------------------- pass 2: this group's 64 columns of both branches
+        const f2 rc2 = two(rc, rc), rg2 = two(rg, rg);
         const float4* const nws = reinterpret_cast<const float4*>(cst + 512);
         const uint32_t r3 = (uint32_t)t % 3u;
         const uint32_t core = lane_q + 128u * ((r3 + 2) % 3u) + 64u * grp, gate = lane_q + 128u * r3 + 64u * grp;
@@ -541,8 +569,8 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const float4 bc = b2s[c4 + j], nc = nws[c4 + j];
-            y[4 * j] = (y[4 * j] + bc.x) * (rc * nc.x); y[4 * j + 1] = (y[4 * j + 1] + bc.y) * (rc * nc.y);
-            y[4 * j + 2] = (y[4 * j + 2] + bc.z) * (rc * nc.z); y[4 * j + 3] = (y[4 * j + 3] + bc.w) * (rc * nc.w);
+            apart((two(y[4 * j], y[4 * j + 1]) + low(bc)) * (rc2 * low(nc)), y[4 * j], y[4 * j + 1]);
+            apart((two(y[4 * j + 2], y[4 * j + 3]) + high(bc)) * (rc2 * high(nc)), y[4 * j + 2], y[4 * j + 3]);
           }
           float z[32];
           tmem_get(gate + 32u * j2, z);
@@ -554,10 +582,9 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const float4 bg = b2s[32 + c4 + j], ng = nws[32 + c4 + j];
-            y[4 * j] = gated_value(y[4 * j], (z[4 * j] + bg.x) * (rg * ng.x));
-            y[4 * j + 1] = gated_value(y[4 * j + 1], (z[4 * j + 1] + bg.y) * (rg * ng.y));
-            y[4 * j + 2] = gated_value(y[4 * j + 2], (z[4 * j + 2] + bg.z) * (rg * ng.z));
-            y[4 * j + 3] = gated_value(y[4 * j + 3], (z[4 * j + 3] + bg.w) * (rg * ng.w));
+            apart(gated_value(two(y[4 * j], y[4 * j + 1]), (two(z[4 * j], z[4 * j + 1]) + low(bg)) * (rg2 * low(ng))), y[4 * j], y[4 * j + 1]);
+            apart(gated_value(two(y[4 * j + 2], y[4 * j + 3]), (two(z[4 * j + 2], z[4 * j + 3]) + high(bg)) * (rg2 * high(ng))),
+                  y[4 * j + 2], y[4 * j + 3]);
           }
           finish(y, 64 * grp + 32 * j2, row0);
         }
@@ -581,7 +608,7 @@ k_mlp(const __grid_constant__ MlpArgs d, const __grid_constant__ MlpMaps maps) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
               const float4 v = b2s[j];
-              y[4 * j] += v.x; y[4 * j + 1] += v.y; y[4 * j + 2] += v.z; y[4 * j + 3] += v.w;
+              add4_to(y + 4 * j, v);
             }
           }
           finish(y, col, row0);
