@@ -293,7 +293,7 @@ struct Gemm {
   }
   void run(Run& R, const int32_t* pair = nullptr) {
     if (d.n_rows == 0 || d.n_blocks == 0) return;
-    double flops = 0, bytes = 4.0 * d.n_rows * 128 * (d.blk[0].n_src + d.n_blocks);
+    double flops = 0, bytes = 4.0 * d.n_rows * 128 * ((pair ? 2 : 1) * d.blk[0].n_src + d.n_blocks);
     for (int j = 0; j < d.n_blocks; ++j) {
       flops += 2.0 * d.n_rows * 128 * 128 * d.blk[j].n_src;
       bytes += 4.0 * d.n_rows * 128 * ((d.blk[j].gate != nullptr) + (d.blk[j].res != nullptr));

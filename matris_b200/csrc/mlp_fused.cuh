@@ -32,12 +32,12 @@
 // two epilogue groups, L1(t) -> 2t mod 3, L2(t) -> 2t+1 mod 3, issued L1(t+1) before L2(t).
 //
 // Measured behind an L2 flush (bench_gemm.py; addend tables of a fifth of the rows), 573,894 rows with z1 and z2 kept: two addends
-// and a residual 0.50 ms, three addends 0.58 (nothing kept: 0.42), no contraction and three addends 0.48, K = 384 gathered with a
-// residual 0.63; GATED_BWD with a residual 0.42, with E too 0.59; FFN forward 0.23, backward 0.18.  One tile alone takes 28 us
-// forward, 21 us backward: the chain of its stages.  With the epilogues' arithmetic two values at a time (f2, common.cuh), 523,000 rows:
-// three addends 0.497 -> 0.483 (nothing kept 0.382 -> 0.364), no contraction 0.439 -> 0.433, FFN forward 0.208 -> 0.202, backward 0.169 -> 0.156.
-// (The addends' own sums that way: 0.523.)  Of the cycles 44 % issue an instruction, the load / store data pipe is busy in 44 %, the
-// tensor pipe in 20 %: 4.5 warps a scheduler that wait for their own chains.
+// and a residual 0.49 ms, three addends 0.53 (nothing kept: 0.40), no contraction and three addends 0.48, K = 384 gathered with a
+// residual 0.63; GATED_BWD with a residual 0.42, with E too 0.59; FFN forward 0.22, backward 0.17.  One tile alone takes 28 us
+// forward, 21 us backward: the chain of its stages.  The epilogues' arithmetic goes two values at a time (f2, common.cuh); 523,000
+// rows: three addends 0.497 -> 0.483 (nothing kept 0.382 -> 0.364), no contraction 0.439 -> 0.433, FFN forward 0.208 -> 0.202,
+// backward 0.169 -> 0.156.  (The addends' own sums that way: 0.523.)  With three addends 44 % of the cycles issue an
+// instruction, the load / store data pipe is busy in 44 %, the tensor pipe in 20 %: 4.5 warps a scheduler wait for their own chains.
 //
 // Warps: 0 MMA, 1 TMA (weights, 16 KB tiles of 64 K values, five slots), 2-9 producers, 10-17 epilogue (two groups of four; the
 // group's branch or tile parity, the warp's lane quarter).  Every mbarrier wait is bounded; on expiry the status word is set, the
