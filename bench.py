@@ -476,13 +476,13 @@ def main():
         ach = gemm_flops / (gemm_ms * 1e-3) / 1e12
         ach_gb = gemm_bytes / (gemm_ms * 1e-3) / 1e9
         n_gemm = sum(per[k][0] for k in GEMM_CALLS if k in per)
-        # DRAM traffic per launch: over the 380 contraction launches of an evaluation of 256 random crystals ncu counts
-        # 189.8 GB for 197.7 GB of algorithmic bytes (A rows read + gate / residual rows read + output rows written);
-        # scaled here to the average launch of the step by its algorithmic bytes.
+        # DRAM traffic per launch: on five forms of the contractions at 573,894 rows, one launch at a time, ncu counts 9.2 GB for
+        # 8.8 GB of algorithmic bytes (A rows read + gate / residual rows read + output rows written; addend tables come on
+        # top); scaled here to the average launch of the step by its algorithmic bytes.
         pk = clocks_peak.summary()
         roofline = {"kernel": "k_linear + k_mlp (mb_gemm, mb_gated_mlp_fwd, mb_mlp_bwd_data)", "bound": "tensor", "achieved": ach,
-                    "peak": peak_tf, "unit": "TFLOP/s", "frac": ach / peak_tf, "traffic": 0.96 * gemm_bytes / n_gemm,
-                    "traffic_note": "bytes per average launch, scaled from ncu captures by the algorithmic bytes",
+                    "peak": peak_tf, "unit": "TFLOP/s", "frac": ach / peak_tf, "traffic": 1.04 * gemm_bytes / n_gemm,
+                    "traffic_note": "bytes per average launch, scaled from ncu captures of single launches by the algorithmic bytes",
                     "peak_source": src + " bf16 sustained",
                     "launches": n_gemm, "avg_launch_ms": gemm_ms / n_gemm,
                     "flops_per_step": gemm_flops, "mma_kind": "kind::f16, 3xBF16 operand split",
