@@ -716,9 +716,15 @@ static void attn_bwd(Run& R, const mb_attn_params& p, const mb_row_graph& g, con
 }
 
 // ------------------------------------------------------------------ refinement layer
-// Up to so many bonds (whatever the device: the memory plan depends on it) the envelopes of all layers come from one launch at the
-// start (84 MB for ten layers at the most), and their gradients go on into the radial basis's in the kernel that forms them: 40 launches
-// less.  More bonds fill the device with a launch of their own.
+// Two lines for launches of few bonds, whatever the device (the memory plan depends on them).
+// Up to FEW_ENVELOPES bonds the envelopes of all layers come from one launch at the start (42 MB for ten layers at the most).  An
+// evaluation with / without it, ms: 156 bonds 2.64 / 2.66, 323 bonds 2.53 / 2.56; 470 - 4,200 bonds between 0.5 % slower and 0.8 % faster;
+// 4,400 bonds 5.36 / 5.32, 6,000 bonds 9.81 / 9.68, 7,100 bonds 7.23 / 7.14, 7,600 bonds 8.51 / 8.45 (the side stream that forms an
+// envelope beside the layer's products costs nothing there, and its rows are still in L2 when they are read).
+constexpr int64_t FEW_ENVELOPES = 4096;
+// Up to FEW_BONDS bonds an envelope's gradient goes on into the radial basis's in the kernel that forms it: 1,248 bonds 4.14 -> 4.03 ms,
+// 2,300 bonds 4.21 -> 4.10, 4,800 bonds 6.45 -> 6.39, 7,800 bonds 7.72 -> 7.62, 8,200 bonds 7.69 -> 7.64; 11,200 bonds 9.50 and 9.49, 15,200 bonds
+// 12.21 -> 12.28, 20,300 bonds 15.61 -> 15.78, where the two separate kernels fill the device.
 constexpr int64_t FEW_BONDS = 8192;
 
 struct RefineInter { float *z1, *z2, *h, *env, *zn, *ze; };
@@ -944,7 +950,7 @@ static int evaluate(Run& R, mb_eval& E) {
       if (line) for (int i = 5; i < 7; ++i) r[i] = A.bottom(T * 128);
     }
   std::vector<float*> envs(2 * (size_t)L, nullptr);  // line, atom refinement of each layer
-  if (E.n_bonds <= FEW_BONDS && 2 * L <= MANY_LINEARS) {
+  if (E.n_bonds <= FEW_ENVELOPES && 2 * L <= MANY_LINEARS) {
     ManyLinears many{};
     int n = 0;
     for (int i = 0; i < L; ++i)

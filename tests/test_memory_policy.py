@@ -81,3 +81,12 @@ def test_sub_batches_and_evaluation_plan_with_the_same_need(shape, gigabytes):
         # no more parts than the memory asks for, but for the balancing
         whole = dry_run(10, g.n_atoms, g.n_struct, g.n_edges, g.n_triplets)
         assert fits or len(ranges) <= math.ceil(whole / (0.93 * 0.9 * gigabytes * 1e9)) + 2
+
+
+@pytest.mark.parametrize("bonds,at_once", [(4096, True), (4097, False), (7123, False), (8192, False)])
+def test_envelopes_of_all_layers_are_held_at_once_for_few_bonds_only(bonds, at_once):
+    """One launch for all layers' envelopes pays for small graphs; from 4,400 bonds on it costs about 1 % of an evaluation.  Seen in the
+    memory of an evaluation that keeps nothing, by the number of layers."""
+    few, many = (dry_run(0, 400, 1, 2 * bonds, 2 * bonds, n_layers=n) for n in (10, 20))
+    rows = (many - few - 10 * 512 * 2 * 400) / (10 * 512 * bonds)  # a layer's rows of 512 bytes for a bond and its two triplets
+    assert 10 <= rows < 10.5 if at_once else 8 <= rows < 8.5  # its features and, at once, two envelopes
