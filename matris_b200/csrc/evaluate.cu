@@ -509,8 +509,8 @@ static void edge_update_bwd(Run& R, const mb_update& p, const mb_row_graph& g, c
       node_sums();
       n.run(R);
     });
-    const int ld = dlogits ? 512 : 256;
-    float* pair = R.ar.bottom((size_t)g.n_edge_rows * ld);
+    // the sums, where a launch of its own forms them, in the place of dz2, which has been read by then ([n_rows, 256] = [n_edge_rows, 512])
+    float* const pair = 2 * g.n_edge_rows <= g.n_rows ? dz2 : R.ar.bottom((size_t)g.n_edge_rows * 512);
     Gemm e(g.n_edge_rows);
     mb_colblock& b = e.block({}, dlogits ? *w_log : p.wet, 0, d_edge, 128);
     b.res = edge_res; b.res_w = edge_w; b.ld_res = 128;
@@ -518,6 +518,7 @@ static void edge_update_bwd(Run& R, const mb_update& p, const mb_row_graph& g, c
     for (int j = 0; j < b.n_src; ++j) b.src[j] = src(j < 2 ? dz1 : dlogits, g.u2d, 128 * (j & 1), 256);
     const bool pairs = pair_linear_fits(&e.d);
     if (!pairs) {  // contraction modes other than the default, weights that are not aligned to 32 bytes
+      const int ld = dlogits ? 512 : 256;
       MB_OP(mb_pair_sum, (int32_t)g.n_edge_rows, g.u2d, g.rev, dz1, dlogits, pair);
       for (int j = 0; j < b.n_src; ++j) b.src[j] = src(pair, nullptr, 128 * j, ld);
     }
@@ -812,9 +813,10 @@ static void refine_bwd(Run& R, const mb_refine_params& p, const mb_row_graph& g,
   // smoothed aggregation; with a gated update dh is finished in registers and leaves as dz2
   const int32_t* src_idx = g.is_atom ? nullptr : g.src;
   float* dz2 = gated ? R.ar.bottom(rows * 256) : nullptr;
-  float* denv = R.ar.bottom((size_t)n_bonds * 128);
+  const bool straight = n_bonds <= FEW_BONDS;  // to the radial basis's gradient
+  float* const denv = straight ? nullptr : R.ar.bottom((size_t)n_bonds * 128);
   R.side(1, [&] {
-    if (R.go() && n_bonds <= FEW_BONDS) {
+    if (straight) {
       R.op("mb_seg_smooth_sum_bwd_env", [&] {
         return smooth_env_bwd_rbf((int32_t)n_bonds, g, it.env, it.h, dagg, drow, p.wenv, d_rbf, R.st);
       });

@@ -123,6 +123,23 @@ def _evaluate(ck, crystals, task, keep=None):
     return res, out, model
 
 
+@pytest.mark.parametrize("mode", ["simt", "tcgen05_tile", "tcgen05_tf32"])
+def test_other_contraction_modes_match_reference(mode):
+    """A whole evaluation in the cross-check modes, whose bond gradients are summed by a launch of their own into the buffer of dz2."""
+    from matris_b200 import ops
+    meta, crystals, z = load_golden("random2_L2")
+    ck = random_checkpoint(golden_config(meta), seed=meta["seed"], jitter=meta["jitter"])
+    try:
+        ops.set_gemm_mode(mode)
+        res = _evaluate(ck, crystals, "efs")[0]
+        assert ops.gemm_status() == 0
+    finally:
+        ops.set_gemm_mode("tcgen05")
+    for k, unit in (("e", 1.0), ("f", 1.0), ("s", GPA)):
+        report(f"mode {mode} {k}", res[k] / unit, z[f"ref32_{k}"] / unit, TOL[k])
+    report(f"mode {mode} F vs fp64 (2e-3 relative)", res["f"], z["ref64_f"], 2e-3 * np.abs(z["ref64_f"]).max())
+
+
 @pytest.mark.parametrize("keep", [True, False], ids=["keep", "recompute"])
 @pytest.mark.parametrize("case", GOLDEN_CASES)
 def test_end_to_end_matches_reference(case, keep):

@@ -90,3 +90,29 @@ def test_envelopes_of_all_layers_are_held_at_once_for_few_bonds_only(bonds, at_o
     few, many = (dry_run(0, 400, 1, 2 * bonds, 2 * bonds, n_layers=n) for n in (10, 20))
     rows = (many - few - 10 * 512 * 2 * 400) / (10 * 512 * bonds)  # a layer's rows of 512 bytes for a bond and its two triplets
     assert 10 <= rows < 10.5 if at_once else 8 <= rows < 8.5  # its features and, at once, two envelopes
+
+
+def layer_workspace(kind, line, bonds):
+    """Bytes a sub-block's forward and backward pass takes: the atom graph of ``bonds`` bonds, or a line graph with two triplets each."""
+    rows = 2 * bonds
+    g = _lib.MbRowGraph(n_rows=rows, n_nodes=bonds if line else 10, n_edge_rows=rows if line else bonds, n_ctr=10 if line else 0,
+                        is_atom=int(not line))
+    need, any_ = C.c_size_t(0), 256
+    if kind == "attention":
+        status = _lib.load().mb_attention_layer(C.byref(_lib.MbAttnParams()), C.byref(g), *[any_] * 2, None, None, *[any_] * 4, None,
+                                                C.byref(need), None)
+    else:
+        atom = any_ if line else None
+        status = _lib.load().mb_refine_layer(C.byref(_lib.MbRefineParams()), C.byref(g), *[any_] * 3, atom, None, None, *[any_] * 5, atom,
+                                             None, C.byref(need), None)
+    assert status == 0
+    return need.value
+
+
+@pytest.mark.parametrize("kind,line,bonds,rows", [("attention", False, 8192, 24), ("attention", False, 16384, 24),
+                                                  ("refine", False, 8192, 23), ("refine", False, 16384, 24),
+                                                  ("refine", True, 8192, 29), ("refine", True, 16384, 30)])
+def test_nothing_is_reserved_that_no_kernel_writes(kind, line, bonds, rows):
+    """Rows of 512 bytes a bond.  The sums of a bond's two directed rows have no buffer of their own (they are formed on the way into
+    their contraction, or laid where dz2 was), and the envelopes' gradient none where it goes straight on (8,192 bonds)."""
+    assert rows <= layer_workspace(kind, line, bonds) / (512 * bonds) < rows + 0.1
