@@ -38,7 +38,6 @@ if ROOT not in sys.path:
     sys.path.insert(0, ROOT)
 
 NUM_LAYERS = 10
-GEMM_CALLS = ("mb_gemm", "mb_gated_mlp_fwd", "mb_mlp_bwd_data")  # the tensor-core entry points
 PER_GPU = {"perov512": 512, "random256": 256, "random64": 64}
 
 
@@ -80,6 +79,31 @@ def flops_per_eval(atoms, edges, triplets, layers):
     """Algorithmic GEMM FLOPs of one forward + backward evaluation (no recompute counted):
     2 (fwd+bwd) * 2 (MAC) * L * (360448 T + 327680 Ed + 163840 Eu + 163840 N), Eu = Ed / 2."""
     return 4.0 * layers * (360448.0 * triplets + 327680.0 * edges + 163840.0 * edges / 2 + 163840.0 * atoms)
+
+
+def profile_sums(records):
+    """Sums over the (name, start, end, meta) records of an instrumented step: {name: [launches, ms]} of all calls, {shape: [launches,
+    ms, flops]} and the totals of the contractions, i.e. of the calls that say how many operations they do."""
+    per, shapes = {}, {}
+    gemm = dict(flops=0.0, ms=0.0, bytes=0.0, launches=0, calls=set())
+    for name, a, b, meta in records:
+        ms = a.elapsed_time(b)
+        d = per.setdefault(name, [0, 0.0])
+        d[0] += 1
+        d[1] += ms
+        if meta and meta["flops"] > 0:
+            gemm["flops"] += meta["flops"]
+            gemm["ms"] += ms
+            gemm["bytes"] += meta["bytes"]  # A rows read once + output rows written
+            gemm["launches"] += 1
+            gemm["calls"].add(name)
+            tag = "gated " if meta.get("fused") else ""
+            s = shapes.setdefault(f"{tag}rows={meta['rows']} K={meta['k']} N={meta['n']}", [0, 0.0, 0.0])
+            s[0] += 1
+            s[1] += ms
+            s[2] += meta["flops"]
+    gemm["calls"] = sorted(gemm["calls"])
+    return per, shapes, gemm
 
 
 class ClockSampler:
@@ -444,22 +468,8 @@ def main():
         step_resident(gather=False)  # rank 0 only: no collective in here
         torch.cuda.synchronize()
         prof, _lib.profile = _lib.profile, None
-        per, shapes = {}, {}
-        gemm_flops, gemm_ms, gemm_bytes = 0.0, 0.0, 0.0
-        for name, a, b, meta in prof:
-            ms = a.elapsed_time(b)
-            d = per.setdefault(name, [0, 0.0])
-            d[0] += 1
-            d[1] += ms
-            if name in GEMM_CALLS:
-                gemm_flops += meta["flops"]
-                gemm_ms += ms
-                gemm_bytes += meta["bytes"]  # A rows read once + output rows written
-                tag = "gated " if meta.get("fused") else ""
-                s = shapes.setdefault(f"{tag}rows={meta['rows']} K={meta['k']} N={meta['n']}", [0, 0.0, 0.0])
-                s[0] += 1
-                s[1] += ms
-                s[2] += meta["flops"]
+        per, shapes, gemm = profile_sums(prof)
+        gemm_flops, gemm_ms, gemm_bytes, n_gemm = gemm["flops"], gemm["ms"], gemm["bytes"], gemm["launches"]
         total_ms = sum(v[1] for v in per.values())
         kernel_table = {k: {"launches": v[0], "ms": round(v[1], 3), "share": round(v[1] / total_ms, 4)}
                         for k, v in sorted(per.items(), key=lambda kv: -kv[1][1])}
@@ -475,12 +485,11 @@ def main():
         src = "measured" if peaks else "fallback"
         ach = gemm_flops / (gemm_ms * 1e-3) / 1e12
         ach_gb = gemm_bytes / (gemm_ms * 1e-3) / 1e9
-        n_gemm = sum(per[k][0] for k in GEMM_CALLS if k in per)
         # DRAM traffic per launch: on five forms of the contractions at 573,894 rows, one launch at a time, ncu counts 9.2 GB for
         # 8.8 GB of algorithmic bytes (A rows read + gate / residual rows read + output rows written; addend tables come on
         # top); scaled here to the average launch of the step by its algorithmic bytes.
         pk = clocks_peak.summary()
-        roofline = {"kernel": "k_linear + k_mlp (mb_gemm, mb_gated_mlp_fwd, mb_mlp_bwd_data)", "bound": "tensor", "achieved": ach,
+        roofline = {"kernel": f"k_linear + k_mlp + k_few ({', '.join(gemm['calls'])})", "bound": "tensor", "achieved": ach,
                     "peak": peak_tf, "unit": "TFLOP/s", "frac": ach / peak_tf, "traffic": 1.04 * gemm_bytes / n_gemm,
                     "traffic_note": "bytes per average launch, scaled from ncu captures of single launches by the algorithmic bytes",
                     "peak_source": src + " bf16 sustained",
