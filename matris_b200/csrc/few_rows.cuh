@@ -40,6 +40,8 @@ template <int MODE> struct FewArgs { typedef MlpArgs T; };
 template <> struct FewArgs<FEW_LINEAR> { typedef FewLinear T; };
 template <> struct FewArgs<FEW_PLAIN_BWD> { typedef FewPlainBwd T; };
 template <> struct FewArgs<FEW_ROW_BWD> { typedef FewRowBwd T; };
+template <typename T> __device__ __forceinline__ const T& few_problem(const T& args, int) { return args; }  // that of a block
+__device__ __forceinline__ const MlpArgs& few_problem(const FewPlainBwd& args, int i) { return args.of[i]; }
 // hi, lo; MLPs: layer 1, layer 2, E's weights (PLAIN_BWD: two of each problem); LINEAR: column blocks
 struct alignas(64) FewMaps { CUtensorMap w[FW_MAX_BLOCKS][2]; };
 
@@ -129,10 +131,7 @@ k_few(const __grid_constant__ typename FewArgs<MODE>::T args, const __grid_const
   constexpr uint32_t X_OPERAND = few_x_bytes(MODE, R), X_LO = X_OPERAND / 2;
   constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)R >> 3) << 17 | ((128u >> 4) << 24), MN_MAJOR_B = 1u << 16;
   constexpr uint32_t COLUMNS = few_columns(MODE, R);
-  const auto& d = [&]() -> const auto& {
-    if constexpr (MODE == FEW_PLAIN_BWD) return args.of[blockIdx.y];
-    else return args;
-  }();
+  const auto& d = few_problem(args, blockIdx.y);
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sm0 = smem_u32(smem);
   if ((sm0 & 1023u) != 0) {

@@ -13,7 +13,7 @@
 
 namespace mb {
 
-constexpr int BM = 128, BN = 128, BK = 16, GEMM_THREADS = 256, LDS = BM + 4;
+constexpr int BM = 128, BK = 16, GEMM_THREADS = 256, LDS = BM + 4;
 
 __global__ void __launch_bounds__(GEMM_THREADS, 2) k_gemm(const __grid_constant__ mb_gemm_desc d) {
   const mb_colblock& cb = d.blk[blockIdx.y];
