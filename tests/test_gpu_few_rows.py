@@ -2,6 +2,7 @@
 does not depend on how many rows a call has."""
 from types import SimpleNamespace
 
+import numpy as np
 import pytest
 import torch
 import torch.nn.functional as F
@@ -131,3 +132,131 @@ def test_sums_of_a_bonds_two_rows_as_operand(count):
     for i in range(count):  # tolerances as above: the same expressions, float32 sums of order one in another order
         report(f"bond sums {count}/{i}: F", one["f"][0], many["f"][i], 2e-6)
         report(f"bond sums {count}/{i}: S", one["s"][0] / GPA, many["s"][i] / GPA, 2e-7)
+
+
+# ------------------------------------------------------------------ sub-blocks: merged launches, row gradients, sums of two rows
+def grouped(key, n):
+    """Row numbers sorted by key (stable) and the start of each key's run."""
+    return np.argsort(key, kind="stable"), np.concatenate([[0], np.cumsum(np.bincount(key, minlength=n))])
+
+
+def line_graph(rows, nodes, seed):
+    """Rows sorted by target node; two target nodes share a centre, so that a centre's sum is of two terms at the most."""
+    r = np.random.default_rng(seed)
+    tgt, src = np.sort(r.integers(0, nodes, rows)), r.integers(0, nodes, rows)
+    perm, src_ptr = grouped(src, nodes)
+    return dict(n_rows=rows, n_nodes=nodes, n_edge_rows=rows, n_ctr=(nodes + 1) // 2, tgt=tgt, src=src, ctr=tgt // 2, src_perm=perm,
+                tgt_ptr=grouped(tgt, nodes)[1], src_ptr=src_ptr)
+
+
+def atom_graph(bonds, nodes, seed):
+    """Two directed rows a bond, sorted by centre."""
+    r = np.random.default_rng(seed)
+    a, b = r.integers(0, nodes, (2, bonds))
+    order, ptr = grouped(np.concatenate([a, b]), nodes)
+    at = np.empty(2 * bonds, dtype=np.int64)
+    at[order] = np.arange(2 * bonds)  # where a directed row went
+    bond, rev = order % bonds, at[(order + bonds) % (2 * bonds)]
+    return dict(n_rows=2 * bonds, n_nodes=nodes, n_edge_rows=bonds, n_ctr=0, is_atom=1, tgt=np.concatenate([a, b])[order],
+                src=np.concatenate([b, a])[order], tgt_ptr=ptr, src_ptr=ptr, src_perm=rev, rev=rev, emap=bond, u2d=at[:bonds])
+
+
+def joined(g, h):
+    """Both graphs as one, the first's rows, nodes and bonds first."""
+    of = dict(tgt="n_nodes", src="n_nodes", ctr="n_ctr", src_perm="n_rows", rev="n_rows", u2d="n_rows", emap="n_edge_rows", tgt_ptr="n_rows",
+              src_ptr="n_rows")
+    out = {k: g[k] + h[k] for k in ("n_rows", "n_nodes", "n_edge_rows", "n_ctr")}
+    out.update({k: np.concatenate([g[k], h[k][int(k.endswith("_ptr")):] + g[of[k]]]) for k in of if k in g})
+    return {**out, "is_atom": g.get("is_atom", 0)}
+
+
+def on_device(g):
+    from matris_b200 import _lib
+    alive = {k: dev(v, torch.int32) for k, v in g.items() if isinstance(v, np.ndarray)}
+    c = _lib.MbRowGraph(**{k: int(v) for k, v in g.items() if not isinstance(v, np.ndarray)}, **{k: _lib.ptr(v) for k, v in alive.items()})
+    return SimpleNamespace(c=c, alive=alive, skip_edge_out=False)
+
+
+@pytest.fixture(scope="module")
+def layer():
+    from matris_b200.model import pack_parameters
+    from matris_b200.weights import full_config, random_checkpoint
+    ck = random_checkpoint(dict(num_layers=1), seed=3, jitter=0.1)
+    return pack_parameters(ck["state_dict"], full_config(ck["config"]), torch.device("cuda"))
+
+
+def sub_block(layer, kind, g, x):
+    """Results and gradients of a sub-block on the first rows of the features x."""
+    from matris_b200.model import AttentionFn, RefineFn
+    line = not g.get("is_atom")
+    bonds = g["n_nodes"] if line else g["n_edge_rows"]
+    node, edge, rbf, atom = (x[k][:n].clone().requires_grad_(True) for k, n in (("node", g["n_nodes"]), ("edge", g["n_edge_rows"]),
+                                                                                ("rbf", bonds), ("atom", g["n_ctr"])))
+    P, rg = getattr(layer.layers[0], f"{kind}_{'line' if line else 'atom'}"), on_device(g)
+    if kind == "attn":
+        leaves, out = [node, edge], AttentionFn.apply(node, edge, P, rg)
+    else:
+        leaves = [node, edge, rbf] + [atom] * line
+        out = RefineFn.apply(node, edge, rbf, atom if line else None, P, rg)
+    grads = torch.autograd.grad(out, leaves, [x["d_node"][:g["n_nodes"]], x["d_edge"][:g["n_edge_rows"]]])
+    return [t.detach() for t in (*out, *grads)]
+
+
+def compare(layer, ops, kind, small, big, seed):
+    both = joined(small, big)
+    n = max(both[k] for k in ("n_nodes", "n_edge_rows", "n_ctr"))
+    x = {k: dev(rnd(n, w, seed=seed + i)) for i, (k, w) in enumerate([("node", 128), ("edge", 128), ("rbf", 7), ("atom", 128),
+                                                                      ("d_node", 128), ("d_edge", 128)])}
+    alone, among = sub_block(layer, kind, small, x), sub_block(layer, kind, both, x)
+    assert ops.gemm_status() == 0
+    for i, (a, b) in enumerate(zip(alone, among)):
+        assert torch.isfinite(a).all() and torch.equal(a, b[:a.shape[0]]), (i, (a - b[:a.shape[0]]).abs().max())
+
+
+def shapes():
+    """(rows, nodes) at the edges of the tiles: row gradients with one output take n rows a tile, with three (the node update's) a third."""
+    n = torch.cuda.get_device_properties(0).multi_processor_count if torch.cuda.is_available() else 3
+    t = n // 3
+    return [(1, 1), (15, 7), (17, 16), (33, 17), (16 * n, 16 * t), (16 * n + 1, 16 * t + 1), (32 * n - 1, 32 * t), (32 * n, 32 * t + 1),
+            (32 * n + 1, 16 * n), (64 * n, 16 * n + 1), (64 * n + 1, 32 * n)]
+
+
+@pytest.mark.parametrize("at", range(11))
+@pytest.mark.parametrize("kind", ["attn", "refine"])
+@pytest.mark.parametrize("which", ["line", "atom"])
+def test_sub_blocks_do_not_depend_on_how_many_rows_there_are(layer, ops, which, kind, at):
+    """Alone, a graph's sub-block takes merged launches (of problems with different numbers of rows), row gradients formed inside the
+    products and sums of a bond's two rows as operand; in front of a large graph, the row kernels and the persistent contractions.  All
+    sums keep their order, so the results of the first graph's rows are the same bit for bit."""
+    rows, nodes = shapes()[at]
+    if which == "line":
+        compare(layer, ops, kind, line_graph(rows, nodes, at), line_graph(50_000, 10_000, 99), 10 * at)
+    else:  # segments of 16 rows and more on both sides: the kernel of the sums of node rows is chosen by that
+        small = atom_graph((rows + 1) // 2, max(1, rows // 20), at) if rows > 40 else atom_graph((rows + 1) // 2, 1, at)
+        compare(layer, ops, kind, small, atom_graph(90_000, 9_600, 99), 10 * at)
+
+
+@pytest.mark.parametrize("bonds", [8192, 8193])
+@pytest.mark.parametrize("which", ["line", "atom"])
+def test_envelope_gradient_either_side_of_its_line(layer, ops, which, bonds):
+    """Up to 8,192 bonds the envelopes' gradient goes straight on into the radial basis's."""
+    if which == "line":
+        compare(layer, ops, "refine", line_graph(3 * bonds, bonds, 1), line_graph(6_000, 2_000, 2), 5)
+    else:
+        compare(layer, ops, "refine", atom_graph(bonds, 700, 1), atom_graph(2_000, 150, 2), 5)
+
+
+def test_energies_either_side_of_the_line_of_merged_envelopes():
+    """156 bonds a structure: 26 of them stay below 4,096 bonds, 27 do not.  No sum of the forward pass depends on the batch."""
+    from matris_b200 import MatRIS, workloads
+    from matris_b200.weights import random_checkpoint
+    c = workloads.cu_fcc((1, 1, 1), sigma=0.05)
+    model = MatRIS.from_dict(random_checkpoint(dict(num_layers=2, reference_energy="mpa"), seed=1, jitter=0.1)).to("cuda")
+    one = model.predict([c], "efs")
+    for count in (26, 27):
+        g = model.graph_converter.batch([c] * count)
+        assert (g.n_bonds <= 4096) == (count == 26)
+        many = model(g, "efs")
+        for i in range(count):
+            assert torch.equal(one["e"][0], many["e"][i])
+            report(f"merged envelopes {count}/{i}: F", one["f"][0], many["f"][i], 2e-6)

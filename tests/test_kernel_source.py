@@ -37,12 +37,25 @@ def test_proxy_fence_before_copies_into_patches_that_threads_stored_to(name, n_r
         assert 0 <= r.find("to_async_proxy()") < r.find("load_patch("), r
 
 
+def test_proxy_fence_before_matrix_instructions_read_what_threads_stored():
+    """The few-row kernel's operands in shared memory are stored by threads: the fence stands between a warp's stores and the arrival
+    that lets the matrix instructions read them."""
+    text = code("few_rows.cuh")
+    arrivals = [m.start() for m in re.finditer(r"mbar_arrive\((?:x|act)_ready", text)]
+    assert len(arrivals) == 3  # row gradients, rows read in place, hidden layer
+    for at in arrivals:
+        before = text[:at]
+        stores = max(before.rfind("st.shared"), before.rfind("few_put4(at"))
+        assert before.rfind("to_async_proxy()") > stores, text[at - 200:at]
+
+
 @pytest.mark.parametrize("name,drains", [
     ("mlp_fused.cuh", ["drain_mma(retired, elected);", "drain_copies(w_ready, ML_W_SLOTS, n);",
                        "if (EPI_RES && !alive) drain_copies(my_full, 2, asked);",
                        "if (!alive) drain_copies(my_conv, 1, conv_asked);", "drain_copies(side_full + 16 * pw, 2, side_asked);"]),
     ("linear_tma.cuh", ["drain_mma(retired, elected);", "drain_copies(w_ready, ML_W_SLOTS, n);",
                         "drain_copies(side_full + 16 * lane, 2, n);", "if (!alive) drain_copies(my_conv, 1, conv_asked);"]),
+    ("few_rows.cuh", ["drain_mma(retired, elected);", "drain_copies(w_full, (uint32_t)n_slots, asked);"]),
     ("gemm_persistent.cuh", ["drain_mma(retired, elected);", "drain_copies(w_ready, w_period, wu);"]),
     ("gemm.cu", ["drain_copies(w_full, 2, n_loads);", '"bar.arrive 1, 160;"', '"bar.sync 1, 160;"'])])
 def test_nothing_is_in_flight_when_a_block_ends(name, drains):
