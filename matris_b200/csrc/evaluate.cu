@@ -1,9 +1,9 @@
 // Whole-model driver: queues every kernel of an evaluation (graph tensors -> energies, forces, stresses, moments) from
 // one host call.
 //
-// What bounds a small system is the host: an evaluation is 600 - 800 launches, and from an interpreter each costs about
-// 20 us (descriptor packing, foreign-function call, tensor allocation, autograd bookkeeping), 13 ms in all, while the
-// device needs 9 ms.  Queued from here a launch costs 2 - 3 us: 4 atoms 13.2 -> 9.2 ms, bound by the device.
+// What bounds a small system is the host: an evaluation is 430 - 640 launches, and from an interpreter each costs about
+// 20 us (descriptor packing, foreign-function call, tensor allocation, autograd bookkeeping).  Queued from here a launch costs
+// 2 - 3 us: when they were 600 - 800, 4 atoms 13.2 -> 9.2 ms, bound by the device ever since.
 //
 // Memory is handed out from two stacks: inputs of the sub-blocks (always needed by the backward pass) and temporaries on the
 // bottom one, internals of the layers that keep them on the top one.  The backward pass pops both in reverse order.  A small
@@ -131,7 +131,7 @@ struct Arena {
 
 // ------------------------------------------------------------------ side streams
 // Two more streams for work that does not feed the next kernel of the caller's stream.  A small system is bound by the chain of its
-// 660 launches, most of which leave most SMs idle: off the chain go a layer's centre and node tables, the logits, the envelopes and
+// launches, most of which leave most SMs idle: off the chain go a layer's centre and node tables, the logits, the envelopes and
 // the other of two feed-forward blocks, in the backward pass the node sums beside the edge gradients.  Device time of an evaluation:
 // 32 atoms 6.5 -> 5.5 ms, 256 atoms 10.4 -> 9.4; 16,000 atoms 624 -> 608 (tails of one launch filled by another), so for all sizes.
 // Taken from a pool for one call and given back when its work is queued (a later user of the same streams queues behind it); the

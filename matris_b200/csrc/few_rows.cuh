@@ -12,7 +12,8 @@
 // (tensor-memory lane) and registers = rows, bias and weights of an epilogue are one register, a row of an addend table, gate,
 // residual or output is one 128-byte access of a warp straight from or to global memory (no staging, no hand-over), and the hidden
 // layer goes back to shared memory as the MN-major B operand of layer 2.  A feature's rows are spread over 16 warps.  A table's row
-// numbers are asked for first of all, in one register of a lane each, and shuffled.
+// numbers are asked for first of all, in one register of a lane each, and shuffled: three addends without a contraction 6.2 -> 5.8 us for
+// 16 rows, 13.2 -> 12.6 for 9,472; with K = 128 7.0 -> 7.1 and 15.6 -> 14.8.
 //
 // The products of a K step are accumulated in the order of the persistent kernels, so that a row's sums do not depend on how many rows
 // a call has.  (w_hi x [x_hi ; x_lo] as one instruction of N = 2 R, the small terms in columns of their own, would save a third of the
@@ -24,11 +25,13 @@
 //
 // Warps 0 - 15: rows in, epilogues; 16: matrix instructions; 17: weights.
 
-// A small evaluation is also bound by its launches, 2.5 us of the host's time each and 3 - 4 of the chain, so a launch takes on more:
-// ROW_BWD is the backward pass from a row's own gradient on (RowBwd, common.cuh), a warp forming the row's dz2 (and the logits'
-// gradients) in registers as the row kernels do; LINEAR takes the column blocks of independent problems, and sums of a bond's two
-// directed rows as operand; PLAIN_BWD two problems.  550 -> 430 launches an evaluation: 4 atoms 3.37 -> 2.91 ms, 32 atoms through the
-// calculator 5.02 -> 4.84.
+// A small evaluation is also bound by its launches, 2.5 us of the host's time each and 3 - 4 of the chain, so a launch takes on
+// more: ROW_BWD is the backward pass from a row's own gradient on (RowBwd, common.cuh), a warp forming the row's dz2 (and the
+// logits' gradients) in registers as the row kernels do; LINEAR takes the column blocks of independent problems, and sums of a
+// bond's two directed rows as operand; PLAIN_BWD two problems.  550 -> 430 launches an evaluation, with the envelopes'
+// (evaluate.cu): 4 atoms 3.37 -> 2.91 ms, 32 atoms through the calculator 5.02 -> 4.84.  Left out again one by one: row gradients
+// 3.0 and 0.4 % slower, LINEAR's problems 5.2 and 2.6 %, PLAIN_BWD's 2.7 and 1.2 %; 572 atoms, where few launches are of few rows,
+// within 0.3 %.
 
 enum FewMode { FEW_GATED_FWD = MLP_GATED_FWD, FEW_PLAIN_FWD = MLP_PLAIN_FWD, FEW_GATED_BWD = MLP_GATED_BWD,
                FEW_PLAIN_BWD = MLP_PLAIN_BWD, FEW_LINEAR = 4, FEW_ROW_BWD = 5 };

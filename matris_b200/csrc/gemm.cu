@@ -672,7 +672,11 @@ static int row_map(const float* p, int64_t ld, int cols, int64_t rows, CUtensorM
   return weight_map(p, ld, cols, out, (int)rows, false, 32);
 }
 
-// rows of a block at the most: dense layers and the products that form their operand themselves gain nothing from 64
+// Rows of a block at the most.  64 pay for the MLPs (with 32 at the most evaluations of 600 - 4,000 bonds take up to 6 % longer).  For dense
+// layers they would save the wide operands 5 % (512 -> 128 at 9,472 rows 11.7 -> 11.2 us, 384 -> 128 10.1 -> 9.5, 256 -> 256 at 4,736 rows
+// 8.4 -> 7.9; the line of 128 -> 128 ... 512 with 64 rows is that with 32), evaluations of 4 - 572 atoms 0.7 % at the most and most of them
+// nothing.  For the products that form their operand themselves it depends: with one output 7,500 - 9,000 triplets gain 0.8 - 2.5 % of an
+// evaluation, with three, each of which forms it anew, 2,800 - 4,000 bonds lose 0.8 - 1.6 %.
 static constexpr int few_most(int mode) { return mode == FEW_LINEAR || mode == FEW_ROW_BWD ? 32 : 64; }
 template <int MODE> static int few_config_mode() {
   MB_CUDA_CHECK(cudaFuncSetAttribute(k_few<MODE, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, FW_SMEM_LIMIT));
@@ -691,10 +695,21 @@ static int few_config() {
 }
 // R of k_few for a launch, 0: the persistent kernels.  A block of k_few takes one tile, so the line lies where its tiles no longer run
 // side by side: 16 rows a block while a multiprocessor gets one at most, then 32 (dense layers with K = 128: two blocks on a
-// multiprocessor), the MLPs then 64.  Back to back, weights in L2, us (persistent kernel / here): gated forward with two addends, 2300
-// rows 17.8 / 7.5, 4700 rows 17.9 / 9.2, 9400 rows 18.2 / 14.3; its backward 13.1 / 6.9, 13.3 / 7.8, 13.6 / 11.4; feed-forward block, 4700
-// rows 10.4 / 5.7, 9400 rows 10.7 / 8.2; dense 128 -> 128 6.1 / 3.4 and 6.1 / 4.1; dense 128 -> 512, 1180 rows 6.2 / 4.1, 2300 rows
-// 6.7 / 5.7; dense 512 -> 128 10.9 / 6.6 and 11 / 7.2.  With 96 rows (14,200) the gated forward spills: 18.9 / 25.
+// multiprocessor), the MLPs then 64.  Back to back, weights in L2, us (persistent kernel / here) at the last launch of each height
+// and the first of the next (148 multiprocessors):
+//                                          2,368 rows    2,369          4,736          4,737          9,472
+//   gated forward, K = 128, two addends     18.7 /  8.1   18.6 /  9.4    18.8 / 10.0    18.8 / 15.2    19.1 / 15.6
+//     three addends, no contraction         16.7 /  6.6   16.7 /  7.9    16.8 /  8.4    16.8 / 12.1    17.0 / 12.6
+//     K = 384 (three slots for weights)     21.9 / 11.5   22.0 / 12.4    22.0 / 13.1    22.0 / 18.6    22.4 / 19.1
+//     the same, nothing kept                20.0 / 11.4   20.0 / 12.1    20.1 / 12.8    20.0 / 17.4    20.4 / 18.0
+//   gated backward                          13.1 /  7.2   13.0 /  7.5    13.2 /  8.0    13.1 / 11.2    13.4 / 11.7
+//     with two more segments (three slots)  16.8 /  9.1   16.8 /  9.3    16.9 /  9.9    16.9 / 14.2    17.1 / 14.6
+//   feed-forward block                      11.9 /  5.3   11.9 /  6.1    11.9 /  6.5    11.9 /  9.0    12.1 /  9.5
+//     its backward                           9.1 /  5.1    9.1 /  5.4     9.1 /  5.7     9.1 /  7.3     9.3 /  7.6
+//   dense 128 -> 128                         6.5 /  3.5    6.5 /  4.2     6.5 /  4.2     6.5 /  5.4     6.6 /  5.8
+//   dense 512 -> 128                        11.3 /  6.8   11.3 /  7.0    11.4 /  7.4
+// and dense 128 -> 512 at 592 rows 6.5 / 3.5, 1,184 rows 6.6 / 4.3, 2,368 rows 6.8 / 6.0.  With 96 rows (14,200) the gated forward
+// spills: 18.9 / 25.
 static uint32_t few_rest(int mode, int r, int n_src, int n_ext) {  // shared memory beside the weight ring
   return (n_src + n_ext) * few_x_bytes(mode, r) + few_hidden(mode, n_src) * few_operand_bytes(r) + few_tail_bytes(r);
 }

@@ -1,6 +1,6 @@
 // Row GEMM with direct outputs (included by gemm.cu inside namespace mb, after mlp_fused.cuh): the descriptors of mb_gemm whose
 // column blocks share one A operand or have a single 128-wide segment each and whose outputs go to their own rows (store or
-// accumulate, no index).  Those are all dense layers of an evaluation; scattered outputs take k_gemm_ps.
+// accumulate, no index).  Those are all dense layers of an evaluation but those of few rows (k_few); scattered outputs take k_gemm_ps.
 //
 // Same machinery as k_mlp (see there): rows by TMA patches in both directions, A split into bf16 hi / lo in four tensor-memory
 // buffers, weights in 16 KB tiles, three accumulator regions used in turn by the column blocks in the order they are finished,
@@ -13,7 +13,8 @@
 // counts.
 //
 // HBM bounds the large launches: 573,894 rows take 0.171 ms for 128 -> 256 (k_gemm_ps 0.214), 0.25 with a gate, 0.36 for
-// 512 -> 128, 0.275 for 128 -> 512.  One tile takes 12 us (15), with K = 512 19 us: the chain of its 16 chunks.
+// 512 -> 128, 0.275 for 128 -> 512.  The smallest launches that k_few leaves are bound by the chain of a tile, back to back 6.8 us for 128 -> 128
+// (9,473 rows), 11.4 for 512 -> 128 (4,737 rows), whose tile has 16 chunks, 6.9 for 128 -> 512 (2,369 rows).
 //
 // PAIR sums the two directed rows of a bond on the way in, instead of a pass that writes the sums and one that reads them back: with
 // K = 512, 117,048 bonds 98 + 87 -> 115 us (92 at the copy rate), with K = 256 49 + 49 -> 62.  The rows are gathered by cp.async

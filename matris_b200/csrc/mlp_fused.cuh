@@ -31,13 +31,15 @@
 // r+1 as soon as L2 gate(t) is done, under the epilogue of t.  GATED_BWD: 0, 1 and 2.  PLAIN_*: tiles alternate between the
 // two epilogue groups, L1(t) -> 2t mod 3, L2(t) -> 2t+1 mod 3, issued L1(t+1) before L2(t).
 //
-// Measured behind an L2 flush (bench_gemm.py; addend tables of a fifth of the rows), 573,894 rows with z1 and z2 kept: two addends
-// and a residual 0.49 ms, three addends 0.53 (nothing kept: 0.40), no contraction and three addends 0.48, K = 384 gathered with a
-// residual 0.63; GATED_BWD with a residual 0.42, with E too 0.59; FFN forward 0.22, backward 0.17.  One tile alone takes 28 us
-// forward, 21 us backward: the chain of its stages.  The epilogues' arithmetic goes two values at a time (f2, common.cuh); 523,000
-// rows: three addends 0.497 -> 0.483 (nothing kept 0.382 -> 0.364), no contraction 0.439 -> 0.433, FFN forward 0.208 -> 0.202,
-// backward 0.169 -> 0.156.  (The addends' own sums that way: 0.523.)  With three addends 44 % of the cycles issue an
-// instruction, the load / store data pipe is busy in 44 %, the tensor pipe in 20 %: 4.5 warps a scheduler wait for their own chains.
+// Measured behind an L2 flush (bench_gemm.py; addend tables of a fifth of the rows), 573,894 rows with z1 and z2 kept: two
+// addends and a residual 0.49 ms, three addends 0.53 (nothing kept: 0.40), no contraction and three addends 0.48, K = 384
+// gathered with a residual 0.63; GATED_BWD with a residual 0.42, with E too 0.59; FFN forward 0.22, backward 0.17.  The smallest
+// launches that k_few leaves (9,473 rows: one tile for half of the multiprocessors) are bound by the chain of a tile's stages:
+// back to back 19.0 us for the gated forward with two addends, 22.5 with K = 384, 13.5 for its backward, 17.2 with E, 12.0 for
+// the FFN, 9.2 for its backward.  The epilogues' arithmetic goes two values at a time (f2, common.cuh); 523,000 rows: three
+// addends 0.497 -> 0.483 (nothing kept 0.382 -> 0.364), no contraction 0.439 -> 0.433, FFN forward 0.208 -> 0.202, backward
+// 0.169 -> 0.156.  (The addends' own sums that way: 0.523.)  With three addends 44 % of the cycles issue an instruction, the
+// load / store data pipe is busy in 44 %, the tensor pipe in 20 %: 4.5 warps a scheduler wait for their own chains.
 //
 // Warps: 0 MMA, 1 TMA (weights, 16 KB tiles of 64 K values, five slots), 2-9 producers, 10-17 epilogue (two groups of four; the
 // group's branch or tile parity, the warp's lane quarter).  Every mbarrier wait is bounded; on expiry the status word is set, the
