@@ -1,7 +1,7 @@
 // Whole-model driver: queues every kernel of an evaluation (graph tensors -> energies, forces, stresses, moments) from
 // one host call.
 //
-// What bounds a small system is the host: an evaluation is 430 - 640 launches, and from an interpreter each costs about
+// What bounds a small system is the host: an evaluation is 440 - 640 launches, and from an interpreter each costs about
 // 20 us (descriptor packing, foreign-function call, tensor allocation, autograd bookkeeping).  Queued from here a launch costs
 // 2 - 3 us: when they were 600 - 800, 4 atoms 13.2 -> 9.2 ms, bound by the device ever since.
 //

@@ -28,10 +28,10 @@
 // A small evaluation is also bound by its launches, 2.5 us of the host's time each and 3 - 4 of the chain, so a launch takes on
 // more: ROW_BWD is the backward pass from a row's own gradient on (RowBwd, common.cuh), a warp forming the row's dz2 (and the
 // logits' gradients) in registers as the row kernels do; LINEAR takes the column blocks of independent problems, and sums of a
-// bond's two directed rows as operand; PLAIN_BWD two problems.  550 -> 430 launches an evaluation, with the envelopes'
-// (evaluate.cu): 4 atoms 3.37 -> 2.91 ms, 32 atoms through the calculator 5.02 -> 4.84.  Left out again one by one: row gradients
-// 3.0 and 0.4 % slower, LINEAR's problems 5.2 and 2.6 %, PLAIN_BWD's 2.7 and 1.2 %; 572 atoms, where few launches are of few rows,
-// within 0.3 %.
+// bond's two directed rows as operand; PLAIN_BWD two problems.  With the envelopes' (evaluate.cu) an evaluation of 4 atoms takes 443
+// launches instead of 660 (32 atoms 494, 572 atoms 599), 3.37 -> 2.91 ms, of 32 atoms through the calculator 5.02 -> 4.84.  Left out
+// again one by one: row gradients 3.0 and 0.4 % slower, LINEAR's problems 5.2 and 2.6 %, PLAIN_BWD's 2.7 and 1.2 %; 572 atoms, where
+// few launches are of few rows, within 0.3 %.
 
 enum FewMode { FEW_GATED_FWD = MLP_GATED_FWD, FEW_PLAIN_FWD = MLP_PLAIN_FWD, FEW_GATED_BWD = MLP_GATED_BWD,
                FEW_PLAIN_BWD = MLP_PLAIN_BWD, FEW_LINEAR = 4, FEW_ROW_BWD = 5 };
